@@ -106,6 +106,37 @@ __device__ __forceinline__ uint32_t sat_pack4(int32_t r0, int32_t r1, int32_t r2
   return b;
 }
 
+// Results in bits 8..15 of a word (8 fraction bits below), saturated to int8 and packed: the 16-bit saturating pack
+// clamps the integer part to [-128, 127] and the byte select drops the fraction (a floor).
+__device__ __forceinline__ uint32_t high_bytes4(int32_t h0, int32_t h1, int32_t h2, int32_t h3) {
+  uint32_t a, b;
+  asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(a) : "r"(h1), "r"(h0));
+  asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(b) : "r"(h3), "r"(h2));
+  return __byte_perm(a, b, 0x7531);
+}
+// byte j of w, sign-extended, times 2^8 (__byte_perm drops the selector's sign-replication bits)
+template <int J>
+__device__ __forceinline__ int32_t sx8_shl8(uint32_t w) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "n"(0x8804 + J * 0x1110));
+  return (int32_t)r;
+}
+__device__ __forceinline__ uint32_t max_s16x2(uint32_t a, uint32_t b) {
+  asm("max.s16x2 %0, %0, %1;" : "+r"(a) : "r"(b));
+  return a;
+}
+__device__ __forceinline__ uint32_t min_s16x2(uint32_t a, uint32_t b) {
+  asm("min.s16x2 %0, %0, %1;" : "+r"(a) : "r"(b));
+  return a;
+}
+// High word of a * m + k. A 32 x 32 -> 64 multiply-add issues at twice the rate of a multiply-high here (2 against 4
+// cycles per warp instruction and scheduler), and its 64-bit addend takes bias, rounding and zero point at once.
+__device__ __forceinline__ int32_t mad_wide_hi(int32_t a, int32_t m, long long k) {
+  long long t;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(t) : "r"(a), "r"(m), "l"(k));
+  return (int32_t)(t >> 32);
+}
+
 __device__ __forceinline__ int32_t sx8(uint32_t word, int j) {
   return (int32_t)(int8_t)(word >> (8 * j));
 }

@@ -1,4 +1,4 @@
-// Bandwidth-bound layer kernels: pooling, rescaled add/sub/mul, 256-entry table,
+// Bandwidth-bound layer kernels: rescaled add/sub/mul, 256-entry table,
 // standalone rescale (also the building block of a rescaled concat), 2x nearest
 // resize. 128-bit accesses wherever the channel count allows; grids sized in
 // whole multiples of the SM count with grid-stride loops.
@@ -19,251 +19,51 @@ inline unsigned grid_for(long long work_items, int per_block = kThreads) {
   return (unsigned)blocks;
 }
 
-// ---- max pool: torq_hl.maxpool2d (PoolingPattern.cpp:128-258) ----
-template <int VEC>  // channels per thread: 16 (uint4) or 1
-__global__ void __launch_bounds__(kThreads) maxpool_kernel(PoolArgs a) {
-  grid_dependency_release();
-  grid_dependency_wait();
-  const int groups = a.C / VEC;
-  const long long total = (long long)a.N * a.OH * a.OW * groups;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    int g = (int)(idx % groups);
-    long long p = idx / groups;
-    int ow = (int)(p % a.OW);
-    long long t = p / a.OW;
-    int oh = (int)(t % a.OH);
-    int n = (int)(t / a.OH);
-    const int8_t* xin = a.x + (size_t)n * a.H * a.W * a.C + g * VEC;
-    if (VEC == 16) {
-      uint32_t best[4] = {0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u};
-      const uint32_t padw = (uint32_t)(a.pad_value & 0xff) * 0x01010101u;
-      for (int kh = 0; kh < a.KH; kh++) {
-        int ih = oh * a.stride_h - a.pad_t + kh;
-        for (int kw = 0; kw < a.KW; kw++) {
-          int iw = ow * a.stride_w - a.pad_l + kw;
-          uint4 v;
-          if (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) v = make_uint4(padw, padw, padw, padw);
-          else v = *reinterpret_cast<const uint4*>(xin + ((size_t)ih * a.W + iw) * a.C);
-          best[0] = __vmaxs4(best[0], v.x);
-          best[1] = __vmaxs4(best[1], v.y);
-          best[2] = __vmaxs4(best[2], v.z);
-          best[3] = __vmaxs4(best[3], v.w);
-        }
-      }
-      *reinterpret_cast<uint4*>(a.out + (size_t)p * a.C + g * 16) = make_uint4(best[0], best[1], best[2], best[3]);
-    } else {
-      int best = -128;
-      for (int kh = 0; kh < a.KH; kh++) {
-        int ih = oh * a.stride_h - a.pad_t + kh;
-        for (int kw = 0; kw < a.KW; kw++) {
-          int iw = ow * a.stride_w - a.pad_l + kw;
-          int v = (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) ? a.pad_value
-                                                               : (int)xin[((size_t)ih * a.W + iw) * a.C];
-          best = max(best, v);
-        }
-      }
-      a.out[(size_t)p * a.C + g] = (int8_t)best;
-    }
-  }
-}
-
-// The same on int16 tensors (the reference's MaxPool2D i16 -> i16): 8 channels per thread, or 1.
-template <int VEC>
-__global__ void __launch_bounds__(kThreads) maxpool_i16_kernel(PoolArgs a) {
-  const int16_t* x = reinterpret_cast<const int16_t*>(a.x);
-  int16_t* out = reinterpret_cast<int16_t*>(a.out);
-  const int groups = a.C / VEC;
-  const long long total = (long long)a.N * a.OH * a.OW * groups;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int g = (int)(idx % groups);
-    const long long p = idx / groups;
-    const int ow = (int)(p % a.OW);
-    const long long t = p / a.OW;
-    const int oh = (int)(t % a.OH);
-    const int n = (int)(t / a.OH);
-    const int16_t* xin = x + (size_t)n * a.H * a.W * a.C + g * VEC;
-    if (VEC == 8) {
-      uint32_t best[4] = {0x80008000u, 0x80008000u, 0x80008000u, 0x80008000u};
-      const uint32_t padw = (uint32_t)(a.pad_value & 0xffff) * 0x00010001u;
-      for (int kh = 0; kh < a.KH; kh++) {
-        const int ih = oh * a.stride_h - a.pad_t + kh;
-        for (int kw = 0; kw < a.KW; kw++) {
-          const int iw = ow * a.stride_w - a.pad_l + kw;
-          uint4 v;
-          if (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) v = make_uint4(padw, padw, padw, padw);
-          else v = *reinterpret_cast<const uint4*>(xin + ((size_t)ih * a.W + iw) * a.C);
-          best[0] = __vmaxs2(best[0], v.x);
-          best[1] = __vmaxs2(best[1], v.y);
-          best[2] = __vmaxs2(best[2], v.z);
-          best[3] = __vmaxs2(best[3], v.w);
-        }
-      }
-      *reinterpret_cast<uint4*>(out + (size_t)p * a.C + g * 8) = make_uint4(best[0], best[1], best[2], best[3]);
-    } else {
-      int best = -32768;
-      for (int kh = 0; kh < a.KH; kh++) {
-        const int ih = oh * a.stride_h - a.pad_t + kh;
-        for (int kw = 0; kw < a.KW; kw++) {
-          const int iw = ow * a.stride_w - a.pad_l + kw;
-          const int v = (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) ? a.pad_value : (int)xin[((size_t)ih * a.W + iw) * a.C];
-          best = max(best, v);
-        }
-      }
-      out[(size_t)p * a.C + g] = (int16_t)best;
-    }
-  }
-}
-
-// reciprocal_scale of the TOSA spec (compiler/torq/Conversions/TosaToTorqHL/Patterns.cpp:796-805)
-__device__ __forceinline__ void reciprocal_scale(uint32_t count, int32_t& mult, int32_t& shift) {
-  int k = 32 - __clz((int)(count - 1));
-  if (count == 1) k = 0;
-  long long numerator = ((1ll << 30) + 1) << k;
-  mult = (int32_t)(numerator / (long long)count);
-  shift = 30 + k;
-}
-
-// ---- average pool: tosa.avg_pool2d acc_type=i32; count excludes padding ----
-// The rescale depends only on the number of taps inside the image, so the block fills a table indexed by that
-// count once (one 64-bit division per entry instead of one per output). Entry {M, 2^(S-30), S-29, count}:
-// TOSA's (v * M + 2^(S-1)) >> S with S = 30 + k >= 30 equals (8v * M + 2^(S+2)) >> (S + 3), and since the constant
-// has a zero low word that is (mulhi(8v, M) + 2^(S-30)) >> (S - 29): exact, 32-bit.
-constexpr int kAvgMaxTaps = 256;
-template <int VEC>  // 16, 4 or 1 channels per thread
-__global__ void __launch_bounds__(kThreads) avgpool_kernel(PoolArgs a) {
-  grid_dependency_release();
-  grid_dependency_wait();
-  __shared__ int4 by_count[kAvgMaxTaps + 1];
-  for (int c = threadIdx.x; c <= a.KH * a.KW; c += blockDim.x) {
-    int32_t mult, shift;
-    reciprocal_scale(c ? (uint32_t)c : 1u, mult, shift);
-    by_count[c] = make_int4(mult, 1 << (shift - 30), shift - 29, c);
-  }
-  __syncthreads();
-  const int groups = a.C / VEC;
-  const long long total = (long long)a.N * a.OH * a.OW * groups;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    int g = (int)(idx % groups);
-    long long p = idx / groups;
-    int ow = (int)(p % a.OW);
-    long long t = p / a.OW;
-    int oh = (int)(t % a.OH);
-    int n = (int)(t / a.OH);
-    const int8_t* xin = a.x + (size_t)n * a.H * a.W * a.C + g * VEC;
-    int acc[VEC];
-#pragma unroll
-    for (int j = 0; j < VEC; j++) acc[j] = 0;
-    int count = 0;
-    for (int kh = 0; kh < a.KH; kh++) {
-      int ih = oh * a.stride_h - a.pad_t + kh;
-      if (ih < 0 || ih >= a.H) continue;
-      for (int kw = 0; kw < a.KW; kw++) {
-        int iw = ow * a.stride_w - a.pad_l + kw;
-        if (iw < 0 || iw >= a.W) continue;
-        count++;
-        const int8_t* px = xin + ((size_t)ih * a.W + iw) * a.C;
-        if (VEC == 16) {
-          const uint4 v = *reinterpret_cast<const uint4*>(px);
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int j = 0; j < 16; j++) acc[j] = __dp4a((int)w[j >> 2], 1 << (8 * (j & 3)), acc[j]);  // adds byte j, sign-extended
-        } else if (VEC == 4) {
-          const uint32_t v = *reinterpret_cast<const uint32_t*>(px);
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc[j] = __dp4a((int)v, 1 << (8 * j), acc[j]);
-        } else {
-          acc[0] += (int)px[0];
-        }
-      }
-    }
-    const int4 k = by_count[count];
-    const int zsum = count * a.input_zp;
-    int q[VEC];
-#pragma unroll
-    for (int j = 0; j < VEC; j++) {
-      const int r = ((__mulhi((acc[j] - zsum) * 8, k.x) + k.y) >> k.z) + a.output_zp;
-      q[j] = max(-128, min(127, r));
-    }
-    if (VEC == 16)
-      *reinterpret_cast<uint4*>(a.out + (size_t)p * a.C + g * 16) =
-          make_uint4(pack4(q[0], q[1], q[2], q[3]), pack4(q[4], q[5], q[6], q[7]), pack4(q[8], q[9], q[10], q[11]),
-                     pack4(q[12], q[13], q[14], q[15]));
-    else if (VEC == 4) *reinterpret_cast<uint32_t*>(a.out + (size_t)p * a.C + g * 4) = pack4(q[0], q[1], q[2], q[3]);
-    else a.out[(size_t)p * a.C + g] = (int8_t)q[0];
-  }
-}
-
-// Large windows over few outputs (the global pool at the end of a classifier: 7x7 -> 1x1): a warp per output pixel
-// and group of 16 channels, the taps spread over the lanes, sums combined by shuffles. Same arithmetic as above.
-__global__ void __launch_bounds__(kThreads) avgpool_warp_kernel(PoolArgs a) {
-  grid_dependency_release();
-  grid_dependency_wait();
-  __shared__ int4 by_count[kAvgMaxTaps + 1];
-  for (int c = threadIdx.x; c <= a.KH * a.KW; c += blockDim.x) {
-    int32_t mult, shift;
-    reciprocal_scale(c ? (uint32_t)c : 1u, mult, shift);
-    by_count[c] = make_int4(mult, 1 << (shift - 30), shift - 29, c);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int groups = a.C / 16;
-  const long long total = (long long)a.N * a.OH * a.OW * groups;
-  const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const int taps = a.KH * a.KW;
-  for (long long idx = warp0; idx < total; idx += nwarps) {
-    const int g = (int)(idx % groups);
-    const long long p = idx / groups;
-    const int ow = (int)(p % a.OW);
-    const long long t = p / a.OW;
-    const int oh = (int)(t % a.OH);
-    const int n = (int)(t / a.OH);
-    const int8_t* xin = a.x + (size_t)n * a.H * a.W * a.C + g * 16;
-    int acc[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++) acc[j] = 0;
-    int count = 0;
-    for (int tap = lane; tap < taps; tap += 32) {
-      const int kh = tap / a.KW, kw = tap - kh * a.KW;
-      const int ih = oh * a.stride_h - a.pad_t + kh, iw = ow * a.stride_w - a.pad_l + kw;
-      if (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) continue;
-      count++;
-      const uint4 v = *reinterpret_cast<const uint4*>(xin + ((size_t)ih * a.W + iw) * a.C);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 16; j++) acc[j] = __dp4a((int)w[j >> 2], 1 << (8 * (j & 3)), acc[j]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      count += __shfl_xor_sync(0xffffffffu, count, o);
-#pragma unroll
-      for (int j = 0; j < 16; j++) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-    }
-    if (lane == 0) {
-      const int4 k = by_count[count];
-      const int zsum = count * a.input_zp;
-      int q[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        const int r = ((__mulhi((acc[j] - zsum) * 8, k.x) + k.y) >> k.z) + a.output_zp;
-        q[j] = max(-128, min(127, r));
-      }
-      *reinterpret_cast<uint4*>(a.out + (size_t)p * a.C + g * 16) =
-          make_uint4(pack4(q[0], q[1], q[2], q[3]), pack4(q[4], q[5], q[6], q[7]), pack4(q[8], q[9], q[10], q[11]),
-                     pack4(q[12], q[13], q[14], q[15]));
-    }
-  }
-}
-
 // ---- add / sub / mul in TOSA form (ElementWiseBinaryPattern.cpp:385-570, MulPattern.cpp:229-238) ----
-// An int8 operand takes 256 values, so its input-side rescale is a 256-entry table (filled here by the
-// same apply_scale_32, one entry per thread): per element two shared-memory loads replace two 64-bit
-// multiply-shift sequences; the output rescale stays arithmetic.
-// EPI: the output rescale, 0 = 64-bit arithmetic, 1 / 2 = the compact 32-bit record (common.cuh) with / without the sign
-// term, chosen by the planner when it can bound |operand sum or product| (it evaluates the same two tables).
+// Four raw table bytes -> one word; lut is indexed by the raw byte.
+__device__ __forceinline__ uint32_t lut_word(const uint8_t* lut, uint32_t w) {
+  const uint32_t b0 = lut[w & 0xff], b1 = lut[(w >> 8) & 0xff], b2 = lut[(w >> 16) & 0xff], b3 = lut[w >> 24];
+  return __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
+}
+
+// add / sub as one linear function of the two bytes: out = clamp((xa * 2^8 * ma + xb * 2^8 * mb + K) >> (32 + F)), the
+// three roundings of the op absorbed in K. The planner takes this form only after it has compared it with the exact op on
+// all 65536 operand pairs (binary_linear_form). Per output: two byte extracts, two multiply-adds and a quarter of the
+// packing, against two 256-entry look-ups (two wavefronts each), a 64-bit or 4-cycle multiply-high and the rounding before:
+// 12.8 M elements 18.9 -> 6 us. HBM-bound at large sizes.
+__global__ void __launch_bounds__(kThreads) binary_linear_kernel(BinaryArgs a) {
+  grid_dependency_release();
+  grid_dependency_wait();
+  const uint32_t lo2 = (uint32_t)((a.clamp_min << a.lin_f) & 0xffff) * 0x10001u;
+  const uint32_t hi2 = (uint32_t)(((a.clamp_max << a.lin_f) | ((1 << a.lin_f) - 1)) & 0xffff) * 0x10001u;
+  const int up = 8 - a.lin_f;  // brings the integer part to the high byte of its 16-bit field
+  auto one = [&](int xa, int xb) { return mad_wide_hi(xb, a.lin_mb, (long long)xa * (long long)a.lin_ma + a.lin_k); };
+  auto word = [&](uint32_t wa, uint32_t wb) {
+    const int h0 = one(sx8_shl8<0>(wa), sx8_shl8<0>(wb)), h1 = one(sx8_shl8<1>(wa), sx8_shl8<1>(wb)),
+              h2 = one(sx8_shl8<2>(wa), sx8_shl8<2>(wb)), h3 = one(sx8_shl8<3>(wa), sx8_shl8<3>(wb));
+    uint32_t p, q;
+    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(p) : "r"(h1), "r"(h0));
+    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(q) : "r"(h3), "r"(h2));
+    // clamped first, so that the shift cannot carry the low field into the integer part of the high one
+    p = min_s16x2(max_s16x2(p, lo2), hi2) << up;
+    q = min_s16x2(max_s16x2(q, lo2), hi2) << up;
+    return __byte_perm(p, q, 0x7531);
+  };
+  const long long nvec = a.n >> 4;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long i = tid; i < nvec; i += stride) {
+    const uint4 va = reinterpret_cast<const uint4*>(a.a)[i];
+    const uint4 vb = reinterpret_cast<const uint4*>(a.b)[i];
+    reinterpret_cast<uint4*>(a.out)[i] = make_uint4(word(va.x, vb.x), word(va.y, vb.y), word(va.z, vb.z), word(va.w, vb.w));
+  }
+  for (long long i = (nvec << 4) + tid; i < a.n; i += stride) a.out[i] = (int8_t)word((uint8_t)a.a[i], (uint8_t)a.b[i]);
+}
+
+// Every other case (mul, or an add without an exact linear form). An int8 operand takes 256 values, so its input-side
+// rescale is a 256-entry table (filled here by the same apply_scale_32, one entry per thread); the output rescale stays
+// arithmetic: EPI 0 = 64-bit, 1 / 2 = the compact 32-bit record (common.cuh) with / without the sign term, chosen by the
+// planner when it can bound |operand sum or product| (it evaluates the same two tables).
 template <int EPI>
 __global__ void __launch_bounds__(kThreads) binary_kernel(BinaryArgs a) {
   grid_dependency_release();
@@ -310,26 +110,18 @@ __global__ void __launch_bounds__(kThreads) binary_kernel(BinaryArgs a) {
 __global__ void __launch_bounds__(kThreads) table_kernel(const int8_t* __restrict__ x,
                                                          const int8_t* __restrict__ table,
                                                          int8_t* __restrict__ out, long long n) {
-  grid_dependency_release();
-  grid_dependency_wait();
   __shared__ uint8_t lut[256];
   // index by the raw byte: entry for byte b is table[(int8)b + 128]
   lut[threadIdx.x] = (uint8_t)table[(int)(int8_t)threadIdx.x + 128];
+  grid_dependency_release();
+  grid_dependency_wait();
   __syncthreads();
   const long long nvec = n >> 4;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = tid; i < nvec; i += stride) {
-    uint4 v = reinterpret_cast<const uint4*>(x)[i];
-    uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      uint32_t r = 0;
-#pragma unroll
-      for (int j = 0; j < 4; j++) r |= (uint32_t)lut[(w[k] >> (8 * j)) & 0xff] << (8 * j);
-      w[k] = r;
-    }
-    reinterpret_cast<uint4*>(out)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    const uint4 v = reinterpret_cast<const uint4*>(x)[i];
+    reinterpret_cast<uint4*>(out)[i] = make_uint4(lut_word(lut, v.x), lut_word(lut, v.y), lut_word(lut, v.z), lut_word(lut, v.w));
   }
   for (long long i = (nvec << 4) + tid; i < n; i += stride) out[i] = (int8_t)lut[(uint8_t)x[i]];
 }
@@ -453,38 +245,9 @@ __global__ void __launch_bounds__(kThreads) resize_nn2x_kernel(const int8_t* __r
 
 }  // namespace
 
-void launch_maxpool(const PoolArgs& a, cudaStream_t stream) {
-  if (a.elem16) {
-    if ((a.C & 7) == 0) maxpool_i16_kernel<8><<<grid_for((long long)a.N * a.OH * a.OW * (a.C / 8)), kThreads, 0, stream>>>(a);
-    else maxpool_i16_kernel<1><<<grid_for((long long)a.N * a.OH * a.OW * a.C), kThreads, 0, stream>>>(a);
-    return;
-  }
-  if ((a.C & 15) == 0) {
-    long long total = (long long)a.N * a.OH * a.OW * (a.C / 16);
-    launch_dependent(maxpool_kernel<16>, dim3(grid_for(total)), dim3(kThreads), 0, stream, a);
-  } else {
-    long long total = (long long)a.N * a.OH * a.OW * a.C;
-    launch_dependent(maxpool_kernel<1>, dim3(grid_for(total)), dim3(kThreads), 0, stream, a);
-  }
-}
-
-void launch_avgpool(const PoolArgs& a, cudaStream_t stream) {
-  if ((a.C & 15) == 0 && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.out & 15) == 0) {
-    long long total = (long long)a.N * a.OH * a.OW * (a.C / 16);
-    // few outputs with many taps each: spread the taps over a warp
-    if (a.KH * a.KW >= 16 && total < 148ll * 2048) launch_dependent(avgpool_warp_kernel, dim3(grid_for(total * 32)), dim3(kThreads), 0, stream, a);
-    else launch_dependent(avgpool_kernel<16>, dim3(grid_for(total)), dim3(kThreads), 0, stream, a);
-  } else if ((a.C & 3) == 0) {
-    long long total = (long long)a.N * a.OH * a.OW * (a.C / 4);
-    launch_dependent(avgpool_kernel<4>, dim3(grid_for(total)), dim3(kThreads), 0, stream, a);
-  } else {
-    long long total = (long long)a.N * a.OH * a.OW * a.C;
-    launch_dependent(avgpool_kernel<1>, dim3(grid_for(total)), dim3(kThreads), 0, stream, a);
-  }
-}
-
 void launch_binary(const BinaryArgs& a, cudaStream_t stream) {
-  if (a.epi == 1) launch_dependent(binary_kernel<1>, dim3(grid_for((a.n + 15) / 16)), dim3(kThreads), 0, stream, a);
+  if (a.lin) launch_dependent(binary_linear_kernel, dim3(grid_for((a.n + 15) / 16)), dim3(kThreads), 0, stream, a);
+  else if (a.epi == 1) launch_dependent(binary_kernel<1>, dim3(grid_for((a.n + 15) / 16)), dim3(kThreads), 0, stream, a);
   else if (a.epi == 2) launch_dependent(binary_kernel<2>, dim3(grid_for((a.n + 15) / 16)), dim3(kThreads), 0, stream, a);
   else launch_dependent(binary_kernel<0>, dim3(grid_for((a.n + 15) / 16)), dim3(kThreads), 0, stream, a);
 }

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <vector>
 
 #include "common.cuh"
 
@@ -98,7 +99,12 @@ struct PoolArgs {
   int pad_value;            // max pool
   int input_zp, output_zp;  // avg pool
   int elem16;               // max pool on int16 tensors (x and out then point to int16 data)
+  const int8_t* lut;        // fused 256-entry table, or null (only where pool_strip_applies)
+  const int4* by_count;     // average pool: pool_avg_records on the device, or null
 };
+bool pool_strip_applies(const PoolArgs& a);  // the window (not the sizes) decides
+// Records {M', -, K} by tap count (index 0 unused) of pool_strip_kernel's average; false when a count has no exact one.
+bool pool_avg_records(int taps, int input_zp, int output_zp, std::vector<int4>& out);
 void launch_maxpool(const PoolArgs& a, cudaStream_t stream);
 void launch_avgpool(const PoolArgs& a, cudaStream_t stream);
 
@@ -113,6 +119,9 @@ struct BinaryArgs {
   int a_lshift, b_lshift;  // (x - zp) << lshift before the input rescale (two-stage input rescale), 0..22
   int epi;                 // output rescale: 0 = 64-bit arithmetic, 1 / 2 = the compact 32-bit record q4 with / without the sign term
   int4 q4;
+  // add / sub as one linear function of the two bytes with lin_f fraction bits in the high word (binary_linear_kernel)
+  int lin, lin_f, lin_ma, lin_mb;
+  long long lin_k;
 };
 void launch_binary(const BinaryArgs& a, cudaStream_t stream);
 

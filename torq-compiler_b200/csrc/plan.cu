@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdlib>
@@ -209,6 +210,52 @@ long long host_apply_scale_32(long long value, int mult, int shift, bool double_
   return (long long)(int32_t)(uint32_t)(unsigned long long)((v * (long long)mult + round) >> shift);
 }
 
+// add / sub of two bytes with three rescales is, up to its roundings, linear in the bytes. Looks for ma, mb, K with
+//   clamp((xa * 2^8 * ma + xb * 2^8 * mb + K) >> (32 + F)) == the op's result for every one of the 65536 operand pairs:
+// ma, mb are the real factors at 2^(24 + F), every pair then bounds K from one or both sides, and any K left between the
+// bounds is exact. The op's own operand roundings are of the order of 2^-20 of a result step, so a K nearly always exists.
+static void binary_linear_form(const tb200_op_t& op, BinaryArgs& a) {
+  a.lin = 0;
+  if (a.kind == 2 || a.clamp_min < -128 || a.clamp_max > 127 || a.clamp_min > a.clamp_max) return;
+  const bool dr = op.double_round != 0;
+  const double out = std::ldexp((double)a.out_mult, -a.out_shift);
+  const double sa = std::ldexp((double)a.a_mult, a.a_lshift - a.a_shift) * out;
+  const double sb = std::ldexp((double)a.b_mult, a.b_lshift - a.b_shift) * out * (a.kind == 1 ? -1.0 : 1.0);
+  int f = 6;
+  while (f >= 2 && std::ldexp(std::max(std::fabs(sa), std::fabs(sb)), 24 + f) >= 2147483000.0) f--;
+  if (f < 2) return;
+  long long ta[256], tb[256];
+  for (int v = -128; v < 128; v++) {
+    ta[v + 128] = host_apply_scale_32((long long)(v - a.a_zp) * (1ll << a.a_lshift), a.a_mult, a.a_shift, dr);
+    tb[v + 128] = host_apply_scale_32((long long)(v - a.b_zp) * (1ll << a.b_lshift), a.b_mult, a.b_shift, dr);
+  }
+  std::vector<int8_t> want(65536);
+  for (int x = 0; x < 256; x++)
+    for (int y = 0; y < 256; y++) {
+      const long long s = a.kind == 1 ? ta[x] - tb[y] : ta[x] + tb[y];
+      const long long r = (int32_t)(host_apply_scale_32(s, a.out_mult, a.out_shift, dr) + a.out_zp);
+      want[x * 256 + y] = (int8_t)std::max<long long>(a.clamp_min, std::min<long long>(a.clamp_max, r));
+    }
+  // DOUBLE_ROUND moves the thresholds of positive and negative values apart by a trace: a trace of extra slope allows for it
+  for (double extra : {std::ldexp(1.0, -26), std::ldexp(1.0, -24), 0.0, std::ldexp(1.0, -22), std::ldexp(1.0, -20)}) {
+    const long long ma = std::llround(std::ldexp(sa * (1.0 + extra), 24 + f)), mb = std::llround(std::ldexp(sb * (1.0 + extra), 24 + f));
+    long long lo = INT64_MIN, hi = INT64_MAX;
+    for (int x = 0; x < 256; x++)
+      for (int y = 0; y < 256; y++) {
+        const long long r = want[x * 256 + y], q = (long long)(x - 128) * 256 * ma + (long long)(y - 128) * 256 * mb;
+        if (r > a.clamp_min) lo = std::max(lo, r * (1ll << (32 + f)) - q);
+        if (r < a.clamp_max) hi = std::min(hi, (r + 1) * (1ll << (32 + f)) - q - 1);
+      }
+    if (lo > hi || lo == INT64_MIN || hi == INT64_MAX || std::max(std::llabs(ma), std::llabs(mb)) >= (1ll << 31)) continue;
+    a.lin = 1;
+    a.lin_f = f;
+    a.lin_ma = (int)ma;
+    a.lin_mb = (int)mb;
+    a.lin_k = lo + (hi - lo) / 2;
+    return;
+  }
+}
+
 // The parameters of a rescaled add / sub / mul without its pointers and size. The operand-side rescales are functions
 // of one byte: both tables are evaluated here as the kernel does, the value that reaches the output rescale is
 // bounded, and the 32-bit form of that rescale is taken when it is exact. False: a left shift outside [0, 22].
@@ -237,6 +284,7 @@ static bool binary_args_of(const tb200_op_t& op, BinaryArgs& a) {
   a.epi = (ma < (1ll << 31) && mb < (1ll << 31) && bound < (1ll << 29))
               ? Builder::q4_params({cp}, {bound}, op.double_round != 0, a.out_zp, a.clamp_min, q4) : 0;
   if (a.epi) a.q4 = q4[0];
+  binary_linear_form(op, a);
   return true;
 }
 
@@ -560,7 +608,16 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       const auto& op = ops[i];
       if (op.kind != TB200_OP_TABLE || op.in0 < 0 || op.in0 >= nt || op.out0 < 0 || op.out0 >= nt) continue;
       const int src = op.in0, pc = producer[src];
-      if (pc < 0 || pc >= i || ops[pc].kind != TB200_OP_CONV2D || uses[src] != 1 || table_after[pc] >= 0 ||
+      if (pc < 0 || pc >= i || !takes_table(ops[pc]) || uses[src] != 1 || table_after[pc] >= 0 ||
+    // the pooling windows with a strip kernel apply a table the same way
+    auto takes_table = [](const tb200_op_t& o) {
+      if (o.kind == TB200_OP_CONV2D) return true;
+      if (o.kind != TB200_OP_MAXPOOL && o.kind != TB200_OP_AVGPOOL) return false;
+      PoolArgs a{};
+      a.KH = o.kh; a.KW = o.kw; a.stride_h = o.stride_h; a.stride_w = o.stride_w;
+      std::vector<int4> rec;
+      return pool_strip_applies(a) && (o.kind == TB200_OP_MAXPOOL || pool_avg_records(o.kh * o.kw, o.in0_zp, o.out_zp, rec));
+    };
           tensors[src].kind != TB200_TENSOR_ACTIVATION || tensors[src].dtype != TB200_I8 || tensors[op.out0].dtype != TB200_I8)
         continue;
       table_after[pc] = i;
@@ -762,7 +819,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
     if (fused_away[i]) {
       step.kernel_name = op.kind == TB200_OP_RMSNORM ? "(norm fused into the previous norm)"
                          : op.kind == TB200_OP_ADD   ? "(add in the convolution's epilogue)"
-                                                     : "(table in the convolution's epilogue)";
+                         : op.kind == TB200_OP_TRANSPOSE || op.kind == TB200_OP_EW ? "(in the op it feeds or follows)"
+                                                     : "(table in the producer's epilogue)";
       step.launches = 0;
       step.launch = [](const ExecContext&) {};
       plan.steps.push_back(std::move(step));
@@ -1346,7 +1404,17 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (!tbl) return b.status;
         size_t t_off = b.add_const(tbl, 256);
         long long n = (long long)b.numel(op.in0);
-        Loc lx = loc(op.in0), lo = loc(op.out0);
+        // a table that is the only reader runs in the pool's kernel
+        const int fused_table = table_after[i];
+        size_t lut_off = 0;
+        if (fused_table >= 0) {
+          const int8_t* tbl = b.const_data<int8_t>(ops[fused_table].table, 256, "table", fused_table);
+          if (!tbl) return b.status;
+          if (b.numel(ops[fused_table].out0) != b.numel(op.out0) || !pool_strip_applies(a))
+            return b.fail(TB200_INVALID_ARGUMENT, "op %d: table wants int8 input/output of equal size", fused_table);
+          lut_off = b.add_const(tbl, 256);
+        }
+        Loc lx = loc(op.in0), lo = loc(fused_table >= 0 ? ops[fused_table].out0 : op.out0);
         step.kernel_name = "table";
         step.launch = [=](const ExecContext& c) {
           launch_table((const int8_t*)lx.resolve(c), (const int8_t*)(c.consts + t_off), (int8_t*)lo.resolve(c), n,
@@ -1358,9 +1426,15 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (!b.valid_id(op.in0) || !b.valid_id(op.out0) || b.numel(op.in0) != b.numel(op.out0))
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: rescale wants input/output of equal size", i);
         if (tensors[op.in0].dtype != TB200_I8 || tensors[op.out0].dtype != TB200_I8 || op.flags != 0) {
+        std::vector<int4> records;
+        size_t rec_off = 0;
+        const bool has_rec = !is_max && pool_strip_applies(a) && pool_avg_records(a.KH * a.KW, a.input_zp, a.output_zp, records);
+        if (has_rec) rec_off = b.add_const(records.data(), records.size() * sizeof(int4));
           // generic form: any of i8 / i16 / i32 in and out, unsigned storage by flag
           auto int_t = [](uint32_t d) { return d == TB200_I8 || d == TB200_I16 || d == TB200_I32; };
           if (!int_t(tensors[op.in0].dtype) || !int_t(tensors[op.out0].dtype))
+          k.lut = fused_table >= 0 ? (const int8_t*)(c.consts + lut_off) : nullptr;
+          k.by_count = has_rec ? (const int4*)(c.consts + rec_off) : nullptr;
             return b.fail(TB200_INVALID_ARGUMENT, "op %d: rescale wants integer tensors", i);
           const auto& x = tensors[op.in0];
           const int C = x.shape[x.rank - 1];
