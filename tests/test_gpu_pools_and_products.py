@@ -1,0 +1,91 @@
+"""The strip pooling kernels, the one-step rescaled add and the tiled products at the sizes where they can go wrong: odd
+frames and channel counts, windows that hang over every edge, tile remainders, folded transposes, scalars and casts."""
+import numpy as np
+import pytest
+from gpu_exec import run_graph_gpu
+from oracle_exec import run_graph
+from torq_b200.bf16 import from_bf16, to_bf16
+from torq_b200.oplist import Graph
+from torq_b200.quant import add_rescale_params
+from torq_b200.runtime import Executable
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(device, g, inputs):
+    for want, got in zip(run_graph(g, inputs), run_graph_gpu(device, g, inputs)):
+        assert want.shape == got.shape and (want == got).all(), int((want != got).sum())
+
+
+@pytest.mark.parametrize("k,s", [(2, 2), (3, 1), (3, 2), (5, 1)])
+@pytest.mark.parametrize("shape", [(1, 5, 7, 3), (2, 9, 6, 20), (1, 13, 11, 32), (3, 40, 33, 64)])
+@pytest.mark.parametrize("table", [False, True])
+def test_strip_pools(device, k, s, shape, table):
+    rng = np.random.default_rng(k * 100 + s)
+    x = rng.integers(-128, 128, shape, dtype=np.int8)
+    t = rng.integers(-128, 128, 256).astype(np.int8)
+    pad = ((k - 1) // 2, k // 2) * 2
+    for kind in ("max", "avg"):
+        g = Graph()
+        xi = g.input(shape)
+        y = g.maxpool2d(xi, (k, k), (s, s), pad, pad_value=-77) if kind == "max" else \
+            g.avg_pool2d(xi, (k, k), (s, s), pad, input_zp=-9, output_zp=5)
+        g.output(g.table(y, t) if table else y)
+        if table:
+            ex = Executable(device, g.serialize())
+            assert ex.launch_count == 1, ex.op_kernels()
+            ex.destroy()
+        _check(device, g, [x])
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 4099])
+@pytest.mark.parametrize("scales", [(0.02, 0.1, 0.05), (0.07, 0.03, 0.09), (0.05, 0.05, 0.02)])
+def test_rescaled_add_covers_every_operand_pair(device, n, scales):
+    rng = np.random.default_rng(n)
+    m0, m1, mo = add_rescale_params(*scales)
+    a, b = (rng.integers(-128, 128, (1, n), dtype=np.int8) for _ in range(2))
+    if n == 4099:  # all 65536 pairs
+        p = np.arange(65536)
+        a, b = (p >> 8).astype(np.uint8).view(np.int8).reshape(1, -1), (p & 255).astype(np.uint8).view(np.int8).reshape(1, -1)
+    for fn, clamp in (("add", (-128, 127)), ("sub", (-100, 90))):
+        g = Graph()
+        g.output(getattr(g, fn)(g.input(a.shape), g.input(b.shape), a_zp=7, a_ms=m0, b_zp=-10, b_ms=m1, out_ms=mo, out_zp=3, clamp=clamp))
+        _check(device, g, [a, b])
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 1, 1), (16, 128, 17), (33, 130, 31), (160, 65, 190), (300, 36, 900), (520, 129, 512)])
+@pytest.mark.parametrize("dtype", ["bf16", "f32", "i16", "i8"])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_tiled_products(device, M, K, N, dtype, transposed):
+    rng = np.random.default_rng(M + K + N)
+    shape_b = (N, K) if transposed else (K, N)
+    if dtype[0] == "i":
+        lim = 128 if dtype == "i8" else 32768
+        a, b = (rng.integers(-lim, lim, s).astype(np.int8 if dtype == "i8" else np.int16) for s in ((M, K), shape_b))
+    else:
+        a, b = (rng.normal(0, 1, s).astype(np.float32) for s in ((M, K), shape_b))
+        if dtype == "bf16":
+            a, b = to_bf16(a), to_bf16(b)
+    g = Graph()
+    ai, bi = g.input((M, K), dtype), g.input(shape_b, dtype)
+    bt = g.transpose(bi, (1, 0)) if transposed else bi
+    g.output(g.matmul_i32(ai, bt, a_zp=3, b_zp=-2) if dtype[0] == "i" else g.matmul_f(ai, bt, "f32"))
+    ex = Executable(device, g.serialize())
+    assert ex.launch_count == 1, ex.op_kernels()
+    ex.destroy()
+    _check(device, g, [a, b])
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 255), (5, 256), (7, 500), (2, 1024), (4, 1100)])
+def test_softmax_with_its_scalar_and_cast(device, rows, cols):
+    x = np.random.default_rng(cols).normal(0, 3, (rows, cols)).astype(np.float32)
+    g = Graph()
+    p = g.softmax(g.ew("mul", g.input(x.shape, "f32"), g.const(np.full((1, 1), 0.37, np.float32))))
+    g.output(g.ew("cast", p, out_dtype="bf16"))
+    if x.size > 1:
+        ex = Executable(device, g.serialize())
+        assert ex.launch_count == 1, ex.op_kernels()
+        ex.destroy()
+    got = from_bf16(run_graph_gpu(device, g, [x])[0])
+    e = np.exp((x * np.float32(0.37)).astype(np.float64) - (x * np.float32(0.37)).max(-1, keepdims=True))
+    assert np.allclose(got, e / e.sum(-1, keepdims=True), rtol=2 ** -7, atol=1e-30)

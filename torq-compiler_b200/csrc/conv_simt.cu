@@ -339,53 +339,6 @@ __global__ void __launch_bounds__(128) conv2d_c16_kernel(ConvArgs a) {
   }
 }
 
-// raw torq_hl.matmul (tests/testdata/tosa_ops/matmul-in-int8-out-int32.mlir, matmul-in-int16-out-int32.mlir,
-// matmul-in-int16-out-int16.mlir): int8 x int8 or int16 x int16, accumulated in int32 with wrap-around, stored as
-// int32 or truncated to int16. A block computes a 64 x 64 tile of the result from 64 x 16 / 16 x 64 tiles of the
-// operands in shared memory; a thread owns a 4 x 4 patch.
-template <typename TIn, typename TOut>
-__global__ void __launch_bounds__(256) matmul_int_kernel(const TIn* __restrict__ a, const TIn* __restrict__ b,
-                                                         TOut* __restrict__ out, int M, int K, int N, int a_zp, int b_zp) {
-  __shared__ int sa[16][64 + 1];  // [k][m]
-  __shared__ int sb[16][64];      // [k][n]
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  int acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0;
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-      const int am = i >> 4, ak = i & 15;  // a: consecutive threads along k
-      sa[ak][am] = (m0 + am < M && k0 + ak < K) ? (int)a[(size_t)(m0 + am) * K + k0 + ak] - a_zp : 0;
-      const int bk = i >> 6, bn = i & 63;  // b: consecutive threads along n
-      sb[bk][bn] = (k0 + bk < K && n0 + bn < N) ? (int)b[(size_t)(k0 + bk) * N + n0 + bn] - b_zp : 0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-      int av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) av[i] = sa[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) bv[j] = sb[k][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] += av[i] * bv[j];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int m = m0 + ty * 4 + i, n = n0 + tx + 16 * j;
-      if (m < M && n < N) out[(size_t)m * N + n] = (TOut)acc[i][j];
-    }
-}
-
 // The 3x3 window over 3 channels (the stem of an image network) with the compact 32-bit epilogue records. A thread
 // owns kStemPix output pixels (adjacent threads adjacent pixels). A kernel row of a pixel is 9 consecutive bytes of
 // the input: three aligned words and two funnel shifts bring them in (pixels whose window leaves the image, or whose
@@ -668,19 +621,6 @@ void launch_fc_rows(const FcRowsArgs& a, cudaStream_t stream) {
 void launch_conv2d_i16(const ConvI16Args& a, cudaStream_t stream) {
   const long long total = (long long)a.N * a.OH * a.OW * a.OC;
   conv2d_i16_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(a);
-}
-
-void launch_matmul_int(const void* a, const void* b, void* out, bool in_i16, bool out_i16, int M, int K, int N, int a_zp,
-                       int b_zp, cudaStream_t stream) {
-  const dim3 grid((N + 63) / 64, (M + 63) / 64);
-  if (!in_i16 && !out_i16)
-    matmul_int_kernel<int8_t, int32_t><<<grid, 256, 0, stream>>>((const int8_t*)a, (const int8_t*)b, (int32_t*)out, M, K, N, a_zp, b_zp);
-  else if (!in_i16)
-    matmul_int_kernel<int8_t, int16_t><<<grid, 256, 0, stream>>>((const int8_t*)a, (const int8_t*)b, (int16_t*)out, M, K, N, a_zp, b_zp);
-  else if (!out_i16)
-    matmul_int_kernel<int16_t, int32_t><<<grid, 256, 0, stream>>>((const int16_t*)a, (const int16_t*)b, (int32_t*)out, M, K, N, a_zp, b_zp);
-  else
-    matmul_int_kernel<int16_t, int16_t><<<grid, 256, 0, stream>>>((const int16_t*)a, (const int16_t*)b, (int16_t*)out, M, K, N, a_zp, b_zp);
 }
 
 }  // namespace tb200

@@ -255,21 +255,57 @@ __global__ void __launch_bounds__(256) table16_kernel(const int16_t* __restrict_
   }
 }
 
-// One warp per row: maximum, exp and sum in fp32, then one multiplication by the reciprocal of the sum.
-__global__ void __launch_bounds__(256) softmax_kernel(const void* __restrict__ x, void* __restrict__ out, long long rows, int cols,
-                                                      int dtype) {
+// One warp per row: maximum, exp and sum in fp32, then one multiplication by the reciprocal of the sum. PER > 0: the row
+// (at most 32 * PER values) stays in registers, so it is read once and every exponential is taken once. The operand may be
+// multiplied by a scalar constant first (f32, rounded as the stand-alone multiplication stores it) and the result, rounded
+// to the operand's type, may be stored as the other float type: what the planner folded in. Types are template parameters:
+// chosen per element they cost more than the arithmetic (512 x 512: 11 -> 4 us).
+template <typename T>
+__device__ __forceinline__ float as_float(T v) {
+  if (sizeof(T) == 4) return v;
+  return __uint_as_float((uint32_t)v << 16);
+}
+template <typename TIn, typename TOut>
+__device__ __forceinline__ void softmax_out(TOut* p, float v) {
+  if (sizeof(TIn) == 2) v = __bfloat162float(__float2bfloat16_rn(v));
+  if (sizeof(TOut) == 4) *reinterpret_cast<float*>(p) = v;
+  else *reinterpret_cast<uint16_t*>(p) = __bfloat16_as_ushort(__float2bfloat16_rn(v));
+}
+template <typename TIn, typename TOut, int PER>
+__global__ void __launch_bounds__(128) softmax_kernel(SoftmaxArgs a) {
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const long long base = row * cols;
-  float m = -INFINITY;
-  for (int c = lane; c < cols; c += 32) m = fmaxf(m, load_float(x, dtype, base + c));
+  if (row >= a.rows) return;
+  const TIn* x = reinterpret_cast<const TIn*>(a.x) + row * a.cols;
+  TOut* out = reinterpret_cast<TOut*>(a.out) + row * a.cols;
+  const float scale = a.scale ? *a.scale : 1.0f;
+  float m = -INFINITY, sum = 0.f;
+  if (PER > 0) {
+    float v[PER > 0 ? PER : 1];
+#pragma unroll
+    for (int j = 0; j < PER; j++) v[j] = lane + 32 * j < a.cols ? as_float(x[lane + 32 * j]) * scale : -INFINITY;
+#pragma unroll
+    for (int j = 0; j < PER; j++) m = fmaxf(m, v[j]);
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+    for (int j = 0; j < PER; j++)
+      if (lane + 32 * j < a.cols) {
+        v[j] = expf(v[j] - m);
+        sum += v[j];
+      }
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float inv = 1.0f / sum;
+#pragma unroll
+    for (int j = 0; j < PER; j++)
+      if (lane + 32 * j < a.cols) softmax_out<TIn>(out + lane + 32 * j, v[j] * inv);
+    return;
+  }
+  for (int c = lane; c < a.cols; c += 32) m = fmaxf(m, as_float(x[c]) * scale);
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  float sum = 0.f;
-  for (int c = lane; c < cols; c += 32) sum += expf(load_float(x, dtype, base + c) - m);
+  for (int c = lane; c < a.cols; c += 32) sum += expf(as_float(x[c]) * scale - m);
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = 1.0f / sum;
-  for (int c = lane; c < cols; c += 32) store_float(out, dtype, base + c, expf(load_float(x, dtype, base + c) - m) * inv);
+  for (int c = lane; c < a.cols; c += 32) softmax_out<TIn>(out + c, expf(as_float(x[c]) * scale - m) * inv);
 }
 
 unsigned grid_for(long long n) {
@@ -342,20 +378,6 @@ __global__ void __launch_bounds__(256) rows_by_index_kernel(const uint8_t* __res
 }  // namespace
 
 namespace {
-// tosa.matmul on floats: one thread per output, products and sums rounded separately (no fused multiply-add), k in order
-__global__ void __launch_bounds__(256) matmul_f_kernel(const void* __restrict__ a, const void* __restrict__ b, void* __restrict__ out,
-                                                       int M, int K, int N, int in_dtype, int out_dtype) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)M * N) return;
-  const int n = (int)(idx % N), m = (int)(idx / N);
-  float acc = 0.f;
-  for (int k = 0; k < K; k++)
-    acc = __fadd_rn(acc, __fmul_rn(load_float(a, in_dtype, (long long)m * K + k), load_float(b, in_dtype, (long long)k * N + n)));
-  store_float(out, out_dtype, idx, acc);
-}
-}  // namespace
-
-namespace {
 // tosa.depthwise_conv2d on floats: one thread per output; products and sums rounded separately, taps in (kh, kw) order,
 // taps outside the frame skipped, the bias added last
 __global__ void __launch_bounds__(256) depthwise_f_kernel(DepthwiseFArgs a) {
@@ -390,18 +412,29 @@ void launch_depthwise_f(const DepthwiseFArgs& a, cudaStream_t stream) {
   depthwise_f_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(a);
 }
 
-void launch_matmul_f(const void* a, const void* b, void* out, int M, int K, int N, int in_dtype, int out_dtype, cudaStream_t stream) {
-  matmul_f_kernel<<<(unsigned)(((long long)M * N + 255) / 256), 256, 0, stream>>>(a, b, out, M, K, N, in_dtype, out_dtype);
-}
-
 void launch_gather_rows(const void* values, const int32_t* idx, void* out, int N, int K, int W, int row_bytes, cudaStream_t stream) {
   rows_by_index_kernel<false><<<grid_for((long long)N * W * row_bytes), 256, 0, stream>>>((const uint8_t*)values, idx, (uint8_t*)out, N, K, W, row_bytes);
 }
 void launch_scatter_rows(const void* updates, const int32_t* idx, void* out, int N, int K, int W, int row_bytes, cudaStream_t stream) {
   rows_by_index_kernel<true><<<grid_for((long long)N * W * row_bytes), 256, 0, stream>>>((const uint8_t*)updates, idx, (uint8_t*)out, N, K, W, row_bytes);
 }
-void launch_softmax(const void* x, void* out, long long rows, int cols, int dtype, cudaStream_t stream) {
-  softmax_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(x, out, rows, cols, dtype);
+void launch_softmax(const SoftmaxArgs& a, cudaStream_t stream) {
+  const unsigned blocks = (unsigned)((a.rows + 3) / 4);
+  auto sized = [&](auto in, auto out) {
+    typedef decltype(in) I;
+    typedef decltype(out) O;
+    if (a.cols <= 256) softmax_kernel<I, O, 8><<<blocks, 128, 0, stream>>>(a);
+    else if (a.cols <= 512) softmax_kernel<I, O, 16><<<blocks, 128, 0, stream>>>(a);
+    else if (a.cols <= 1024) softmax_kernel<I, O, 32><<<blocks, 128, 0, stream>>>(a);
+    else softmax_kernel<I, O, 0><<<blocks, 128, 0, stream>>>(a);
+  };
+  if (a.dtype == TB200_F32) {
+    if (a.out_dtype == TB200_F32) sized(0.f, 0.f);
+    else sized(0.f, (uint16_t)0);
+  } else {
+    if (a.out_dtype == TB200_F32) sized((uint16_t)0, 0.f);
+    else sized((uint16_t)0, (uint16_t)0);
+  }
 }
 void launch_table16(const int16_t* x, const int16_t* table, int32_t* out, long long n, cudaStream_t stream) {
   table16_kernel<<<grid_for(n), 256, 0, stream>>>(x, table, out, n);

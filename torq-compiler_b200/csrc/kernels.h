@@ -88,9 +88,9 @@ bool depthwise3x3_supported(const DwArgs& a);
 // Packs [3][3][C] weights into [3 rows][variants][C] words; returns the word count written.
 size_t depthwise3x3_pack(const int8_t* w, int C, int stride, uint32_t* out);
 
-// raw int8 x int8 -> int32 matmul, b is [K][N]
+// raw integer matmul (matmul_tile.cu), b is [K][N], or [N][K] when b_transposed
 void launch_matmul_int(const void* a, const void* b, void* out, bool in_i16, bool out_i16, int M, int K, int N, int a_zp,
-                       int b_zp, cudaStream_t stream);
+                       int b_zp, bool b_transposed, cudaStream_t stream);
 
 struct PoolArgs {
   const int8_t* x;
@@ -352,7 +352,8 @@ void launch_reduce(const ReduceArgs& a, cudaStream_t stream);
 // (the caller has copied values to out first). Indices outside [0, K) give zero rows / are skipped.
 void launch_gather_rows(const void* values, const int32_t* idx, void* out, int N, int K, int W, int row_bytes, cudaStream_t stream);
 void launch_scatter_rows(const void* updates, const int32_t* idx, void* out, int N, int K, int W, int row_bytes, cudaStream_t stream);
-void launch_matmul_f(const void* a, const void* b, void* out, int M, int K, int N, int in_dtype, int out_dtype, cudaStream_t stream);
+void launch_matmul_f(const void* a, const void* b, void* out, int M, int K, int N, int in_dtype, int out_dtype, bool b_transposed,
+                     cudaStream_t stream);
 struct DepthwiseFArgs {
   const void* x;     // [N, H, W, C]
   const void* w;     // [KH, KW, C, M]
@@ -362,7 +363,15 @@ struct DepthwiseFArgs {
   int N, H, W, C, M, KH, KW, OH, OW, stride_h, stride_w, dil_h, dil_w, pad_t, pad_l;
 };
 void launch_depthwise_f(const DepthwiseFArgs& a, cudaStream_t stream);
-void launch_softmax(const void* x, void* out, long long rows, int cols, int dtype, cudaStream_t stream);
+struct SoftmaxArgs {
+  const void* x;
+  void* out;
+  const float* scale;  // a scalar the operand is multiplied by first, or null
+  long long rows;
+  int cols, dtype;     // of the operand
+  int out_dtype;
+};
+void launch_softmax(const SoftmaxArgs& a, cudaStream_t stream);
 void launch_table16(const int16_t* x, const int16_t* table, int32_t* out, long long n, cudaStream_t stream);
 
 void launch_resize_nn2x(const int8_t* x, int8_t* out, int N, int H, int W, int C, cudaStream_t stream);

@@ -585,6 +585,11 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   std::vector<char> defer_finalize(ops.size(), 0);
   std::vector<int> norm_second(ops.size(), -1);    // rmsnorm op -> the rmsnorm op fused into it
   std::vector<int> extra_out(ops.size(), -1);      // tensor an op writes on behalf of the op fused into it
+  std::vector<int> extra_in(ops.size(), -1);       // tensor an op reads on behalf of the op fused into it
+  // Attention written op by op: a rank-2 transpose that only feeds a matmul's second operand (the product reads the
+  // untransposed tensor), the multiplication of softmax's operand by a scalar, and the cast of its result.
+  std::vector<int> folded_transpose(ops.size(), -1);  // matmul op -> the tensor its transposed operand is read from
+  std::vector<int> softmax_scale(ops.size(), -1), softmax_cast(ops.size(), -1);  // softmax op -> the ew op fused into it
   {
     std::vector<int> uses(nt, 0), producer(nt, -1);
     for (int i = 0; i < (int)ops.size(); i++) {
@@ -604,11 +609,6 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         concat_into[a] = op.out0;
     }
     const char* no_fuse = getenv("TB200_NO_TABLE_FUSION");
-    for (int i = 0; i < (int)ops.size() && !(no_fuse && *no_fuse && *no_fuse != '0'); i++) {
-      const auto& op = ops[i];
-      if (op.kind != TB200_OP_TABLE || op.in0 < 0 || op.in0 >= nt || op.out0 < 0 || op.out0 >= nt) continue;
-      const int src = op.in0, pc = producer[src];
-      if (pc < 0 || pc >= i || !takes_table(ops[pc]) || uses[src] != 1 || table_after[pc] >= 0 ||
     // the pooling windows with a strip kernel apply a table the same way
     auto takes_table = [](const tb200_op_t& o) {
       if (o.kind == TB200_OP_CONV2D) return true;
@@ -618,6 +618,11 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       std::vector<int4> rec;
       return pool_strip_applies(a) && (o.kind == TB200_OP_MAXPOOL || pool_avg_records(o.kh * o.kw, o.in0_zp, o.out_zp, rec));
     };
+    for (int i = 0; i < (int)ops.size() && !(no_fuse && *no_fuse && *no_fuse != '0'); i++) {
+      const auto& op = ops[i];
+      if (op.kind != TB200_OP_TABLE || op.in0 < 0 || op.in0 >= nt || op.out0 < 0 || op.out0 >= nt) continue;
+      const int src = op.in0, pc = producer[src];
+      if (pc < 0 || pc >= i || !takes_table(ops[pc]) || uses[src] != 1 || table_after[pc] >= 0 ||
           tensors[src].kind != TB200_TENSOR_ACTIVATION || tensors[src].dtype != TB200_I8 || tensors[op.out0].dtype != TB200_I8)
         continue;
       table_after[pc] = i;
@@ -671,6 +676,55 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         break;
       }
     }
+    for (int i = 0; i < (int)ops.size(); i++) {
+      const auto& op = ops[i];
+      auto inter = [&](int id) { return id >= 0 && id < nt && tensors[id].kind == TB200_TENSOR_ACTIVATION && uses[id] == 1 && producer[id] >= 0; };
+      // what the fused op reads must still hold its value here: an input, a constant, or an intermediate (kept alive through extra_in)
+      auto readable = [&](int id) { return id >= 0 && id < nt && tensors[id].kind != TB200_TENSOR_STATE && tensors[id].kind != TB200_TENSOR_OUTPUT; };
+      if ((op.kind == TB200_OP_MATMUL_F || (op.kind == TB200_OP_MATMUL_I32 && op.weights < 0)) && inter(op.in1)) {
+        const int t = producer[op.in1];
+        const auto& tr = ops[t];
+        if (t < i && tr.kind == TB200_OP_TRANSPOSE && readable(tr.in0) && tensors[tr.in0].rank == 2 && tensors[op.in1].rank == 2 &&
+            tr.i0 == 1 && tr.i1 == 0 && tensors[tr.in0].dtype == tensors[op.in1].dtype &&
+            tensors[tr.in0].shape[0] == tensors[op.in1].shape[1] && tensors[tr.in0].shape[1] == tensors[op.in1].shape[0]) {
+          folded_transpose[i] = tr.in0;
+          extra_in[i] = tr.in0;
+          fused_away[t] = 1;
+        }
+      }
+      if (op.kind == TB200_OP_SOFTMAX && op.in0 >= 0 && op.in0 < nt && op.out0 >= 0 && op.out0 < nt) {
+        if (inter(op.in0)) {
+          const int t = producer[op.in0];
+          const auto& mu = ops[t];
+          if (t < i && mu.kind == TB200_OP_EW && mu.i0 == TB200_EW_MUL && readable(mu.in0) && readable(mu.in1)) {
+            for (int side = 0; side < 2; side++) {
+              const int x = side ? mu.in1 : mu.in0, s = side ? mu.in0 : mu.in1;
+              // bf16 operands keep their own op: the scalar would be bf16 too
+              if (tensors[s].kind != TB200_TENSOR_CONSTANT || b.numel(s) != 1 || tensors[s].dtype != TB200_F32 ||
+                  b.numel(x) != b.numel(op.in0) || b.numel(x) == 1 || tensors[x].dtype != TB200_F32 || tensors[op.in0].dtype != TB200_F32)
+                continue;
+              softmax_scale[i] = t;
+              extra_in[i] = x;
+              fused_away[t] = 1;
+              break;
+            }
+          }
+        }
+        if (inter(op.out0)) {
+          for (int j = i + 1; j < (int)ops.size(); j++) {
+            const auto& ca = ops[j];
+            if (ca.in0 != op.out0) continue;
+            if (ca.kind == TB200_OP_EW && ca.i0 == TB200_EW_CAST && ca.in1 < 0 && !(ca.flags & TB200_FLAG_BOOL_RESULT) && ca.out0 >= 0 && ca.out0 < nt &&
+                (tensors[ca.out0].dtype == TB200_BF16 || tensors[ca.out0].dtype == TB200_F32) && b.numel(ca.out0) == b.numel(op.out0)) {
+              softmax_cast[i] = j;
+              extra_out[i] = ca.out0;
+              fused_away[j] = 1;
+            }
+            break;
+          }
+        }
+      }
+    }
     const char* no_dec = getenv("TB200_NO_DECODER_FUSION");
     for (int i = 0; i + 1 < (int)ops.size() && !(no_dec && *no_dec && *no_dec != '0'); i++) {
       const auto& op = ops[i];
@@ -704,7 +758,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   }
   for (int i = 0; i < (int)ops.size(); i++) {
     const auto& op = ops[i];
-    int ins[3] = {op.in0, op.in1, op.in2};
+    int ins[4] = {op.in0, op.in1, op.in2, extra_in[i]};
     int outs[3] = {op.out0, op.out1, extra_out[i]};
     for (int id : ins)
       if (id >= 0) {
@@ -1309,11 +1363,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           const int M = ta.shape[0], K = ta.shape[1], N = tb.shape[1];
           if (tb.shape[0] != K || to.shape[0] != M || to.shape[1] != N)
             return b.fail(TB200_INVALID_ARGUMENT, "op %d: matmul shape mismatch", i);
-          Loc lx = loc(op.in0), lw = loc(op.in1), lo = loc(op.out0);
+          const bool tb_fold = folded_transpose[i] >= 0;  // [N, K] as the transpose's own operand holds it
+          Loc lx = loc(op.in0), lw = loc(tb_fold ? folded_transpose[i] : op.in1), lo = loc(op.out0);
           const int azp = op.in0_zp, bzp = op.weight_zp;
           step.kernel_name = "matmul_int";
           step.launch = [=](const ExecContext& c) {
-            launch_matmul_int(lx.resolve(c), lw.resolve(c), lo.resolve(c), in16, out16, M, K, N, azp, bzp, c.stream);
+            launch_matmul_int(lx.resolve(c), lw.resolve(c), lo.resolve(c), in16, out16, M, K, N, azp, bzp, tb_fold, c.stream);
           };
           break;
         }
@@ -1330,7 +1385,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         int azp = op.in0_zp, bzp = op.weight_zp;
         step.kernel_name = "matmul_int";
         step.launch = [=](const ExecContext& c) {
-          launch_matmul_int(lx.resolve(c), c.consts + w_off, lo.resolve(c), false, false, M, K, N, azp, bzp, c.stream);
+          launch_matmul_int(lx.resolve(c), c.consts + w_off, lo.resolve(c), false, false, M, K, N, azp, bzp, false, c.stream);
         };
         break;
       }
@@ -1357,13 +1412,29 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (o.shape[0] != a.N || o.shape[1] != a.OH || o.shape[2] != a.OW || o.shape[3] != a.C)
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: pooling output shape mismatch", i);
         a.pad_value = op.pad_value; a.input_zp = op.in0_zp; a.output_zp = op.out_zp;
-        Loc lx = loc(op.in0), lo = loc(op.out0);
+        // a table that is the only reader runs in the pool's kernel
+        const int fused_table = table_after[i];
+        size_t lut_off = 0;
+        if (fused_table >= 0) {
+          const int8_t* tbl = b.const_data<int8_t>(ops[fused_table].table, 256, "table", fused_table);
+          if (!tbl) return b.status;
+          if (b.numel(ops[fused_table].out0) != b.numel(op.out0) || !pool_strip_applies(a))
+            return b.fail(TB200_INVALID_ARGUMENT, "op %d: table wants int8 input/output of equal size", fused_table);
+          lut_off = b.add_const(tbl, 256);
+        }
+        Loc lx = loc(op.in0), lo = loc(fused_table >= 0 ? ops[fused_table].out0 : op.out0);
         const bool is_max = op.kind == TB200_OP_MAXPOOL;
         if (!is_max && (long long)a.KH * a.KW > 256)  // the kernel's per-count rescale table
           return b.fail(TB200_UNIMPLEMENTED, "op %d: average pooling windows above 256 taps are not supported", i);
+        std::vector<int4> records;
+        size_t rec_off = 0;
+        const bool has_rec = !is_max && pool_strip_applies(a) && pool_avg_records(a.KH * a.KW, a.input_zp, a.output_zp, records);
+        if (has_rec) rec_off = b.add_const(records.data(), records.size() * sizeof(int4));
         step.kernel_name = is_max ? "maxpool" : "avgpool";
         step.launch = [=](const ExecContext& c) {
           PoolArgs k = a;
+          k.lut = fused_table >= 0 ? (const int8_t*)(c.consts + lut_off) : nullptr;
+          k.by_count = has_rec ? (const int4*)(c.consts + rec_off) : nullptr;
           k.x = (const int8_t*)lx.resolve(c);
           k.out = (int8_t*)lo.resolve(c);
           if (is_max) launch_maxpool(k, c.stream);
@@ -1404,17 +1475,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (!tbl) return b.status;
         size_t t_off = b.add_const(tbl, 256);
         long long n = (long long)b.numel(op.in0);
-        // a table that is the only reader runs in the pool's kernel
-        const int fused_table = table_after[i];
-        size_t lut_off = 0;
-        if (fused_table >= 0) {
-          const int8_t* tbl = b.const_data<int8_t>(ops[fused_table].table, 256, "table", fused_table);
-          if (!tbl) return b.status;
-          if (b.numel(ops[fused_table].out0) != b.numel(op.out0) || !pool_strip_applies(a))
-            return b.fail(TB200_INVALID_ARGUMENT, "op %d: table wants int8 input/output of equal size", fused_table);
-          lut_off = b.add_const(tbl, 256);
-        }
-        Loc lx = loc(op.in0), lo = loc(fused_table >= 0 ? ops[fused_table].out0 : op.out0);
+        Loc lx = loc(op.in0), lo = loc(op.out0);
         step.kernel_name = "table";
         step.launch = [=](const ExecContext& c) {
           launch_table((const int8_t*)lx.resolve(c), (const int8_t*)(c.consts + t_off), (int8_t*)lo.resolve(c), n,
@@ -1426,15 +1487,9 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (!b.valid_id(op.in0) || !b.valid_id(op.out0) || b.numel(op.in0) != b.numel(op.out0))
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: rescale wants input/output of equal size", i);
         if (tensors[op.in0].dtype != TB200_I8 || tensors[op.out0].dtype != TB200_I8 || op.flags != 0) {
-        std::vector<int4> records;
-        size_t rec_off = 0;
-        const bool has_rec = !is_max && pool_strip_applies(a) && pool_avg_records(a.KH * a.KW, a.input_zp, a.output_zp, records);
-        if (has_rec) rec_off = b.add_const(records.data(), records.size() * sizeof(int4));
           // generic form: any of i8 / i16 / i32 in and out, unsigned storage by flag
           auto int_t = [](uint32_t d) { return d == TB200_I8 || d == TB200_I16 || d == TB200_I32; };
           if (!int_t(tensors[op.in0].dtype) || !int_t(tensors[op.out0].dtype))
-          k.lut = fused_table >= 0 ? (const int8_t*)(c.consts + lut_off) : nullptr;
-          k.by_count = has_rec ? (const int4*)(c.consts + rec_off) : nullptr;
             return b.fail(TB200_INVALID_ARGUMENT, "op %d: rescale wants integer tensors", i);
           const auto& x = tensors[op.in0];
           const int C = x.shape[x.rank - 1];
@@ -1916,9 +1971,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             to.shape[0] != ta.shape[0] || to.shape[1] != tb.shape[1])
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: matmul_f wants [M, K] x [K, N] of bf16 or f32 -> [M, N] of f32 or bf16", i);
         const int M = ta.shape[0], K = ta.shape[1], N = tb.shape[1], idt = (int)ta.dtype, odt = (int)to.dtype;
-        Loc la = loc(op.in0), lb = loc(op.in1), lo = loc(op.out0);
+        const bool tb_fold = folded_transpose[i] >= 0;
+        Loc la = loc(op.in0), lb = loc(tb_fold ? folded_transpose[i] : op.in1), lo = loc(op.out0);
         step.kernel_name = "matmul_f";
-        step.launch = [=](const ExecContext& c) { launch_matmul_f(la.resolve(c), lb.resolve(c), lo.resolve(c), M, K, N, idt, odt, c.stream); };
+        step.launch = [=](const ExecContext& c) {
+          launch_matmul_f(la.resolve(c), lb.resolve(c), lo.resolve(c), M, K, N, idt, odt, tb_fold, c.stream);
+        };
         break;
       }
       case TB200_OP_DEPTHWISE_F: {
@@ -2047,11 +2105,21 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             (tensors[op.in0].dtype != TB200_BF16 && tensors[op.in0].dtype != TB200_F32) || b.numel(op.in0) != b.numel(op.out0))
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: softmax wants bf16 or f32 tensors of equal size", i);
         const auto& x = tensors[op.in0];
-        const int cols = x.shape[x.rank - 1], dt = (int)x.dtype;
-        const long long rows = (long long)(b.numel(op.in0) / cols);
-        Loc lx = loc(op.in0), lo = loc(op.out0);
+        SoftmaxArgs a{};
+        a.cols = x.shape[x.rank - 1]; a.dtype = (int)x.dtype;
+        a.rows = (long long)(b.numel(op.in0) / a.cols);
+        // the multiplication by a scalar in front and the cast behind run in the same launch
+        const int pre = softmax_scale[i], post = softmax_cast[i];
+        const int src = pre >= 0 ? (b.numel(ops[pre].in0) == b.numel(op.in0) ? ops[pre].in0 : ops[pre].in1) : op.in0;
+        const int dst = post >= 0 ? ops[post].out0 : op.out0;
+        a.out_dtype = (int)tensors[dst].dtype;
+        Loc lx = loc(src), lo = loc(dst), ls = pre >= 0 ? loc(src == ops[pre].in0 ? ops[pre].in1 : ops[pre].in0) : Loc{};
         step.kernel_name = "softmax";
-        step.launch = [=](const ExecContext& c) { launch_softmax(lx.resolve(c), lo.resolve(c), rows, cols, dt, c.stream); };
+        step.launch = [=](const ExecContext& c) {
+          SoftmaxArgs k = a;
+          k.x = lx.resolve(c); k.out = lo.resolve(c); k.scale = (const float*)ls.resolve(c);
+          launch_softmax(k, c.stream);
+        };
         break;
       }
       case TB200_OP_TABLE16: {
