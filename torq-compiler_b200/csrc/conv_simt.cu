@@ -282,8 +282,8 @@ __global__ void __launch_bounds__(128) conv2d_smallic_kernel(ConvArgs a) {
 // Weight rows are Kpad bytes apart (K = TAPS * 16 is a multiple of 16, Kpad of 32).
 template <int TAPS>
 __global__ void __launch_bounds__(128) conv2d_c16_kernel(ConvArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   extern __shared__ uint4 w16[];  // [OC][TAPS]
   for (int i = threadIdx.x; i < a.OC * TAPS; i += blockDim.x) {
     const int oc = i / TAPS, t = i - oc * TAPS;
@@ -348,8 +348,8 @@ __global__ void __launch_bounds__(128) conv2d_c16_kernel(ConvArgs a) {
 constexpr int kStemPix = 4;
 template <int EPI, bool LUT>
 __global__ void __launch_bounds__(128) conv2d_stem333_kernel(ConvArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   extern __shared__ __align__(16) uint32_t stem_s[];  // [OC][8] weight words (word 7 zero), [OC] Q4 records, 256-byte table
   uint4* w_s = reinterpret_cast<uint4*>(stem_s);
   int4* q_s = reinterpret_cast<int4*>(stem_s + (size_t)a.OC * 8);

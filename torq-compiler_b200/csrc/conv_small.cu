@@ -1,0 +1,358 @@
+// Small convolutions and products (one image, a few hundred rows): warp-level int8 matrix instructions on fragments that
+// go from L2 straight to registers.
+//
+// What bounds such a call is not arithmetic (a whole MobileNetV2 layer on one image is 1..10 M multiply-adds, well under
+// a microsecond on any path) but the chain of latencies between the launch and the last store. The persistent tcgen05
+// kernel's chain - tensor-map fetch, TMEM allocation, TMA into shared memory, MMA, commit, TMEM read, staging, TMA store -
+// takes 5.8 .. 8.3 us per layer however little there is to do. Here a warp owns a 16 x 32 tile of the result, fetches its
+// operands with 16-byte loads (all of them in flight at once), multiplies with mma.sync and stores from registers: one
+// memory round trip, no barrier. A long K is split over up to eight warps of a block, whose sums meet in shared memory
+// once, so that a layer with few result tiles still has enough loads in flight.
+// Measured, one image: 3x3 56x56 x 64 -> 64 7.3 -> 3.0 us, 14x14 x 576 -> 96 6.6 -> 2.3 us, 3x3 20x20 x 128 -> 128
+// 7.4 -> 2.7 us, 112x112 x 16 -> 96 6.9 -> 4.0 us.
+//
+// Fragments. The K order of a product is free as long as both operands agree, so lane (g = lane / 4, t = lane % 4) takes
+// the 16 contiguous bytes 16 t .. 16 t + 15 of a 64-byte K step of row g: words 0 / 1 of them are its fragment of the
+// first k32 instruction, words 2 / 3 of the second. Likewise the columns: fragment column f of instruction j is channel
+// 8 (f / 2) + 2 j + f % 2 of the warp's 32, so that a lane ends with eight consecutive channels of a row and stores eight
+// bytes. The weights are laid out in exactly that order by conv_small_pack: a warp's load is 512 contiguous bytes.
+#include <string.h>
+
+#include "kernels.h"
+#include "dependent_launch.cuh"
+
+namespace tb200 {
+namespace {
+
+constexpr int kTileM = 16, kTileN = 32, kStepBytes = 64;
+constexpr int kSumPitch = kTileN + 4;  // words per row of a partial tile: rows land on different banks
+
+__device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Four consecutive channels of one row: rescale, clamp, table, and the residual add; q[j] are the channels' Q4 records.
+__device__ __forceinline__ uint32_t finish4(const ConvSmallArgs& a, const int (&acc)[4], const int4 (&q)[4], int chan, const int8_t* lut,
+                                            uint32_t other) {
+  int r[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    if (a.epi == 1) {
+      r[j] = scale_q4_sign(acc[j], q[j]);
+    } else if (a.epi == 2) {
+      r[j] = scale_q4(acc[j], q[j]);
+    } else {
+      const ChanParams cp = a.chan[chan + j];
+      r[j] = scale_cp<false>(acc[j] + cp.bias, cp) + a.out_zp;
+    }
+    r[j] = max(a.clamp_min, min(a.clamp_max, r[j]));
+  }
+  uint32_t w = pack4(r[0], r[1], r[2], r[3]);
+  if (a.lut) w = pack4(lut[(w & 0xff) ^ 0x80], lut[(w >> 8 & 0xff) ^ 0x80], lut[(w >> 16 & 0xff) ^ 0x80], lut[(w >> 24) ^ 0x80]);
+  if (a.res) {  // as binary_linear_kernel, clamped after the fraction is dropped
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int h = mad_wide_hi(sx8(other, j) * 256, a.add_m_other, (long long)(sx8(w, j) * 256) * (long long)a.add_m_self + a.add_k);
+      r[j] = max(a.add_clamp_min, min(a.add_clamp_max, h >> a.add_f));
+    }
+    w = pack4(r[0], r[1], r[2], r[3]);
+  }
+  return w;
+}
+
+// up to 8 bytes of a row at a channel offset; `full` = all of them exist and the address is 8-byte aligned
+__device__ __forceinline__ void store_bytes(int8_t* p, uint32_t w, int n) {
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    if (j < n) p[j] = (int8_t)(w >> (8 * j));
+}
+__device__ __forceinline__ uint32_t load_bytes(const int8_t* p, int n) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    if (j < n) w |= (uint32_t)(uint8_t)p[j] << (8 * j);
+  return w;
+}
+
+// MODE: what a row of the product is - kRows: lda bytes of memory; kConv: the taps of an output pixel, IC a multiple of 16;
+// kStem: the 27 bytes under a 3 x 3 window of 3 channels, one k32 instruction: lane t = 0 .. 2 holds the first eight of the nine
+// bytes of kernel row t (consecutive in memory), lane 3 the three ninth bytes.
+// U = K steps whose loads are in flight together; SPLIT: several warps share a tile.
+enum { kRows = 0, kConv = 1, kStem = 2 };
+template <int MODE, int U, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 256 : 128, SPLIT ? 2 : 4) conv_small_kernel(const ConvSmallArgs a) {
+  extern __shared__ int sums[];  // [tiles of the block][warps of a tile][16][kSumPitch], only with more than one warp per tile
+  __shared__ int8_t lut[256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int ks_log2 = SPLIT ? a.ks_log2 : 0, ks_n = 1 << ks_log2;
+  const int ks = warp & (ks_n - 1), slot = warp >> ks_log2;
+  const int tile = blockIdx.x * ((int)(blockDim.x >> 5) >> ks_log2) + slot;
+  const int mt = tile / a.n_tiles, nt = tile - mt * a.n_tiles;
+  const bool live = mt < a.m_tiles;
+  const int8_t* wp = a.w + ((size_t)(live ? nt : 0) * a.steps * 4) * 512 + lane * 16;
+  // the channels this thread finishes: eight of two rows, or (several warps per tile) four of every (8 ks_n)-th row
+  const int chan = (live ? nt : 0) * kTileN + (SPLIT ? 4 * (lane & 7) : 8 * t);
+  int4 q[SPLIT ? 4 : 8];
+  if (a.epi) {
+#pragma unroll
+    for (int j = 0; j < (SPLIT ? 4 : 8); j++) q[j] = __ldg(a.q4 + chan + j);
+  }
+  if (a.lut)
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = a.lut[i];
+
+  // the two rows of this lane
+  int px[2];
+  int ih0[2], iw0[2];
+  bool row_ok[2];
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const int row = mt * kTileM + g + 8 * r;
+    row_ok[r] = live && row < a.M;
+    if (MODE != kRows) {
+      const int pix = row_ok[r] ? row : 0;
+      const int n = pix / (a.OH * a.OW), rem = pix - n * (a.OH * a.OW), oh = rem / a.OW, ow = rem - oh * a.OW;
+      ih0[r] = oh * a.stride - a.pad_t;
+      iw0[r] = ow * a.stride - a.pad_l;
+      px[r] = ((n * a.H + ih0[r]) * a.W + iw0[r]) * a.IC;  // may lie outside: only dereferenced inside
+    } else {
+      px[r] = row * a.lda;
+    }
+  }
+  const uint32_t fill = (uint32_t)(a.input_zp & 0xff) * 0x01010101u;  // a tap outside the frame reads the zero point
+  auto load_a = [&](int step, uint4 (&v)[2]) {
+    const int c = 4 * step + t;  // 16-byte chunk of the K axis (tap-major)
+    const bool in_k = c < a.chunks;
+    if (MODE == kStem) {
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        v[r] = make_uint4(fill, fill, 0, 0);
+        if (!row_ok[r]) continue;
+        if (t < 3) {
+          if ((unsigned)(ih0[r] + t) >= (unsigned)a.H) continue;
+          const int off = px[r] + t * a.W * 3;
+          if (iw0[r] >= 0 && iw0[r] + 2 < a.W && (off & ~3) + 12 <= a.x_bytes) {
+            const uint32_t* p = reinterpret_cast<const uint32_t*>(a.x + (off & ~3));
+            const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], sh = (uint32_t)(off & 3) * 8;
+            v[r].x = __funnelshift_r(w0, w1, sh);
+            v[r].y = __funnelshift_r(w1, w2, sh);
+          } else {
+            uint32_t b[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) b[j] = (unsigned)(iw0[r] + j / 3) < (unsigned)a.W ? (uint32_t)(uint8_t)a.x[off + j] : fill & 0xff;
+            v[r].x = b[0] | b[1] << 8 | b[2] << 16 | b[3] << 24;
+            v[r].y = b[4] | b[5] << 8 | b[6] << 16 | b[7] << 24;
+          }
+        } else if ((unsigned)(iw0[r] + 2) < (unsigned)a.W) {
+          uint32_t b[3];
+#pragma unroll
+          for (int kh = 0; kh < 3; kh++) b[kh] = (unsigned)(ih0[r] + kh) < (unsigned)a.H ? (uint32_t)(uint8_t)a.x[px[r] + kh * a.W * 3 + 8] : fill & 0xff;
+          v[r].x = b[0] | b[1] << 8 | b[2] << 16;
+        }
+      }
+    } else if (MODE == kConv) {
+      const int tap = (int)(((unsigned)c * (unsigned)a.inv_icb) >> 20), icb = c - tap * a.icb;
+      const int kh = (int)(((unsigned)tap * (unsigned)a.inv_kw) >> 20), kw = tap - kh * a.KW;
+      const int off = (kh * a.W + kw) * a.IC + icb * 16;
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        v[r] = make_uint4(fill, fill, fill, fill);
+        if (in_k && row_ok[r] && (unsigned)(ih0[r] + kh) < (unsigned)a.H && (unsigned)(iw0[r] + kw) < (unsigned)a.W)
+          v[r] = *reinterpret_cast<const uint4*>(a.x + (px[r] + off));
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        v[r] = make_uint4(0, 0, 0, 0);
+        if (in_k && row_ok[r]) v[r] = *reinterpret_cast<const uint4*>(a.x + (px[r] + c * 16));
+      }
+    }
+  };
+  int acc[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc[j][i] = 0;
+
+  bool waited = false;
+  for (int s0 = ks; s0 < a.steps; s0 += U * ks_n) {
+    uint4 b[U][4], v[U][2];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int s = s0 + u * ks_n;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        b[u][j] = make_uint4(0, 0, 0, 0);
+        if (s < a.steps) b[u][j] = __ldg(reinterpret_cast<const uint4*>(wp + ((size_t)s * 4 + j) * 512));
+      }
+    }
+    if (!waited) {  // the weights and constants belong to the program: only the activations wait for the launch before
+      grid_dependency_wait();
+      grid_dependency_release();
+      waited = true;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) load_a(s0 + u * ks_n, v[u]);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        mma_s8(acc[j], v[u][0].x, v[u][1].x, v[u][0].y, v[u][1].y, b[u][j].x, b[u][j].y);
+        if (MODE != kStem) mma_s8(acc[j], v[u][0].z, v[u][1].z, v[u][0].w, v[u][1].w, b[u][j].z, b[u][j].w);
+      }
+  }
+  if (!waited) grid_dependency_wait();
+
+  if constexpr (!SPLIT) {
+    if (a.lut) __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      if (!row_ok[r]) continue;
+      const long long off = (long long)(mt * kTileM + g + 8 * r) * a.ldc + chan;
+      const int left = a.N - chan;
+      const bool vec = a.vec && left >= 8;
+      uint32_t o[2] = {0, 0};
+      if (a.res) {
+        if (vec) {
+          const uint2 ov = *reinterpret_cast<const uint2*>(a.res + off);
+          o[0] = ov.x;
+          o[1] = ov.y;
+        } else {
+          o[0] = load_bytes(a.res + off, left);
+          o[1] = load_bytes(a.res + off + 4, left - 4);
+        }
+      }
+      uint32_t w[2];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int four[4] = {acc[2 * h][2 * r], acc[2 * h][2 * r + 1], acc[2 * h + 1][2 * r], acc[2 * h + 1][2 * r + 1]};
+        const int4 qs[4] = {q[4 * h], q[4 * h + 1], q[4 * h + 2], q[4 * h + 3]};
+        w[h] = finish4(a, four, qs, chan + 4 * h, lut, o[h]);
+      }
+      if (vec) {
+        *reinterpret_cast<uint2*>(a.out + off) = make_uint2(w[0], w[1]);
+      } else {
+        store_bytes(a.out + off, w[0], left);
+        store_bytes(a.out + off + 4, w[1], left - 4);
+      }
+    }
+    return;
+  } else {
+  // several warps per tile: every warp leaves its sums, then each takes its share of the rows
+  int* mine = sums + (warp * kTileM) * kSumPitch;
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      *reinterpret_cast<int4*>(mine + (g + 8 * r) * kSumPitch + 8 * t + 4 * h) =
+          make_int4(acc[2 * h][2 * r], acc[2 * h][2 * r + 1], acc[2 * h + 1][2 * r], acc[2 * h + 1][2 * r + 1]);
+  __syncthreads();
+  if (!live) return;
+  const int* first = sums + ((slot << a.ks_log2) * kTileM) * kSumPitch;
+  for (int lr = ks * 4 + (lane >> 3); lr < kTileM; lr += 4 * ks_n) {
+    const int row = mt * kTileM + lr;
+    if (row >= a.M) break;
+    int four[4] = {0, 0, 0, 0};
+#pragma unroll 4
+    for (int k = 0; k < ks_n; k++) {
+      const int4 p = *reinterpret_cast<const int4*>(first + (k * kTileM + lr) * kSumPitch + 4 * (lane & 7));
+      four[0] += p.x;
+      four[1] += p.y;
+      four[2] += p.z;
+      four[3] += p.w;
+    }
+    const long long off = (long long)row * a.ldc + chan;
+    const int left = a.N - chan;
+    if (left <= 0) break;
+    const bool vec = a.vec && left >= 4;
+    const uint32_t o = !a.res ? 0u : vec ? *reinterpret_cast<const uint32_t*>(a.res + off) : load_bytes(a.res + off, left);
+    const int4 qs[4] = {q[0], q[1], q[2], q[3]};
+    const uint32_t w = finish4(a, four, qs, chan, lut, o);
+    if (vec) *reinterpret_cast<uint32_t*>(a.out + off) = w;
+    else store_bytes(a.out + off, w, left);
+  }
+  }
+}
+
+int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+}  // namespace
+
+int conv_small_steps(int taps, int IC) { return ceil_div((long long)taps * (IC / 16), kStepBytes / 16); }
+int conv_small_columns(int OC) { return ceil_div(OC, kTileN) * kTileN; }
+
+// The line to the tcgen05 kernel. A warp's tile costs about (steps + 5) * 0.18 ns of the whole chip beyond the 2 us that
+// every launch takes (measured over batches of 2 .. 23 of the layers of both networks), the tcgen05 kernel about 7 us up to
+// the same sizes: (tiles, steps, here / there in us) 1600, 6: 5.2 / 7.3; 4800, 1: 7.7 / 8.2; 3200, 5: 9.4 / 9.2;
+// 3200, 6: 9.9 / 7.4; 2300, 18: 11.2 / 10.9.
+constexpr long long kSmallCost = 29000;
+
+bool conv_small_applies(long long M, int OC, int taps, int IC) {
+  if (small_kernels_off() || IC % 16 != 0 || taps < 1 || taps > 64 || (long long)taps * (IC / 16) > 4096) return false;
+  const long long tiles = (long long)ceil_div(M, kTileM) * ceil_div(OC, kTileN);
+  return tiles * (conv_small_steps(taps, IC) + 5) <= kSmallCost && M * IC < (1ll << 30);
+}
+
+void conv_small_pack(const int8_t* w, int OC, int taps, int IC, int8_t* out) {
+  const int steps = conv_small_steps(taps, IC), n_tiles = ceil_div(OC, kTileN), chunks = taps * (IC / 16);
+  const long long K = (long long)taps * IC;
+  for (int nt = 0; nt < n_tiles; nt++)
+    for (int s = 0; s < steps; s++)
+      for (int j = 0; j < 4; j++)
+        for (int lane = 0; lane < 32; lane++) {
+          const int f = lane >> 2, c = 4 * s + (lane & 3);
+          const int oc = nt * kTileN + 8 * (f >> 1) + 2 * j + (f & 1);
+          int8_t* o = out + ((((size_t)nt * steps + s) * 4 + j) * 32 + lane) * 16;
+          if (oc < OC && c < chunks) memcpy(o, w + (size_t)oc * K + (size_t)c * 16, 16);
+          else memset(o, 0, 16);
+        }
+}
+
+void conv_small_pack_stem(const int8_t* w, int OC, int8_t* out) {
+  for (int i = 0; i < conv_small_columns(OC) * kStepBytes; i++) out[i] = 0;
+  for (int nt = 0; nt < ceil_div(OC, kTileN); nt++)
+    for (int j = 0; j < 4; j++)
+      for (int lane = 0; lane < 32; lane++) {
+        const int f = lane >> 2, t = lane & 3, oc = nt * kTileN + 8 * (f >> 1) + 2 * j + (f & 1);
+        if (oc >= OC) continue;
+        int8_t* o = out + (((size_t)nt * 4 + j) * 32 + lane) * 16;
+        for (int i = 0; i < (t < 3 ? 8 : 3); i++) o[i] = w[(size_t)oc * 27 + (t < 3 ? 9 * t + i : 9 * i + 8)];
+      }
+}
+
+cudaError_t launch_conv_small(const ConvSmallArgs& args, cudaStream_t stream) {
+  ConvSmallArgs a = args;
+  const int taps = a.KH * a.KW;
+  a.m_tiles = ceil_div(a.M, kTileM);
+  a.n_tiles = ceil_div(a.N, kTileN);
+  a.steps = a.mode == kStem ? 1 : conv_small_steps(taps, a.IC);
+  a.icb = a.mode == kStem ? 1 : a.IC / 16;
+  a.chunks = taps * a.icb;
+  a.inv_icb = ((1 << 20) + a.icb - 1) / a.icb;
+  a.inv_kw = ((1 << 20) + a.KW - 1) / a.KW;
+  a.vec = a.ldc % 8 == 0 && ((uintptr_t)a.out & 7) == 0 && ((uintptr_t)a.res & 7) == 0;
+  // K is split over 2 or 4 warps while the grid stays within about twelve warps per SM, over 8 (whose sums take longer to
+  // meet) only up to six. One layer, us with 1 / 2 / 4 / 8 warps per tile: 98 tiles, 3 steps 3.0 / 2.3 / 2.0 / 2.1;
+  // 392 tiles, 9 steps 4.4 / 3.6 / 3.0 / 4.9; 100 tiles, 18 steps 6.7 / 3.9 / 2.9 / 2.7; 1600 tiles, 3 steps 4.5 / 5.7 / 6.4.
+  const long long tiles = (long long)a.m_tiles * a.n_tiles;
+  a.ks_log2 = 0;
+  while (a.ks_log2 < 3 && (1 << a.ks_log2) < a.steps && (tiles << (a.ks_log2 + 1)) <= (a.ks_log2 == 2 ? 6ll : 12ll) * current_sm_count())
+    a.ks_log2++;
+  const int ks_n = 1 << a.ks_log2;
+  const int per_warp = ceil_div(a.steps, ks_n);
+  const int warps = ks_n > 4 ? ks_n : 4;
+  const dim3 grid((unsigned)ceil_div(tiles, warps / ks_n)), block(warps * 32);
+  const size_t smem = ks_n > 1 ? (size_t)warps * kTileM * kSumPitch * 4 : 0;
+  const int u = per_warp < 3 ? per_warp : 3;  // more than three steps in flight do not fit 128 registers
+  using Kernel = void (*)(ConvSmallArgs);
+  static const Kernel kernels[2][2][3] = {
+      {{conv_small_kernel<kRows, 1, false>, conv_small_kernel<kRows, 2, false>, conv_small_kernel<kRows, 3, false>},
+       {conv_small_kernel<kRows, 1, true>, conv_small_kernel<kRows, 2, true>, conv_small_kernel<kRows, 3, true>}},
+      {{conv_small_kernel<kConv, 1, false>, conv_small_kernel<kConv, 2, false>, conv_small_kernel<kConv, 3, false>},
+       {conv_small_kernel<kConv, 1, true>, conv_small_kernel<kConv, 2, true>, conv_small_kernel<kConv, 3, true>}}};
+  const Kernel kernel = a.mode == kStem ? conv_small_kernel<kStem, 1, false> : kernels[a.mode == kConv][ks_n > 1][u - 1];
+  return launch_dependent_if(true, kernel, grid, block, smem, stream, a);
+}
+
+}  // namespace tb200

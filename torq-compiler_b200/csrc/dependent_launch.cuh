@@ -24,11 +24,11 @@ inline bool dependent_launch_enabled() {
   return v != 0;
 }
 
-// Measured on MobileNetV2: with every launch programmatic the batch-256 step gains 1.3 %, the batch-1 inference
-// (64 launches of a few microseconds each) loses 17 % - a programmatic edge costs about a microsecond that only a
-// kernel with a real tail pays back. So the attribute is set for launches of at least kDependentMinBlocks blocks
-// (or tiles, for the persistent kernels, which pass `large` themselves).
-constexpr long long kDependentMinBlocks = 4 * 148;
+// A kernel lets the next one in only after its own wait has returned (grid_dependency_wait before grid_dependency_release):
+// releasing first let chains of short kernels stack up a dozen deep, holding the registers and block slots of the one that
+// had work. Measured on one-image inferences (56 and 120 launches of a few microseconds): released first 269 and 313 us,
+// released after the wait 256 and 287 us, fully serialised 274 and 393 us.
+constexpr long long kDependentMinBlocks = 4 * 148;  // persistent kernels: tiles x 2 from which their tail is worth overlapping
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent_if(bool large, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
@@ -49,8 +49,7 @@ inline cudaError_t launch_dependent_if(bool large, void (*kernel)(KArgs...), dim
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                     Args&&... args) {
-  const long long blocks = (long long)grid.x * grid.y * grid.z;
-  return launch_dependent_if(blocks >= kDependentMinBlocks, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+  return launch_dependent_if(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 }  // namespace tb200

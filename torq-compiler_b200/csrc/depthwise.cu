@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(128, 4) dw3x3_kernel(DwArgs a) {
 // rows, the weights and the per-channel records are then paid once per 14 rows instead of once per 8.
 template <int STRIDE, int EPI, int ROWS>
 __global__ void __launch_bounds__(128, STRIDE == 1 ? 6 : 8) dw3x3_tile_kernel(DwArgs a, int cg_log2, int cchunks) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   constexpr int TW = STRIDE == 1 ? 2 : 1;
   constexpr int NCOL = STRIDE == 1 ? 4 : 3;
   constexpr int NR = (ROWS - 1) * STRIDE + 3;
@@ -312,6 +312,72 @@ __global__ void __launch_bounds__(128, STRIDE == 1 ? 6 : 8) dw3x3_tile_kernel(Dw
   }
 }
 
+// Few outputs (one frame, a small batch of small ones): bound by the chain of latencies, not by issue slots. A thread makes
+// one row of TW outputs of four channels and reads its 3 x NCOL words straight into registers, all in flight at once (the
+// rows that neighbours share come from L1): no tile, no barrier, and weights and constants arrive before the launch
+// ahead has finished. One frame, 80 x 80 x 96 at stride 2: 3.8 -> 2.1 us; 10 x 10 x 576: 3.5 -> 1.7 us.
+template <int STRIDE, int EPI>
+__global__ void __launch_bounds__(128) dw3x3_few_kernel(DwArgs a) {
+  constexpr int TW = STRIDE == 1 ? 2 : 1;
+  constexpr int NCOL = STRIDE == 1 ? 4 : 3;
+  const int Cw = a.C >> 2, strips = (a.OW + TW - 1) / TW;
+  const int q = blockIdx.x * 128 + threadIdx.x;
+  const int strip = q / Cw, g = q - strip * Cw;
+  const bool live = strip < strips;
+  const int oh = blockIdx.y, n = blockIdx.z, ow0 = strip * TW, c = 4 * (live ? g : 0);
+  uint32_t wq[3][TW][4];
+#pragma unroll
+  for (int kh = 0; kh < 3; kh++)
+#pragma unroll
+    for (int v = 0; v < TW; v++) {
+      const uint4 w = __ldg(reinterpret_cast<const uint4*>(a.wq + ((size_t)(kh * TW + v) * a.C + c)));
+      wq[kh][v][0] = w.x; wq[kh][v][1] = w.y; wq[kh][v][2] = w.z; wq[kh][v][3] = w.w;
+    }
+  int4 cq[EPI != 0 ? 4 : 1];
+  ChanParams cp[EPI != 0 ? 1 : 4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (EPI != 0) cq[EPI != 0 ? k : 0] = __ldg(a.q4 + c + k);
+    else cp[EPI != 0 ? 0 : k] = a.chan[c + k];
+  }
+  const uint32_t zpw = (uint32_t)(a.input_zp & 0xff) * 0x01010101u;
+  const uint32_t lo2 = (uint32_t)(a.clamp_min & 0xffff) * 0x10001u, hi2 = (uint32_t)(a.clamp_max & 0xffff) * 0x10001u;
+  const uint32_t* x32 = reinterpret_cast<const uint32_t*>(a.x);
+  const int ih0 = oh * STRIDE - a.pad_t, iw0 = ow0 * STRIDE - a.pad_l;
+  grid_dependency_wait();
+  grid_dependency_release();
+  if (!live) return;
+  uint32_t x[3][4];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const bool row_in = (unsigned)(ih0 + i) < (unsigned)a.H;
+    const int row = ((n * a.H + ih0 + i) * a.W + iw0) * Cw + g;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      x[i][k] = zpw;
+      if (k < NCOL && row_in && (unsigned)(iw0 + k) < (unsigned)a.W) x[i][k] = x32[row + k * Cw];
+    }
+  }
+  uint32_t win[3][4];
+#pragma unroll
+  for (int i = 0; i < 3; i++) transpose4x4(x[i][0], x[i][1], x[i][2], x[i][3], win[i]);
+  uint32_t* o32 = reinterpret_cast<uint32_t*>(a.out) + ((n * a.OH + oh) * a.OW + ow0) * Cw + g;
+#pragma unroll
+  for (int v = 0; v < TW; v++) {
+    int r[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      int acc = EPI != 0 ? 0 : cp[EPI != 0 ? 0 : k].bias;
+#pragma unroll
+      for (int kh = 0; kh < 3; kh++) acc = __dp4a((int)win[kh][k], (int)wq[kh][v][k], acc);
+      if (EPI == 1) r[k] = scale_q4_sign(acc, cq[EPI != 0 ? k : 0]);
+      else if (EPI == 2) r[k] = scale_q4(acc, cq[EPI != 0 ? k : 0]);
+      else r[k] = scale_cp<false>(acc, cp[EPI != 0 ? 0 : k]) + a.out_zp;
+    }
+    if (v == 0 || ow0 + 1 < a.OW) o32[v * Cw] = clamp_pack4(r[0], r[1], r[2], r[3], lo2, hi2);
+  }
+}
+
 // One thread per (output pixel, VEC consecutive channels); taps outside the image are skipped.
 template <int VEC>
 __global__ void __launch_bounds__(256) depthwise_generic_kernel(DwArgs a) {
@@ -421,6 +487,26 @@ static bool dw_tile_shape(const DwArgs& a, int& cg_log2, int& tiles, int& cchunk
 
 void launch_depthwise(const DwArgs& a, cudaStream_t stream) {
   int cg_log2 = 0, tiles = 0, cchunks = 0;
+  // Threads of dw3x3_few_kernel from which its nine or twelve loads per output row cost more than the tile's barrier (threads,
+  // few / tile in us): 26 k 2.0 / 3.5; 86 k 3.0 / 4.2; 115 k 3.7 / 4.2; 153 k 3.7 / 4.3; 165 k 4.9 / 5.1; 220 k 5.8 / 5.4;
+  // 307 k 7.6 / 5.4.
+  constexpr long long kFewThreads = 160000;
+  const int few_strips = a.stride_h == 1 ? (a.OW + 1) / 2 : a.OW;
+  if (a.wq && depthwise3x3_supported(a) && a.OH <= 65535 && a.N <= 65535 && !small_kernels_off() &&
+      (long long)few_strips * (a.C >> 2) * a.OH * a.N <= kFewThreads) {
+    const dim3 grid((unsigned)((few_strips * (a.C >> 2) + 127) / 128), (unsigned)a.OH, (unsigned)a.N);
+    auto go = [&](auto kern) { launch_dependent_if(true, kern, grid, dim3(128), 0, stream, a); };
+    if (a.stride_h == 1) {
+      if (a.epi == 1) go(dw3x3_few_kernel<1, 1>);
+      else if (a.epi == 2) go(dw3x3_few_kernel<1, 2>);
+      else go(dw3x3_few_kernel<1, 0>);
+    } else {
+      if (a.epi == 1) go(dw3x3_few_kernel<2, 1>);
+      else if (a.epi == 2) go(dw3x3_few_kernel<2, 2>);
+      else go(dw3x3_few_kernel<2, 0>);
+    }
+    return;
+  }
   if (a.wq && depthwise3x3_supported(a) && dw_tile_shape(a, cg_log2, tiles, cchunks)) {
     const int S = a.stride_h, tw = S == 1 ? 2 : 1, sw = 128 >> cg_log2;
     static const bool rows8 = getenv("TB200_DW_ROWS8") != nullptr;  // A/B switch

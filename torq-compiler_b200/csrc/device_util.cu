@@ -50,4 +50,9 @@ unsigned long long wait_limit_ns() {
   return (unsigned long long)ms * 1000000ull;
 }
 
+bool small_kernels_off() {
+  const char* e = getenv("TB200_NO_SMALL");
+  return e && *e && *e != '0';
+}
+
 }  // namespace tb200

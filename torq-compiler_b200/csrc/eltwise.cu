@@ -32,8 +32,8 @@ __device__ __forceinline__ uint32_t lut_word(const uint8_t* lut, uint32_t w) {
 // packing, against two 256-entry look-ups (two wavefronts each), a 64-bit or 4-cycle multiply-high and the rounding before:
 // 12.8 M elements 18.9 -> 6 us. HBM-bound at large sizes.
 __global__ void __launch_bounds__(kThreads) binary_linear_kernel(BinaryArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   const uint32_t lo2 = (uint32_t)((a.clamp_min << a.lin_f) & 0xffff) * 0x10001u;
   const uint32_t hi2 = (uint32_t)(((a.clamp_max << a.lin_f) | ((1 << a.lin_f) - 1)) & 0xffff) * 0x10001u;
   const int up = 8 - a.lin_f;  // brings the integer part to the high byte of its 16-bit field
@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(kThreads) binary_linear_kernel(BinaryArgs a) {
 // planner when it can bound |operand sum or product| (it evaluates the same two tables).
 template <int EPI>
 __global__ void __launch_bounds__(kThreads) binary_kernel(BinaryArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   __shared__ int ta[256], tb[256];  // indexed by the raw byte
   {
     const bool dr = a.double_round != 0;
@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(kThreads) table_kernel(const int8_t* __restric
   __shared__ uint8_t lut[256];
   // index by the raw byte: entry for byte b is table[(int8)b + 128]
   lut[threadIdx.x] = (uint8_t)table[(int)(int8_t)threadIdx.x + 128];
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   __syncthreads();
   const long long nvec = n >> 4;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(kThreads) table_kernel(const int8_t* __restric
 
 // ---- standalone rescale i8 -> i8 (PatternUtils.cpp:426-435,3441-3451) ----
 __global__ void __launch_bounds__(kThreads) rescale_kernel(RescaleArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   const long long total = a.rows * a.C;
   const bool dr = a.double_round != 0;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(kThreads) rescale_kernel(RescaleArgs a) {
 // (multiplier 2^30, shift 30, equal zero points, full clamp range), i.e. a strided copy
 template <bool IDENT>
 __global__ void __launch_bounds__(kThreads) rescale_vec16_kernel(RescaleArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   const int cv = a.C >> 4;
   const long long total = a.rows * cv;
   const bool dr = a.double_round != 0;
@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(kThreads) rescale_vec16_kernel(RescaleArgs a) 
 // Per-tensor constants: the rescale is a function of the input byte alone, so it runs as a 256-entry table
 // in shared memory (one entry per thread, filled by the same requant), 16 channels per thread.
 __global__ void __launch_bounds__(kThreads) rescale_lut_vec16_kernel(RescaleArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   __shared__ uint8_t lut[256];  // indexed by the raw byte
   {
     const ChanParams cp = a.chan[0];
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(kThreads) rescale_lut_vec16_kernel(RescaleArgs
 // ---- nearest 2x (PatternUtils.cpp:489-491): out[y,x] = in[y/2, x/2] ----
 __global__ void __launch_bounds__(kThreads) resize_nn2x_vec16_kernel(const int8_t* __restrict__ x, int8_t* __restrict__ out,
                                                                      int N, int H, int W, int C) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   const int cv = C >> 4;
   const long long total = (long long)N * 2 * H * 2 * W * cv;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;

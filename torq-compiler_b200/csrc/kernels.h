@@ -18,6 +18,7 @@ int current_sm_count();  // SMs of the current device
 // mark_used_on_device has been called with the same flag while the same device was current.
 bool first_use_on_device(std::atomic<unsigned long long>& done);
 void mark_used_on_device(std::atomic<unsigned long long>& done);
+bool small_kernels_off();  // TB200_NO_SMALL=1 (A/B aid): small problems take the kernels of the large ones
 // Limit of every bounded wait inside the kernels, from TB200_WAIT_LIMIT_MS (default 2000 ms).
 unsigned long long wait_limit_ns();
 
@@ -211,6 +212,34 @@ struct ConvTcArgs {
   const int8_t* lut;      // 256-entry table applied to the int8 result, or null
 };
 cudaError_t launch_conv_i8_tc(const ConvTcArgs& a, GemmTcState* st, cudaStream_t stream);
+
+// ---- small convolutions and products (conv_small.cu) ----
+struct ConvSmallArgs {
+  const int8_t* x;        // [N, H, W, IC], or rows of lda bytes
+  const int8_t* w;        // conv_small_pack
+  const ChanParams* chan; // [conv_small_columns(N)], bias holds bias - izp * sum of all taps (a tap outside the frame reads izp)
+  const int4* q4;         // [conv_small_columns(N)] when epi != 0
+  int8_t* out;            // M rows of ldc bytes
+  const int8_t* res;      // other operand of an add behind the result (layout of out), or null
+  const int8_t* lut;      // 256-entry table applied to the int8 result, or null
+  long long ldc;
+  int lda, M, N;          // rows (pixels) and output channels
+  int mode;               // 0 = rows, 1 = convolution with IC % 16 == 0, 2 = 3 x 3 over 3 channels
+  int x_bytes;            // size of the input (mode 2 reads it in aligned words)
+  int H, W, IC, KH, KW, OH, OW, stride, pad_t, pad_l;
+  int input_zp, out_zp, clamp_min, clamp_max, epi;
+  int add_m_self, add_m_other, add_f, add_clamp_min, add_clamp_max;  // BinaryArgs::lin_*
+  long long add_k;
+  // filled by the launcher
+  int m_tiles, n_tiles, steps, chunks, icb, inv_icb, inv_kw, ks_log2, vec;
+};
+bool conv_small_applies(long long M, int OC, int taps, int IC);  // is this the faster kernel for the size
+int conv_small_steps(int taps, int IC);
+int conv_small_columns(int OC);
+// [OC][taps][IC] -> conv_small_columns(OC) * conv_small_steps(taps, IC) * 64 bytes
+void conv_small_pack(const int8_t* w, int OC, int taps, int IC, int8_t* out);
+void conv_small_pack_stem(const int8_t* w, int OC, int8_t* out);  // [OC][27] -> conv_small_columns(OC) * 64 bytes (mode 2)
+cudaError_t launch_conv_small(const ConvSmallArgs& a, cudaStream_t stream);
 
 // ---- decoder kernels (decoder.cu): bf16 tensors are passed as uint16_t bit patterns ----
 void launch_embed(const int32_t* tok, const int8_t* table, const uint16_t* scale, uint16_t* out, int B, int H, int V,

@@ -299,14 +299,14 @@ bool force_simt() {
 // Rows of a 1x1 convolution / FullyConnected product that are read as one row against block-diagonal weights
 // (row m' of the product then holds the outputs of pixels r*m' .. r*m'+r-1 back to back, which is exactly their dense
 // NHWC placement, so nothing else changes).
+static int bytes16_row_group(long long K) {  // rows that together are a multiple of 16 bytes
+  int g16 = 16;
+  while (K % g16 != 0) g16 >>= 1;  // gcd(K, 16)
+  return 16 / g16;
+}
 static int pointwise_row_group(long long M, long long K, int OC) {
   // TMA wants a row pitch that is a multiple of 16 bytes
-  int rgroup = 1;
-  if (K % 16 != 0) {
-    int g16 = 16;
-    while (K % g16 != 0) g16 >>= 1;  // gcd(K, 16)
-    rgroup = 16 / g16;
-  }
+  int rgroup = bytes16_row_group(K);
   // Short rows make poor TMA boxes (the copy engine works row by row): widen them the same way while the grouped
   // row stays within one 128-byte swizzle row.
   while (rgroup * 2 <= 8 && K * rgroup * 2 <= 128 && M % (rgroup * 2) == 0 && OC * rgroup * 2 <= 512) rgroup *= 2;
@@ -325,6 +325,12 @@ static bool pointwise_takes_gemm_tc(long long M, long long K, int OC, int weight
   if (M <= 4 && K % 16 == 0 && K <= 12288) return false;  // fc_rows_dp4a
   const int r = pointwise_row_group(M, K, OC);
   return r <= 8 && M % r == 0 && (long long)OC * r <= 65536 && gemm_tc_supported(M / r, OC * r, (int)K * r, K * r);
+}
+
+// Whether such a product is one for the small-problem kernel.
+static bool pointwise_takes_small(long long M, long long K, int OC) {
+  const int r = bytes16_row_group(K);
+  return M % r == 0 && conv_small_applies(M / r, OC * r, 1, (int)K * r);
 }
 
 bool decode_per_op() {
@@ -578,6 +584,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   std::vector<char> fused_away(ops.size(), 0);
   std::vector<int> add_after(ops.size(), -1);      // conv op -> index of the add fused into its epilogue
   std::vector<char> add_self_is_a(ops.size(), 0);  // the convolution's result is the add's first operand
+  std::vector<char> add_fits_small(ops.size(), 0); // the fused add runs in the small-problem kernel
   // Decoder graphs run op by op: (1) a split-K gemv_w8 whose only reader is the next op (rmsnorm, rope_kv or
   // geglu) leaves its per-slice sums in scratch and the reader finalizes them as it loads; (2) an rmsnorm
   // directly followed by an rmsnorm of its result runs as one launch. Same arithmetic, fewer launches.
@@ -634,11 +641,13 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
     // there, the product never goes to memory. The add's own checks (and its 32-bit output rescale, which the
     // fused form requires) happen when the convolution is planned; what cannot be fused there fails the plan
     // no differently from the stand-alone op.
-    // Off unless TB200_ADD_FUSION=1: measured on MobileNetV2 at batch 256 the fused form is no faster (1.693 ms per
+    // Small problems are bound by their chain of launches: there an add in linear form between two intermediates always
+    // moves into the convolution. Otherwise off unless TB200_ADD_FUSION=1: measured on MobileNetV2 at batch 256 the fused form is no faster (1.693 ms per
     // step against 1.678 with the ten adds as their own launches) - the step is bound by integer issue slots, and the
     // add's table look-ups, rescale and repacking cost the same slots wherever they run.
     const char* do_add = getenv("TB200_ADD_FUSION");
-    for (int i = 0; i < (int)ops.size() && do_add && *do_add && *do_add != '0'; i++) {
+    const bool all_adds = do_add && *do_add && *do_add != '0';
+    for (int i = 0; i < (int)ops.size(); i++) {
       const auto& op = ops[i];
       if (op.kind != TB200_OP_ADD || op.in0 < 0 || op.in0 >= nt || op.in1 < 0 || op.in1 >= nt || op.out0 < 0 || op.out0 >= nt ||
           op.in0 == op.in1)
@@ -669,6 +678,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         // the fused form exists for the 32-bit output rescale only
         BinaryArgs probe{};
         if (!binary_args_of(op, probe) || probe.epi == 0) continue;
+        add_fits_small[pc] = probe.lin && pointwise_takes_small(M, x.shape[3], OC);
+        if (!all_adds && !(add_fits_small[pc] && tensors[other].kind == TB200_TENSOR_ACTIVATION)) continue;
         add_after[pc] = i;
         add_self_is_a[pc] = side == 0;
         fused_away[i] = 1;
@@ -1021,6 +1032,74 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           };
           break;
         }
+        // Small problems (conv_small.cu): the same two families of products, on kernels that are latency-bound differently.
+        // The step keeps the name of the family, whichever kernel the size picks.
+        auto plan_small = [&](const char* family, int rows_per_group) {
+          const int G = rows_per_group;  // rows read as one (block-diagonal weights) to make a row a multiple of 16 bytes
+          ConvSmallArgs sa{};
+          const bool stem = !pointwise && IC == 3;
+          sa.mode = pointwise ? 0 : stem ? 2 : 1;
+          sa.x_bytes = (int)b.numel(op.in0);
+          sa.M = (int)(M / G); sa.N = OC * G; sa.ldc = (long long)OC * G; sa.lda = (int)K * G;
+          sa.H = H; sa.W = W; sa.IC = pointwise ? (int)K * G : IC; sa.KH = KH; sa.KW = KW; sa.OH = OH; sa.OW = OW;
+          sa.stride = fc ? 1 : op.stride_h; sa.pad_t = fc ? 0 : op.pad_t; sa.pad_l = fc ? 0 : op.pad_l;
+          sa.input_zp = op.in0_zp; sa.out_zp = op.out_zp; sa.clamp_min = op.clamp_min; sa.clamp_max = op.clamp_max;
+          std::vector<int4> q4;
+          sa.epi = Builder::q4_params(cp, acc_bound, dr != 0, op.out_zp, op.clamp_min, q4);
+          const int cols = conv_small_columns(sa.N);
+          ChanParams none{};
+          none.shift = 34; none.hshift = 2; none.rnd = 1ll << 33;
+          std::vector<ChanParams> cps(cols, none);
+          std::vector<int4> q4s(cols, make_int4(0, 0, 0, 1));
+          std::vector<int8_t> grouped;
+          const int8_t* ws = w;
+          for (int j = 0; j < G; j++)
+            for (int oc = 0; oc < OC; oc++) {
+              cps[(size_t)j * OC + oc] = cp[oc];
+              if (sa.epi) q4s[(size_t)j * OC + oc] = q4[oc];
+            }
+          if (G > 1) {
+            grouped.assign((size_t)G * OC * G * K, 0);
+            for (int j = 0; j < G; j++)
+              for (int oc = 0; oc < OC; oc++) memcpy(grouped.data() + ((size_t)j * OC + oc) * G * K + (size_t)j * K, w + (size_t)oc * K, (size_t)K);
+            ws = grouped.data();
+          }
+          std::vector<int8_t> wp((size_t)cols * (stem ? 1 : conv_small_steps(KH * KW, sa.IC)) * 64);
+          if (stem) conv_small_pack_stem(ws, sa.N, wp.data());
+          else conv_small_pack(ws, sa.N, KH * KW, sa.IC, wp.data());
+          const size_t w_off = b.add_const(wp.data(), wp.size());
+          const size_t c_off = b.add_const(cps.data(), cps.size() * sizeof(ChanParams));
+          const size_t q_off = sa.epi ? b.add_const(q4s.data(), q4s.size() * sizeof(int4)) : 0;
+          const int fused_add = add_after[i];
+          Loc lx = loc(op.in0), lo = loc(fused_add >= 0 ? ops[fused_add].out0 : result_id), lres{};
+          if (fused_add >= 0) {
+            BinaryArgs add{};
+            binary_args_of(ops[fused_add], add);
+            const bool self_a = add_self_is_a[i] != 0;
+            sa.add_m_self = self_a ? add.lin_ma : add.lin_mb;
+            sa.add_m_other = self_a ? add.lin_mb : add.lin_ma;
+            sa.add_f = add.lin_f; sa.add_k = add.lin_k;
+            sa.add_clamp_min = add.clamp_min; sa.add_clamp_max = add.clamp_max;
+            lres = loc(self_a ? ops[fused_add].in1 : ops[fused_add].in0);
+          }
+          step.kernel_name = family;
+          step.launch = [=](const ExecContext& c) {
+            ConvSmallArgs k = sa;
+            k.x = (const int8_t*)lx.resolve(c);
+            k.out = (int8_t*)lo.resolve(c);
+            k.w = (const int8_t*)(c.consts + w_off);
+            k.chan = (const ChanParams*)(c.consts + c_off);
+            k.q4 = k.epi ? (const int4*)(c.consts + q_off) : nullptr;
+            k.lut = has_lut ? (const int8_t*)(c.consts + lut_off) : nullptr;
+            k.res = fused_add >= 0 ? (const int8_t*)lres.resolve(c) : nullptr;
+            const cudaError_t e = launch_conv_small(k, c.stream);
+            if (e != cudaSuccess && c.launch_error) *c.launch_error = e;
+          };
+        };
+        if (add_after[i] >= 0 ? add_fits_small[i] != 0 : pointwise && pointwise_takes_gemm_tc(M, K, OC, op.weight_zp) && pointwise_takes_small(M, K, OC)) {
+          plan_small("gemm_i8_tcgen05", bytes16_row_group(K));
+          break;
+        }
         const int rgroup = pointwise_row_group(M, K, OC);
         if (pointwise && op.weight_zp == 0 && !force_simt() && rgroup <= 8 && M % rgroup == 0 &&
             (long long)OC * rgroup <= 65536 && gemm_tc_supported(M / rgroup, OC * rgroup, (int)K * rgroup, K * rgroup)) {
@@ -1091,6 +1170,14 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         // of padding, its weights the original ones placed at [(j, oc)][kh][kp][(h, c)] and zero elsewhere. 1 / G of
         // the rows per pixel through the copy engine; the zero parts cost tensor-core work that is free here. Border classes, bias folding and the
         // epilogue constants follow from the transformed op as for any convolution.
+        if (!fc && !pointwise && op.weight_zp == 0 && !force_simt() &&
+            conv_tc_supported(N, H, W, IC, OC, KH, KW, op.stride_h, op.stride_w, op.dil_h, op.dil_w, OH, OW) &&
+            (IC != 16 || conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).halo ||
+             conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).s2) &&
+            conv_small_applies(M, OC, KH * KW, IC)) {
+          plan_small("conv_igemm_i8_tcgen05", 1);
+          break;
+        }
         std::vector<int8_t> w_pairs;
         static const bool no_pairs = getenv("TB200_CONV_NO_PAIRS") != nullptr;  // A/B switch
         int group = 0;  // pixels per row of the rewritten convolution: 4 for 16 channels where the width allows, else 2
@@ -1249,6 +1336,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           break;
         }
 
+        // the stem of an image network on a small frame
+        if (!fc && IC == 3 && KH == 3 && KW == 3 && op.stride_h == op.stride_w && op.dil_h == 1 && op.dil_w == 1 && op.weight_zp == 0 &&
+            !force_simt() && conv_small_applies(M, OC, 1, 16)) {
+          plan_small("conv2d_stem333_dp4a", 1);
+          break;
+        }
         const int Kpad = (int)((K + 31) / 32 * 32);
         std::vector<int8_t> packed((size_t)OC * Kpad, 0);
         for (int oc = 0; oc < OC; oc++) memcpy(packed.data() + (size_t)oc * Kpad, w + (size_t)oc * K, (size_t)K);

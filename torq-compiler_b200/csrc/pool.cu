@@ -46,8 +46,8 @@ constexpr int kStripThreads = 128;
 // VW: 32-bit words of channels per thread (4 or 1), or 0 for a single channel.
 template <int VW, int K, int S, int ROWS, bool AVG, bool LUT>
 __global__ void __launch_bounds__(kStripThreads) pool_strip_kernel(PoolArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   __shared__ uint8_t lut_s[256];
   if (LUT) {
     for (int i = threadIdx.x; i < 256; i += kStripThreads) lut_s[i] = (uint8_t)a.lut[(int)(int8_t)i + 128];
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(kStripThreads) pool_strip_kernel(PoolArgs a) {
 // I: index type, 32 bits where the tensor allows (a 64-bit division costs more than a window of loads)
 template <int VEC, typename I>  // channels per thread: 16 (uint4) or 1
 __global__ void __launch_bounds__(kThreads) maxpool_kernel(PoolArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   const int groups = a.C / VEC;
   const I total = (I)a.N * a.OH * a.OW * groups;
   for (I idx = (I)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (I)gridDim.x * blockDim.x) {
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kThreads) maxpool_kernel(PoolArgs a) {
 // The same on int16 tensors (the reference's MaxPool2D i16 -> i16): 8 channels per thread, or 1.
 template <int VEC, typename I>
 __global__ void __launch_bounds__(kThreads) maxpool_i16_kernel(PoolArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   const int16_t* x = reinterpret_cast<const int16_t*>(a.x);
   int16_t* out = reinterpret_cast<int16_t*>(a.out);
   const int groups = a.C / VEC;
@@ -287,8 +287,8 @@ __device__ __forceinline__ void reciprocal_scale(uint32_t count, int32_t& mult, 
 constexpr int kAvgMaxTaps = 256;
 template <int VEC, typename I>  // 16, 4 or 1 channels per thread
 __global__ void __launch_bounds__(kThreads) avgpool_kernel(PoolArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   __shared__ int4 by_count[kAvgMaxTaps + 1];
   for (int c = threadIdx.x; c <= a.KH * a.KW; c += blockDim.x) {
     int32_t mult, shift;
@@ -352,8 +352,8 @@ __global__ void __launch_bounds__(kThreads) avgpool_kernel(PoolArgs a) {
 // Large windows over few outputs (the global pool at the end of a classifier: 7x7 -> 1x1): a warp per output pixel
 // and group of 16 channels, the taps spread over the lanes, sums combined by shuffles. Same arithmetic as above.
 __global__ void __launch_bounds__(kThreads) avgpool_warp_kernel(PoolArgs a) {
-  grid_dependency_release();
   grid_dependency_wait();
+  grid_dependency_release();
   __shared__ int4 by_count[kAvgMaxTaps + 1];
   for (int c = threadIdx.x; c <= a.KH * a.KW; c += blockDim.x) {
     int32_t mult, shift;
