@@ -1,0 +1,91 @@
+"""The op-by-op decode kernels (decode_linear.cu) where they can go wrong: tile and token remainders, one and many K groups, K slices
+that meet in a cluster, products that walk their tiles with the arg max riding along, caches shorter and longer than a round of
+keys, one to four query heads. Against fp32 torch."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_exec import run_graph_gpu
+from torq_b200.bf16 import from_bf16, to_bf16
+from torq_b200.oplist import Graph
+from torq_b200.runtime import Executable
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf(t):
+    return t.to(torch.bfloat16).to(torch.float32)
+
+
+def _product(rng, B, K, N):
+    x = to_bf16(rng.normal(0, 1, (B, K)).astype(np.float32))
+    w = rng.integers(-128, 128, (N, K), dtype=np.int8)
+    s = to_bf16(rng.uniform(0.5, 1.5, N).astype(np.float32) / (73.0 * np.sqrt(K)))
+    want = (torch.from_numpy(from_bf16(x)) @ torch.from_numpy(w.astype(np.float32)).T) * torch.from_numpy(from_bf16(s))
+    return x, w, s, want
+
+
+@pytest.mark.parametrize("B,K,N", [(1, 64, 1), (3, 64, 33), (8, 192, 32), (9, 8192, 31), (16, 6912, 100), (32, 6912, 1152), (25, 4096, 70),
+                                   (2, 128, 60001), (32, 1152, 30001)])
+def test_products(device, B, K, N):
+    rng = np.random.default_rng(B + K + N)
+    x, w, s, want = _product(rng, B, K, N)
+    g = Graph()
+    y = g.gemv_w8(g.input((B, K), "bf16"), w, s, out_dtype="f32")
+    g.output(y), g.output(g.argmax(y))
+    got, ids = run_graph_gpu(device, g, [x])
+    assert np.abs(got - want.numpy()).max() <= 1e-5 * np.abs(want.numpy()).max()
+    assert (ids == got.argmax(-1)).all()
+
+
+@pytest.mark.parametrize("B,K,I", [(1, 64, 1), (5, 1152, 17), (32, 1152, 6912), (17, 4096, 100)])
+def test_geglu_behind_the_product(device, B, K, I):
+    rng = np.random.default_rng(B + K + I)
+    x, w, s, want = _product(rng, B, K, 2 * I)
+    g = Graph()
+    g.output(g.geglu(g.gemv_w8(g.input((B, K), "bf16"), w, s)))
+    ex = Executable(device, g.serialize())
+    assert ex.launch_count == 1, ex.op_kernels()
+    ex.destroy()
+    got = from_bf16(run_graph_gpu(device, g, [x])[0])
+    want = _bf(want)
+    want = (_bf(torch.nn.functional.gelu(want[:, :I], approximate="tanh")) * want[:, I:]).numpy()
+    assert (np.abs(got - want) <= 2.0 ** -6 * np.maximum(np.abs(want), 0.05)).all()
+
+
+@pytest.mark.parametrize("n_q,B,window", [(1, 1, 0), (2, 3, 20), (4, 9, 130)])
+def test_attention_over_short_and_long_caches(device, n_q, B, window):
+    rng = np.random.default_rng(n_q)
+    D, T = 256, 700
+    g = Graph()
+    qkv, pos_in = g.input((B, (n_q + 2) * D), "bf16"), g.input((1,), "i32")
+    kc, vc = g.state((B, T, D), "bf16"), g.state((B, T, D), "bf16")
+    one = to_bf16(np.zeros(D, np.float32))
+    q = g.rope_kv(qkv, pos_in, one, one, kc, vc, n_q=n_q, n_kv=1, head_dim=D, theta=10000.0, eps=1e-6)
+    g.output(q), g.output(g.attn_decode(q, pos_in, kc, vc, n_q=n_q, n_kv=1, head_dim=D, window=window, scale=D ** -0.5))
+    ex = Executable(device, g.serialize())
+    d_in, d_pos = device.alloc(B * (n_q + 2) * D * 2), device.alloc(4)
+    outs = [device.alloc(B * n_q * D * 2) for _ in range(2)]
+    half = D // 2
+    inv = torch.pow(torch.tensor(10000.0), -torch.arange(half, dtype=torch.float32) / half)
+    K, V = torch.zeros(B, T, D), torch.zeros(B, T, D)
+    for pos in range(600):
+        t = torch.from_numpy(rng.normal(0, 1, (B, (n_q + 2) * D)).astype(np.float32))
+        bits = to_bf16(t.numpy())
+        d_in.upload(bits), d_pos.upload(np.array([pos], np.int32))
+        ex.dispatch([d_in, d_pos], outs)
+        t = torch.from_numpy(from_bf16(bits))
+        k = t[:, n_q * D:(n_q + 1) * D]
+        k = _bf(k * torch.rsqrt((k * k).mean(-1, keepdim=True) + 1e-6))
+        cs, sn = torch.cos(pos * inv), torch.sin(pos * inv)
+        K[:, pos] = _bf(torch.cat([k[:, :half] * cs - k[:, half:] * sn, k[:, half:] * cs + k[:, :half] * sn], -1))
+        V[:, pos] = t[:, (n_q + 1) * D:]
+        if pos in (0, 1, 15, 16, 127, 128, 129, 512, 599):
+            qg, got = (from_bf16(o.download((B, n_q * D), np.uint16)) for o in outs)
+            lo = max(0, pos - window + 1) if window else 0
+            p = torch.softmax(torch.einsum("bhd,btd->bht", torch.from_numpy(qg).reshape(B, n_q, D) * D ** -0.5, K[:, lo:pos + 1]), -1)
+            want = torch.einsum("bht,btd->bhd", p, V[:, lo:pos + 1]).reshape(B, -1).numpy()
+            assert np.abs(got - want).max() <= 2.0 ** -6 * np.abs(want).max(), pos
+    for b in [d_in, d_pos] + outs:
+        b.free()
+    ex.destroy()

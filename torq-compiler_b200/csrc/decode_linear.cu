@@ -1,0 +1,885 @@
+// The products and the attention of a decode step run op by op: int8 weights on bf16 activations of up to 32 tokens, and one
+// query per sequence against its cache. Every one of them moves a few MB, a microsecond or two of HBM time, so what bounds a
+// step is how early the bytes are asked for and how few launches stand in a row:
+//   * each kernel asks for its weights (or cache lines) before it waits for the kernel ahead of it: the weights belong to
+//     the program, so they stream in while the activations are still being made;
+//   * a long K is split over the warps of a block and, where the activations would not fit shared memory, over the blocks of
+//     a cluster; the fp32 sums meet in shared memory (the cluster's through distributed shared memory), in one fixed order,
+//     and the finished bf16 values leave the kernel - no partial sums in global memory;
+//   * the op behind a product runs in its epilogue where a block holds what it needs: GeGLU (a warp's tile is 16 gate rows
+//     and the 16 matching up rows), head norm + RoPE + cache append (a cluster of eight blocks holds a head), the arg max
+//     over the logits.
+// Measured at the Gemma-3-1B shape, 32 sequences at position 1024, us per launch before -> after: see each kernel.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "dependent_launch.cuh"
+#include "kernels.h"
+
+namespace tb200 {
+namespace {
+
+__device__ __forceinline__ float bf2f(uint16_t v) { return __uint_as_float((uint32_t)v << 16); }
+__device__ __forceinline__ uint16_t f2bf(float f) { return __bfloat16_as_ushort(__float2bfloat16_rn(f)); }
+__device__ __forceinline__ float rbf(float f) { return bf2f(f2bf(f)); }
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {  // zeros when not valid
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+// a float of another block of the cluster, at the address the same float has in this block
+__device__ __forceinline__ float ld_peer(uint32_t addr, int rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_peer(uint32_t addr, int rank, float v) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Four signed bytes -> bf16 pairs (k, k+1) and (k+2, k+3), exact. 0x4300 | u is 128 + u for the seven low bits, and the top
+// bit turns the 128 that is taken off again into 256.
+__device__ __forceinline__ void s8x4_to_bf16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
+  const uint32_t p = __byte_perm(w, 0x43434343u, 0x4140), q = __byte_perm(w, 0x43434343u, 0x4342);
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(p & 0xff7fff7fu), "r"(p & 0xff80ff80u));
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"(q & 0xff7fff7fu), "r"(q & 0xff80ff80u));
+}
+__device__ __forceinline__ float gelu_tanh(float x) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// y[b, n] = sum_k x[b, k] * W[n, k] * scale[n]: weights are the 16-row operand of mma.sync m16n8k16 (bf16, fp32
+// accumulation), tokens the 8-column one. A warp works on a tile of 32 weight rows (each activation fragment read from shared
+// memory then serves two instructions: at 32 tokens these reads bounded a 16-row tile) and one of TK groups of 64-byte
+// blocks of K, whose weights it copies into a ring of its own (cp.async; nothing but the warp itself waits for them). The
+// activations of the block's K range are staged once per block. TK depends on N and K alone, and a result is the sum of its
+// TK groups in order, so it does not depend on the mode or on how groups are spread over warps and blocks.
+//   kStore: bf16 or fp32 results.                      kGeglu: bf16(bf16(gelu(gate)) * up), tiles of 16 gate and 16 up rows.
+//   kRope:  a cluster of eight blocks is one head of 256: head norm, RoPE, q out / cache append (arithmetic of rope_kv_kernel).
+//   kStream: one group and a warp per tile, blocks stay and walk the tiles (the LM head); fp32 or bf16 results and, with
+//            cand_v, the block's arg-max candidates per token.
+// ---------------------------------------------------------------------------------------------------------------
+enum { kStore = 0, kGeglu = 1, kRope = 2, kStream = 3 };
+constexpr int kTileRows = 32, kBlk = 64, kStageBytes = kTileRows * kBlk, kStreamStages = 4;
+
+template <int NT, int MODE>
+__global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  constexpr int kTok = NT * 8, kPitch = kTok + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+  const int kg = warp % a.kg, rt = warp / a.kg;
+  const int rank = a.ck > 1 ? blockIdx.x % a.ck : 0;  // K slice of this block (clusters are consecutive blocks)
+  const int row_block = a.ck > 1 ? blockIdx.x / a.ck : blockIdx.x;
+  const int blocks = a.K / kBlk, tk = a.kg * a.ck;
+  const int kb0 = blocks * (rank * a.kg) / tk, kb1 = blocks * (rank * a.kg + a.kg) / tk;  // K blocks of this thread block
+  const int group = rank * a.kg + kg;
+  const int wb0 = blocks * group / tk, nb = blocks * (group + 1) / tk - wb0;  // and of this warp
+  const int tile0 = MODE == kStream ? blockIdx.x * a.rt + rt : row_block * a.rt + rt;
+  const int tile_step = gridDim.x * a.rt;
+  const int tiles = (MODE == kStream) ? (tile0 < a.tiles ? (a.tiles - tile0 + tile_step - 1) / tile_step : 0) : tile0 < a.tiles ? 1 : 0;
+  const int total = tiles * nb;
+  const uint32_t x_addr = smem_u32(sm), ring = x_addr + (uint32_t)a.x_bytes + (uint32_t)(warp * a.stages) * kStageBytes;
+
+  // ---- weights: this warp's first blocks, before anything else ----
+  auto weight_row = [&](int tile, int r) { return MODE == kGeglu ? (r < 16 ? tile * 16 + r : a.N / 2 + tile * 16 + r - 16) : tile * kTileRows + r; };
+  auto row_valid = [&](int tile, int r) { return MODE == kGeglu ? tile * 16 + (r & 15) < a.N / 2 : tile * kTileRows + r < a.N; };
+  int is_tile = tile0, is_kb = 0, is_stage = 0;
+  auto issue = [&]() {
+    // lane -> 16-byte piece tig of rows g, g + 8, g + 16, g + 24
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int r = g + 8 * j;
+      const bool v = row_valid(is_tile, r);
+      cp_async16(ring + is_stage * kStageBytes + r * kBlk + tig * 16, a.W + (v ? (size_t)weight_row(is_tile, r) * a.K : 0) + (size_t)(wb0 + is_kb) * kBlk + tig * 16, v);
+    }
+    if (++is_kb == nb) { is_kb = 0; is_tile += tile_step; }
+    if (++is_stage == a.stages) is_stage = 0;
+  };
+  int issued = 0;
+  for (; issued < a.stages && issued < total; issued++) {
+    issue();
+    cp_commit();
+  }
+  float rope_c = 0.f, rope_s = 0.f, norm_w = 0.f;
+  int pos = 0;
+  const int head = MODE == kRope ? blockIdx.x / 8 : 0, part = MODE == kRope ? blockIdx.x % 8 : 0;
+  const bool is_q = head < a.n_q, is_k = head == a.n_q;
+  if (MODE == kRope) {
+    if (is_q || is_k) norm_w = 1.0f + bf2f(__ldg((is_q ? a.qw : a.kw) + part * 32 + lane));
+  }
+  // the scales of the block's rows, read once per step and so always from HBM
+  float* scale_s = reinterpret_cast<float*>(sm + a.scale_off);
+  if (MODE != kStream)
+    for (int i = threadIdx.x; i < a.rt * kTileRows; i += blockDim.x) {
+      const int t = row_block * a.rt + i / kTileRows;
+      scale_s[i] = row_valid(t, i % kTileRows) ? bf2f(__ldg(a.scale + weight_row(t, i % kTileRows))) : 0.f;
+    }
+  if (a.ck > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
+  grid_dependency_wait();
+  grid_dependency_release();
+
+  // ---- activations of K blocks [kb0, kb1); tokens beyond B read as zero ----
+  {
+    const int vec = (kb1 - kb0) * 8;  // 16-byte pieces per token
+    for (int b = warp; b < kTok; b += (int)(blockDim.x >> 5)) {
+      const uint16_t* src = a.x + (b < a.B ? (size_t)b * a.K : 0) + kb0 * kBlk;
+      const uint32_t dst = x_addr + (uint32_t)(b * a.x_pitch);
+#pragma unroll 4
+      for (int c = lane; c < vec; c += 32) cp_async16(dst + 16 * c, src + 8 * c, b < a.B);
+    }
+    cp_commit();
+    if (MODE == kRope) {  // while they arrive: the position's rotation for this lane's row
+      pos = __ldcg(a.pos);
+      pos = pos < 0 ? 0 : (pos >= a.T ? a.T - 1 : pos);
+      const int i = (part & 3) * 32 + lane;
+      const float inv_freq = powf(a.theta, -(float)i / 128.0f);
+      sincosf((float)pos * inv_freq, &rope_s, &rope_c);
+    }
+    cp_wait<0>();
+  }
+  __syncthreads();
+
+  float c[2][NT][4];
+  float best_v[NT][2];
+  int best_i[NT][2];
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    best_v[t][0] = best_v[t][1] = -INFINITY;
+    best_i[t][0] = best_i[t][1] = 0x7fffffff;
+#pragma unroll
+    for (int j = 0; j < 4; j++) c[0][t][j] = c[1][t][j] = 0.f;
+  }
+  const uint32_t xrow = x_addr + (uint32_t)(g * a.x_pitch + (wb0 - kb0) * kBlk * 2 + tig * 32);
+  int stage = 0, kb = 0, tile = tile0;
+  for (int i = 0; i < total; i++) {
+    if (MODE == kStream) {  // the ring is a.stages deep and one group is committed per block from here on
+      if (i >= a.stages) cp_wait<kStreamStages - 1>();
+      __syncwarp();
+    }
+    const uint32_t src = ring + stage * kStageBytes + g * kBlk + tig * 16;
+    const uint4 w0 = lds128(src), w1 = lds128(src + 8 * kBlk), w2 = lds128(src + 16 * kBlk), w3 = lds128(src + 24 * kBlk);
+    if (MODE == kStream) {
+      __syncwarp();  // read by every lane before any of them refills the stage
+      if (issued < total) {
+        issue();
+        issued++;
+      }
+      cp_commit();
+    }
+    const uint32_t ww[4][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}, {w2.x, w2.y, w2.z, w2.w}, {w3.x, w3.y, w3.z, w3.w}};
+    uint4 x0[NT], x1[NT];
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      const uint32_t xa = xrow + (uint32_t)(t * 8 * a.x_pitch + kb * kBlk * 2);
+      x0[t] = lds128(xa);
+      x1[t] = lds128(xa + 16);
+    }
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      uint32_t f[4][2];
+#pragma unroll
+      for (int r = 0; r < 4; r++) s8x4_to_bf16x4(ww[r][m], f[r][0], f[r][1]);
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        const uint32_t b0 = m == 0 ? x0[t].x : m == 1 ? x0[t].z : m == 2 ? x1[t].x : x1[t].z;
+        const uint32_t b1 = m == 0 ? x0[t].y : m == 1 ? x0[t].w : m == 2 ? x1[t].y : x1[t].w;
+        mma_bf16(c[0][t], f[0][0], f[1][0], f[0][1], f[1][1], b0, b1);
+        mma_bf16(c[1][t], f[2][0], f[3][0], f[2][1], f[3][1], b0, b1);
+      }
+    }
+    if (++stage == a.stages) stage = 0;
+    if (++kb == nb) {
+      kb = 0;
+      if (MODE == kStream) {
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int n = tile * kTileRows + 16 * mt + 8 * h + g;
+            const float s = n < a.N ? bf2f(__ldg(a.scale + n)) : 0.f;
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+#pragma unroll
+              for (int e = 0; e < 2; e++) {
+                const int b = 8 * t + 2 * tig + e;
+                const float v = c[mt][t][2 * h + e] * s;
+                if (n < a.N && b < a.B) {
+                  if (a.y_f32) ((float*)a.y)[(size_t)b * a.N + n] = v;
+                  else ((uint16_t*)a.y)[(size_t)b * a.N + n] = f2bf(v);
+                  if (v > best_v[t][e]) {  // a warp's rows come in rising order: ties keep the lower index
+                    best_v[t][e] = v;
+                    best_i[t][e] = n;
+                  }
+                }
+                c[mt][t][2 * h + e] = 0.f;
+              }
+          }
+        tile += tile_step;
+      }
+    }
+  }
+
+  if constexpr (MODE == kStream) {
+    if (!a.cand_v) return;
+    // best of the block per token, lowest row on ties
+    __syncthreads();
+    float* sv = reinterpret_cast<float*>(sm);
+    int* si = reinterpret_cast<int*>(sm) + 16 * kTok;
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        float v = best_v[t][e];
+        int n = best_i[t][e];
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+          const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+          const int on = __shfl_xor_sync(0xffffffffu, n, o);
+          if (ov > v || (ov == v && on < n)) {
+            v = ov;
+            n = on;
+          }
+        }
+        if (g == 0) {
+          sv[warp * kTok + 8 * t + 2 * tig + e] = v;
+          si[warp * kTok + 8 * t + 2 * tig + e] = n;
+        }
+      }
+    __syncthreads();
+    if ((int)threadIdx.x < a.B) {
+      float v = sv[threadIdx.x];
+      int n = si[threadIdx.x];
+      for (int w = 1; w < (int)(blockDim.x >> 5); w++) {
+        const float ov = sv[w * kTok + threadIdx.x];
+        const int on = si[w * kTok + threadIdx.x];
+        if (ov > v || (ov == v && on < n)) {
+          v = ov;
+          n = on;
+        }
+      }
+      a.cand_v[threadIdx.x * gridDim.x + blockIdx.x] = v;
+      a.cand_i[threadIdx.x * gridDim.x + blockIdx.x] = n;
+    }
+    return;
+  } else {
+  // ---- the groups' sums meet: [tile of the block][group of the block][32 rows][tokens], over the staged operands ----
+  __syncthreads();
+  float* sums = reinterpret_cast<float*>(sm);
+  float* mine = sums + (rt * a.kg + kg) * (kTileRows * kPitch);
+#pragma unroll
+  for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) mine[(16 * mt + g + 8 * (j >> 1)) * kPitch + 8 * t + 2 * tig + (j & 1)] = c[mt][t][j];
+  __syncthreads();
+  // the block's groups, in order
+  auto block_sum = [&](int r_t, int row, int tok) {
+    const float* at = sums + r_t * a.kg * (kTileRows * kPitch) + row * kPitch + tok;
+    float v = at[0];
+#pragma unroll 4
+    for (int k = 1; k < a.kg; k++) v += at[k * (kTileRows * kPitch)];
+    return v;
+  };
+  const int warps = blockDim.x >> 5;
+  // Results are numbered i = tile of the block * B + token, 32 rows each. In a cluster block i % ck finishes result i: the others
+  // store their sums into its shared memory, 128 contiguous bytes a warp (reading them over one by one, a word per lane
+  // and request, took up to 40 us), and it adds the blocks' sums in order.
+  float* recv = reinterpret_cast<float*>(sm + a.recv_off);  // [block of the cluster][i / ck][32]
+  const int share = (a.rt * a.B + a.ck - 1) / a.ck;
+  if (MODE != kRope && a.ck > 1) {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    for (int i = warp; i < a.rt * a.B; i += warps)
+      st_peer(smem_u32(recv + (rank * share + i / a.ck) * 32 + lane), i % a.ck, block_sum(i / a.B, lane, i % a.B));
+    cluster_sync();
+  }
+  auto sum_of = [&](int i, int row) {
+    if (a.ck <= 1) return block_sum(i / a.B, row, i % a.B);
+    float v = recv[(i / a.ck) * 32 + row];
+    for (int q = 1; q < a.ck; q++) v += recv[(q * share + i / a.ck) * 32 + row];
+    return v;
+  };
+  if constexpr (MODE == kStore) {
+    for (int i = warp * a.ck + rank; i < a.rt * a.B; i += warps * a.ck) {
+      const int r_t = i / a.B, b = i - r_t * a.B, n = (row_block * a.rt + r_t) * kTileRows + lane;
+      const float v = sum_of(i, lane) * scale_s[r_t * kTileRows + lane];
+      if (n >= a.N) continue;
+      if (a.y_f32) ((float*)a.y)[(size_t)b * a.N + n] = v;
+      else ((uint16_t*)a.y)[(size_t)b * a.N + n] = f2bf(v);
+    }
+  } else if constexpr (MODE == kGeglu) {
+    const int I = a.N / 2, r = lane & 15;  // half a warp per token
+    for (int i = (warp * 2 + (lane >> 4)) * a.ck + rank; i < a.rt * a.B; i += 2 * warps * a.ck) {
+      const int r_t = i / a.B, b = i - r_t * a.B, n = (row_block * a.rt + r_t) * 16 + r;
+      if (n >= I) continue;
+      const float* sc = scale_s + r_t * kTileRows;
+      const float gate = rbf(sum_of(i, r) * sc[r]), up = rbf(sum_of(i, 16 + r) * sc[16 + r]);
+      ((uint16_t*)a.y)[(size_t)b * I + n] = f2bf(rbf(gelu_tanh(gate)) * up);
+    }
+  } else {
+    // one head of 256 rows per cluster, 32 rows per block: lane = row
+    float* ss = sums + a.kg * (kTileRows * kPitch);  // [tokens] sum of squares of this block's rows
+    float* nv = ss + kTok;                           // [tokens][32] normalised values
+    const float scale = scale_s[lane];
+    for (int b = warp; b < a.B; b += warps) {
+      const float v = rbf(block_sum(0, lane, b) * scale);
+      nv[b * 32 + lane] = v;
+      const float s = warp_sum(v * v);
+      if (lane == 0) ss[b] = s;
+    }
+    cluster_sync();
+    if (is_q || is_k)
+      for (int b = warp; b < a.B; b += warps) {
+        float s = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; q++) s += ld_peer(smem_u32(ss + b), q);
+        nv[b * 32 + lane] = rbf(nv[b * 32 + lane] * rsqrtf(s / 256.0f + a.eps) * norm_w);
+      }
+    cluster_sync();
+    for (int b = warp; b < a.B; b += warps) {
+      const float own = nv[b * 32 + lane];
+      float v = own;
+      if (is_q || is_k) {
+        const float other = ld_peer(smem_u32(nv + b * 32 + lane), part ^ 4);
+        v = part < 4 ? own * rope_c - other * rope_s : own * rope_c + other * rope_s;
+      }
+      uint16_t* dst = is_q ? a.q_out + ((size_t)b * a.n_q + head) * 256 : (is_k ? a.kcache : a.vcache) + ((size_t)b * a.T + pos) * 256;
+      dst[part * 32 + lane] = f2bf(v);
+    }
+  }
+  if (MODE == kRope) cluster_sync();  // no block leaves while another may read its values
+  }
+}
+
+// Head norm, RoPE and cache append on finished q/k/v values, head size 256: a warp per (sequence, head). The same arithmetic in the
+// same order as the epilogue of linear_w8_kernel.
+__global__ void __launch_bounds__(128) rope_head_kernel(const uint16_t* __restrict__ qkv, const int32_t* __restrict__ pos_p,
+                                                        const uint16_t* __restrict__ qw, const uint16_t* __restrict__ kw,
+                                                        uint16_t* __restrict__ q_out, uint16_t* __restrict__ kcache,
+                                                        uint16_t* __restrict__ vcache, int B, int n_q, int n_kv, int T, float theta, float eps) {
+  const int heads = n_q + 2 * n_kv, lane = threadIdx.x & 31;
+  const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (item >= B * heads) {
+    grid_dependency_wait();
+    return;
+  }
+  const int b = item / heads, h = item - b * heads;
+  const bool is_q = h < n_q, is_k = !is_q && h < n_q + n_kv;
+  float w[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) w[j] = (is_q || is_k) ? 1.0f + bf2f(__ldg((is_q ? qw : kw) + 32 * j + lane)) : 0.f;
+  grid_dependency_wait();
+  grid_dependency_release();
+  int pos = __ldcg(pos_p);
+  pos = pos < 0 ? 0 : (pos >= T ? T - 1 : pos);
+  float v[8], s = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    v[j] = bf2f(__ldcg(qkv + (size_t)item * 256 + 32 * j + lane));
+    s += warp_sum(v[j] * v[j]);
+  }
+  uint16_t* dst = is_q ? q_out + ((size_t)b * n_q + h) * 256
+                       : (is_k ? kcache : vcache) + (((size_t)b * T + pos) * n_kv + (is_k ? h - n_q : h - n_q - n_kv)) * 256;
+  if (!is_q && !is_k) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) dst[32 * j + lane] = f2bf(v[j]);
+    return;
+  }
+  const float inv = rsqrtf(s / 256.0f + eps);
+#pragma unroll
+  for (int j = 0; j < 8; j++) v[j] = rbf(v[j] * inv * w[j]);
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float inv_freq = powf(theta, -(float)(32 * j + lane) / 128.0f);
+    float sn, cs;
+    sincosf((float)pos * inv_freq, &sn, &cs);
+    dst[32 * j + lane] = f2bf(v[j] * cs - v[j + 4] * sn);
+    dst[128 + 32 * j + lane] = f2bf(v[j + 4] * cs + v[j] * sn);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// One query per head against the cache of its sequence (one KV head of 256, up to 4 query heads). A cluster of eight blocks is
+// one sequence; a block takes an eighth of the visible keys, a warp 16 keys at a time, copied to shared memory at once (rows
+// 64 and 16 bytes apart modulo 128: no bank is hit twice): scores = heads (4 of 16 rows used) x 8 keys, whose accumulator layout is at once the operand layout of the
+// second product, values (16 dims) x heads. The probabilities enter that product as three bf16 terms whose sum is the fp32
+// number exactly (columns 0-3 and 4-7 of one instruction, columns 0-3 of another), so nothing is lost against an fp32
+// product. Warps merge in shared memory, blocks through distributed shared memory: one launch, no partial sums in memory.
+// What bounds it is the cache's way from HBM: its lines are prefetched before the wait for the kernel ahead.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int kAttnBlocks = 8, kAttnWarps = 4, kAttnCol = 256 + 8;
+constexpr int kKeyPitch = 512 + 64, kValPitch = 512 + 16, kAttnWarpBytes = 16 * (kKeyPitch + kValPitch);
+static_assert(8 * kAttnCol * 4 <= kAttnWarpBytes, "the warps' results take the place of their keys and values");
+
+__global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_cluster_kernel(const uint16_t* __restrict__ q, const int32_t* __restrict__ pos_p,
+                                                                          const uint16_t* kcache, const uint16_t* vcache,
+                                                                          uint16_t* __restrict__ out, int n_q, int T, int window, float scale) {
+  extern __shared__ __align__(128) unsigned char kv_s[];  // [warp][16 keys, 16 values], later [warp][8 columns][kAttnCol] results
+  __shared__ float part_ml[kAttnWarps][4][2];
+  __shared__ float blk_acc[4][256];
+  __shared__ float blk_ml[4][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int rank = blockIdx.x, b = blockIdx.y;
+  int t0, t1;
+  auto slice = [&](int pos) {
+    pos = pos < 0 ? 0 : (pos >= T ? T - 1 : pos);
+    const int t_lo = window > 0 ? max(0, pos - window + 1) : 0;
+    const int per = ((pos + 1 - t_lo + kAttnBlocks - 1) / kAttnBlocks + 15) & ~15;
+    t0 = t_lo + rank * per;
+    t1 = min(pos + 1, t0 + per);
+  };
+  slice(__ldcg(pos_p));  // for the prefetch only: read again behind the wait
+  const uint16_t* kc = kcache + (size_t)b * T * 256;
+  const uint16_t* vc = vcache + (size_t)b * T * 256;
+  for (int row = t0 + 16 * warp + (lane & 15); row < t1; row += 16 * kAttnWarps) {
+    const uint16_t* p = (lane < 16 ? kc : vc) + (size_t)row * 256;
+#pragma unroll
+    for (int j = 0; j < 4; j++) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 64 * j));
+  }
+  grid_dependency_wait();
+  grid_dependency_release();
+  slice(__ldcg(pos_p));
+  const uint32_t ks = smem_u32(kv_s) + warp * kAttnWarpBytes, vs = ks + 16 * kKeyPitch;
+  auto copy = [&](const uint16_t* src, int t, uint32_t dst, int pitch) {  // a row is 32 pieces of 16 bytes: one per lane
+#pragma unroll
+    for (int r = 0; r < 16; r++) cp_async16(dst + r * pitch + lane * 16, src + (size_t)min(t + r, t1 - 1) * 256 + lane * 8, true);
+    cp_commit();
+  };
+  const int t_first = t0 + 16 * warp;
+  if (t_first < t1) {
+    copy(kc, t_first, ks, kKeyPitch);
+    copy(vc, t_first, vs, kValPitch);
+  }
+  uint4 qf[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    qf[j] = make_uint4(0, 0, 0, 0);
+    if (g < n_q) qf[j] = __ldcg(reinterpret_cast<const uint4*>(q + ((size_t)b * n_q + g) * 256 + 32 * j + 8 * t4));
+  }
+  float m = -INFINITY, l = 0.f, acc[16][4];
+#pragma unroll
+  for (int j = 0; j < 16; j++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) acc[j][e] = 0.f;
+  for (int t = t_first; t < t1; t += 16 * kAttnWarps) {
+    if (t != t_first) {
+      __syncwarp();  // every lane has read the round before
+      copy(kc, t, ks, kKeyPitch);
+      copy(vc, t, vs, kValPitch);
+    }
+    cp_wait<1>();
+    __syncwarp();
+    // ---- scores of 2 x 8 keys ----
+    float s[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      uint4 kf[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) kf[j] = lds128(ks + (8 * u + g) * kKeyPitch + 64 * j + 16 * t4);
+      float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        mma_bf16(c0, qf[j].x, 0u, qf[j].y, 0u, kf[j].x, kf[j].y);
+        mma_bf16(c1, qf[j].z, 0u, qf[j].w, 0u, kf[j].z, kf[j].w);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; e++) s[u][e] = t + 8 * u + 2 * t4 + e < t1 ? (c0[e] + c1[e]) * scale : -INFINITY;
+    }
+    float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float m_new = fmaxf(m, mx), corr = expf(m - m_new);
+    m = m_new;
+    float p[2][2];
+    l *= corr;
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        p[u][e] = expf(s[u][e] - m_new);
+        l += p[u][e];
+      }
+    const float corr0 = __shfl_sync(0xffffffffu, corr, ((2 * t4) & 3) * 4), corr1 = __shfl_sync(0xffffffffu, corr, ((2 * t4 + 1) & 3) * 4);
+    uint32_t b_hm[2], b_lo[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      uint16_t hm[2], lo[2];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const float x = __shfl_sync(0xffffffffu, p[u][e], lane & 15);
+        const float hi = rbf(x), mid = rbf(x - hi);
+        hm[e] = g < 4 ? f2bf(hi) : f2bf(mid);
+        lo[e] = g < 4 ? f2bf((x - hi) - mid) : (uint16_t)0;
+      }
+      b_hm[u] = hm[0] | (uint32_t)hm[1] << 16;
+      b_lo[u] = lo[0] | (uint32_t)lo[1] << 16;
+    }
+    // ---- values ----
+    cp_wait<0>();
+    __syncwarp();
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+      uint4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        v[k] = lds128(vs + (2 * t4 + (k & 1) + 8 * (k >> 1)) * kValPitch + 128 * d + 16 * g);
+      const uint32_t r[4][4] = {{v[0].x, v[0].y, v[0].z, v[0].w}, {v[1].x, v[1].y, v[1].z, v[1].w}, {v[2].x, v[2].y, v[2].z, v[2].w}, {v[3].x, v[3].y, v[3].z, v[3].w}};
+#pragma unroll
+      for (int j = 0; j < 4; j++) {  // row g: dim 64 d + 8 g + j, row g + 8: dim 64 d + 8 g + 4 + j
+        const uint32_t sel = j & 1 ? 0x7632 : 0x5410;
+        const uint32_t a0 = __byte_perm(r[0][j >> 1], r[1][j >> 1], sel), a1 = __byte_perm(r[0][2 + (j >> 1)], r[1][2 + (j >> 1)], sel);
+        const uint32_t a2 = __byte_perm(r[2][j >> 1], r[3][j >> 1], sel), a3 = __byte_perm(r[2][2 + (j >> 1)], r[3][2 + (j >> 1)], sel);
+        float(&c)[4] = acc[4 * d + j];
+        c[0] *= corr0; c[1] *= corr1; c[2] *= corr0; c[3] *= corr1;
+        mma_bf16(c, a0, a1, a2, a3, b_hm[0], b_hm[1]);
+        mma_bf16(c, a0, a1, a2, a3, b_lo[0], b_lo[1]);
+      }
+    }
+  }
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  if (t4 == 0 && g < 4) {
+    part_ml[warp][g][0] = m;
+    part_ml[warp][g][1] = l;
+  }
+  __syncwarp();
+  float(*part)[kAttnCol] = reinterpret_cast<float(*)[kAttnCol]>(kv_s + warp * kAttnWarpBytes);
+#pragma unroll
+  for (int j = 0; j < 16; j++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) part[2 * t4 + (e & 1)][16 * j + g + 8 * (e >> 1)] = acc[j][e];
+  __syncthreads();
+  for (int h = 0; h < n_q; h++) {
+    float mm = -INFINITY, ll = 0.f, e[kAttnWarps];
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; w++) mm = fmaxf(mm, part_ml[w][h][0]);
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; w++) {
+      e[w] = part_ml[w][h][1] > 0.f ? expf(part_ml[w][h][0] - mm) : 0.f;
+      ll += part_ml[w][h][1] * e[w];
+    }
+#pragma unroll
+    for (int i = threadIdx.x; i < 256; i += kAttnWarps * 32) {
+      float o = 0.f;
+#pragma unroll
+      for (int w = 0; w < kAttnWarps; w++) {
+        const float* p = reinterpret_cast<const float*>(kv_s + w * kAttnWarpBytes);
+        o += (p[h * kAttnCol + i] + p[(h + 4) * kAttnCol + i]) * e[w];
+      }
+      blk_acc[h][i] = o;
+    }
+    if (threadIdx.x == 0) {
+      blk_ml[h][0] = mm;
+      blk_ml[h][1] = ll;
+    }
+  }
+  cluster_sync();
+  for (int i = rank * (kAttnWarps * 32) + threadIdx.x; i < n_q * 256; i += kAttnBlocks * kAttnWarps * 32) {
+    const int h = i >> 8, at = i & 255;
+    float mr[kAttnBlocks], lr[kAttnBlocks], ar[kAttnBlocks], mm = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < kAttnBlocks; r++) {
+      mr[r] = ld_peer(smem_u32(&blk_ml[h][0]), r);
+      lr[r] = ld_peer(smem_u32(&blk_ml[h][1]), r);
+      ar[r] = ld_peer(smem_u32(&blk_acc[h][at]), r);
+      mm = fmaxf(mm, mr[r]);
+    }
+    float ll = 0.f, o = 0.f;
+#pragma unroll
+    for (int r = 0; r < kAttnBlocks; r++)
+      if (lr[r] > 0.f) {
+        const float e = expf(mr[r] - mm);
+        ll += lr[r] * e;
+        o += ar[r] * e;
+      }
+    // place i of a column: tile (d, j) x row
+    const int dim = 64 * (at >> 6) + 8 * (at & 7) + 4 * (at >> 3 & 1) + (at >> 4 & 3);
+    out[((size_t)b * n_q + h) * 256 + dim] = f2bf(o / ll);
+  }
+  cluster_sync();
+}
+
+// best of the blocks' candidates, [B][count] values and rows: a warp per token
+__global__ void __launch_bounds__(32) argmax_candidates_kernel(const float* __restrict__ pv, const int32_t* __restrict__ pi, int count,
+                                                               int32_t* __restrict__ out) {
+  grid_dependency_wait();
+  grid_dependency_release();
+  const int b = blockIdx.x;
+  float v = -INFINITY;
+  int n = 0x7fffffff;
+  auto take = [&](float ov, int on) {
+    if (ov > v || (ov == v && on < n)) {
+      v = ov;
+      n = on;
+    }
+  };
+  for (int c = threadIdx.x; c < count; c += 32) take(__ldcg(pv + b * count + c), __ldcg(pi + b * count + c));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) take(__shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, n, o));
+  if (threadIdx.x == 0) out[b] = n;
+}
+
+// y = [res +] bf16(x * rsqrt(mean(x^2) + eps) * (1 + w)), optionally followed by the same norm (w2, no residual) of y: a block per row, four
+// elements a thread, the row in registers (H a multiple of 4, up to 4096).
+template <int V>
+__global__ void __launch_bounds__(512) rmsnorm_row_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ res,
+                                                          const uint16_t* __restrict__ w, uint16_t* __restrict__ out,
+                                                          const uint16_t* __restrict__ w2, uint16_t* __restrict__ out2, int H, float eps,
+                                                          float eps2) {
+  __shared__ float red[2][16];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  auto four = [](const uint2& u, float (&f)[4]) {
+    f[0] = __uint_as_float(u.x << 16);
+    f[1] = __uint_as_float(u.x & 0xffff0000u);
+    f[2] = __uint_as_float(u.y << 16);
+    f[3] = __uint_as_float(u.y & 0xffff0000u);
+  };
+  uint2 wv[V], wv2[V];
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const int i = 4 * (threadIdx.x + k * blockDim.x);
+    wv[k] = wv2[k] = make_uint2(0, 0);
+    if (i < H) {
+      wv[k] = __ldg(reinterpret_cast<const uint2*>(w + i));
+      if (w2) wv2[k] = __ldg(reinterpret_cast<const uint2*>(w2 + i));
+    }
+  }
+  grid_dependency_wait();
+  grid_dependency_release();
+  const size_t base = (size_t)blockIdx.x * H;
+  float v[V][4], r[V][4], ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const int i = 4 * (threadIdx.x + k * blockDim.x);
+    uint2 u = make_uint2(0, 0), ur = make_uint2(0, 0);
+    if (i < H) {
+      u = __ldcg(reinterpret_cast<const uint2*>(x + base + i));
+      if (res) ur = __ldcg(reinterpret_cast<const uint2*>(res + base + i));
+    }
+    four(u, v[k]);
+    four(ur, r[k]);
+#pragma unroll
+    for (int e = 0; e < 4; e++) ss += v[k][e] * v[k][e];
+  }
+  auto total = [&](float s, int slot) {
+    s = warp_sum(s);
+    if (lane == 0) red[slot][warp] = s;
+    __syncthreads();
+    return warp_sum(lane < warps ? red[slot][lane] : 0.f);
+  };
+  const float inv = rsqrtf(total(ss, 0) / (float)H + eps);
+  float ss2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const int i = 4 * (threadIdx.x + k * blockDim.x);
+    float f[4];
+    four(wv[k], f);
+    uint16_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const float n = rbf(v[k][e] * inv * (1.0f + f[e]));
+      o[e] = res ? f2bf(r[k][e] + n) : f2bf(n);
+      v[k][e] = bf2f(o[e]);
+      ss2 += i < H ? v[k][e] * v[k][e] : 0.f;
+    }
+    if (i < H) *reinterpret_cast<uint2*>(out + base + i) = make_uint2(o[0] | (uint32_t)o[1] << 16, o[2] | (uint32_t)o[3] << 16);
+  }
+  if (!w2) return;
+  const float inv2 = rsqrtf(total(ss2, 1) / (float)H + eps2);
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const int i = 4 * (threadIdx.x + k * blockDim.x);
+    float f[4];
+    four(wv2[k], f);
+    uint16_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[e] = f2bf(v[k][e] * inv2 * (1.0f + f[e]));
+    if (i < H) *reinterpret_cast<uint2*>(out2 + base + i) = make_uint2(o[0] | (uint32_t)o[1] << 16, o[2] | (uint32_t)o[3] << 16);
+  }
+}
+
+int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+// groups of K of a product: enough warps to ask for every weight at once, none without a 64-byte block
+int linear_groups(int N, int K) {
+  const int tiles = ceil_div(N, kTileRows), blocks = K / kBlk;
+  const int cap = K <= 4096 ? 16 : 32;
+  int tk = 1;
+  while (tk * 2 <= blocks && tk < cap && (long long)tiles * tk * 2 <= 12 * 148) tk *= 2;
+  return tk;
+}
+
+struct LinearShape {
+  int tk, kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, smem, tiles, grid;
+  bool ok;
+};
+constexpr int kSmemMax = 227 * 1024 - 1024;
+
+LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
+  LinearShape s{};
+  if (K % kBlk != 0 || K < kBlk || B < 1 || B > 32 || N < 1) return s;
+  const int tok = ceil_div(B, 8) * 8, blocks = K / kBlk;
+  s.tk = linear_groups(N, K);
+  if (mode == kStore && s.tk == 1) mode = kStream;
+  s.tiles = mode == kGeglu ? ceil_div(N / 2, 16) : ceil_div(N, kTileRows);
+  auto fit = [&](int kg, int ck, int rt, int stages) {
+    s.kg = kg; s.ck = ck; s.rt = rt; s.stages = stages;
+    int widest = 0;
+    for (int r = 0; r < ck; r++) widest = std::max(widest, blocks * (r * kg + kg) / s.tk - blocks * (r * kg) / s.tk);
+    s.x_pitch = (widest * kBlk * 2 + 127) / 128 * 128 + 16;
+    s.x_bytes = (tok * s.x_pitch + 127) / 128 * 128;
+    const int warps = kg * rt;
+    const int sums = warps * kTileRows * (tok + 1) * 4 + (mode == kRope ? tok * 33 * 4 : 0);
+    s.scale_off = std::max(s.x_bytes + warps * stages * kStageBytes, mode == kStream ? 16 * tok * 8 : (sums + 127) / 128 * 128);
+    s.recv_off = s.scale_off + rt * kTileRows * 4;
+    s.smem = s.recv_off + (ck > 1 ? (rt * B + ck - 1) / ck * ck * 128 : 0);
+    return s.smem <= kSmemMax;
+  };
+  if (mode == kStream) {
+    for (int rt = 16; rt >= 1; rt /= 2)
+      if (fit(1, 1, rt, kStreamStages)) {
+        s.grid = std::min(sms, ceil_div(s.tiles, rt));
+        s.ok = true;
+        return s;
+      }
+    return s;
+  }
+  const int stages = ceil_div(blocks, s.tk);  // every block of a warp has its own place
+  if (stages > 64) return s;
+  if (mode == kRope) {
+    s.ok = s.tk <= 16 && fit(s.tk, 1, 1, stages);
+    s.grid = s.tiles;
+    return s;
+  }
+  // the fewest blocks per cluster whose activations leave room; more while that fills idle SMs
+  for (int ck = 1; ck <= 8 && ck <= s.tk; ck *= 2) {
+    const int kg = s.tk / ck;
+    if (kg > 16) continue;
+    int rt = std::max(1, std::min(ceil_div((long long)s.tiles * ck, sms), 16 / kg));
+    while (rt > 1 && !fit(kg, ck, rt, stages)) rt--;
+    if (!fit(kg, ck, rt, stages)) continue;
+    s.grid = ceil_div(s.tiles, rt) * ck;
+    s.ok = true;
+    return s;
+  }
+  return s;
+}
+
+template <int NT, int MODE>
+cudaError_t launch_linear_as(const LinearArgs& a, const LinearShape& s, int cluster, cudaStream_t stream) {
+  auto kernel = linear_w8_kernel<NT, MODE>;
+  static std::atomic<unsigned long long> attr_done{0};
+  if (first_use_on_device(attr_done)) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    if (e != cudaSuccess) return e;
+    mark_used_on_device(attr_done);
+  }
+  return launch_dependent_cluster(cluster, kernel, dim3(s.grid), dim3(s.kg * s.rt * 32), (size_t)s.smem, stream, !a.serial, a);
+}
+template <int MODE>
+cudaError_t launch_linear_mode(const LinearArgs& args, const LinearShape& s, cudaStream_t stream) {
+  LinearArgs a = args;
+  a.kg = s.kg; a.ck = s.ck; a.rt = s.rt; a.stages = s.stages; a.x_pitch = s.x_pitch; a.x_bytes = s.x_bytes; a.scale_off = s.scale_off; a.recv_off = s.recv_off; a.tiles = s.tiles;
+  const int cluster = MODE == kRope ? 8 : s.ck;
+  switch ((a.B + 7) / 8) {
+    case 1: return launch_linear_as<1, MODE>(a, s, cluster, stream);
+    case 2: return launch_linear_as<2, MODE>(a, s, cluster, stream);
+    case 3: return launch_linear_as<3, MODE>(a, s, cluster, stream);
+    default: return launch_linear_as<4, MODE>(a, s, cluster, stream);
+  }
+}
+
+}  // namespace
+
+bool linear_w8_applies(int B, int N, int K) { return linear_shape(B, N, K, kStore, 148).ok; }
+bool linear_geglu_applies(int B, int N, int K) { return N % 2 == 0 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kGeglu, 148).ok; }
+bool linear_rope_applies(int B, int N, int K, int n_q, int n_kv, int D) {
+  return n_kv == 1 && D == 256 && N == (n_q + 2) * 256 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kRope, 148).ok;
+}
+// whether the arg max over the results can ride along, and the candidates' bytes
+size_t linear_argmax_scratch(int B, int N, int K) {
+  const LinearShape s = linear_shape(B, N, K, kStore, current_sm_count());
+  return s.ok && s.tk == 1 ? (size_t)B * s.grid * 8 : 0;
+}
+
+cudaError_t launch_linear(const LinearArgs& a, cudaStream_t stream) {
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kStore, current_sm_count());
+  if (!s.ok) return cudaErrorInvalidConfiguration;
+  return s.tk == 1 ? launch_linear_mode<kStream>(a, s, stream) : launch_linear_mode<kStore>(a, s, stream);
+}
+cudaError_t launch_linear_geglu(const LinearArgs& a, cudaStream_t stream) {
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kGeglu, current_sm_count());
+  return s.ok ? launch_linear_mode<kGeglu>(a, s, stream) : cudaErrorInvalidConfiguration;
+}
+cudaError_t launch_linear_rope(const LinearArgs& a, cudaStream_t stream) {
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kRope, current_sm_count());
+  return s.ok ? launch_linear_mode<kRope>(a, s, stream) : cudaErrorInvalidConfiguration;
+}
+cudaError_t launch_linear_argmax(LinearArgs a, void* scratch, int32_t* out, cudaStream_t stream) {
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kStore, current_sm_count());
+  if (!s.ok || s.tk != 1) return cudaErrorInvalidConfiguration;
+  a.cand_v = (float*)scratch;
+  a.cand_i = (int32_t*)scratch + (size_t)a.B * s.grid;
+  const cudaError_t e = launch_linear_mode<kStream>(a, s, stream);
+  if (e != cudaSuccess) return e;
+  return launch_dependent(argmax_candidates_kernel, dim3(a.B), dim3(32), 0, stream, a.cand_v, a.cand_i, s.grid, out);
+}
+
+void launch_rope_heads(const uint16_t* qkv, const int32_t* pos, const uint16_t* qw, const uint16_t* kw, uint16_t* q_out, uint16_t* kcache,
+                       uint16_t* vcache, int B, int n_q, int n_kv, int T, float theta, float eps, cudaStream_t stream) {
+  launch_dependent(rope_head_kernel, dim3(ceil_div((long long)B * (n_q + 2 * n_kv), 4)), dim3(128), 0, stream, qkv, pos, qw, kw, q_out, kcache, vcache,
+                   B, n_q, n_kv, T, theta, eps);
+}
+
+void launch_attn_decode(const uint16_t* q, const int32_t* pos, const uint16_t* kcache, const uint16_t* vcache, uint16_t* out, int B, int n_q,
+                        int T, int window, float scale, cudaStream_t stream) {
+  static std::atomic<unsigned long long> attr_done{0};
+  if (first_use_on_device(attr_done)) {
+    cudaFuncSetAttribute(attn_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnWarps * kAttnWarpBytes);
+    mark_used_on_device(attr_done);
+  }
+  launch_dependent_cluster(kAttnBlocks, attn_cluster_kernel, dim3(kAttnBlocks, B), dim3(kAttnWarps * 32), kAttnWarps * kAttnWarpBytes, stream, true, q, pos, kcache, vcache, out,
+                           n_q, T, window, scale);
+}
+
+bool rmsnorm_row_applies(int H) { return H % 4 == 0 && H <= 4096; }
+void launch_rmsnorm_row(const uint16_t* x, const uint16_t* res, const uint16_t* w, uint16_t* out, const uint16_t* w2, uint16_t* out2, int rows,
+                        int H, float eps, float eps2, cudaStream_t stream) {
+  const int threads = std::min(512, ceil_div(ceil_div(H, 4), 32) * 32);
+  if (H <= 4 * 512) launch_dependent(rmsnorm_row_kernel<1>, dim3(rows), dim3(threads), 0, stream, x, res, w, out, w2, out2, H, eps, eps2);
+  else launch_dependent(rmsnorm_row_kernel<2>, dim3(rows), dim3(threads), 0, stream, x, res, w, out, w2, out2, H, eps, eps2);
+}
+
+}  // namespace tb200

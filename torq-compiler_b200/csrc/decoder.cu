@@ -17,6 +17,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace tb200 {
@@ -41,9 +42,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   float t = lane < nw ? red[lane] : 0.f;
   return warp_sum(t);
 }
-// One launch helper for every kernel of this file. (Launching them as programmatic dependents of one
-// another - blocks resident early, griddepcontrol.wait before the first memory access - was measured on
-// B200 inside the captured graph of a decode step: 4-6 % slower at batches 8 and 32, so it is not used.)
+// One launch helper for the kernels of this file, which run one after the other.
 template <typename... KArgs, typename... Args>
 void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   kernel<<<grid, block, smem, stream>>>(KArgs(args)...);
@@ -59,11 +58,14 @@ __device__ __forceinline__ float s8_to_float(uint32_t word, int j) {
 __global__ void __launch_bounds__(128) embed_kernel(const int32_t* __restrict__ tok, const int8_t* __restrict__ table,
                                                     const uint16_t* __restrict__ scale, uint16_t* __restrict__ out,
                                                     int H, int V, float mult) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const int b = blockIdx.x;
   int t = tok[b];
   t = t < 0 ? 0 : (t >= V ? V - 1 : t);
-  const float s = bf2f(scale[t]);
   const int8_t* row = table + (size_t)t * H;
+  const float s = bf2f(scale[t]);
+#pragma unroll 4
   for (int i = threadIdx.x; i < H; i += blockDim.x)
     out[(size_t)b * H + i] = f2bf(bf2f(f2bf((float)row[i] * s)) * mult);
 }
@@ -85,74 +87,6 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const uint16_t* __restric
     const float n = bf2f(f2bf(bf2f(x[base + i]) * inv * (1.0f + bf2f(w[i]))));
     out[base + i] = res ? f2bf(bf2f(res[base + i]) + n) : f2bf(n);
   }
-}
-
-// One element of a bf16 [B, N] operand: the tensor itself, or the finalized sum of split-K partials.
-__device__ __forceinline__ float operand_at(const uint16_t* __restrict__ x, const GemvPartials& gp, size_t bn, size_t idx,
-                                            int n) {
-  if (gp.splits == 0) return bf2f(x[idx]);
-  float s = 0.f;
-#pragma unroll 4
-  for (int sp = 0; sp < gp.splits; sp++) s += __ldg(gp.partial + (size_t)sp * bn + idx);
-  return bf2f(f2bf(s * bf2f(__ldg(gp.scale + n))));
-}
-
-// rmsnorm_kernel, its input optionally split-K partials, and optionally a second norm (no residual) of the
-// result in the same launch: out2 = bf16( out * rsqrt(mean(out^2) + eps2) * (1 + w2) ). One block per row,
-// the row kept in shared memory as fp32.
-__global__ void __launch_bounds__(1024) rmsnorm_fused_kernel(const uint16_t* __restrict__ x, GemvPartials gp,
-                                                            const uint16_t* __restrict__ res,
-                                                            const uint16_t* __restrict__ w, uint16_t* __restrict__ out,
-                                                            const uint16_t* __restrict__ w2, uint16_t* __restrict__ out2,
-                                                            int rows, int H, float eps, float eps2) {
-  extern __shared__ float row_s[];
-  __shared__ float red[32];
-  const size_t base = (size_t)blockIdx.x * H;
-  const size_t bn = (size_t)rows * H;
-  float ss = 0.f;
-  if (gp.splits > 0 && H <= 4 * (int)blockDim.x) {
-    // up to four elements per thread: slices outermost, so that 4 x 8 loads are in flight together;
-    // every element still adds its slices in order
-    float a[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* p0 = gp.partial + base + threadIdx.x;
-#pragma unroll 8
-    for (int sp = 0; sp < gp.splits; sp++) {
-#pragma unroll
-      for (int e = 0; e < 4; e++)
-        if ((int)threadIdx.x + e * (int)blockDim.x < H) a[e] += __ldg(p0 + (size_t)sp * bn + e * blockDim.x);
-    }
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const int i = threadIdx.x + e * blockDim.x;
-      if (i < H) {
-        const float v = bf2f(f2bf(a[e] * bf2f(__ldg(gp.scale + i))));
-        row_s[i] = v;
-        ss += v * v;
-      }
-    }
-  } else {
-    for (int i = threadIdx.x; i < H; i += blockDim.x) {
-      const float v = operand_at(x, gp, bn, base + i, i);
-      row_s[i] = v;
-      ss += v * v;
-    }
-  }
-  ss = block_sum(ss, red);
-  const float inv = rsqrtf(ss / (float)H + eps);
-  float ss2 = 0.f;
-  for (int i = threadIdx.x; i < H; i += blockDim.x) {
-    const float n = bf2f(f2bf(row_s[i] * inv * (1.0f + bf2f(w[i]))));
-    const uint16_t o = res ? f2bf(bf2f(res[base + i]) + n) : f2bf(n);
-    out[base + i] = o;
-    const float ov = bf2f(o);
-    row_s[i] = ov;
-    ss2 += ov * ov;
-  }
-  if (!w2) return;
-  __syncthreads();  // red is reused
-  ss2 = block_sum(ss2, red);
-  const float inv2 = rsqrtf(ss2 / (float)H + eps2);
-  for (int i = threadIdx.x; i < H; i += blockDim.x) out2[base + i] = f2bf(row_s[i] * inv2 * (1.0f + bf2f(w2[i])));
 }
 
 // Split-K GEMV / skinny GEMM with int8 weights: one warp per output row n and K slice.
@@ -345,7 +279,7 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const uint16_t* __restrict
                                                       const uint16_t* __restrict__ qw, const uint16_t* __restrict__ kw,
                                                       uint16_t* __restrict__ q_out, uint16_t* __restrict__ kcache,
                                                       uint16_t* __restrict__ vcache, int n_q, int n_kv, int D, int T,
-                                                      float theta, float eps, GemvPartials gp) {
+                                                      float theta, float eps) {
   __shared__ float red[32];
   __shared__ float hv[512];
   const int b = blockIdx.x, h = blockIdx.y;  // h: q heads, then k heads, then v heads
@@ -353,18 +287,17 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const uint16_t* __restrict
   pos = pos < 0 ? 0 : (pos >= T ? T - 1 : pos);
   const int width = (n_q + 2 * n_kv) * D;
   const size_t src = (size_t)b * width + (size_t)h * D;  // element offset of this head in qkv
-  const size_t bn = (size_t)gridDim.x * width;
   const bool is_q = h < n_q, is_k = !is_q && h < n_q + n_kv;
   if (!is_q && !is_k) {  // v head: plain copy into the cache
     const int hk = h - n_q - n_kv;
     uint16_t* dst = vcache + (((size_t)b * T + pos) * n_kv + hk) * D;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) dst[i] = f2bf(operand_at(qkv, gp, bn, src + i, h * D + i));
+    for (int i = threadIdx.x; i < D; i += blockDim.x) dst[i] = qkv[src + i];
     return;
   }
   const uint16_t* w = is_q ? qw : kw;
   float ss = 0.f;
   for (int i = threadIdx.x; i < D; i += blockDim.x) {
-    const float v = operand_at(qkv, gp, bn, src + i, h * D + i);
+    const float v = bf2f(qkv[src + i]);
     hv[i] = v;
     ss += v * v;
   }
@@ -385,134 +318,18 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const uint16_t* __restrict
   }
 }
 
-// Split-T single-query attention (one KV head shared by n_q query heads, D = 256):
-// block = (batch b, T slice), warp w = query head w. Each warp keeps a running (max, sum,
-// acc[D]) over its slice and writes it to scratch; attn_combine_kernel merges the slices.
-constexpr int kAttnD = 256;
-__global__ void __launch_bounds__(128) attn_partial_kernel(const uint16_t* __restrict__ q, const int32_t* __restrict__ pos_p,
-                                                           const uint16_t* __restrict__ kcache,
-                                                           const uint16_t* __restrict__ vcache, float* __restrict__ part,
-                                                           int n_q, int T, int window, float scale) {
-  const int b = blockIdx.x, sp = blockIdx.y, S = gridDim.y;
-  const int h = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (h >= n_q) return;
-  int pos = pos_p[0];
-  pos = pos < 0 ? 0 : (pos >= T ? T - 1 : pos);
-  const int t_lo = window > 0 ? max(0, pos - window + 1) : 0;
-  const int span = pos + 1 - t_lo;
-  const int per = (span + S - 1) / S;
-  const int t0 = t_lo + sp * per, t1 = min(pos + 1, t0 + per);
-  // this lane's 8 dims of the query, pre-scaled
-  float qv[8];
-  {
-    const uint4 qq = *reinterpret_cast<const uint4*>(q + ((size_t)b * n_q + h) * kAttnD + lane * 8);
-    const uint32_t w[4] = {qq.x, qq.y, qq.z, qq.w};
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      qv[2 * j] = __uint_as_float(w[j] << 16) * scale;
-      qv[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u) * scale;
-    }
-  }
-  float m = -INFINITY, l = 0.f, acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) acc[j] = 0.f;
-  // four keys per round: their score reductions interleave and one rescale serves all four
-  // and the next pass's rows are loaded before this pass's arithmetic (registers as the second buffer)
-  uint4 kk[4], vv[4], nk[4], nv[4];
-  auto load_round = [&](int t, uint4 (&kd)[4], uint4 (&vd)[4]) {
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const size_t off = ((size_t)b * T + min(t + u, t1 - 1)) * kAttnD + lane * 8;
-      kd[u] = __ldg(reinterpret_cast<const uint4*>(kcache + off));
-      vd[u] = __ldg(reinterpret_cast<const uint4*>(vcache + off));
-    }
-  };
-  if (t0 < t1) load_round(t0, kk, vv);
-  for (int t = t0; t < t1; t += 4) {
-    if (t + 4 < t1) load_round(t + 4, nk, nv);
-    float s[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t kw[4] = {kk[u].x, kk[u].y, kk[u].z, kk[u].w};
-      float d = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        d = fmaf(qv[2 * j], __uint_as_float(kw[j] << 16), d);
-        d = fmaf(qv[2 * j + 1], __uint_as_float(kw[j] & 0xffff0000u), d);
-      }
-      s[u] = d;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int u = 0; u < 4; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
-#pragma unroll
-    for (int u = 1; u < 4; u++)
-      if (t + u >= t1) s[u] = -INFINITY;  // past the slice: weight 0
-    const float m_new = fmaxf(fmaxf(m, s[0]), fmaxf(fmaxf(s[1], s[2]), s[3]));
-    const float corr = expf(m - m_new);
-    float p[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) p[u] = expf(s[u] - m_new);
-    l = l * corr + ((p[0] + p[1]) + (p[2] + p[3]));
-#pragma unroll
-    for (int j = 0; j < 8; j++) acc[j] *= corr;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t vw[4] = {vv[u].x, vv[u].y, vv[u].z, vv[u].w};
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        acc[2 * j] = fmaf(p[u], __uint_as_float(vw[j] << 16), acc[2 * j]);
-        acc[2 * j + 1] = fmaf(p[u], __uint_as_float(vw[j] & 0xffff0000u), acc[2 * j + 1]);
-      }
-    }
-    m = m_new;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      kk[u] = nk[u];
-      vv[u] = nv[u];
-    }
-  }
-  float* dst = part + (((size_t)b * n_q + h) * S + sp) * (kAttnD + 2);
-  if (lane == 0) {
-    dst[0] = m;
-    dst[1] = l;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; j++) dst[2 + lane * 8 + j] = acc[j];
-}
-
-__global__ void __launch_bounds__(256) attn_combine_kernel(const float* __restrict__ part, uint16_t* __restrict__ out,
-                                                           int S) {
-  const int bh = blockIdx.x, d = threadIdx.x;  // one block per (b, head), one thread per dim
-  const float* p = part + (size_t)bh * S * (kAttnD + 2);
-  float m = -INFINITY;
-  for (int s = 0; s < S; s++) m = fmaxf(m, p[(size_t)s * (kAttnD + 2)]);
-  float l = 0.f, o = 0.f;
-  for (int s = 0; s < S; s++) {
-    const float* ps = p + (size_t)s * (kAttnD + 2);
-    if (ps[1] > 0.f) {
-      const float c = expf(ps[0] - m);
-      l += ps[1] * c;
-      o += ps[2 + d] * c;
-    }
-  }
-  out[(size_t)bh * kAttnD + d] = f2bf(o / l);
-}
-
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
   return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
 }
 // out[b, i] = bf16( bf16(gelu_tanh(gate)) * up ), gate = gu[b, i], up = gu[b, I + i]
 __global__ void __launch_bounds__(256) geglu_kernel(const uint16_t* __restrict__ gu, uint16_t* __restrict__ out, int B,
-                                                    int I, GemvPartials gp) {
+                                                    int I) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)B * I) return;
   const int i = (int)(idx % I);
   const size_t b = idx / I;
-  const size_t bn = (size_t)B * 2 * I;
-  const float g = operand_at(gu, gp, bn, b * 2 * I + i, i), u = operand_at(gu, gp, bn, b * 2 * I + I + i, I + i);
+  const float g = bf2f(gu[b * 2 * I + i]), u = bf2f(gu[b * 2 * I + I + i]);
   out[idx] = f2bf(bf2f(f2bf(gelu_tanh(g))) * u);
 }
 
@@ -721,7 +538,7 @@ __global__ void argmax_final_kernel(const float* __restrict__ pv, const int32_t*
 
 void launch_embed(const int32_t* tok, const int8_t* table, const uint16_t* scale, uint16_t* out, int B, int H, int V,
                   float mult, cudaStream_t stream) {
-  launch_k(embed_kernel, dim3(B), dim3(128), 0, stream, tok, table, scale, out, H, V, mult);
+  launch_dependent(embed_kernel, dim3(B), dim3(128), 0, stream, tok, table, scale, out, H, V, mult);
 }
 
 void launch_rmsnorm(const uint16_t* x, const uint16_t* res, const uint16_t* w, uint16_t* out, int rows, int H, float eps,
@@ -774,19 +591,8 @@ bool gemv_w8_splits_fit(int B, int N, int K, int splits) {
 
 size_t gemv_w8_scratch_bytes(int B, int N, int splits) { return splits > 1 ? (size_t)splits * B * N * sizeof(float) : 0; }
 
-int gemv_w8_used_splits(int B, int N, int K, int splits) {
-  const int slice = gemv_use_mma(B, K) ? gemv_mma_slice(N, K, splits) : ((K + splits - 1) / splits + 511) / 512 * 512;
-  return (K + slice - 1) / slice;
-}
-
-void launch_rmsnorm_fused(const uint16_t* x, GemvPartials gp, const uint16_t* res, const uint16_t* w, uint16_t* out,
-                          const uint16_t* w2, uint16_t* out2, int rows, int H, float eps, float eps2,
-                          cudaStream_t stream) {
-  launch_k(rmsnorm_fused_kernel, dim3(rows), dim3(1024), (size_t)H * sizeof(float), stream, x, gp, res, w, out, w2, out2, rows, H, eps, eps2);
-}
-
 void launch_gemv_w8(const uint16_t* x, const int8_t* W, const uint16_t* scale, void* y, int y_f32, float* scratch, int B,
-                    int N, int K, int splits, cudaStream_t stream, bool finalize) {
+                    int N, int K, int splits, cudaStream_t stream) {
   if (gemv_use_mma(B, K)) {
     const int slice = gemv_mma_slice(N, K, splits);
     const int used = (K + slice - 1) / slice;
@@ -807,7 +613,7 @@ void launch_gemv_w8(const uint16_t* x, const int8_t* W, const uint16_t* scale, v
     else if (nt == 2) run(gemv_w8_mma_kernel<2>);
     else if (nt == 3) run(gemv_w8_mma_kernel<3>);
     else run(gemv_w8_mma_kernel<4>);
-    if (used > 1 && finalize) {
+    if (used > 1) {
       const size_t total = (size_t)B * N;
       launch_k(gemv_finalize_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, scratch, scale, y, B, N, used, y_f32);
     }
@@ -821,7 +627,7 @@ void launch_gemv_w8(const uint16_t* x, const int8_t* W, const uint16_t* scale, v
   else if (B <= 8) launch_k(gemv_w8_kernel<8>, dim3(grid), dim3(256), 0, stream, x, W, scale, y, scratch, B, N, K, slice, y_f32);
   else if (B <= 16) launch_k(gemv_w8_kernel<16>, dim3(grid), dim3(256), 0, stream, x, W, scale, y, scratch, B, N, K, slice, y_f32);
   else launch_k(gemv_w8_kernel<32>, dim3(grid), dim3(256), 0, stream, x, W, scale, y, scratch, B, N, K, slice, y_f32);
-  if (used > 1 && finalize) {
+  if (used > 1) {
     const size_t total = (size_t)B * N;
     launch_k(gemv_finalize_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, scratch, scale, y, B, N, used, y_f32);
   }
@@ -829,30 +635,17 @@ void launch_gemv_w8(const uint16_t* x, const int8_t* W, const uint16_t* scale, v
 
 void launch_rope_kv(const uint16_t* qkv, const int32_t* pos, const uint16_t* qw, const uint16_t* kw, uint16_t* q_out,
                     uint16_t* kcache, uint16_t* vcache, int B, int n_q, int n_kv, int D, int T, float theta, float eps,
-                    cudaStream_t stream, GemvPartials gp) {
-  launch_k(rope_kv_kernel, dim3(dim3(B, n_q + 2 * n_kv)), dim3(128), 0, stream, qkv, pos, qw, kw, q_out, kcache, vcache, n_q, n_kv, D, T,
-                                                              theta, eps, gp);
+                    cudaStream_t stream) {
+  if (D == 256) {
+    launch_rope_heads(qkv, pos, qw, kw, q_out, kcache, vcache, B, n_q, n_kv, T, theta, eps, stream);
+    return;
+  }
+  launch_k(rope_kv_kernel, dim3(B, n_q + 2 * n_kv), dim3(128), 0, stream, qkv, pos, qw, kw, q_out, kcache, vcache, n_q, n_kv, D, T, theta, eps);
 }
 
-int attn_decode_splits(int B) {
-  static int forced = -1;  // TB200_ATTN_SPLITS: T slices of the split-T attention (1..64), else by batch
-  if (forced < 0) { const char* e = getenv("TB200_ATTN_SPLITS"); forced = e && atoi(e) > 0 && atoi(e) <= 64 ? atoi(e) : 0; }
-  if (forced) return forced;
-  return B >= 16 ? 16 : 32;
-}
-size_t attn_decode_scratch_bytes(int B, int n_q, int splits) {
-  return (size_t)B * n_q * splits * (kAttnD + 2) * sizeof(float);
-}
-void launch_attn_decode(const uint16_t* q, const int32_t* pos, const uint16_t* kcache, const uint16_t* vcache,
-                        uint16_t* out, float* scratch, int B, int n_q, int T, int window, float scale, int splits,
-                        cudaStream_t stream) {
-  launch_k(attn_partial_kernel, dim3(dim3(B, splits)), dim3(128), 0, stream, q, pos, kcache, vcache, scratch, n_q, T, window, scale);
-  launch_k(attn_combine_kernel, dim3(B * n_q), dim3(kAttnD), 0, stream, scratch, out, splits);
-}
-
-void launch_geglu(const uint16_t* gu, uint16_t* out, int B, int I, cudaStream_t stream, GemvPartials gp) {
+void launch_geglu(const uint16_t* gu, uint16_t* out, int B, int I, cudaStream_t stream) {
   const size_t total = (size_t)B * I;
-  launch_k(geglu_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, gu, out, B, I, gp);
+  launch_k(geglu_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, gu, out, B, I);
 }
 
 void launch_gemv_q8b(const uint16_t* x, const int8_t* W, const uint16_t* scale, const int8_t* zp, uint16_t* y, int B, int N,
@@ -939,7 +732,8 @@ extern "C" int tb200_gemv_w8_noalloc(int cuda_ordinal, void* stream, const void*
     fprintf(stderr, "tb200_gemv_w8_noalloc: x and W must be 16-byte aligned, y and the scales aligned to their element\n");
     return 3;
   }
-  if (splits <= 0) splits = gemv_w8_splits(B, N, K);
+  const bool own_choice = splits <= 0;
+  if (own_choice) splits = gemv_w8_splits(B, N, K);
   if (!gemv_w8_splits_fit(B, N, K, splits)) {
     fprintf(stderr,
             "tb200_gemv_w8_noalloc: %d slices of K = %d leave a slice of the input too long for the tensor-core kernel's "
@@ -974,6 +768,12 @@ extern "C" int tb200_gemv_w8_noalloc(int cuda_ordinal, void* stream, const void*
     scratch = g_noalloc_scratch_ptr[cuda_ordinal];
   }
   (void)cudaGetLastError();  // an earlier, unrelated error of the host must not be reported as this call's
+  if (own_choice && linear_w8_applies(B, N, K)) {  // as an executable's gemv_w8: no partial sums in memory at all
+    LinearArgs a{};
+    a.x = (const uint16_t*)x_bf16; a.W = (const int8_t*)w_i8; a.scale = (const uint16_t*)scale_bf16;
+    a.y = y; a.y_f32 = y_is_f32 ? 1 : 0; a.B = B; a.N = N; a.K = K; a.serial = 1;
+    return launch_linear(a, (cudaStream_t)stream) == cudaSuccess ? 0 : 13;
+  }
   launch_gemv_w8((const uint16_t*)x_bf16, (const int8_t*)w_i8, (const uint16_t*)scale_bf16, y, y_is_f32 ? 1 : 0, scratch,
                  B, N, K, splits, (cudaStream_t)stream);
   return cudaGetLastError() == cudaSuccess ? 0 : 13;

@@ -250,40 +250,59 @@ int gemv_w8_splits(int B, int N, int K);
 size_t gemv_w8_scratch_bytes(int B, int N, int splits);
 // false when a caller-chosen slice count leaves K slices the tensor-core kernel cannot stage in shared memory
 bool gemv_w8_splits_fit(int B, int N, int K, int splits);
-// y bf16, or fp32 when y_f32. finalize == false with more than one K slice in use leaves the per-slice
-// sums in scratch ([slice][B][N] fp32) for a consumer kernel that takes a GemvPartials.
+// y bf16, or fp32 when y_f32
 void launch_gemv_w8(const uint16_t* x, const int8_t* W, const uint16_t* scale, void* y, int y_f32, float* scratch, int B,
-                    int N, int K, int splits, cudaStream_t stream, bool finalize = true);
-int gemv_w8_used_splits(int B, int N, int K, int splits);  // K slices that launch_gemv_w8 really launches
-// A bf16 [B, N] operand that is still the per-slice partial sums of a split-K product: the consumer adds
-// the slices in order, applies the row scale and rounds to bf16, exactly as the finalize kernel would.
-// splits == 0: the operand is an ordinary bf16 tensor.
-struct GemvPartials {
-  const float* partial;
-  const uint16_t* scale;
-  int splits;
-};
-// First norm as launch_rmsnorm (x may be partial sums); with w2 a second norm without residual of the
-// first result goes to out2 in the same launch. H * 4 bytes of shared memory: H <= 8192.
-void launch_rmsnorm_fused(const uint16_t* x, GemvPartials gp, const uint16_t* res, const uint16_t* w, uint16_t* out,
-                          const uint16_t* w2, uint16_t* out2, int rows, int H, float eps, float eps2,
-                          cudaStream_t stream);
+                    int N, int K, int splits, cudaStream_t stream);
 void launch_rope_kv(const uint16_t* qkv, const int32_t* pos, const uint16_t* qw, const uint16_t* kw, uint16_t* q_out,
                     uint16_t* kcache, uint16_t* vcache, int B, int n_q, int n_kv, int D, int T, float theta, float eps,
-                    cudaStream_t stream, GemvPartials gp = GemvPartials{nullptr, nullptr, 0});
-int attn_decode_splits(int B);
-size_t attn_decode_scratch_bytes(int B, int n_q, int splits);
-void launch_attn_decode(const uint16_t* q, const int32_t* pos, const uint16_t* kcache, const uint16_t* vcache,
-                        uint16_t* out, float* scratch, int B, int n_q, int T, int window, float scale, int splits,
-                        cudaStream_t stream);
-void launch_geglu(const uint16_t* gu, uint16_t* out, int B, int I, cudaStream_t stream,
-                  GemvPartials gp = GemvPartials{nullptr, nullptr, 0});
+                    cudaStream_t stream);
+void launch_geglu(const uint16_t* gu, uint16_t* out, int B, int I, cudaStream_t stream);
 // block-quantised GEMV: W [N, K] int8, scale bf16 and zp int8 (or null) [N, K / bs], bs a multiple of 16, batch <= 8
 void launch_gemv_q8b(const uint16_t* x, const int8_t* W, const uint16_t* scale, const int8_t* zp, uint16_t* y, int B, int N,
                      int K, int bs, cudaStream_t stream);
 void launch_act_bf16(const uint16_t* x, uint16_t* out, long long n, int fn, cudaStream_t stream);  // fn: see TB200_OP_ACT_BF16
 size_t argmax_scratch_bytes(int B);
 void launch_argmax(const void* logits, int is_f32, int32_t* out, void* scratch, int B, int V, cudaStream_t stream);
+
+// ---- products, attention and norms of a decode step run op by op (decode_linear.cu) ----
+struct LinearArgs {
+  const uint16_t* x;      // bf16 [B, K], B <= 32
+  const int8_t* W;        // [N, K], K % 64 == 0
+  const uint16_t* scale;  // bf16 [N]
+  void* y;                // bf16 or fp32 [B, N] (geglu: bf16 [B, N / 2])
+  int y_f32, B, N, K;
+  int serial;             // W may still be being written: start only when everything before has finished
+  // head norm + RoPE + cache append behind the product (launch_linear_rope)
+  const int32_t* pos;
+  const uint16_t* qw;
+  const uint16_t* kw;
+  uint16_t* q_out;
+  uint16_t* kcache;
+  uint16_t* vcache;
+  int n_q, T;
+  float theta, eps;
+  // filled by the launcher
+  float* cand_v;
+  int32_t* cand_i;
+  int kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, tiles;
+};
+bool linear_w8_applies(int B, int N, int K);
+bool linear_geglu_applies(int B, int N, int K);
+bool linear_rope_applies(int B, int N, int K, int n_q, int n_kv, int D);
+size_t linear_argmax_scratch(int B, int N, int K);  // 0 = the arg max does not ride along
+cudaError_t launch_linear(const LinearArgs& a, cudaStream_t stream);
+cudaError_t launch_linear_geglu(const LinearArgs& a, cudaStream_t stream);
+cudaError_t launch_linear_rope(const LinearArgs& a, cudaStream_t stream);
+cudaError_t launch_linear_argmax(LinearArgs a, void* scratch, int32_t* out, cudaStream_t stream);  // fp32 or bf16 logits to y as well
+void launch_rope_heads(const uint16_t* qkv, const int32_t* pos, const uint16_t* qw, const uint16_t* kw, uint16_t* q_out, uint16_t* kcache,
+                       uint16_t* vcache, int B, int n_q, int n_kv, int T, float theta, float eps, cudaStream_t stream);  // head size 256
+// one KV head of 256, up to 4 query heads
+void launch_attn_decode(const uint16_t* q, const int32_t* pos, const uint16_t* kcache, const uint16_t* vcache, uint16_t* out, int B, int n_q,
+                        int T, int window, float scale, cudaStream_t stream);
+bool rmsnorm_row_applies(int H);
+// rmsnorm; with w2 a second norm without residual of its result goes to out2
+void launch_rmsnorm_row(const uint16_t* x, const uint16_t* res, const uint16_t* w, uint16_t* out, const uint16_t* w2, uint16_t* out2, int rows,
+                        int H, float eps, float eps2, cudaStream_t stream);
 
 // ---- whole decode step as one persistent kernel (decode_step.cu) ----
 // Byte offsets: weights and norm vectors into the constant image, caches into the arena.

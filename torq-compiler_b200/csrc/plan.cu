@@ -585,11 +585,11 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   std::vector<int> add_after(ops.size(), -1);      // conv op -> index of the add fused into its epilogue
   std::vector<char> add_self_is_a(ops.size(), 0);  // the convolution's result is the add's first operand
   std::vector<char> add_fits_small(ops.size(), 0); // the fused add runs in the small-problem kernel
-  // Decoder graphs run op by op: (1) a split-K gemv_w8 whose only reader is the next op (rmsnorm, rope_kv or
-  // geglu) leaves its per-slice sums in scratch and the reader finalizes them as it loads; (2) an rmsnorm
-  // directly followed by an rmsnorm of its result runs as one launch. Same arithmetic, fewer launches.
-  std::vector<int> partials_from(ops.size(), -1);  // reader op -> the gemv_w8 op whose partial sums it takes
-  std::vector<char> defer_finalize(ops.size(), 0);
+  // Decoder graphs run op by op: (1) geglu, rope_kv and argmax run in the epilogue of the gemv_w8 right in front of them when they
+  // are its only reader (decode_linear.cu) - the reader's step launches both; (2) an rmsnorm directly followed by an rmsnorm of
+  // its result runs as one launch. Same arithmetic in the same order, fewer launches.
+  std::vector<int> gemv_before(ops.size(), -1);    // reader op -> the gemv_w8 op that runs in its step
+  std::vector<char> gemv_deferred(ops.size(), 0);
   std::vector<int> norm_second(ops.size(), -1);    // rmsnorm op -> the rmsnorm op fused into it
   std::vector<int> extra_out(ops.size(), -1);      // tensor an op writes on behalf of the op fused into it
   std::vector<int> extra_in(ops.size(), -1);       // tensor an op reads on behalf of the op fused into it
@@ -743,22 +743,21 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       auto ok2d = [&](int id, int dtype) {
         return id >= 0 && id < nt && tensors[id].rank == 2 && tensors[id].dtype == dtype;
       };
-      if (op.kind == TB200_OP_GEMV_W8 && ok2d(op.in0, TB200_BF16) && ok2d(op.out0, TB200_BF16) && ok2d(op.weights, TB200_I8) &&
-          tensors[op.out0].kind == TB200_TENSOR_ACTIVATION && uses[op.out0] == 1 && nx.in0 == op.out0 && op.i1 == 0 &&
-          (nx.kind == TB200_OP_RMSNORM || nx.kind == TB200_OP_ROPE_KV || nx.kind == TB200_OP_GEGLU)) {
+      if (op.kind == TB200_OP_GEMV_W8 && ok2d(op.in0, TB200_BF16) && ok2d(op.weights, TB200_I8) && op.i0 <= 0 && op.i1 == 0 && nx.in0 == op.out0) {
         const int B = tensors[op.in0].shape[0], N = tensors[op.weights].shape[0], K = tensors[op.weights].shape[1];
-        const bool plain = K == tensors[op.in0].shape[1] && K > 0 && K % 16 == 0 && B >= 1 && B <= 32 && N >= 1;
-        if (plain && !(nx.kind == TB200_OP_RMSNORM && N > 8192)) {
-          const int splits = op.i0 > 0 ? op.i0 : gemv_w8_splits(B, N, K);
-          if (gemv_w8_used_splits(B, N, K, splits) > 1) {
-            defer_finalize[i] = 1;
-            partials_from[i + 1] = i;
-          }
+        const bool own = ok2d(op.out0, TB200_BF16) && tensors[op.out0].kind == TB200_TENSOR_ACTIVATION && uses[op.out0] == 1;
+        const bool plain = K == tensors[op.in0].shape[1] && K > 0 && B >= 1 && B <= 32 && N >= 1;
+        if (plain && ((nx.kind == TB200_OP_GEGLU && own && linear_geglu_applies(B, N, K)) ||
+                      (nx.kind == TB200_OP_ROPE_KV && own && linear_rope_applies(B, N, K, nx.i0, nx.i1, nx.i2)) ||
+                      (nx.kind == TB200_OP_ARGMAX && nx.i1 <= 1 && ok2d(op.out0, TB200_F32) && linear_argmax_scratch(B, N, K) > 0))) {
+          gemv_deferred[i] = 1;
+          gemv_before[i + 1] = i;
+          extra_in[i + 1] = op.in0;
         }
       }
       if (op.kind == TB200_OP_RMSNORM && nx.kind == TB200_OP_RMSNORM && !fused_away[i] && nx.in0 == op.out0 && nx.in1 < 0 &&
           ok2d(op.in0, TB200_BF16) && ok2d(op.out0, TB200_BF16) && ok2d(nx.out0, TB200_BF16) && nx.out0 != op.out0 &&
-          tensors[op.in0].shape[1] <= 8192 && tensors[nx.out0].shape[0] == tensors[op.out0].shape[0] &&
+          rmsnorm_row_applies(tensors[op.in0].shape[1]) && tensors[nx.out0].shape[0] == tensors[op.out0].shape[0] &&
           tensors[nx.out0].shape[1] == tensors[op.out0].shape[1] && tensors[op.out0].shape[1] == tensors[op.in0].shape[1] &&
           tensors[op.out0].shape[0] == tensors[op.in0].shape[0]) {
         norm_second[i] = i + 1;
@@ -856,12 +855,18 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   }
 
   size_t scratch_need = 0;
-  struct DeferredGemv { size_t scale_off; int splits; };
-  std::vector<DeferredGemv> deferred(ops.size(), DeferredGemv{0, 0});
-  // the operand a reader of deferred partial sums passes to its kernel
-  auto partials_of = [&](int reader) {
-    const int src = partials_from[reader];
-    return src >= 0 ? deferred[src] : DeferredGemv{0, 0};
+  struct LinearStep { Loc x; size_t w_off, s_off; int B, N, K; };
+  std::vector<LinearStep> linear(ops.size(), LinearStep{});  // deferred gemv_w8 ops
+  auto linear_args = [](const LinearStep& l, const ExecContext& c) {
+    LinearArgs k{};
+    k.x = (const uint16_t*)l.x.resolve(c);
+    k.W = (const int8_t*)(c.consts + l.w_off);
+    k.scale = (const uint16_t*)(c.consts + l.s_off);
+    k.B = l.B; k.N = l.N; k.K = l.K;
+    return k;
+  };
+  auto report = [](cudaError_t e, const ExecContext& c) {
+    if (e != cudaSuccess && c.launch_error) *c.launch_error = e;
   };
   bool needs_fusion = false;  // the graph holds ops that exist only inside the fused decode step
   // ---- one step per op ----
@@ -1723,9 +1728,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         Loc lx = loc(op.in0), lr = loc(op.in1), lo = loc(op.out0);
         const float eps = op.f0;
         const bool has_res = op.in1 >= 0;
-        const DeferredGemv dg = partials_of(i);
         const int second = norm_second[i];
-        if (dg.splits > 0 || second >= 0) {
+        if (rmsnorm_row_applies(H)) {
           size_t w2_off = 0;
           Loc lo2{};
           float eps2 = 0.f;
@@ -1734,15 +1738,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             lo2 = loc(ops[second].out0);
             eps2 = ops[second].f0;
           }
-          step.kernel_name = second >= 0 ? (dg.splits > 0 ? "rmsnorm_pair_from_partials" : "rmsnorm_pair")
-                                         : "rmsnorm_from_partials";
+          step.kernel_name = second >= 0 ? "rmsnorm_pair" : "rmsnorm";
           step.launch = [=](const ExecContext& c) {
-            const GemvPartials gp{dg.splits > 0 ? (const float*)c.scratch : nullptr,
-                                  dg.splits > 0 ? (const uint16_t*)(c.consts + dg.scale_off) : nullptr, dg.splits};
-            launch_rmsnorm_fused((const uint16_t*)lx.resolve(c), gp, has_res ? (const uint16_t*)lr.resolve(c) : nullptr,
-                                 (const uint16_t*)(c.consts + w_off), (uint16_t*)lo.resolve(c),
-                                 second >= 0 ? (const uint16_t*)(c.consts + w2_off) : nullptr,
-                                 second >= 0 ? (uint16_t*)lo2.resolve(c) : nullptr, rows, H, eps, eps2, c.stream);
+            launch_rmsnorm_row((const uint16_t*)lx.resolve(c), has_res ? (const uint16_t*)lr.resolve(c) : nullptr,
+                               (const uint16_t*)(c.consts + w_off), (uint16_t*)lo.resolve(c),
+                               second >= 0 ? (const uint16_t*)(c.consts + w2_off) : nullptr,
+                               second >= 0 ? (uint16_t*)lo2.resolve(c) : nullptr, rows, H, eps, eps2, c.stream);
           };
           break;
         }
@@ -1769,19 +1770,36 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         size_t w_off, s_off;
         if (!b.add_raw_const(op.weights, (size_t)N * K, "weights", i, w_off)) return b.status;
         if (!b.add_raw_const(op.bias, (size_t)N * 2, "scales", i, s_off)) return b.status;
+        if (op.i0 <= 0 && op.i1 == 0 && K == tensors[op.in0].shape[1] && linear_w8_applies(B, N, K)) {
+          const LinearStep l{loc(op.in0), w_off, s_off, B, N, K};
+          if (gemv_deferred[i]) {
+            linear[i] = l;
+            step.kernel_name = "gemv_w8_splitk_partials";
+            step.launches = 0;
+            step.launch = [](const ExecContext&) {};
+            break;
+          }
+          const Loc ly = loc(op.out0);
+          step.kernel_name = "gemv_w8";
+          step.launch = [=](const ExecContext& c) {
+            LinearArgs k = linear_args(l, c);
+            k.y = ly.resolve(c);
+            k.y_f32 = y_f32;
+            report(launch_linear(k, c.stream), c);
+          };
+          break;
+        }
         const int splits = op.i0 > 0 ? op.i0 : gemv_w8_splits(B, N, K);
         if (!gemv_w8_splits_fit(B, N, K, splits))
           return b.fail(TB200_OUT_OF_RANGE, "op %d: %d K slices leave a slice longer than the tensor-core gemv_w8 can stage", i, splits);
         scratch_need = std::max(scratch_need, gemv_w8_scratch_bytes(B, N, splits));
         Loc lx = loc(op.in0), lo = loc(op.out0);
-        const bool finalize = !defer_finalize[i];
-        if (!finalize) deferred[i] = DeferredGemv{s_off, gemv_w8_used_splits(B, N, K, splits)};
-        step.kernel_name = !finalize ? "gemv_w8_splitk_partials" : splits > 1 ? "gemv_w8_splitk" : "gemv_w8";
-        step.launches = splits > 1 && finalize ? 2 : 1;
+        step.kernel_name = splits > 1 ? "gemv_w8_splitk" : "gemv_w8";
+        step.launches = splits > 1 ? 2 : 1;
         step.launch = [=](const ExecContext& c) {
           launch_gemv_w8((const uint16_t*)lx.resolve(c), (const int8_t*)(c.consts + w_off),
                          (const uint16_t*)(c.consts + s_off), lo.resolve(c), y_f32, (float*)c.scratch, B, N, K, splits,
-                         c.stream, finalize);
+                         c.stream);
         };
         break;
       }
@@ -1802,14 +1820,27 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (!b.add_raw_const(op.bias, (size_t)D * 2, "k_norm weight", i, kw_off)) return b.status;
         Loc lx = loc(op.in0), lp = loc(op.in1), lq = loc(op.out0), lk = loc(op.out1), lv = loc(op.in2);
         const float theta = op.f0, eps = op.f1;
-        const DeferredGemv dg = partials_of(i);
-        step.kernel_name = dg.splits > 0 ? "rope_kv_from_partials" : "rope_kv";
+        if (gemv_before[i] >= 0) {
+          const LinearStep l = linear[gemv_before[i]];
+          step.kernel_name = "rope_kv_from_partials";
+          step.launch = [=](const ExecContext& c) {
+            LinearArgs k = linear_args(l, c);
+            k.pos = (const int32_t*)lp.resolve(c);
+            k.qw = (const uint16_t*)(c.consts + qw_off);
+            k.kw = (const uint16_t*)(c.consts + kw_off);
+            k.q_out = (uint16_t*)lq.resolve(c);
+            k.kcache = (uint16_t*)lk.resolve(c);
+            k.vcache = (uint16_t*)lv.resolve(c);
+            k.n_q = n_q; k.T = T; k.theta = theta; k.eps = eps;
+            report(launch_linear_rope(k, c.stream), c);
+          };
+          break;
+        }
+        step.kernel_name = "rope_kv";
         step.launch = [=](const ExecContext& c) {
-          const GemvPartials gp{dg.splits > 0 ? (const float*)c.scratch : nullptr,
-                                dg.splits > 0 ? (const uint16_t*)(c.consts + dg.scale_off) : nullptr, dg.splits};
           launch_rope_kv((const uint16_t*)lx.resolve(c), (const int32_t*)lp.resolve(c), (const uint16_t*)(c.consts + qw_off),
                          (const uint16_t*)(c.consts + kw_off), (uint16_t*)lq.resolve(c), (uint16_t*)lk.resolve(c),
-                         (uint16_t*)lv.resolve(c), B, n_q, n_kv, D, T, theta, eps, c.stream, gp);
+                         (uint16_t*)lv.resolve(c), B, n_q, n_kv, D, T, theta, eps, c.stream);
         };
         break;
       }
@@ -1825,16 +1856,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (tensors[op.in0].shape[1] != n_q * D || b.numel(op.out0) != (size_t)B * n_q * D ||
             tensors[op.in2].shape[0] != B || tensors[op.in2].shape[2] != D || b.numel(op.weights) != b.numel(op.in2))
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: attn_decode shape mismatch", i);
-        const int splits = attn_decode_splits(B);
-        scratch_need = std::max(scratch_need, attn_decode_scratch_bytes(B, n_q, splits));
         Loc lq = loc(op.in0), lp = loc(op.in1), lk = loc(op.in2), lv = plan.tensor_loc[op.weights], lo = loc(op.out0);
         const float scale = op.f0;
         step.kernel_name = "attn_decode_splitT";
-        step.launches = 2;
         step.launch = [=](const ExecContext& c) {
           launch_attn_decode((const uint16_t*)lq.resolve(c), (const int32_t*)lp.resolve(c), (const uint16_t*)lk.resolve(c),
-                             (const uint16_t*)lv.resolve(c), (uint16_t*)lo.resolve(c), (float*)c.scratch, B, n_q, T, window,
-                             scale, splits, c.stream);
+                             (const uint16_t*)lv.resolve(c), (uint16_t*)lo.resolve(c), B, n_q, T, window, scale, c.stream);
         };
         break;
       }
@@ -1844,12 +1871,19 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: geglu wants bf16 [B,2I] -> bf16 [B,I]", i);
         const int B = tensors[op.out0].shape[0], I = tensors[op.out0].shape[1];
         Loc lx = loc(op.in0), lo = loc(op.out0);
-        const DeferredGemv dg = partials_of(i);
-        step.kernel_name = dg.splits > 0 ? "geglu_from_partials" : "geglu";
+        if (gemv_before[i] >= 0) {
+          const LinearStep l = linear[gemv_before[i]];
+          step.kernel_name = "geglu_from_partials";
+          step.launch = [=](const ExecContext& c) {
+            LinearArgs k = linear_args(l, c);
+            k.y = lo.resolve(c);
+            report(launch_linear_geglu(k, c.stream), c);
+          };
+          break;
+        }
+        step.kernel_name = "geglu";
         step.launch = [=](const ExecContext& c) {
-          const GemvPartials gp{dg.splits > 0 ? (const float*)c.scratch : nullptr,
-                                dg.splits > 0 ? (const uint16_t*)(c.consts + dg.scale_off) : nullptr, dg.splits};
-          launch_geglu((const uint16_t*)lx.resolve(c), (uint16_t*)lo.resolve(c), B, I, c.stream, gp);
+          launch_geglu((const uint16_t*)lx.resolve(c), (uint16_t*)lo.resolve(c), B, I, c.stream);
         };
         break;
       }
@@ -1864,6 +1898,17 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         Loc lx = loc(op.in0), lo = loc(op.out0);
         step.kernel_name = "argmax";
         step.launches = 2;
+        if (gemv_before[i] >= 0) {  // the product leaves candidates of every block behind its logits
+          const LinearStep l = linear[gemv_before[i]];
+          scratch_need = std::max(scratch_need, linear_argmax_scratch(l.B, l.N, l.K));
+          step.launch = [=](const ExecContext& c) {
+            LinearArgs k = linear_args(l, c);
+            k.y = lx.resolve(c);
+            k.y_f32 = 1;
+            report(launch_linear_argmax(k, c.scratch, (int32_t*)lo.resolve(c), c.stream), c);
+          };
+          break;
+        }
         step.launch = [=](const ExecContext& c) {
           launch_argmax(lx.resolve(c), is_f32, (int32_t*)lo.resolve(c), c.scratch, B, V, c.stream);
         };
