@@ -76,12 +76,32 @@ __device__ __forceinline__ uint32_t load_bytes(const int8_t* p, int n) {
   return w;
 }
 
+// 16 bytes from byte offset off of x (4-byte aligned, total bytes); bytes past the end are undefined
+__device__ __forceinline__ uint4 load16_any(const int8_t* x, int off, int total) {
+  const int w0 = off & ~3;
+  const uint32_t sh = (uint32_t)(off & 3) * 8;
+  uint32_t w[5];
+#pragma unroll
+  for (int i = 0; i < 5; i++) {
+    w[i] = 0;
+    const int at = w0 + 4 * i;
+    if (at + 4 <= total) {
+      w[i] = *reinterpret_cast<const uint32_t*>(x + at);
+    } else {
+      for (int j = 0; at + j < total; j++) w[i] |= (uint32_t)(uint8_t)x[at + j] << (8 * j);
+    }
+  }
+  return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
+}
+
 // MODE: what a row of the product is - kRows: lda bytes of memory; kConv: the taps of an output pixel, IC a multiple of 16;
 // kStem: the 27 bytes under a 3 x 3 window of 3 channels, one k32 instruction: lane t = 0 .. 2 holds the first eight of the nine
 // bytes of kernel row t (consecutive in memory), lane 3 the three ninth bytes.
 // U = K steps whose loads are in flight together; SPLIT: several warps share a tile.
 enum { kRows = 0, kConv = 1, kStem = 2 };
-template <int MODE, int U, bool SPLIT>
+// RAGGED: rows or channels that are no multiple of 16 bytes - the 16 bytes of a chunk come from five aligned words and may run on
+// into the next pixel's, whose weights here are zero.
+template <int MODE, int U, bool SPLIT, bool RAGGED>
 __global__ void __launch_bounds__(SPLIT ? 256 : 128, SPLIT ? 2 : 4) conv_small_kernel(const ConvSmallArgs a) {
   extern __shared__ int sums[];  // [tiles of the block][warps of a tile][16][kSumPitch], only with more than one warp per tile
   __shared__ int8_t lut[256];
@@ -159,13 +179,13 @@ __global__ void __launch_bounds__(SPLIT ? 256 : 128, SPLIT ? 2 : 4) conv_small_k
       for (int r = 0; r < 2; r++) {
         v[r] = make_uint4(fill, fill, fill, fill);
         if (in_k && row_ok[r] && (unsigned)(ih0[r] + kh) < (unsigned)a.H && (unsigned)(iw0[r] + kw) < (unsigned)a.W)
-          v[r] = *reinterpret_cast<const uint4*>(a.x + (px[r] + off));
+          v[r] = RAGGED ? load16_any(a.x, px[r] + off, a.x_bytes) : *reinterpret_cast<const uint4*>(a.x + (px[r] + off));
       }
     } else {
 #pragma unroll
       for (int r = 0; r < 2; r++) {
         v[r] = make_uint4(0, 0, 0, 0);
-        if (in_k && row_ok[r]) v[r] = *reinterpret_cast<const uint4*>(a.x + (px[r] + c * 16));
+        if (in_k && row_ok[r]) v[r] = RAGGED ? load16_any(a.x, px[r] + c * 16, a.x_bytes) : *reinterpret_cast<const uint4*>(a.x + (px[r] + c * 16));
       }
     }
   };
@@ -279,7 +299,7 @@ int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace
 
-int conv_small_steps(int taps, int IC) { return ceil_div((long long)taps * (IC / 16), kStepBytes / 16); }
+int conv_small_steps(int taps, int IC) { return ceil_div((long long)taps * ceil_div(IC, 16), kStepBytes / 16); }
 int conv_small_columns(int OC) { return ceil_div(OC, kTileN) * kTileN; }
 
 // The line to the tcgen05 kernel. A warp's tile costs about (steps + 5) * 0.18 ns of the whole chip beyond the 2 us that
@@ -289,13 +309,15 @@ int conv_small_columns(int OC) { return ceil_div(OC, kTileN) * kTileN; }
 constexpr long long kSmallCost = 29000;
 
 bool conv_small_applies(long long M, int OC, int taps, int IC) {
-  if (small_kernels_off() || IC % 16 != 0 || taps < 1 || taps > 64 || (long long)taps * (IC / 16) > 4096) return false;
+  if (small_kernels_off() || IC < 1 || taps < 1 || taps > 64 || (long long)taps * ceil_div(IC, 16) > 4096) return false;
   const long long tiles = (long long)ceil_div(M, kTileM) * ceil_div(OC, kTileN);
-  return tiles * (conv_small_steps(taps, IC) + 5) <= kSmallCost && M * IC < (1ll << 30);
+  // unaligned rows take five loads for one: worth it up to half of that (3x3 28x28 x 100 -> 77, cost 12 k, 8.8 us against 12.9
+  // padded; FullyConnected 500 x 1001 -> 1003, 21 k, 19.4 us against about 11)
+  return tiles * (conv_small_steps(taps, IC) + 5) <= (IC % 16 ? kSmallCost / 2 : kSmallCost) && M * IC < (1ll << 30);
 }
 
 void conv_small_pack(const int8_t* w, int OC, int taps, int IC, int8_t* out) {
-  const int steps = conv_small_steps(taps, IC), n_tiles = ceil_div(OC, kTileN), chunks = taps * (IC / 16);
+  const int steps = conv_small_steps(taps, IC), n_tiles = ceil_div(OC, kTileN), icb = ceil_div(IC, 16), chunks = taps * icb;
   const long long K = (long long)taps * IC;
   for (int nt = 0; nt < n_tiles; nt++)
     for (int s = 0; s < steps; s++)
@@ -304,8 +326,10 @@ void conv_small_pack(const int8_t* w, int OC, int taps, int IC, int8_t* out) {
           const int f = lane >> 2, c = 4 * s + (lane & 3);
           const int oc = nt * kTileN + 8 * (f >> 1) + 2 * j + (f & 1);
           int8_t* o = out + ((((size_t)nt * steps + s) * 4 + j) * 32 + lane) * 16;
-          if (oc < OC && c < chunks) memcpy(o, w + (size_t)oc * K + (size_t)c * 16, 16);
-          else memset(o, 0, 16);
+          memset(o, 0, 16);
+          if (oc >= OC || c >= chunks) continue;
+          const int tap = c / icb, ic = (c - tap * icb) * 16;
+          memcpy(o, w + (size_t)oc * K + (size_t)tap * IC + ic, (size_t)(IC - ic < 16 ? IC - ic : 16));
         }
 }
 
@@ -327,7 +351,7 @@ cudaError_t launch_conv_small(const ConvSmallArgs& args, cudaStream_t stream) {
   a.m_tiles = ceil_div(a.M, kTileM);
   a.n_tiles = ceil_div(a.N, kTileN);
   a.steps = a.mode == kStem ? 1 : conv_small_steps(taps, a.IC);
-  a.icb = a.mode == kStem ? 1 : a.IC / 16;
+  a.icb = a.mode == kStem ? 1 : ceil_div(a.IC, 16);
   a.chunks = taps * a.icb;
   a.inv_icb = ((1 << 20) + a.icb - 1) / a.icb;
   a.inv_kw = ((1 << 20) + a.KW - 1) / a.KW;
@@ -346,12 +370,13 @@ cudaError_t launch_conv_small(const ConvSmallArgs& args, cudaStream_t stream) {
   const size_t smem = ks_n > 1 ? (size_t)warps * kTileM * kSumPitch * 4 : 0;
   const int u = per_warp < 3 ? per_warp : 3;  // more than three steps in flight do not fit 128 registers
   using Kernel = void (*)(ConvSmallArgs);
-  static const Kernel kernels[2][2][3] = {
-      {{conv_small_kernel<kRows, 1, false>, conv_small_kernel<kRows, 2, false>, conv_small_kernel<kRows, 3, false>},
-       {conv_small_kernel<kRows, 1, true>, conv_small_kernel<kRows, 2, true>, conv_small_kernel<kRows, 3, true>}},
-      {{conv_small_kernel<kConv, 1, false>, conv_small_kernel<kConv, 2, false>, conv_small_kernel<kConv, 3, false>},
-       {conv_small_kernel<kConv, 1, true>, conv_small_kernel<kConv, 2, true>, conv_small_kernel<kConv, 3, true>}}};
-  const Kernel kernel = a.mode == kStem ? conv_small_kernel<kStem, 1, false> : kernels[a.mode == kConv][ks_n > 1][u - 1];
+  static const Kernel kernels[2][2][2][3] = {  // [ragged][convolution][split][U - 1]
+      {{{conv_small_kernel<kRows, 1, false, false>, conv_small_kernel<kRows, 2, false, false>, conv_small_kernel<kRows, 3, false, false>}, {conv_small_kernel<kRows, 1, true, false>, conv_small_kernel<kRows, 2, true, false>, conv_small_kernel<kRows, 3, true, false>}},
+       {{conv_small_kernel<kConv, 1, false, false>, conv_small_kernel<kConv, 2, false, false>, conv_small_kernel<kConv, 3, false, false>}, {conv_small_kernel<kConv, 1, true, false>, conv_small_kernel<kConv, 2, true, false>, conv_small_kernel<kConv, 3, true, false>}}},
+      {{{conv_small_kernel<kRows, 1, false, true>, conv_small_kernel<kRows, 2, false, true>, conv_small_kernel<kRows, 3, false, true>}, {conv_small_kernel<kRows, 1, true, true>, conv_small_kernel<kRows, 2, true, true>, conv_small_kernel<kRows, 3, true, true>}},
+       {{conv_small_kernel<kConv, 1, false, true>, conv_small_kernel<kConv, 2, false, true>, conv_small_kernel<kConv, 3, false, true>}, {conv_small_kernel<kConv, 1, true, true>, conv_small_kernel<kConv, 2, true, true>, conv_small_kernel<kConv, 3, true, true>}}}};
+  const bool ragged = a.IC % 16 != 0;
+  const Kernel kernel = a.mode == kStem ? conv_small_kernel<kStem, 1, false, false> : kernels[ragged][a.mode == kConv][ks_n > 1][u - 1];
   return launch_dependent_if(true, kernel, grid, block, smem, stream, a);
 }
 

@@ -213,6 +213,10 @@ struct ConvTcArgs {
 };
 cudaError_t launch_conv_i8_tc(const ConvTcArgs& a, GemmTcState* st, cudaStream_t stream);
 
+// ---- rows that are no multiple of 16 bytes (ragged_rows.cu): x 4-byte, padded and trimmed buffers 16-byte aligned ----
+void launch_pad_rows(const int8_t* x, int8_t* out, long long rows, int K, int pitch, cudaStream_t stream);
+void launch_trim_rows(const int8_t* x, int8_t* out, long long rows, int N, int pitch, cudaStream_t stream);
+
 // ---- small convolutions and products (conv_small.cu) ----
 struct ConvSmallArgs {
   const int8_t* x;        // [N, H, W, IC], or rows of lda bytes
@@ -224,8 +228,8 @@ struct ConvSmallArgs {
   const int8_t* lut;      // 256-entry table applied to the int8 result, or null
   long long ldc;
   int lda, M, N;          // rows (pixels) and output channels
-  int mode;               // 0 = rows, 1 = convolution with IC % 16 == 0, 2 = 3 x 3 over 3 channels
-  int x_bytes;            // size of the input (mode 2 reads it in aligned words)
+  int mode;               // 0 = rows, 1 = convolution, 2 = 3 x 3 over 3 channels
+  int x_bytes;            // size of the input (mode 2 and ragged rows read it in aligned words)
   int H, W, IC, KH, KW, OH, OW, stride, pad_t, pad_l;
   int input_zp, out_zp, clamp_min, clamp_max, epi;
   int add_m_self, add_m_other, add_f, add_clamp_min, add_clamp_max;  // BinaryArgs::lin_*

@@ -299,6 +299,9 @@ bool force_simt() {
 // Rows of a 1x1 convolution / FullyConnected product that are read as one row against block-diagonal weights
 // (row m' of the product then holds the outputs of pixels r*m' .. r*m'+r-1 back to back, which is exactly their dense
 // NHWC placement, so nothing else changes).
+// Result bytes from which cutting a padded result back beats byte stores from the product: 1000 x 1003 26.2 -> 19.7 us,
+// 4096 x 8190 328 -> 59 us; below, the second launch costs what it saves.
+constexpr long long kTrimBytes = 1 << 18;
 static int bytes16_row_group(long long K) {  // rows that together are a multiple of 16 bytes
   int g16 = 16;
   while (K % g16 != 0) g16 >>= 1;  // gcd(K, 16)
@@ -327,10 +330,16 @@ static bool pointwise_takes_gemm_tc(long long M, long long K, int OC, int weight
   return r <= 8 && M % r == 0 && (long long)OC * r <= 65536 && gemm_tc_supported(M / r, OC * r, (int)K * r, K * r);
 }
 
+// That kernel reads rows of any length, but 16-byte loads are cheaper: pairs of rows when that makes them a multiple of 16 (more
+// than two would multiply the arithmetic by more than the loads cost).
+static int pointwise_small_group(long long M, long long K) {
+  const int r = bytes16_row_group(K);
+  return r <= 2 && M % r == 0 ? r : 1;
+}
 // Whether such a product is one for the small-problem kernel.
 static bool pointwise_takes_small(long long M, long long K, int OC) {
-  const int r = bytes16_row_group(K);
-  return M % r == 0 && conv_small_applies(M / r, OC * r, 1, (int)K * r);
+  const int r = pointwise_small_group(M, K);
+  return conv_small_applies(M / r, OC * r, 1, (int)K * r);
 }
 
 bool decode_per_op() {
@@ -873,6 +882,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   for (int i = 0; i < (int)ops.size(); i++) {
     const auto& op = ops[i];
     Step step;
+    std::function<void(const ExecContext&)> before, after;  // launches around the op's own
     // a constant tensor used as a runtime operand (the generic tensor ops) is uploaded as it is
     auto loc = [&](int id) {
       if (id < 0) return Loc{};
@@ -991,7 +1001,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           if (o.shape[0] != N || o.shape[1] != OH || o.shape[2] != OW || o.shape[3] != OC)
             return b.fail(TB200_INVALID_ARGUMENT, "op %d: conv2d output shape is not %dx%dx%dx%d", i, N, OH, OW, OC);
         }
-        const long long K = (long long)KH * KW * IC;
+        long long K = (long long)KH * KW * IC;
         const int8_t* w = b.const_data<int8_t>(op.weights, (size_t)OC * K, "weights", i);
         if (!w) return b.status;
         if (op.in0_zp < -128 || op.in0_zp > 127) return b.fail(TB200_INVALID_ARGUMENT, "op %d: input_zp outside int8", i);
@@ -1016,27 +1026,6 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         const bool pointwise = fc || (KH == 1 && KW == 1 && op.stride_h == 1 && op.stride_w == 1 && op.pad_t == 0 &&
                                       op.pad_b == 0 && op.pad_l == 0 && op.pad_r == 0);
         const long long M = (long long)N * OH * OW;
-        // At most four rows: a weight-streaming dp4a kernel instead of 128-row tensor-core tiles (the weights are the
-        // only traffic that counts there; 4 x K bytes of activations fit any SM's shared memory up to K = 12288)
-        if (pointwise && op.weight_zp == 0 && !force_simt() && M <= 4 && K % 16 == 0 && K <= 12288) {
-          FcRowsArgs fa{};
-          fa.M = (int)M; fa.N = OC; fa.K = (int)K;
-          fa.out_zp = op.out_zp; fa.clamp_min = op.clamp_min; fa.clamp_max = op.clamp_max; fa.hi_shift = b.last_hi_shift;
-          const size_t w_off = b.add_const(w, (size_t)OC * K);
-          const size_t c_off = b.add_const(cp.data(), cp.size() * sizeof(ChanParams));
-          Loc lx = loc(op.in0), lo = loc(result_id);
-          step.kernel_name = "fc_rows_dp4a";
-          step.launch = [=](const ExecContext& c) {
-            FcRowsArgs k = fa;
-            k.x = (const int8_t*)lx.resolve(c);
-            k.out = (int8_t*)lo.resolve(c);
-            k.w = (const int8_t*)(c.consts + w_off);
-            k.chan = (const ChanParams*)(c.consts + c_off);
-            k.lut = has_lut ? (const int8_t*)(c.consts + lut_off) : nullptr;
-            launch_fc_rows(k, c.stream);
-          };
-          break;
-        }
         // Small problems (conv_small.cu): the same two families of products, on kernels that are latency-bound differently.
         // The step keeps the name of the family, whichever kernel the size picks.
         auto plan_small = [&](const char* family, int rows_per_group) {
@@ -1101,8 +1090,77 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             if (e != cudaSuccess && c.launch_error) *c.launch_error = e;
           };
         };
-        if (add_after[i] >= 0 ? add_fits_small[i] != 0 : pointwise && pointwise_takes_gemm_tc(M, K, OC, op.weight_zp) && pointwise_takes_small(M, K, OC)) {
-          plan_small("gemm_i8_tcgen05", bytes16_row_group(K));
+        const bool few_rows = M <= 4 && K % 16 == 0 && K <= 12288;  // fc_rows below
+        if (add_after[i] >= 0 ? add_fits_small[i] != 0
+                              : pointwise && op.weight_zp == 0 && !force_simt() && !few_rows && pointwise_takes_small(M, K, OC)) {
+          plan_small("gemm_i8_tcgen05", pointwise_small_group(M, K));
+          break;
+        }
+        const int IC16 = (IC + 15) / 16 * 16, OC16 = (OC + 15) / 16 * 16;
+        const bool conv_on_tc = !fc && !pointwise && op.weight_zp == 0 && !force_simt() && IC > 4 &&
+                                conv_tc_supported(N, H, W, IC16, OC16, KH, KW, op.stride_h, op.stride_w, op.dil_h, op.dil_w, OH, OW);
+        if (conv_on_tc &&
+            (IC != 16 || OC != OC16 || conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).halo ||
+             conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).s2) &&
+            conv_small_applies(M, OC, KH * KW, IC)) {
+          plan_small("conv_igemm_i8_tcgen05", 1);
+          break;
+        }
+        // Rows that are no multiple of 16 bytes (ragged_rows.cu): the layer runs on padded copies in scratch. A product whose rows
+        // can be read in groups needs no padded input; a result of few bytes leaves the product through byte stores faster
+        // than through a second launch.
+        Loc x_loc = loc(op.in0), y_loc = loc(result_id);
+        std::vector<int8_t> w_ragged;
+        if (add_after[i] < 0 && op.weight_zp == 0 && !force_simt() && (pointwise || conv_on_tc)) {
+          const bool pad = IC != IC16 && (!pointwise || !pointwise_takes_gemm_tc(M, K, OC, 0));
+          const int ICn = pad ? IC16 : IC;
+          const bool trim = OC != OC16 && (!pointwise || (M > 4 && OC * pointwise_row_group(M, ICn, OC) % 16 != 0 && M * OC >= kTrimBytes));
+          if (pad || trim) {
+            const int OCn = trim ? OC16 : OC, ic = IC, oc = OC;
+            w_ragged.assign((size_t)OCn * KH * KW * ICn, 0);
+            for (int r = 0; r < OC * KH * KW; r++) memcpy(w_ragged.data() + (size_t)r * ICn, w + (size_t)r * IC, (size_t)IC);
+            w = w_ragged.data();
+            ChanParams none{};
+            none.shift = 34; none.hshift = 2; none.rnd = 1ll << 33;
+            cp.resize(OCn, none);
+            acc_bound.resize(OCn, 0);
+            const long long in_rows = (long long)N * H * W;
+            const size_t x_bytes = pad ? ((size_t)in_rows * ICn + 255) / 256 * 256 : 0;
+            scratch_need = std::max(scratch_need, x_bytes + (trim ? (size_t)M * OCn : 0));
+            if (pad) {
+              const Loc from = x_loc;
+              x_loc = Loc{Loc::SCRATCH, 0};
+              before = [=](const ExecContext& c) { launch_pad_rows((const int8_t*)from.resolve(c), (int8_t*)c.scratch, in_rows, ic, ICn, c.stream); };
+            }
+            if (trim) {
+              const Loc to = y_loc, from = Loc{Loc::SCRATCH, x_bytes};
+              y_loc = from;
+              after = [=](const ExecContext& c) { launch_trim_rows((const int8_t*)from.resolve(c), (int8_t*)to.resolve(c), M, oc, OCn, c.stream); };
+            }
+            IC = ICn;
+            OC = OCn;
+            K = (long long)KH * KW * IC;
+          }
+        }
+        // At most four rows: a weight-streaming dp4a kernel instead of 128-row tensor-core tiles (the weights are the
+        // only traffic that counts there; 4 x K bytes of activations fit any SM's shared memory up to K = 12288)
+        if (pointwise && op.weight_zp == 0 && !force_simt() && M <= 4 && K % 16 == 0 && K <= 12288) {
+          FcRowsArgs fa{};
+          fa.M = (int)M; fa.N = OC; fa.K = (int)K;
+          fa.out_zp = op.out_zp; fa.clamp_min = op.clamp_min; fa.clamp_max = op.clamp_max; fa.hi_shift = b.last_hi_shift;
+          const size_t w_off = b.add_const(w, (size_t)OC * K);
+          const size_t c_off = b.add_const(cp.data(), cp.size() * sizeof(ChanParams));
+          Loc lx = x_loc, lo = y_loc;
+          step.kernel_name = "fc_rows_dp4a";
+          step.launch = [=](const ExecContext& c) {
+            FcRowsArgs k = fa;
+            k.x = (const int8_t*)lx.resolve(c);
+            k.out = (int8_t*)lo.resolve(c);
+            k.w = (const int8_t*)(c.consts + w_off);
+            k.chan = (const ChanParams*)(c.consts + c_off);
+            k.lut = has_lut ? (const int8_t*)(c.consts + lut_off) : nullptr;
+            launch_fc_rows(k, c.stream);
+          };
           break;
         }
         const int rgroup = pointwise_row_group(M, K, OC);
@@ -1140,16 +1198,16 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           const bool has_q4 = ga.epi != 0;
           // a residual add fused behind the product: the result is the add's, the other operand is read in the epilogue
           const int fused_add = add_after[i];
-          int out_id = result_id;
+          Loc lout = y_loc;
           Loc lres{};
           if (fused_add >= 0) {
             if (!binary_args_of(ops[fused_add], ga.add) || ga.add.epi == 0)
               return b.fail(TB200_INTERNAL, "op %d: fused add lost its 32-bit rescale", fused_add);
             ga.add_self_is_a = add_self_is_a[i];
-            out_id = ops[fused_add].out0;
+            lout = loc(ops[fused_add].out0);
             lres = loc(add_self_is_a[i] ? ops[fused_add].in1 : ops[fused_add].in0);
           }
-          Loc lx = loc(op.in0), lo = loc(out_id);
+          Loc lx = x_loc, lo = lout;
           std::shared_ptr<GemmTcState> st(gemm_tc_state_new(), gemm_tc_state_free);
           step.kernel_name = "gemm_i8_tcgen05";
           step.launch = [=](const ExecContext& c) {
@@ -1175,14 +1233,6 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         // of padding, its weights the original ones placed at [(j, oc)][kh][kp][(h, c)] and zero elsewhere. 1 / G of
         // the rows per pixel through the copy engine; the zero parts cost tensor-core work that is free here. Border classes, bias folding and the
         // epilogue constants follow from the transformed op as for any convolution.
-        if (!fc && !pointwise && op.weight_zp == 0 && !force_simt() &&
-            conv_tc_supported(N, H, W, IC, OC, KH, KW, op.stride_h, op.stride_w, op.dil_h, op.dil_w, OH, OW) &&
-            (IC != 16 || conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).halo ||
-             conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).s2) &&
-            conv_small_applies(M, OC, KH * KW, IC)) {
-          plan_small("conv_igemm_i8_tcgen05", 1);
-          break;
-        }
         std::vector<int8_t> w_pairs;
         static const bool no_pairs = getenv("TB200_CONV_NO_PAIRS") != nullptr;  // A/B switch
         int group = 0;  // pixels per row of the rewritten convolution: 4 for 16 channels where the width allows, else 2
@@ -1317,7 +1367,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             nz_off = b.add_const(nonzero.data(), nonzero.size());
             ca.ncc = (int)cmasks.size();
           }
-          Loc lx = loc(op.in0), lo = loc(result_id);
+          Loc lx = x_loc, lo = y_loc;
           std::shared_ptr<GemmTcState> st(gemm_tc_state_new(), gemm_tc_state_free);
           step.kernel_name = "conv_igemm_i8_tcgen05";
           step.launch = [=](const ExecContext& c) {
@@ -1365,8 +1415,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         a.epi = fc ? 0 : Builder::q4_params(cp, acc_bound, dr != 0, op.out_zp, op.clamp_min, q4s);
         const size_t q_off = a.epi ? b.add_const(q4s.data(), q4s.size() * sizeof(int4)) : 0;
         const bool has_q4s = a.epi != 0;
-        a.x_bytes = (long long)b.numel(op.in0);
-        Loc lx = loc(op.in0), lo = loc(result_id);
+        a.x_bytes = (long long)N * H * W * IC;
+        Loc lx = x_loc, lo = y_loc;
         step.kernel_name = conv2d_simt_kernel_name(a);
         step.launch = [=](const ExecContext& c) {
           ConvArgs k = a;
@@ -2318,6 +2368,14 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       }
       default:
         return b.fail(TB200_UNIMPLEMENTED, "op %d: kind %u is not implemented", i, op.kind);
+    }
+    if (before || after) {
+      step.launches += (before ? 1 : 0) + (after ? 1 : 0);
+      step.launch = [before, own = std::move(step.launch), after](const ExecContext& c) {
+        if (before) before(c);
+        own(c);
+        if (after) after(c);
+      };
     }
     plan.launch_count += step.launches;
     plan.steps.push_back(std::move(step));

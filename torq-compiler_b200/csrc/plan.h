@@ -28,12 +28,13 @@ struct ExecContext {
 
 // Where a tensor lives at dispatch time.
 struct Loc {
-  enum Kind { ARENA, IO, CONST, NONE } kind = NONE;
-  size_t offset = 0;  // byte offset in arena / const image, or io index
+  enum Kind { ARENA, IO, CONST, SCRATCH, NONE } kind = NONE;
+  size_t offset = 0;  // byte offset in arena / const image / scratch, or io index
   void* resolve(const ExecContext& c) const {
     switch (kind) {
       case ARENA: return c.arena + offset;
       case CONST: return c.consts + offset;
+      case SCRATCH: return c.scratch + offset;
       case IO: return c.io[offset];
       default: return nullptr;
     }
