@@ -13,6 +13,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "dependent_launch.cuh"
 #include "kernels.h"
@@ -93,6 +94,7 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 // ---------------------------------------------------------------------------------------------------------------
 enum { kStore = 0, kGeglu = 1, kRope = 2, kStream = 3 };
 constexpr int kTileRows = 32, kBlk = 64, kStageBytes = kTileRows * kBlk, kStreamStages = 4;
+constexpr int kRopeTokens = 8;  // most tokens a warp finishes in the RoPE epilogue
 
 template <int NT, int MODE>
 __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
@@ -132,12 +134,16 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     issue();
     cp_commit();
   }
-  float rope_c = 0.f, rope_s = 0.f, norm_w = 0.f;
+  float rope_c = 0.f, rope_s = 0.f, norm_w = 0.f, norm_w_other = 0.f;
   int pos = 0;
   const int head = MODE == kRope ? blockIdx.x / 8 : 0, part = MODE == kRope ? blockIdx.x % 8 : 0;
   const bool is_q = head < a.n_q, is_k = head == a.n_q;
   if (MODE == kRope) {
-    if (is_q || is_k) norm_w = 1.0f + bf2f(__ldg((is_q ? a.qw : a.kw) + part * 32 + lane));
+    if (is_q || is_k) {
+      const uint16_t* w = (is_q ? a.qw : a.kw) + lane;
+      norm_w = 1.0f + bf2f(__ldg(w + part * 32));
+      norm_w_other = 1.0f + bf2f(__ldg(w + (part ^ 4) * 32));
+    }
   }
   // the scales of the block's rows, read once per step and so always from HBM
   float* scale_s = reinterpret_cast<float*>(sm + a.scale_off);
@@ -146,7 +152,7 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
       const int t = row_block * a.rt + i / kTileRows;
       scale_s[i] = row_valid(t, i % kTileRows) ? bf2f(__ldg(a.scale + weight_row(t, i % kTileRows))) : 0.f;
     }
-  if (a.ck > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
+  if (MODE == kRope || a.ck > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
   grid_dependency_wait();
   grid_dependency_release();
 
@@ -171,7 +177,10 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
   }
   __syncthreads();
 
-  float c[2][NT][4];
+  // independent chains of accumulation: a dependent matrix instruction waits about 130 cycles here
+  constexpr int kSets = NT == 1 ? 4 : NT == 2 ? 2 : 1;
+  float cs[kSets][2][NT][4];
+  auto& c = cs[0];
   float best_v[NT][2];
   int best_i[NT][2];
 #pragma unroll
@@ -179,8 +188,24 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     best_v[t][0] = best_v[t][1] = -INFINITY;
     best_i[t][0] = best_i[t][1] = 0x7fffffff;
 #pragma unroll
-    for (int j = 0; j < 4; j++) c[0][t][j] = c[1][t][j] = 0.f;
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int q = 0; q < kSets; q++) cs[q][0][t][j] = cs[q][1][t][j] = 0.f;
   }
+  auto fold = [&]() {  // the chains into the first, which the others start from zero after
+    if (kSets == 1) return;
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+      for (int t = 0; t < NT; t++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (kSets == 4) c[mt][t][j] = (c[mt][t][j] + cs[1 % kSets][mt][t][j]) + (cs[2 % kSets][mt][t][j] + cs[3 % kSets][mt][t][j]);
+          else c[mt][t][j] += cs[1 % kSets][mt][t][j];
+#pragma unroll
+          for (int q = 1; q < kSets; q++) cs[q][mt][t][j] = 0.f;
+        }
+  };
   const uint32_t xrow = x_addr + (uint32_t)(g * a.x_pitch + (wb0 - kb0) * kBlk * 2 + tig * 32);
   int stage = 0, kb = 0, tile = tile0;
   for (int i = 0; i < total; i++) {
@@ -215,13 +240,14 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
       for (int t = 0; t < NT; t++) {
         const uint32_t b0 = m == 0 ? x0[t].x : m == 1 ? x0[t].z : m == 2 ? x1[t].x : x1[t].z;
         const uint32_t b1 = m == 0 ? x0[t].y : m == 1 ? x0[t].w : m == 2 ? x1[t].y : x1[t].w;
-        mma_bf16(c[0][t], f[0][0], f[1][0], f[0][1], f[1][1], b0, b1);
-        mma_bf16(c[1][t], f[2][0], f[3][0], f[2][1], f[3][1], b0, b1);
+        mma_bf16(cs[m % kSets][0][t], f[0][0], f[1][0], f[0][1], f[1][1], b0, b1);
+        mma_bf16(cs[m % kSets][1][t], f[2][0], f[3][0], f[2][1], f[3][1], b0, b1);
       }
     }
     if (++stage == a.stages) stage = 0;
     if (++kb == nb) {
       kb = 0;
+      fold();
       if (MODE == kStream) {
 #pragma unroll
         for (int mt = 0; mt < 2; mt++)
@@ -314,26 +340,27 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     return v;
   };
   const int warps = blockDim.x >> 5;
+  auto tile_of = [&](int i) { return (i * a.inv_b) >> 16; };  // i / B for i < 16 * 32
   // Results are numbered i = tile of the block * B + token, 32 rows each. In a cluster block i % ck finishes result i: the others
   // store their sums into its shared memory, 128 contiguous bytes a warp (reading them over one by one, a word per lane
   // and request, took up to 40 us), and it adds the blocks' sums in order.
   float* recv = reinterpret_cast<float*>(sm + a.recv_off);  // [block of the cluster][i / ck][32]
-  const int share = (a.rt * a.B + a.ck - 1) / a.ck;
+  const int ck_log2 = __ffs(a.ck) - 1, share = (a.rt * a.B + a.ck - 1) >> ck_log2;
   if (MODE != kRope && a.ck > 1) {
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     for (int i = warp; i < a.rt * a.B; i += warps)
-      st_peer(smem_u32(recv + (rank * share + i / a.ck) * 32 + lane), i % a.ck, block_sum(i / a.B, lane, i % a.B));
+      st_peer(smem_u32(recv + (rank * share + (i >> ck_log2)) * 32 + lane), i & (a.ck - 1), block_sum(tile_of(i), lane, i - tile_of(i) * a.B));
     cluster_sync();
   }
   auto sum_of = [&](int i, int row) {
-    if (a.ck <= 1) return block_sum(i / a.B, row, i % a.B);
-    float v = recv[(i / a.ck) * 32 + row];
-    for (int q = 1; q < a.ck; q++) v += recv[(q * share + i / a.ck) * 32 + row];
+    if (a.ck <= 1) return block_sum(tile_of(i), row, i - tile_of(i) * a.B);
+    float v = recv[(i >> ck_log2) * 32 + row];
+    for (int q = 1; q < a.ck; q++) v += recv[(q * share + (i >> ck_log2)) * 32 + row];
     return v;
   };
   if constexpr (MODE == kStore) {
     for (int i = warp * a.ck + rank; i < a.rt * a.B; i += warps * a.ck) {
-      const int r_t = i / a.B, b = i - r_t * a.B, n = (row_block * a.rt + r_t) * kTileRows + lane;
+      const int r_t = tile_of(i), b = i - r_t * a.B, n = (row_block * a.rt + r_t) * kTileRows + lane;
       const float v = sum_of(i, lane) * scale_s[r_t * kTileRows + lane];
       if (n >= a.N) continue;
       if (a.y_f32) ((float*)a.y)[(size_t)b * a.N + n] = v;
@@ -341,45 +368,61 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     }
   } else if constexpr (MODE == kGeglu) {
     const int I = a.N / 2, r = lane & 15;  // half a warp per token
-    for (int i = (warp * 2 + (lane >> 4)) * a.ck + rank; i < a.rt * a.B; i += 2 * warps * a.ck) {
-      const int r_t = i / a.B, b = i - r_t * a.B, n = (row_block * a.rt + r_t) * 16 + r;
-      if (n >= I) continue;
-      const float* sc = scale_s + r_t * kTileRows;
-      const float gate = rbf(sum_of(i, r) * sc[r]), up = rbf(sum_of(i, 16 + r) * sc[16 + r]);
-      ((uint16_t*)a.y)[(size_t)b * I + n] = f2bf(rbf(gelu_tanh(gate)) * up);
-    }
+    const int step = 2 * warps * a.ck, count = a.rt * a.B;
+    auto finish = [&](int i0, auto in_flight) {
+      constexpr int U = decltype(in_flight)::value;
+      float gate[U], up[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u * step < count ? i0 + u * step : i0;
+        const float* sc = scale_s + tile_of(i) * kTileRows;
+        gate[u] = rbf(sum_of(i, r) * sc[r]);
+        up[u] = rbf(sum_of(i, 16 + r) * sc[16 + r]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u * step, r_t = tile_of(i), n = (row_block * a.rt + r_t) * 16 + r;
+        if (i < count && n < I) ((uint16_t*)a.y)[(size_t)(i - r_t * a.B) * I + n] = f2bf(rbf(gelu_tanh(gate[u])) * up[u]);
+      }
+    };
+    int i0 = (warp * 2 + (lane >> 4)) * a.ck + rank;
+    for (; i0 + step < count; i0 += 2 * step) finish(i0, std::integral_constant<int, 2>());
+    if (i0 < count) finish(i0, std::integral_constant<int, 1>());
   } else {
     // one head of 256 rows per cluster, 32 rows per block: lane = row
-    float* ss = sums + a.kg * (kTileRows * kPitch);  // [tokens] sum of squares of this block's rows
-    float* nv = ss + kTok;                           // [tokens][32] normalised values
+    // rank = 32 rows of the head; rows i and i + 128 rotate together, so blocks part and part ^ 4 exchange their values
+    float* ss = sums + a.kg * (kTileRows * kPitch);  // [block][tokens] sums of squares
+    float* nv = ss + 8 * kTok;                       // [tokens][32] the partner's values
     const float scale = scale_s[lane];
-    for (int b = warp; b < a.B; b += warps) {
-      const float v = rbf(block_sum(0, lane, b) * scale);
-      nv[b * 32 + lane] = v;
-      const float s = warp_sum(v * v);
-      if (lane == 0) ss[b] = s;
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    float own[kRopeTokens];
+#pragma unroll
+    for (int u = 0; u < kRopeTokens; u++) {
+      const int b = warp + u * warps;
+      if (b >= a.B) break;
+      own[u] = rbf(block_sum(0, lane, b) * scale);
+      st_peer(smem_u32(nv + b * 32 + lane), part ^ 4, own[u]);
+      const float q = warp_sum(own[u] * own[u]);
+      if (lane < 8) st_peer(smem_u32(ss + part * kTok + b), lane, q);
     }
     cluster_sync();
-    if (is_q || is_k)
-      for (int b = warp; b < a.B; b += warps) {
-        float s = 0.f;
 #pragma unroll
-        for (int q = 0; q < 8; q++) s += ld_peer(smem_u32(ss + b), q);
-        nv[b * 32 + lane] = rbf(nv[b * 32 + lane] * rsqrtf(s / 256.0f + a.eps) * norm_w);
-      }
-    cluster_sync();
-    for (int b = warp; b < a.B; b += warps) {
-      const float own = nv[b * 32 + lane];
-      float v = own;
+    for (int u = 0; u < kRopeTokens; u++) {
+      const int b = warp + u * warps;
+      if (b >= a.B) break;
+      float v = own[u];
       if (is_q || is_k) {
-        const float other = ld_peer(smem_u32(nv + b * 32 + lane), part ^ 4);
-        v = part < 4 ? own * rope_c - other * rope_s : own * rope_c + other * rope_s;
+        float q = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) q += ss[k * kTok + b];
+        const float inv = rsqrtf(q / 256.0f + a.eps);
+        const float mine = rbf(own[u] * inv * norm_w), other = rbf(nv[b * 32 + lane] * inv * norm_w_other);
+        v = part < 4 ? mine * rope_c - other * rope_s : mine * rope_c + other * rope_s;
       }
       uint16_t* dst = is_q ? a.q_out + ((size_t)b * a.n_q + head) * 256 : (is_k ? a.kcache : a.vcache) + ((size_t)b * a.T + pos) * 256;
       dst[part * 32 + lane] = f2bf(v);
     }
   }
-  if (MODE == kRope) cluster_sync();  // no block leaves while another may read its values
   }
 }
 
@@ -445,25 +488,44 @@ static_assert(8 * kAttnCol * 4 <= kAttnWarpBytes, "the warps' results take the p
 
 __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_cluster_kernel(const uint16_t* __restrict__ q, const int32_t* __restrict__ pos_p,
                                                                           const uint16_t* kcache, const uint16_t* vcache,
-                                                                          uint16_t* __restrict__ out, int n_q, int T, int window, float scale) {
+                                                                          uint16_t* __restrict__ out, int n_q, int T, int window, float scale, int early) {
   extern __shared__ __align__(128) unsigned char kv_s[];  // [warp][16 keys, 16 values], later [warp][8 columns][kAttnCol] results
   __shared__ float part_ml[kAttnWarps][4][2];
-  __shared__ float blk_acc[4][256];
-  __shared__ float blk_ml[4][2];
+  __shared__ float recv_acc[kAttnBlocks][kAttnWarps * 32];  // every block's sums of the outputs this block finishes
+  __shared__ float recv_ml[kAttnBlocks][4][2];              // and every block's (max, sum) per head
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int rank = blockIdx.x, b = blockIdx.y;
-  int t0, t1;
-  auto slice = [&](int pos) {
-    pos = pos < 0 ? 0 : (pos >= T ? T - 1 : pos);
+  int t0, t1, pos;
+  auto slice = [&](int p) {
+    pos = p < 0 ? 0 : (p >= T ? T - 1 : p);
     const int t_lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int per = ((pos + 1 - t_lo + kAttnBlocks - 1) / kAttnBlocks + 15) & ~15;
     t0 = t_lo + rank * per;
     t1 = min(pos + 1, t0 + per);
   };
-  slice(__ldcg(pos_p));  // for the prefetch only: read again behind the wait
   const uint16_t* kc = kcache + (size_t)b * T * 256;
   const uint16_t* vc = vcache + (size_t)b * T * 256;
-  for (int row = t0 + 16 * warp + (lane & 15); row < t1; row += 16 * kAttnWarps) {
+  const uint32_t ks = smem_u32(kv_s) + warp * kAttnWarpBytes, vs = ks + 16 * kKeyPitch;
+  auto copy_row = [&](const uint16_t* src, int t, uint32_t dst) {  // a row is 32 pieces of 16 bytes: one per lane
+    cp_async16(dst + lane * 16, src + (size_t)t * 256 + lane * 8, true);
+  };
+  auto copy = [&](const uint16_t* src, int t, uint32_t dst, int pitch) {
+#pragma unroll
+    for (int r = 0; r < 16; r++) copy_row(src, min(t + r, t1 - 1), dst + r * pitch);
+    cp_commit();
+  };
+  // The rows of earlier steps are final, so they may be read before the wait when the launch ahead is the append of row pos
+  // (early); anything else only pulls them towards L2. What depends on the launch ahead is read again behind the wait.
+  slice(__ldcg(pos_p));
+  const int pos_seen = pos;
+  if (early) {
+    if (t0 + 16 * warp < t1) {
+      copy(kc, t0 + 16 * warp, ks, kKeyPitch);
+      copy(vc, t0 + 16 * warp, vs, kValPitch);
+    }
+  }
+  for (int row = t0 + 16 * (warp + (early ? kAttnWarps : 0)) + (lane & 15); row < t1; row += 16 * kAttnWarps) {
     const uint16_t* p = (lane < 16 ? kc : vc) + (size_t)row * 256;
 #pragma unroll
     for (int j = 0; j < 4; j++) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 64 * j));
@@ -471,16 +533,21 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_cluster_kernel(const 
   grid_dependency_wait();
   grid_dependency_release();
   slice(__ldcg(pos_p));
-  const uint32_t ks = smem_u32(kv_s) + warp * kAttnWarpBytes, vs = ks + 16 * kKeyPitch;
-  auto copy = [&](const uint16_t* src, int t, uint32_t dst, int pitch) {  // a row is 32 pieces of 16 bytes: one per lane
-#pragma unroll
-    for (int r = 0; r < 16; r++) cp_async16(dst + r * pitch + lane * 16, src + (size_t)min(t + r, t1 - 1) * 256 + lane * 8, true);
-    cp_commit();
-  };
   const int t_first = t0 + 16 * warp;
-  if (t_first < t1) {
-    copy(kc, t_first, ks, kKeyPitch);
-    copy(vc, t_first, vs, kValPitch);
+  if (!early || pos != pos_seen) {
+    cp_wait<0>();
+    __syncwarp();
+    if (t_first < t1) {
+      copy(kc, t_first, ks, kKeyPitch);
+      copy(vc, t_first, vs, kValPitch);
+    }
+  } else if (t_first < t1 && t_first + 16 >= t1 && t1 - 1 == pos) {  // the new row, and its copies that fill the round
+    cp_wait<0>();
+    __syncwarp();
+    for (int r = pos - t_first; r < 16; r++) copy_row(kc, pos, ks + r * kKeyPitch);
+    cp_commit();
+    for (int r = pos - t_first; r < 16; r++) copy_row(vc, pos, vs + r * kValPitch);
+    cp_commit();
   }
   uint4 qf[8];
 #pragma unroll
@@ -581,54 +648,52 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attn_cluster_kernel(const 
 #pragma unroll
     for (int e = 0; e < 4; e++) part[2 * t4 + (e & 1)][16 * j + g + 8 * (e >> 1)] = acc[j][e];
   __syncthreads();
-  for (int h = 0; h < n_q; h++) {
+  // warp = head: the block's sums go to the blocks that finish them, 128 contiguous bytes a store
+  const int share = n_q * (256 / kAttnBlocks);
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (warp < n_q) {
     float mm = -INFINITY, ll = 0.f, e[kAttnWarps];
 #pragma unroll
-    for (int w = 0; w < kAttnWarps; w++) mm = fmaxf(mm, part_ml[w][h][0]);
+    for (int w = 0; w < kAttnWarps; w++) mm = fmaxf(mm, part_ml[w][warp][0]);
 #pragma unroll
     for (int w = 0; w < kAttnWarps; w++) {
-      e[w] = part_ml[w][h][1] > 0.f ? expf(part_ml[w][h][0] - mm) : 0.f;
-      ll += part_ml[w][h][1] * e[w];
+      e[w] = part_ml[w][warp][1] > 0.f ? expf(part_ml[w][warp][0] - mm) : 0.f;
+      ll += part_ml[w][warp][1] * e[w];
+    }
+    if (lane < kAttnBlocks) {
+      st_peer(smem_u32(&recv_ml[rank][warp][0]), lane, mm);
+      st_peer(smem_u32(&recv_ml[rank][warp][1]), lane, ll);
     }
 #pragma unroll
-    for (int i = threadIdx.x; i < 256; i += kAttnWarps * 32) {
+    for (int k = 0; k < 8; k++) {
+      const int i = 32 * k + lane, at = warp * 256 + 32 * k;
       float o = 0.f;
 #pragma unroll
       for (int w = 0; w < kAttnWarps; w++) {
         const float* p = reinterpret_cast<const float*>(kv_s + w * kAttnWarpBytes);
-        o += (p[h * kAttnCol + i] + p[(h + 4) * kAttnCol + i]) * e[w];
+        o += (p[warp * kAttnCol + i] + p[(warp + 4) * kAttnCol + i]) * e[w];
       }
-      blk_acc[h][i] = o;
-    }
-    if (threadIdx.x == 0) {
-      blk_ml[h][0] = mm;
-      blk_ml[h][1] = ll;
+      st_peer(smem_u32(&recv_acc[rank][at % share + lane]), at / share, o);
     }
   }
   cluster_sync();
-  for (int i = rank * (kAttnWarps * 32) + threadIdx.x; i < n_q * 256; i += kAttnBlocks * kAttnWarps * 32) {
-    const int h = i >> 8, at = i & 255;
-    float mr[kAttnBlocks], lr[kAttnBlocks], ar[kAttnBlocks], mm = -INFINITY;
+  if ((int)threadIdx.x < share) {
+    const int h = (rank * share + threadIdx.x) >> 8, at = (rank * share + threadIdx.x) & 255;
+    float mm = -INFINITY;
 #pragma unroll
-    for (int r = 0; r < kAttnBlocks; r++) {
-      mr[r] = ld_peer(smem_u32(&blk_ml[h][0]), r);
-      lr[r] = ld_peer(smem_u32(&blk_ml[h][1]), r);
-      ar[r] = ld_peer(smem_u32(&blk_acc[h][at]), r);
-      mm = fmaxf(mm, mr[r]);
-    }
+    for (int r = 0; r < kAttnBlocks; r++) mm = fmaxf(mm, recv_ml[r][h][0]);
     float ll = 0.f, o = 0.f;
 #pragma unroll
     for (int r = 0; r < kAttnBlocks; r++)
-      if (lr[r] > 0.f) {
-        const float e = expf(mr[r] - mm);
-        ll += lr[r] * e;
-        o += ar[r] * e;
+      if (recv_ml[r][h][1] > 0.f) {
+        const float e = expf(recv_ml[r][h][0] - mm);
+        ll += recv_ml[r][h][1] * e;
+        o += recv_acc[r][threadIdx.x] * e;
       }
-    // place i of a column: tile (d, j) x row
+    // place `at` of a column: tile (d, j) x row
     const int dim = 64 * (at >> 6) + 8 * (at & 7) + 4 * (at >> 3 & 1) + (at >> 4 & 3);
     out[((size_t)b * n_q + h) * 256 + dim] = f2bf(o / ll);
   }
-  cluster_sync();
 }
 
 // best of the blocks' candidates, [B][count] values and rows: a warp per token
@@ -761,7 +826,7 @@ LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
     s.x_pitch = (widest * kBlk * 2 + 127) / 128 * 128 + 16;
     s.x_bytes = (tok * s.x_pitch + 127) / 128 * 128;
     const int warps = kg * rt;
-    const int sums = warps * kTileRows * (tok + 1) * 4 + (mode == kRope ? tok * 33 * 4 : 0);
+    const int sums = warps * kTileRows * (tok + 1) * 4 + (mode == kRope ? tok * 40 * 4 : 0);
     s.scale_off = std::max(s.x_bytes + warps * stages * kStageBytes, mode == kStream ? 16 * tok * 8 : (sums + 127) / 128 * 128);
     s.recv_off = s.scale_off + rt * kTileRows * 4;
     s.smem = s.recv_off + (ck > 1 ? (rt * B + ck - 1) / ck * ck * 128 : 0);
@@ -779,22 +844,30 @@ LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
   const int stages = ceil_div(blocks, s.tk);  // every block of a warp has its own place
   if (stages > 64) return s;
   if (mode == kRope) {
-    s.ok = s.tk <= 16 && fit(s.tk, 1, 1, stages);
+    s.ok = s.tk <= 16 && s.tk * kRopeTokens >= tok && fit(s.tk, 1, 1, stages);
     s.grid = s.tiles;
     return s;
   }
-  // the fewest blocks per cluster whose activations leave room; more while that fills idle SMs
-  for (int ck = 1; ck <= 8 && ck <= s.tk; ck *= 2) {
-    const int kg = s.tk / ck;
-    if (kg > 16) continue;
-    int rt = std::max(1, std::min(ceil_div((long long)s.tiles * ck, sms), 16 / kg));
-    while (rt > 1 && !fit(kg, ck, rt, stages)) rt--;
-    if (!fit(kg, ck, rt, stages)) continue;
-    s.grid = ceil_div(s.tiles, rt) * ck;
-    s.ok = true;
-    return s;
-  }
-  return s;
+  // The fewest blocks per cluster whose activations leave room and whose clusters are all resident at once (a second wave cost
+  // 7 us): clusters do not cross a GPC, of which eight with 16 SMs are counted on.
+  auto one_wave = [&]() {
+    const int clusters = s.grid / s.ck, per_sm = std::max(1, std::min(2048 / (s.kg * s.rt * 32), kSmemMax / s.smem));
+    return s.ck == 1 ? s.grid <= sms * per_sm : clusters <= 8 * (16 / s.ck) * std::min(per_sm, 2);
+  };
+  for (int pass = 0; pass < 2; pass++)
+    for (int ck = 1; ck <= 8 && ck <= s.tk; ck *= 2) {
+      const int kg = s.tk / ck;
+      if (kg > 16) continue;
+      int rt = std::max(1, std::min(ceil_div((long long)s.tiles * ck, sms), 16 / kg));
+      while (rt > 1 && !fit(kg, ck, rt, stages)) rt--;
+      for (; rt <= 16 / kg && fit(kg, ck, rt, stages); rt++) {
+        s.grid = ceil_div(s.tiles, rt) * ck;
+        if (pass == 0 && !one_wave()) continue;
+        s.ok = true;
+        return s;
+      }
+    }
+  return LinearShape{};
 }
 
 template <int NT, int MODE>
@@ -811,7 +884,7 @@ cudaError_t launch_linear_as(const LinearArgs& a, const LinearShape& s, int clus
 template <int MODE>
 cudaError_t launch_linear_mode(const LinearArgs& args, const LinearShape& s, cudaStream_t stream) {
   LinearArgs a = args;
-  a.kg = s.kg; a.ck = s.ck; a.rt = s.rt; a.stages = s.stages; a.x_pitch = s.x_pitch; a.x_bytes = s.x_bytes; a.scale_off = s.scale_off; a.recv_off = s.recv_off; a.tiles = s.tiles;
+  a.kg = s.kg; a.ck = s.ck; a.rt = s.rt; a.stages = s.stages; a.x_pitch = s.x_pitch; a.x_bytes = s.x_bytes; a.scale_off = s.scale_off; a.recv_off = s.recv_off; a.inv_b = (65536 + a.B - 1) / a.B; a.tiles = s.tiles;
   const int cluster = MODE == kRope ? 8 : s.ck;
   switch ((a.B + 7) / 8) {
     case 1: return launch_linear_as<1, MODE>(a, s, cluster, stream);
@@ -864,14 +937,14 @@ void launch_rope_heads(const uint16_t* qkv, const int32_t* pos, const uint16_t* 
 }
 
 void launch_attn_decode(const uint16_t* q, const int32_t* pos, const uint16_t* kcache, const uint16_t* vcache, uint16_t* out, int B, int n_q,
-                        int T, int window, float scale, cudaStream_t stream) {
+                        int T, int window, float scale, bool early, cudaStream_t stream) {
   static std::atomic<unsigned long long> attr_done{0};
   if (first_use_on_device(attr_done)) {
     cudaFuncSetAttribute(attn_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnWarps * kAttnWarpBytes);
     mark_used_on_device(attr_done);
   }
   launch_dependent_cluster(kAttnBlocks, attn_cluster_kernel, dim3(kAttnBlocks, B), dim3(kAttnWarps * 32), kAttnWarps * kAttnWarpBytes, stream, true, q, pos, kcache, vcache, out,
-                           n_q, T, window, scale);
+                           n_q, T, window, scale, early ? 1 : 0);
 }
 
 bool rmsnorm_row_applies(int H) { return H % 4 == 0 && H <= 4096; }

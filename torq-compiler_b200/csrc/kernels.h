@@ -288,7 +288,7 @@ struct LinearArgs {
   // filled by the launcher
   float* cand_v;
   int32_t* cand_i;
-  int kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, tiles;
+  int kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, inv_b, tiles;
 };
 bool linear_w8_applies(int B, int N, int K);
 bool linear_geglu_applies(int B, int N, int K);
@@ -300,9 +300,10 @@ cudaError_t launch_linear_rope(const LinearArgs& a, cudaStream_t stream);
 cudaError_t launch_linear_argmax(LinearArgs a, void* scratch, int32_t* out, cudaStream_t stream);  // fp32 or bf16 logits to y as well
 void launch_rope_heads(const uint16_t* qkv, const int32_t* pos, const uint16_t* qw, const uint16_t* kw, uint16_t* q_out, uint16_t* kcache,
                        uint16_t* vcache, int B, int n_q, int n_kv, int T, float theta, float eps, cudaStream_t stream);  // head size 256
-// one KV head of 256, up to 4 query heads
+// one KV head of 256, up to 4 query heads; early: the launch right ahead is the append of row pos to these caches and nothing else
+// still writes them
 void launch_attn_decode(const uint16_t* q, const int32_t* pos, const uint16_t* kcache, const uint16_t* vcache, uint16_t* out, int B, int n_q,
-                        int T, int window, float scale, cudaStream_t stream);
+                        int T, int window, float scale, bool early, cudaStream_t stream);
 bool rmsnorm_row_applies(int H);
 // rmsnorm; with w2 a second norm without residual of its result goes to out2
 void launch_rmsnorm_row(const uint16_t* x, const uint16_t* res, const uint16_t* w, uint16_t* out, const uint16_t* w2, uint16_t* out2, int rows,

@@ -395,13 +395,11 @@ bool try_fuse_decode_step(Builder& b, Plan& plan, size_t& scratch_need) {
   const int Tlen = T[first_rope.out1].shape[1];
   const float eps = lo[0]->f0, attn_scale = lo[3]->f0;
   if (!decode_step_supported(B, H, n_q, n_kv, D, I, V)) return false;
-  // Measured on the 1B shape: the fused step wins at 1 and 2 sequences (1.17 ms against 1.43 ms at 2); from 3 on
-  // the per-op path with the tensor-core GEMV is faster (1.44 ms against 1.57 ms at 3, 1.44 against 1.70 at 4,
-  // 1.47 against 2.83 at 8). Tensor-parallel shards exist only in fused form. TB200_DECODE_FUSED_MAX_B moves
-  // the threshold.
+  // Tensor-parallel shards exist only in this form. On one GPU the op-by-op kernels are faster at every batch (measured per
+  // step: 3 layers 108 us against 128 at one sequence, 115 against 166 at two); TB200_DECODE_FUSED_MAX_B moves the threshold.
   {
     const char* e = getenv("TB200_DECODE_FUSED_MAX_B");
-    const int max_b = e ? atoi(e) : 2;
+    const int max_b = e ? atoi(e) : 0;
     if (!tp_graph && B > max_b) return false;
   }
   int dev = 0, sms = 0;
@@ -1908,10 +1906,13 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: attn_decode shape mismatch", i);
         Loc lq = loc(op.in0), lp = loc(op.in1), lk = loc(op.in2), lv = plan.tensor_loc[op.weights], lo = loc(op.out0);
         const float scale = op.f0;
+        // the append right in front of it, to the same caches at the same position: a launch of its own at head size 256
+        const bool early = i > 0 && ops[i - 1].kind == TB200_OP_ROPE_KV && ops[i - 1].out1 == op.in2 && ops[i - 1].in2 == op.weights &&
+                           ops[i - 1].in1 == op.in1;
         step.kernel_name = "attn_decode_splitT";
         step.launch = [=](const ExecContext& c) {
           launch_attn_decode((const uint16_t*)lq.resolve(c), (const int32_t*)lp.resolve(c), (const uint16_t*)lk.resolve(c),
-                             (const uint16_t*)lv.resolve(c), (uint16_t*)lo.resolve(c), B, n_q, T, window, scale, c.stream);
+                             (const uint16_t*)lv.resolve(c), (uint16_t*)lo.resolve(c), B, n_q, T, window, scale, early, c.stream);
         };
         break;
       }
