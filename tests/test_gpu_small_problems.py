@@ -73,3 +73,15 @@ def test_add_between_intermediates_rides_in_the_convolution(device, S, K, OC, co
     assert ex.launch_count == 2, ex.op_kernels()
     ex.destroy()
     _both(device, g, [rng.integers(-128, 128, (1, S, S, K), dtype=np.int8)], monkeypatch)
+
+
+@pytest.mark.parametrize("M,K,N", [(5, 4096, 256), (64, 4096, 4096), (65, 2064, 1024), (128, 1040, 2500), (100, 1001, 2077), (17, 8192, 8192), (321, 2048, 2600)])
+@pytest.mark.parametrize("table", [False, True])
+def test_few_dozen_rows(device, M, K, N, table, monkeypatch):
+    rng = np.random.default_rng(M + K + N)
+    g = Graph()
+    m, s = _ms(rng, N, K)
+    y = g.fully_connected(g.input((M, K)), rng.integers(-127, 128, (N, K), dtype=np.int8), np.round(rng.normal(0, 900, N)).astype(np.int32), m, s,
+                          input_zp=-7, out_zp=3)
+    g.output(g.table(y, rng.permutation(np.arange(-128, 128)).astype(np.int8)) if table else y)
+    _both(device, g, [rng.integers(-128, 128, (M, K), dtype=np.int8)], monkeypatch)

@@ -18,6 +18,8 @@
 // bytes. The weights are laid out in exactly that order by conv_small_pack: a warp's load is 512 contiguous bytes.
 #include <string.h>
 
+#include <atomic>
+
 #include "kernels.h"
 #include "dependent_launch.cuh"
 
@@ -295,6 +297,176 @@ __global__ void __launch_bounds__(SPLIT ? 256 : 128, SPLIT ? 2 : 4) conv_small_k
   }
 }
 
+// ---- products of a few dozen rows ----
+// Between the sizes above and those that fill the chip with 128-row tiles a product is bound by how fast its weights arrive:
+// FullyConnected 64 x 4096 -> 4096 is 17 MB of weights, 2.6 us of HBM time, and took 17.5 us on 32 tiles of the tcgen05 kernel,
+// now 9.9.
+// A block takes 64 rows x 128 columns and one of ck slices of K (a cluster), so that every SM streams weights. Chunks of 256
+// bytes of K - weights in fragment order, rows at a pitch of 64 bytes modulo 128 - pass through three shared-memory stages by
+// cp.async, two of them in flight. A warp is 32 columns x one of the chunk's four steps x all 64 rows: a weight fragment
+// then serves four instructions (eight warps with two steps each left the shared-memory reads' latency in the open). The sums are integers: they meet in shared memory, within the block and pushed through
+// the cluster, and each block of the cluster finishes its share of the rows.
+constexpr int kMidM = 64, kMidN = 128, kMidThreads = 512, kMidStages = 3, kMidSteps = 4;
+constexpr int kMidPitch = kMidSteps * kStepBytes + 64;
+constexpr int kMidX = kMidM * kMidPitch, kMidW = kMidSteps * 2048 * (kMidN / kTileN), kMidStage = kMidX + kMidW;
+constexpr int kMidSumPitch = kMidN + 4;  // words
+constexpr int kMidRecv = kMidM * kMidN * 4, kMidSmem = kMidStages * kMidStage + kMidRecv;
+constexpr int kMidGroups = kMidThreads / 128;  // warps that share a chunk's steps
+static_assert(kMidGroups * kMidM * kMidSumPitch * 4 <= kMidStages * kMidStage, "the sums take the stages' place");
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {  // zeros when not valid
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(kMidThreads, 1) rows_mid_kernel(const ConvSmallArgs a) {
+  extern __shared__ __align__(128) unsigned char mid_s[];
+  __shared__ int8_t lut[256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int ck = 1 << a.ks_log2, rank = blockIdx.x & (ck - 1), nb = blockIdx.x >> a.ks_log2, row0 = blockIdx.y * kMidM;
+  const int nt = warp & 3, kg = warp >> 2;
+  const int s_begin = a.steps * rank >> a.ks_log2, s_end = a.steps * (rank + 1) >> a.ks_log2;  // steps of 64 bytes of K
+  const int chunks = (s_end - s_begin + kMidSteps - 1) / kMidSteps;
+  if (ck > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
+  const uint32_t base = smem_u32(mid_s);
+  // A thread copies piece threadIdx.x of each of the chunk's four weight tiles and pieces of two rows; pointers and limits are kept
+  // (worked out anew for every copy they were 230 of 280 instructions per warp and chunk).
+  static_assert(kMidThreads == 512 && kMidSteps == 4 && kMidN == 4 * kTileN && kMidM == 64, "the copies below");
+  const int w_step = threadIdx.x >> 7, x_row = threadIdx.x >> 4, x_piece = threadIdx.x & 15;
+  const int8_t* wp = a.w + ((size_t)nb * 4 * a.steps + s_begin + w_step) * 2048 + (threadIdx.x & 127) * 16;
+  const size_t w_tile = (size_t)a.steps * 2048;
+  const int w_tiles = min(4, a.n_tiles - 4 * nb);
+  const int8_t* xp = a.x + (long long)(row0 + x_row) * a.lda + s_begin * kStepBytes + x_piece * 16;
+  const long long x_next = 32ll * a.lda;
+  const bool x_ok0 = row0 + x_row < a.M, x_ok1 = row0 + x_row + 32 < a.M;
+  int w_left = s_end - s_begin - w_step;                              // steps from this thread's on
+  int x_left = min(a.chunks, s_end * 4) - s_begin * 4 - x_piece;      // pieces from this thread's on
+  uint32_t w_dst = base + kMidX + threadIdx.x * 16, x_dst = base + x_row * kMidPitch + x_piece * 16;
+  const uint32_t w_end = w_dst + kMidStages * kMidStage, x_end = x_dst + kMidStages * kMidStage;
+  auto load_w = [&]() {
+#pragma unroll
+    for (int i = 0; i < 4; i++) cp_async16(w_dst + i * 8192, w_left > 0 && i < w_tiles ? wp + i * w_tile : a.w, w_left > 0 && i < w_tiles);
+    wp += kMidSteps * 2048;
+    w_left -= kMidSteps;
+    w_dst += kMidStage;
+    if (w_dst == w_end) w_dst -= kMidStages * kMidStage;
+  };
+  auto load_x = [&]() {
+    cp_async16(x_dst, x_left > 0 && x_ok0 ? xp : a.x, x_left > 0 && x_ok0);
+    cp_async16(x_dst + 32 * kMidPitch, x_left > 0 && x_ok1 ? xp + x_next : a.x, x_left > 0 && x_ok1);
+    xp += kMidSteps * kStepBytes;
+    x_left -= kMidSteps * 4;
+    x_dst += kMidStage;
+    if (x_dst == x_end) x_dst -= kMidStages * kMidStage;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load_w();
+  load_w();
+  if (a.lut)
+    for (int i = threadIdx.x; i < 256; i += kMidThreads) lut[i] = a.lut[i];
+  grid_dependency_wait();
+  grid_dependency_release();
+  load_x();
+  load_x();
+  int acc[4][4][4];
+#pragma unroll
+  for (int m = 0; m < 4; m++)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc[m][j][i] = 0;
+  uint32_t stage = base;
+  for (int c = 0; c < chunks; c++) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // chunk c has arrived for everyone, and chunk c - 1 has been read by everyone
+    load_w();
+    load_x();
+    const uint32_t xs = stage + g * kMidPitch + t * 16, ws = stage + kMidX + nt * 8192 + lane * 16;
+    stage = stage == base + (kMidStages - 1) * kMidStage ? base : stage + kMidStage;
+#pragma unroll
+    for (int u = 0; u < kMidSteps / kMidGroups; u++) {
+      const int s = kMidGroups * u + kg;
+      uint4 b[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) b[j] = lds128(ws + s * 2048 + j * 512);
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        const uint4 v0 = lds128(xs + (16 * m) * kMidPitch + s * kStepBytes), v1 = lds128(xs + (16 * m + 8) * kMidPitch + s * kStepBytes);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          mma_s8(acc[m][j], v0.x, v1.x, v0.y, v1.y, b[j].x, b[j].y);
+          mma_s8(acc[m][j], v0.z, v1.z, v0.w, v1.w, b[j].z, b[j].w);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  int* sums = reinterpret_cast<int*>(mid_s);
+#pragma unroll
+  for (int m = 0; m < 4; m++)
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        *reinterpret_cast<int4*>(sums + (kg * kMidM + 16 * m + g + 8 * r) * kMidSumPitch + nt * 32 + 8 * t + 4 * h) =
+            make_int4(acc[m][2 * h][2 * r], acc[m][2 * h][2 * r + 1], acc[m][2 * h + 1][2 * r], acc[m][2 * h + 1][2 * r + 1]);
+  __syncthreads();
+  const int share_log2 = 6 - a.ks_log2;  // rows a block of the cluster finishes
+  int* recv = reinterpret_cast<int*>(mid_s + kMidStages * kMidStage);  // [block of the cluster][its rows][columns]
+  auto block_sum = [&](int row, int col) {
+    int4 v = make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int k = 0; k < kMidGroups; k++) {
+      const int4 p = *reinterpret_cast<const int4*>(sums + (k * kMidM + row) * kMidSumPitch + col);
+      v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+    }
+    return v;
+  };
+  if (ck > 1) {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    for (int row = warp; row < kMidM; row += kMidThreads / 32) {
+      if (row0 + row >= a.M) break;
+      const int4 v = block_sum(row, 4 * lane);
+      const uint32_t local = smem_u32(recv + (((rank << share_log2) + (row & ((1 << share_log2) - 1))) * kMidN) + 4 * lane);
+      uint32_t remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(row >> share_log2));
+      asm volatile("st.shared::cluster.v4.s32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  const int chan = nb * kMidN + 4 * lane, left = a.N - chan;
+  if (left <= 0) return;
+  int4 q[4];
+  if (a.epi)
+#pragma unroll
+    for (int j = 0; j < 4; j++) q[j] = __ldg(a.q4 + chan + j);
+  for (int r = warp; r < 1 << share_log2; r += kMidThreads / 32) {
+    const int row = (rank << share_log2) + r;
+    if (row0 + row >= a.M) break;
+    int four[4];
+    if (ck > 1) {
+      four[0] = four[1] = four[2] = four[3] = 0;
+      for (int k = 0; k < ck; k++) {
+        const int4 v = *reinterpret_cast<const int4*>(recv + ((k << share_log2) + r) * kMidN + 4 * lane);
+        four[0] += v.x; four[1] += v.y; four[2] += v.z; four[3] += v.w;
+      }
+    } else {
+      const int4 v = block_sum(row, 4 * lane);
+      four[0] = v.x; four[1] = v.y; four[2] = v.z; four[3] = v.w;
+    }
+    const uint32_t w = finish4(a, four, q, chan, lut, 0u);
+    int8_t* o = a.out + (long long)(row0 + row) * a.ldc + chan;
+    if (a.vec && left >= 4) *reinterpret_cast<uint32_t*>(o) = w;
+    else store_bytes(o, w, left);
+  }
+}
+
 int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace
@@ -378,6 +550,44 @@ cudaError_t launch_conv_small(const ConvSmallArgs& args, cudaStream_t stream) {
   const bool ragged = a.IC % 16 != 0;
   const Kernel kernel = a.mode == kStem ? conv_small_kernel<kStem, 1, false, false> : kernels[ragged][a.mode == kConv][ks_n > 1][u - 1];
   return launch_dependent_if(true, kernel, grid, block, smem, stream, a);
+}
+
+namespace {
+// log2 of the K slices: while they fill idle SMs and a slice keeps two chunks; clusters of eight are slower even where they
+// fit (64 x 4096 -> 4096, us by slices: 20.2 / 13.4 / 9.9 / 19.7)
+int mid_slices(long long M, int N, int K) {
+  const long long blocks = (long long)ceil_div(N, kMidN) * ceil_div(M, kMidM);
+  const int steps = conv_small_steps(1, K);
+  int ks = 0;
+  while (ks < 2 && blocks << (ks + 1) <= current_sm_count() && steps >> (ks + 1) >= 2 * kMidSteps) ks++;
+  return ks;
+}
+}  // namespace
+// A chunk takes about 1.1 us, the tcgen05 kernel about 0.9 us for the same K but a few more to start: ahead of it with K split
+// over blocks, or with a short K while every block has an SM of its own. Here / there in us: 64 x 4096 -> 4096 9.9 / 17.5,
+// 128 x 4096 -> 4096 13.8 / 17.8, 256 x 1024 -> 4096 9.0 / 10.2, 128 x 2048 -> 8192 13.1 / 14.8; without either
+// 256 x 4096 -> 4096 21.3 / 18.4, 128 x 8192 -> 8192 37.7 / 30.8.
+bool rows_mid_applies(long long M, int N, int K) {
+  if (small_kernels_off() || K % 16 != 0 || M <= 4 || N < 256 || K < 512 || K > (1 << 20)) return false;
+  const long long blocks = (long long)ceil_div(N, kMidN) * ceil_div(M, kMidM);
+  return blocks <= current_sm_count() && (mid_slices(M, N, K) > 0 || K <= 2560);
+}
+cudaError_t launch_rows_mid(const ConvSmallArgs& args, cudaStream_t stream) {
+  ConvSmallArgs a = args;
+  a.n_tiles = ceil_div(a.N, kTileN);
+  a.steps = conv_small_steps(1, a.IC);
+  a.chunks = a.IC / 16;
+  a.vec = a.ldc % 4 == 0 && ((uintptr_t)a.out & 3) == 0;
+  const int nb = ceil_div(a.N, kMidN), mb = ceil_div(a.M, kMidM);
+  a.ks_log2 = mid_slices(a.M, a.N, a.IC);
+  static std::atomic<unsigned long long> attr_done{0};
+  if (first_use_on_device(attr_done)) {
+    const cudaError_t e = cudaFuncSetAttribute(rows_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMidSmem);
+    if (e != cudaSuccess) return e;
+    mark_used_on_device(attr_done);
+  }
+  return launch_dependent_cluster(1 << a.ks_log2, rows_mid_kernel, dim3((unsigned)(nb << a.ks_log2), (unsigned)mb), dim3(kMidThreads), (size_t)kMidSmem,
+                                  stream, true, a);
 }
 
 }  // namespace tb200

@@ -244,6 +244,9 @@ int conv_small_columns(int OC);
 void conv_small_pack(const int8_t* w, int OC, int taps, int IC, int8_t* out);
 void conv_small_pack_stem(const int8_t* w, int OC, int8_t* out);  // [OC][27] -> conv_small_columns(OC) * 64 bytes (mode 2)
 cudaError_t launch_conv_small(const ConvSmallArgs& a, cudaStream_t stream);
+// products of a few dozen rows (mode 0, no add behind them; weights packed as above)
+bool rows_mid_applies(long long M, int N, int K);
+cudaError_t launch_rows_mid(const ConvSmallArgs& a, cudaStream_t stream);
 
 // ---- decoder kernels (decoder.cu): bf16 tensors are passed as uint16_t bit patterns ----
 void launch_embed(const int32_t* tok, const int8_t* table, const uint16_t* scale, uint16_t* out, int B, int H, int V,

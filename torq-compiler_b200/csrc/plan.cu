@@ -1026,7 +1026,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         const long long M = (long long)N * OH * OW;
         // Small problems (conv_small.cu): the same two families of products, on kernels that are latency-bound differently.
         // The step keeps the name of the family, whichever kernel the size picks.
-        auto plan_small = [&](const char* family, int rows_per_group) {
+        auto plan_small = [&](const char* family, int rows_per_group, Loc x_at, cudaError_t (*launcher)(const ConvSmallArgs&, cudaStream_t)) {
           const int G = rows_per_group;  // rows read as one (block-diagonal weights) to make a row a multiple of 16 bytes
           ConvSmallArgs sa{};
           const bool stem = !pointwise && IC == 3;
@@ -1063,7 +1063,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           const size_t c_off = b.add_const(cps.data(), cps.size() * sizeof(ChanParams));
           const size_t q_off = sa.epi ? b.add_const(q4s.data(), q4s.size() * sizeof(int4)) : 0;
           const int fused_add = add_after[i];
-          Loc lx = loc(op.in0), lo = loc(fused_add >= 0 ? ops[fused_add].out0 : result_id), lres{};
+          Loc lx = x_at, lo = loc(fused_add >= 0 ? ops[fused_add].out0 : result_id), lres{};
           if (fused_add >= 0) {
             BinaryArgs add{};
             binary_args_of(ops[fused_add], add);
@@ -1084,14 +1084,14 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             k.q4 = k.epi ? (const int4*)(c.consts + q_off) : nullptr;
             k.lut = has_lut ? (const int8_t*)(c.consts + lut_off) : nullptr;
             k.res = fused_add >= 0 ? (const int8_t*)lres.resolve(c) : nullptr;
-            const cudaError_t e = launch_conv_small(k, c.stream);
+            const cudaError_t e = launcher(k, c.stream);
             if (e != cudaSuccess && c.launch_error) *c.launch_error = e;
           };
         };
         const bool few_rows = M <= 4 && K % 16 == 0 && K <= 12288;  // fc_rows below
         if (add_after[i] >= 0 ? add_fits_small[i] != 0
                               : pointwise && op.weight_zp == 0 && !force_simt() && !few_rows && pointwise_takes_small(M, K, OC)) {
-          plan_small("gemm_i8_tcgen05", pointwise_small_group(M, K));
+          plan_small("gemm_i8_tcgen05", pointwise_small_group(M, K), loc(op.in0), launch_conv_small);
           break;
         }
         const int IC16 = (IC + 15) / 16 * 16, OC16 = (OC + 15) / 16 * 16;
@@ -1101,7 +1101,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             (IC != 16 || OC != OC16 || conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).halo ||
              conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).s2) &&
             conv_small_applies(M, OC, KH * KW, IC)) {
-          plan_small("conv_igemm_i8_tcgen05", 1);
+          plan_small("conv_igemm_i8_tcgen05", 1, loc(op.in0), launch_conv_small);
           break;
         }
         // Rows that are no multiple of 16 bytes (ragged_rows.cu): the layer runs on padded copies in scratch. A product whose rows
@@ -1109,10 +1109,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         // than through a second launch.
         Loc x_loc = loc(op.in0), y_loc = loc(result_id);
         std::vector<int8_t> w_ragged;
+        bool mid = false;  // a product of a few dozen rows
         if (add_after[i] < 0 && op.weight_zp == 0 && !force_simt() && (pointwise || conv_on_tc)) {
-          const bool pad = IC != IC16 && (!pointwise || !pointwise_takes_gemm_tc(M, K, OC, 0));
+          const bool pad = IC != IC16 && (!pointwise || !pointwise_takes_gemm_tc(M, K, OC, 0) || rows_mid_applies(M, OC, IC16));
           const int ICn = pad ? IC16 : IC;
-          const bool trim = OC != OC16 && (!pointwise || (M > 4 && OC * pointwise_row_group(M, ICn, OC) % 16 != 0 && M * OC >= kTrimBytes));
+          mid = pointwise && rows_mid_applies(M, OC, ICn);
+          const bool trim = OC != OC16 && !mid && (!pointwise || (M > 4 && OC * pointwise_row_group(M, ICn, OC) % 16 != 0 && M * OC >= kTrimBytes));
           if (pad || trim) {
             const int OCn = trim ? OC16 : OC, ic = IC, oc = OC;
             w_ragged.assign((size_t)OCn * KH * KW * ICn, 0);
@@ -1139,6 +1141,10 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             OC = OCn;
             K = (long long)KH * KW * IC;
           }
+        }
+        if (mid) {
+          plan_small("gemm_i8_tcgen05", 1, x_loc, launch_rows_mid);
+          break;
         }
         // At most four rows: a weight-streaming dp4a kernel instead of 128-row tensor-core tiles (the weights are the
         // only traffic that counts there; 4 x K bytes of activations fit any SM's shared memory up to K = 12288)
@@ -1392,7 +1398,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         // the stem of an image network on a small frame
         if (!fc && IC == 3 && KH == 3 && KW == 3 && op.stride_h == op.stride_w && op.dil_h == 1 && op.dil_w == 1 && op.weight_zp == 0 &&
             !force_simt() && conv_small_applies(M, OC, 1, 16)) {
-          plan_small("conv2d_stem333_dp4a", 1);
+          plan_small("conv2d_stem333_dp4a", 1, loc(op.in0), launch_conv_small);
           break;
         }
         const int Kpad = (int)((K + 31) / 32 * 32);
