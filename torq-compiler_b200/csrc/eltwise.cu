@@ -126,6 +126,62 @@ __global__ void __launch_bounds__(kThreads) table_kernel(const int8_t* __restric
   for (long long i = (nvec << 4) + tid; i < n; i += stride) out[i] = (int8_t)lut[(uint8_t)x[i]];
 }
 
+// ---- concatenation along the channels (ConcatOpPattern: every operand rescaled to the result's scale) ----
+// All operands of a chain in one launch that writes whole rows. Bound by memory: a copy per operand wrote pieces of 16 .. 256
+// bytes of every row and paid a launch for each - the 38 copies of YOLOv8n took 388 us at 64 frames, 13 launches of this
+// kernel take 257 us (128 us of HBM time). A thread
+// has kConcatFlight units in flight; a unit's row comes from one 32-bit division.
+constexpr int kConcatFlight = 4;
+template <bool LUT>
+__global__ void __launch_bounds__(kThreads) concat_kernel(const __grid_constant__ ConcatArgs a) {
+  __shared__ uint8_t lut[LUT ? kConcatMax : 1][256];
+  if (LUT) {
+    for (int o = 0; o < a.n; o++)
+      if (a.lut[o]) lut[LUT ? o : 0][threadIdx.x] = a.lut[o][threadIdx.x];
+    __syncthreads();
+  }
+  grid_dependency_wait();
+  grid_dependency_release();
+  const long long total = a.rows * a.row_units, stride = (long long)gridDim.x * kThreads;
+  for (long long i0 = (long long)blockIdx.x * kThreads + threadIdx.x; i0 < total; i0 += kConcatFlight * stride) {
+    uint4 v[kConcatFlight];
+    int op[kConcatFlight];
+#pragma unroll
+    for (int u = 0; u < kConcatFlight; u++) {
+      const long long i = i0 + u * stride;
+      v[u] = make_uint4(0, 0, 0, 0);
+      op[u] = 0;
+      if (i < total) {
+        long long r;
+        if (total < (1ll << 32)) r = (uint32_t)i / (uint32_t)a.row_units;
+        else r = i / a.row_units;
+        const int c = (int)(i - r * a.row_units);
+        const int8_t* x = a.x[0];
+        int units = a.units[0], at = c;
+#pragma unroll
+        for (int o = 1; o < kConcatMax; o++)
+          if (o < a.n && c >= a.first[o]) {
+            x = a.x[o];
+            units = a.units[o];
+            at = c - a.first[o];
+            op[u] = o;
+          }
+        v[u] = __ldcs(reinterpret_cast<const uint4*>(x) + r * units + at);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kConcatFlight; u++) {
+      const long long i = i0 + u * stride;
+      if (i >= total) break;
+      if (LUT && a.lut[op[u]]) {
+        const uint8_t* t = lut[LUT ? op[u] : 0];
+        v[u] = make_uint4(lut_word(t, v[u].x), lut_word(t, v[u].y), lut_word(t, v[u].z), lut_word(t, v[u].w));
+      }
+      reinterpret_cast<uint4*>(a.out)[i] = v[u];
+    }
+  }
+}
+
 // ---- standalone rescale i8 -> i8 (PatternUtils.cpp:426-435,3441-3451) ----
 __global__ void __launch_bounds__(kThreads) rescale_kernel(RescaleArgs a) {
   grid_dependency_wait();
@@ -254,6 +310,15 @@ void launch_binary(const BinaryArgs& a, cudaStream_t stream) {
 
 void launch_table(const int8_t* x, const int8_t* table, int8_t* out, long long n, cudaStream_t stream) {
   launch_dependent(table_kernel, dim3(grid_for((n + 15) / 16)), dim3(kThreads), 0, stream, x, table, out, n);
+}
+
+void launch_concat(const ConcatArgs& a, cudaStream_t stream) {
+  bool lut = false;
+  for (int o = 0; o < a.n; o++) lut |= a.lut[o] != nullptr;
+  const long long blocks = (a.rows * a.row_units + kThreads - 1) / kThreads, most = 8ll * current_sm_count();
+  const dim3 grid((unsigned)(blocks < most ? blocks : most));
+  if (lut) launch_dependent(concat_kernel<true>, grid, dim3(kThreads), 0, stream, a);
+  else launch_dependent(concat_kernel<false>, grid, dim3(kThreads), 0, stream, a);
 }
 
 void launch_rescale(const RescaleArgs& a, cudaStream_t stream) {

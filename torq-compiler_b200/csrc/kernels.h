@@ -139,6 +139,18 @@ struct RescaleArgs {
 };
 void launch_rescale(const RescaleArgs& a, cudaStream_t stream);
 
+// concatenation of up to kConcatMax operands along the last axis, each copied or mapped through a 256-entry table
+constexpr int kConcatMax = 8;
+struct ConcatArgs {
+  const int8_t* x[kConcatMax];    // [rows, 16 * units]
+  const uint8_t* lut[kConcatMax]; // indexed by the raw byte, or null = as they are
+  int units[kConcatMax], first[kConcatMax];  // 16-byte units per row of the operand, and of the result in front of it
+  int n, row_units;
+  long long rows;
+  int8_t* out;
+};
+void launch_concat(const ConcatArgs& a, cudaStream_t stream);
+
 // ---- tensor-core GEMM (gemm_tcgen05.cu) ----
 struct GemmTcGeometry {
   int row_bytes;  // bytes of K per shared-memory row: 32, 64 or 128

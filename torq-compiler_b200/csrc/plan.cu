@@ -585,6 +585,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   // place: the inner result becomes the leading columns of the outer one (same storage, the outer
   // row stride) and the outer op only adds its second operand.
   std::vector<int> concat_into(nt, -1);  // inner result tensor -> outer result tensor
+  struct ConcatLeaf { int id, mult, shift, in_zp, out_zp; bool double_round; };
+  std::vector<std::vector<ConcatLeaf>> concat_leaves(ops.size());  // last concat of a chain -> all operands of the chain, in order
   // A 256-entry table that is the only reader of a convolution's result (the reference fuses the same
   // pair: OptimizeSwishActivationPattern.cpp:100-190) is applied in the convolution's epilogue.
   std::vector<int> table_after(ops.size(), -1);  // conv op -> index of its fused table op
@@ -621,6 +623,44 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         continue;
       if (op.in0_mult == (1 << 30) && op.in0_shift == 30 && op.in0_zp == op.out_zp && tensors[a].dtype == TB200_I8)
         concat_into[a] = op.out0;
+    }
+    // The last concatenation of a chain copies all operands of the chain at once (concat_kernel) when they are intermediates in
+    // 16-byte units; operands that are the caller's own buffers keep their copies.
+    for (int i = 0; i < (int)ops.size(); i++) {
+      const auto& last = ops[i];
+      if (last.kind != TB200_OP_CONCAT || last.out0 < 0 || last.out0 >= nt || concat_into[last.out0] >= 0) continue;
+      std::vector<ConcatLeaf> leaves;
+      std::vector<int> inner;
+      bool fits = true;
+      for (int at = i;;) {
+        const auto& op = ops[at];
+        fits = fits && op.in0 >= 0 && op.in0 < nt && op.in1 >= 0 && op.in1 < nt;
+        if (!fits) break;
+        leaves.push_back({op.in1, op.in1_mult, op.in1_shift, op.in1_zp, op.out_zp, op.double_round != 0});
+        if (concat_into[op.in0] == op.out0) {
+          at = producer[op.in0];
+          inner.push_back(at);
+          continue;
+        }
+        leaves.push_back({op.in0, op.in0_mult, op.in0_shift, op.in0_zp, op.out_zp, op.double_round != 0});
+        break;
+      }
+      std::reverse(leaves.begin(), leaves.end());
+      fits = fits && leaves.size() <= (size_t)kConcatMax && tensors[last.out0].dtype == TB200_I8;
+      int channels = 0;
+      for (const auto& l : leaves) {
+        if (!fits) break;
+        const auto& t = tensors[l.id];
+        fits = t.kind == TB200_TENSOR_ACTIVATION && t.dtype == TB200_I8 && t.rank >= 1 && t.shape[t.rank - 1] % 16 == 0 && l.shift >= 2 && l.shift <= 62;
+        channels += fits ? t.shape[t.rank - 1] : 0;
+      }
+      const auto& o = tensors[last.out0];
+      if (!fits || o.rank < 1 || o.shape[o.rank - 1] != channels) continue;
+      const size_t rows = b.numel(last.out0) / channels;
+      for (const auto& l : leaves) fits = fits && b.numel(l.id) == rows * tensors[l.id].shape[tensors[l.id].rank - 1];
+      if (!fits) continue;
+      concat_leaves[i] = std::move(leaves);
+      for (int k : inner) fused_away[k] = 1;
     }
     const char* no_fuse = getenv("TB200_NO_TABLE_FUSION");
     // the pooling windows with a strip kernel apply a table the same way
@@ -807,6 +847,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       if (tensors[op.out0].kind == TB200_TENSOR_ACTIVATION) root[op.out0] = root[op.in0];
     }
   }
+  for (int i = 0; i < (int)ops.size(); i++)
+    for (const auto& l : concat_leaves[i]) last_use[root[l.id]] = std::max(last_use[root[l.id]], i);
   auto bytes_of = [&](int id) {
     size_t n = b.numel(id);
     switch (tensors[id].dtype) {
@@ -897,6 +939,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
     if (fused_away[i]) {
       step.kernel_name = op.kind == TB200_OP_RMSNORM ? "(norm fused into the previous norm)"
                          : op.kind == TB200_OP_ADD   ? "(add in the convolution's epilogue)"
+                         : op.kind == TB200_OP_CONCAT ? "(in the concatenation behind it)"
                          : op.kind == TB200_OP_TRANSPOSE || op.kind == TB200_OP_EW ? "(in the op it feeds or follows)"
                                                      : "(table in the producer's epilogue)";
       step.launches = 0;
@@ -1701,6 +1744,40 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: concat (channel axis) shape mismatch", i);
         for (int s : {op.in0_shift, op.in1_shift})
           if (s < 2 || s > 62) return b.fail(TB200_INVALID_ARGUMENT, "op %d: rescale shift %d outside [2,62]", i, s);
+        if (!concat_leaves[i].empty()) {
+          ConcatArgs ca{};
+          ca.n = (int)concat_leaves[i].size();
+          ca.rows = (long long)rows;
+          std::vector<Loc> from;
+          std::vector<size_t> lut_off;
+          for (int k = 0; k < ca.n; k++) {
+            const ConcatLeaf& l = concat_leaves[i][k];
+            ca.units[k] = tensors[l.id].shape[tensors[l.id].rank - 1] / 16;
+            ca.first[k] = ca.row_units;
+            ca.row_units += ca.units[k];
+            from.push_back(loc(l.id));
+            lut_off.push_back(SIZE_MAX);
+            if (l.mult == (1 << 30) && l.shift == 30 && l.in_zp == l.out_zp) continue;
+            uint8_t table[256];
+            for (int v = 0; v < 256; v++) {
+              const long long r = host_apply_scale_32((int)(int8_t)v - l.in_zp, l.mult, l.shift, l.double_round) + l.out_zp;
+              table[v] = (uint8_t)(int8_t)std::max(-128ll, std::min(127ll, r));
+            }
+            lut_off.back() = b.add_const(table, 256);
+          }
+          const Loc to = loc(op.out0);
+          step.kernel_name = "concat_rescale";
+          step.launch = [=](const ExecContext& c) {
+            ConcatArgs k = ca;
+            for (int q = 0; q < k.n; q++) {
+              k.x[q] = (const int8_t*)from[q].resolve(c);
+              k.lut[q] = lut_off[q] == SIZE_MAX ? nullptr : (const uint8_t*)(c.consts + lut_off[q]);
+            }
+            k.out = (int8_t*)to.resolve(c);
+            launch_concat(k, c.stream);
+          };
+          break;
+        }
         ChanParams p0{}, p1{};
         p0.mult = op.in0_mult; p0.shift = op.in0_shift; p1.mult = op.in1_mult; p1.shift = op.in1_shift;
         Builder::fill_rounding(p0, op.double_round != 0);
