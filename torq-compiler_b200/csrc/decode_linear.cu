@@ -17,6 +17,7 @@
 
 #include "dependent_launch.cuh"
 #include "kernels.h"
+#include "linear_shape.h"
 
 namespace tb200 {
 namespace {
@@ -92,9 +93,6 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 //   kStream: one group and a warp per tile, blocks stay and walk the tiles (the LM head); fp32 or bf16 results and, with
 //            cand_v, the block's arg-max candidates per token.
 // ---------------------------------------------------------------------------------------------------------------
-enum { kStore = 0, kGeglu = 1, kRope = 2, kStream = 3 };
-constexpr int kTileRows = 32, kBlk = 64, kStageBytes = kTileRows * kBlk, kStreamStages = 4;
-constexpr int kRopeTokens = 8;  // most tokens a warp finishes in the RoPE epilogue
 
 template <int NT, int MODE>
 __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
@@ -152,7 +150,9 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
       const int t = row_block * a.rt + i / kTileRows;
       scale_s[i] = row_valid(t, i % kTileRows) ? bf2f(__ldg(a.scale + weight_row(t, i % kTileRows))) : 0.f;
     }
-  if (MODE == kRope || a.ck > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
+  // Waited for before the first remote store: it says that the block runs, not how far it is, so a peer may only store into
+  // memory that nothing else of the block uses (recv_off).
+  if (MODE == kRope || a.ck > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   grid_dependency_wait();
   grid_dependency_release();
 
@@ -391,8 +391,8 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
   } else {
     // one head of 256 rows per cluster, 32 rows per block: lane = row
     // rank = 32 rows of the head; rows i and i + 128 rotate together, so blocks part and part ^ 4 exchange their values
-    float* ss = sums + a.kg * (kTileRows * kPitch);  // [block][tokens] sums of squares
-    float* nv = ss + 8 * kTok;                       // [tokens][32] the partner's values
+    float* ss = recv;            // [block][tokens] sums of squares
+    float* nv = ss + 8 * kTok;   // [tokens][32] the partner's values
     const float scale = scale_s[lane];
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     float own[kRopeTokens];
@@ -793,81 +793,6 @@ __global__ void __launch_bounds__(512) rmsnorm_row_kernel(const uint16_t* __rest
     for (int e = 0; e < 4; e++) o[e] = f2bf(v[k][e] * inv2 * (1.0f + f[e]));
     if (i < H) *reinterpret_cast<uint2*>(out2 + base + i) = make_uint2(o[0] | (uint32_t)o[1] << 16, o[2] | (uint32_t)o[3] << 16);
   }
-}
-
-int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
-
-// groups of K of a product: enough warps to ask for every weight at once, none without a 64-byte block
-int linear_groups(int N, int K) {
-  const int tiles = ceil_div(N, kTileRows), blocks = K / kBlk;
-  const int cap = K <= 4096 ? 16 : 32;
-  int tk = 1;
-  while (tk * 2 <= blocks && tk < cap && (long long)tiles * tk * 2 <= 12 * 148) tk *= 2;
-  return tk;
-}
-
-struct LinearShape {
-  int tk, kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, smem, tiles, grid;
-  bool ok;
-};
-constexpr int kSmemMax = 227 * 1024 - 1024;
-
-LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
-  LinearShape s{};
-  if (K % kBlk != 0 || K < kBlk || B < 1 || B > 32 || N < 1) return s;
-  const int tok = ceil_div(B, 8) * 8, blocks = K / kBlk;
-  s.tk = linear_groups(N, K);
-  if (mode == kStore && s.tk == 1) mode = kStream;
-  s.tiles = mode == kGeglu ? ceil_div(N / 2, 16) : ceil_div(N, kTileRows);
-  auto fit = [&](int kg, int ck, int rt, int stages) {
-    s.kg = kg; s.ck = ck; s.rt = rt; s.stages = stages;
-    int widest = 0;
-    for (int r = 0; r < ck; r++) widest = std::max(widest, blocks * (r * kg + kg) / s.tk - blocks * (r * kg) / s.tk);
-    s.x_pitch = (widest * kBlk * 2 + 127) / 128 * 128 + 16;
-    s.x_bytes = (tok * s.x_pitch + 127) / 128 * 128;
-    const int warps = kg * rt;
-    const int sums = warps * kTileRows * (tok + 1) * 4 + (mode == kRope ? tok * 40 * 4 : 0);
-    s.scale_off = std::max(s.x_bytes + warps * stages * kStageBytes, mode == kStream ? 16 * tok * 8 : (sums + 127) / 128 * 128);
-    s.recv_off = s.scale_off + rt * kTileRows * 4;
-    s.smem = s.recv_off + (ck > 1 ? (rt * B + ck - 1) / ck * ck * 128 : 0);
-    return s.smem <= kSmemMax;
-  };
-  if (mode == kStream) {
-    for (int rt = 16; rt >= 1; rt /= 2)
-      if (fit(1, 1, rt, kStreamStages)) {
-        s.grid = std::min(sms, ceil_div(s.tiles, rt));
-        s.ok = true;
-        return s;
-      }
-    return s;
-  }
-  const int stages = ceil_div(blocks, s.tk);  // every block of a warp has its own place
-  if (stages > 64) return s;
-  if (mode == kRope) {
-    s.ok = s.tk <= 16 && s.tk * kRopeTokens >= tok && fit(s.tk, 1, 1, stages);
-    s.grid = s.tiles;
-    return s;
-  }
-  // The fewest blocks per cluster whose activations leave room and whose clusters are all resident at once (a second wave cost
-  // 7 us): clusters do not cross a GPC, of which eight with 16 SMs are counted on.
-  auto one_wave = [&]() {
-    const int clusters = s.grid / s.ck, per_sm = std::max(1, std::min(2048 / (s.kg * s.rt * 32), kSmemMax / s.smem));
-    return s.ck == 1 ? s.grid <= sms * per_sm : clusters <= 8 * (16 / s.ck) * std::min(per_sm, 2);
-  };
-  for (int pass = 0; pass < 2; pass++)
-    for (int ck = 1; ck <= 8 && ck <= s.tk; ck *= 2) {
-      const int kg = s.tk / ck;
-      if (kg > 16) continue;
-      int rt = std::max(1, std::min(ceil_div((long long)s.tiles * ck, sms), 16 / kg));
-      while (rt > 1 && !fit(kg, ck, rt, stages)) rt--;
-      for (; rt <= 16 / kg && fit(kg, ck, rt, stages); rt++) {
-        s.grid = ceil_div(s.tiles, rt) * ck;
-        if (pass == 0 && !one_wave()) continue;
-        s.ok = true;
-        return s;
-      }
-    }
-  return LinearShape{};
 }
 
 template <int NT, int MODE>

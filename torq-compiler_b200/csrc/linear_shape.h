@@ -1,0 +1,101 @@
+// How a product of decode_linear.cu is cut into warps, blocks and clusters, and what lies where in a block's shared memory.
+// Host code only, so that the layout can be checked without a GPU.
+//
+// Shared memory of a block, in order:
+//   [0, x_bytes)                  staged activations
+//   [x_bytes, + rings)            every warp's weight ring; both are overwritten by the groups' sums once all warps have multiplied
+//   [scale_off, + rt * 32 * 4)    scales of the block's rows
+//   [recv_off, smem)              what other blocks of the cluster store into this one: nothing else uses it, because a peer that
+//                                 is ahead stores while this block is still staging or multiplying
+#pragma once
+#include <algorithm>
+
+namespace tb200 {
+
+// modes of linear_w8_kernel
+enum { kStore = 0, kGeglu = 1, kRope = 2, kStream = 3 };
+constexpr int kTileRows = 32, kBlk = 64, kStageBytes = kTileRows * kBlk, kStreamStages = 4;
+constexpr int kRopeTokens = 8;  // most tokens a warp finishes in the RoPE epilogue
+constexpr int kSmemMax = 227 * 1024 - 1024;
+
+inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+// groups of K of a product: enough warps to ask for every weight at once, none without a 64-byte block
+inline int linear_groups(int N, int K) {
+  const int tiles = ceil_div(N, kTileRows), blocks = K / kBlk;
+  const int cap = K <= 4096 ? 16 : 32;
+  int tk = 1;
+  while (tk * 2 <= blocks && tk < cap && (long long)tiles * tk * 2 <= 12 * 148) tk *= 2;
+  return tk;
+}
+
+struct LinearShape {
+  int tk, kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, smem, tiles, grid;
+  bool ok;
+};
+
+// bytes other blocks store into one: the RoPE epilogue's sums of squares and partner values, or the sums of a cluster's K slices
+inline int linear_recv_bytes(int B, int mode, int ck, int rt) {
+  if (mode == kRope) return ceil_div(B, 8) * 8 * (8 + 32) * 4;
+  return ck > 1 ? (rt * B + ck - 1) / ck * ck * 128 : 0;
+}
+
+inline LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
+  LinearShape s{};
+  if (K % kBlk != 0 || K < kBlk || B < 1 || B > 32 || N < 1) return s;
+  const int tok = ceil_div(B, 8) * 8, blocks = K / kBlk;
+  s.tk = linear_groups(N, K);
+  if (mode == kStore && s.tk == 1) mode = kStream;
+  s.tiles = mode == kGeglu ? ceil_div(N / 2, 16) : ceil_div(N, kTileRows);
+  auto fit = [&](int kg, int ck, int rt, int stages) {
+    s.kg = kg; s.ck = ck; s.rt = rt; s.stages = stages;
+    int widest = 0;
+    for (int r = 0; r < ck; r++) widest = std::max(widest, blocks * (r * kg + kg) / s.tk - blocks * (r * kg) / s.tk);
+    s.x_pitch = (widest * kBlk * 2 + 127) / 128 * 128 + 16;
+    s.x_bytes = (tok * s.x_pitch + 127) / 128 * 128;
+    const int warps = kg * rt;
+    const int sums = warps * kTileRows * (tok + 1) * 4;
+    s.scale_off = std::max(s.x_bytes + warps * stages * kStageBytes, mode == kStream ? 16 * tok * 8 : (sums + 127) / 128 * 128);
+    s.recv_off = s.scale_off + rt * kTileRows * 4;
+    s.smem = s.recv_off + linear_recv_bytes(B, mode, ck, rt);
+    return s.smem <= kSmemMax;
+  };
+  if (mode == kStream) {
+    for (int rt = 16; rt >= 1; rt /= 2)
+      if (fit(1, 1, rt, kStreamStages)) {
+        s.grid = std::min(sms, ceil_div(s.tiles, rt));
+        s.ok = true;
+        return s;
+      }
+    return s;
+  }
+  const int stages = ceil_div(blocks, s.tk);  // every block of a warp has its own place
+  if (stages > 64) return s;
+  if (mode == kRope) {
+    s.ok = s.tk <= 16 && s.tk * kRopeTokens >= tok && fit(s.tk, 1, 1, stages);
+    s.grid = s.tiles;
+    return s;
+  }
+  // The fewest blocks per cluster whose activations leave room and whose clusters are all resident at once (a second wave cost
+  // 7 us): clusters do not cross a GPC, of which eight with 16 SMs are counted on.
+  auto one_wave = [&]() {
+    const int clusters = s.grid / s.ck, per_sm = std::max(1, std::min(2048 / (s.kg * s.rt * 32), kSmemMax / s.smem));
+    return s.ck == 1 ? s.grid <= sms * per_sm : clusters <= 8 * (16 / s.ck) * std::min(per_sm, 2);
+  };
+  for (int pass = 0; pass < 2; pass++)
+    for (int ck = 1; ck <= 8 && ck <= s.tk; ck *= 2) {
+      const int kg = s.tk / ck;
+      if (kg > 16) continue;
+      int rt = std::max(1, std::min(ceil_div((long long)s.tiles * ck, sms), 16 / kg));
+      while (rt > 1 && !fit(kg, ck, rt, stages)) rt--;
+      for (; rt <= 16 / kg && fit(kg, ck, rt, stages); rt++) {
+        s.grid = ceil_div(s.tiles, rt) * ck;
+        if (pass == 0 && !one_wave()) continue;
+        s.ok = true;
+        return s;
+      }
+    }
+  return LinearShape{};
+}
+
+}  // namespace tb200
