@@ -45,6 +45,17 @@ def test_small_convolution(device, case, clamp, table, monkeypatch):
     _both(device, g, [rng.integers(-128, 128, (N, H, W, IC), dtype=np.int8)], monkeypatch)
 
 
+@pytest.mark.parametrize("IC,kh,kw", [(6048, 3, 3), (7216, 3, 3), (8512, 2, 2), (7008, 2, 3)])
+def test_channels_beyond_a_short_reciprocal(device, IC, kh, kw, monkeypatch):
+    """Chunks of the K axis whose tap a 20-bit reciprocal got wrong, with every tap at a border of the frame somewhere."""
+    rng = np.random.default_rng(IC)
+    g = Graph()
+    m, s = _ms(rng, 32, kh * kw * IC)
+    g.output(g.conv2d(g.input((1, 4, 4, IC)), rng.integers(-127, 128, (32, kh, kw, IC), dtype=np.int8), np.full(32, 50, np.int32), m, s,
+                      pad=(kh // 2, kh // 2, kw // 2, kw // 2), input_zp=-9, out_zp=4))
+    _both(device, g, [rng.integers(-128, 128, (1, 4, 4, IC), dtype=np.int8)], monkeypatch)
+
+
 @pytest.mark.parametrize("C,H,W,st,clamp", [(4, 1, 1, 1, (-128, 127)), (20, 5, 7, 1, (-128, 127)), (36, 9, 8, 2, (4, 127)), (128, 6, 33, 1, (-20, 90)),
                                             (16, 12, 3, 2, (-128, 127))])
 def test_few_depthwise_outputs(device, C, H, W, st, clamp, monkeypatch):

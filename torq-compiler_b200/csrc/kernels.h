@@ -247,7 +247,8 @@ struct ConvSmallArgs {
   int add_m_self, add_m_other, add_f, add_clamp_min, add_clamp_max;  // BinaryArgs::lin_*
   long long add_k;
   // filled by the launcher
-  int m_tiles, n_tiles, steps, chunks, icb, inv_icb, inv_kw, ks_log2, vec;
+  int m_tiles, n_tiles, steps, chunks, icb, ks_log2, vec;
+  uint32_t inv_icb, inv_kw;  // divide_constant
 };
 bool conv_small_applies(long long M, int OC, int taps, int IC);  // is this the faster kernel for the size
 int conv_small_steps(int taps, int IC);
