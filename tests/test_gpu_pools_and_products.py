@@ -38,6 +38,22 @@ def test_strip_pools(device, k, s, shape, table):
         _check(device, g, [x])
 
 
+@pytest.mark.parametrize("kind", ["max", "avg"])
+@pytest.mark.parametrize("shape", [(65535, 2, 2, 4), (65536, 2, 2, 4), (1, 131070, 2, 3), (1, 131074, 2, 3)])
+def test_table_behind_a_pool_at_the_strips_grid_limits(device, kind, shape):
+    """More images or rows than a strip's grid takes: the pool and its table run as two launches."""
+    rng = np.random.default_rng(shape[1])
+    x = rng.integers(-128, 128, shape, dtype=np.int8)
+    g = Graph()
+    xi = g.input(shape)
+    y = g.maxpool2d(xi, (2, 2), (2, 2)) if kind == "max" else g.avg_pool2d(xi, (2, 2), (2, 2), input_zp=-9, output_zp=5)
+    g.output(g.table(y, rng.integers(-128, 128, 256).astype(np.int8)))
+    ex = Executable(device, g.serialize())
+    assert ex.launch_count == (1 if max(shape[0], shape[1] // 2) <= 65535 else 2), ex.op_kernels()
+    ex.destroy()
+    _check(device, g, [x])
+
+
 @pytest.mark.parametrize("n", [1, 15, 16, 4099])
 @pytest.mark.parametrize("scales", [(0.02, 0.1, 0.05), (0.07, 0.03, 0.09), (0.05, 0.05, 0.02)])
 def test_rescaled_add_covers_every_operand_pair(device, n, scales):

@@ -103,7 +103,7 @@ struct PoolArgs {
   const int8_t* lut;        // fused 256-entry table, or null (only where pool_strip_applies)
   const int4* by_count;     // average pool: pool_avg_records on the device, or null
 };
-bool pool_strip_applies(const PoolArgs& a);  // the window (not the sizes) decides
+bool pool_strip_applies(const PoolArgs& a);  // by window and strides, element type, N and OH (grid limits); the rest is not looked at
 // Records {M', -, K} by tap count (index 0 unused) of pool_strip_kernel's average; false when a count has no exact one.
 bool pool_avg_records(int taps, int input_zp, int output_zp, std::vector<int4>& out);
 void launch_maxpool(const PoolArgs& a, cudaStream_t stream);

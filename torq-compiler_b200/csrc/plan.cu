@@ -663,12 +663,13 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       for (int k : inner) fused_away[k] = 1;
     }
     const char* no_fuse = getenv("TB200_NO_TABLE_FUSION");
-    // the pooling windows with a strip kernel apply a table the same way
-    auto takes_table = [](const tb200_op_t& o) {
+    // the pools that run as strips (a rule on the window and the sizes, so asked with both) apply a table the same way
+    auto takes_table = [&](const tb200_op_t& o) {
       if (o.kind == TB200_OP_CONV2D) return true;
-      if (o.kind != TB200_OP_MAXPOOL && o.kind != TB200_OP_AVGPOOL) return false;
+      if ((o.kind != TB200_OP_MAXPOOL && o.kind != TB200_OP_AVGPOOL) || !b.valid_id(o.out0) || tensors[o.out0].rank != 4) return false;
       PoolArgs a{};
       a.KH = o.kh; a.KW = o.kw; a.stride_h = o.stride_h; a.stride_w = o.stride_w;
+      a.N = tensors[o.out0].shape[0]; a.OH = tensors[o.out0].shape[1];
       std::vector<int4> rec;
       return pool_strip_applies(a) && (o.kind == TB200_OP_MAXPOOL || pool_avg_records(o.kh * o.kw, o.in0_zp, o.out_zp, rec));
     };
