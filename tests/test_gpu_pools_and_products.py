@@ -92,6 +92,19 @@ def test_tiled_products(device, M, K, N, dtype, transposed):
     _check(device, g, [a, b])
 
 
+@pytest.mark.parametrize("M,K,N", [(65536 * 64 + 5, 3, 2), (2, 3, 65536 * 64 + 5)])
+@pytest.mark.parametrize("dtype", ["bf16", "i8"])
+def test_products_of_more_tiles_than_a_second_grid_dimension_takes(device, M, K, N, dtype):
+    rng = np.random.default_rng(K)
+    a, b = (rng.integers(-128, 128, s, dtype=np.int8) for s in ((M, K), (K, N)))
+    if dtype == "bf16":
+        a, b = to_bf16(a.astype(np.float32)), to_bf16(b.astype(np.float32))
+    g = Graph()
+    ai, bi = g.input((M, K), dtype), g.input((K, N), dtype)
+    g.output(g.matmul_i32(ai, bi, a_zp=3, b_zp=-2) if dtype == "i8" else g.matmul_f(ai, bi, "f32"))
+    _check(device, g, [a, b])
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 1), (3, 255), (5, 256), (7, 500), (2, 1024), (4, 1100)])
 def test_softmax_with_its_scalar_and_cast(device, rows, cols):
     x = np.random.default_rng(cols).normal(0, 3, (rows, cols)).astype(np.float32)

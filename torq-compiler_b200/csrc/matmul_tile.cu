@@ -60,14 +60,14 @@ template <> struct AccOf<uint16_t> { typedef float type; };
 
 template <typename TIn, typename TOut, bool TB, int R>
 __global__ void __launch_bounds__(256) matmul_tile_kernel(const TIn* __restrict__ a, const TIn* __restrict__ b, TOut* __restrict__ out,
-                                                          int M, int K, int N, int a_zp, int b_zp) {
+                                                          int M, int K, int N, int n_tiles, int a_zp, int b_zp) {
   typedef typename AccOf<TIn>::type Acc;
   constexpr int T = 16 * R;
   constexpr int kKC = 128 / R;  // k per stage: two groups of four elements per thread and operand whatever the tile
   constexpr int kPitch = kKC + 4;
   __shared__ __align__(16) Acc as[T][kPitch], bs[T][kPitch];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * T, n0 = blockIdx.x * T;
+  const int m0 = (int)(blockIdx.x / (unsigned)n_tiles) * T, n0 = (int)(blockIdx.x % (unsigned)n_tiles) * T;
   constexpr int kQuads = T * kKC / 4;            // groups of four elements per operand and stage
   constexpr int kPer = kQuads / 256;             // per thread
   const bool ka = (K & 3) == 0, na = (N & 3) == 0;  // four elements of a row are aligned to their size
@@ -167,7 +167,8 @@ void run(const void* a, const void* b, void* out, int M, int K, int N, int a_zp,
   auto tiles = [&](int t) { return (long long)((M + t - 1) / t) * ((N + t - 1) / t); };
   const int sms = current_sm_count();
   auto go = [&](auto kern, int t) {
-    kern<<<dim3((unsigned)((N + t - 1) / t), (unsigned)((M + t - 1) / t)), 256, 0, stream>>>((const TIn*)a, (const TIn*)b, (TOut*)out, M, K, N, a_zp, b_zp);
+    // one grid dimension: the second ends at 65535 tiles
+    kern<<<(unsigned)tiles(t), 256, 0, stream>>>((const TIn*)a, (const TIn*)b, (TOut*)out, M, K, N, (N + t - 1) / t, a_zp, b_zp);
   };
   if (tiles(64) >= sms) {
     if (tb) go(matmul_tile_kernel<TIn, TOut, true, 4>, 64);
