@@ -56,6 +56,24 @@ def test_channels_beyond_a_short_reciprocal(device, IC, kh, kw, monkeypatch):
     _both(device, g, [rng.integers(-128, 128, (1, 4, 4, IC), dtype=np.int8)], monkeypatch)
 
 
+def test_stem_of_few_pixels_on_a_frame_beyond_two_gigabytes(device):
+    """A wide stride leaves few output pixels, but the offsets into the frame need 64 bits."""
+    from oracle import oracle_np as onp
+    rng = np.random.default_rng(5)
+    S, st, OC = 26760, 110, 16
+    x = np.frombuffer(rng.bytes(S * S * 3), np.int8).reshape(1, S, S, 3)
+    w = rng.integers(-127, 128, (OC, 3, 3, 3), dtype=np.int8)
+    m, s = _ms(rng, OC, 27)
+    g = Graph()
+    g.output(g.conv2d(g.input(x.shape), w, np.full(OC, 50, np.int32), m, s, stride=(st, st), input_zp=-9, out_zp=4))
+    got = run_graph_gpu(device, g, [x])[0][0]
+    n = (S - 3) // st + 1
+    taps = [x[0, kh:kh + st * n:st, kw:kw + st * n:st][:n, :n].astype(np.int64) + 9 for kh in range(3) for kw in range(3)]
+    acc = sum(np.einsum("hwi,oi->hwo", t, w.reshape(OC, 9, 3)[:, k].astype(np.int64)) for k, t in enumerate(taps)) + 50
+    want = onp.requant(onp.wrap32(acc.reshape(-1, OC)), m, s, 4, -128, 127)
+    assert (got.reshape(-1, OC) == want).all()
+
+
 @pytest.mark.parametrize("C,H,W,st,clamp", [(4, 1, 1, 1, (-128, 127)), (20, 5, 7, 1, (-128, 127)), (36, 9, 8, 2, (4, 127)), (128, 6, 33, 1, (-20, 90)),
                                             (16, 12, 3, 2, (-128, 127))])
 def test_few_depthwise_outputs(device, C, H, W, st, clamp, monkeypatch):

@@ -1439,9 +1439,10 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           break;
         }
 
-        // the stem of an image network on a small frame
+        // the stem of an image network on few output pixels (its kernel's offsets into the frame have 32 bits, and a wide stride can
+        // leave few pixels of a frame beyond that)
         if (!fc && IC == 3 && KH == 3 && KW == 3 && op.stride_h == op.stride_w && op.dil_h == 1 && op.dil_w == 1 && op.weight_zp == 0 &&
-            !force_simt() && conv_small_applies(M, OC, 1, 16)) {
+            !force_simt() && conv_small_applies(M, OC, 1, 16) && b.numel(op.in0) < (size_t)INT32_MAX) {
           plan_small("conv2d_stem333_dp4a", 1, loc(op.in0), launch_conv_small);
           break;
         }
