@@ -118,3 +118,21 @@ def test_softmax_with_its_scalar_and_cast(device, rows, cols):
     got = from_bf16(run_graph_gpu(device, g, [x])[0])
     e = np.exp((x * np.float32(0.37)).astype(np.float64) - (x * np.float32(0.37)).max(-1, keepdims=True))
     assert np.allclose(got, e / e.sum(-1, keepdims=True), rtol=2 ** -7, atol=1e-30)
+
+
+@pytest.mark.parametrize("cols", [200, 500, 1000, 1025, 3000])
+def test_folded_scalar_rounds_as_the_multiplication_does(device, cols):
+    """softmax(x * s) in one launch against the same two ops apart (the product is an output too): the same bits."""
+    x = np.random.default_rng(cols).normal(0, 20, (64, cols)).astype(np.float32)
+    got = []
+    for apart in (False, True):
+        g = Graph()
+        y = g.ew("mul", g.input(x.shape, "f32"), g.const(np.full((1, 1), 0.37, np.float32)))
+        g.output(g.softmax(y))
+        if apart:
+            g.output(y)
+        ex = Executable(device, g.serialize())
+        assert ex.launch_count == 1 + apart, ex.op_kernels()
+        ex.destroy()
+        got.append(run_graph_gpu(device, g, [x])[0])
+    assert (got[0].view(np.uint32) == got[1].view(np.uint32)).all(), int((got[0] != got[1]).sum())

@@ -279,11 +279,12 @@ __global__ void __launch_bounds__(128) softmax_kernel(SoftmaxArgs a) {
   const TIn* x = reinterpret_cast<const TIn*>(a.x) + row * a.cols;
   TOut* out = reinterpret_cast<TOut*>(a.out) + row * a.cols;
   const float scale = a.scale ? *a.scale : 1.0f;
+  auto scaled = [&](int c) { return __fmul_rn(as_float(x[c]), scale); };  // rounded: not contracted with the subtraction behind it
   float m = -INFINITY, sum = 0.f;
   if (PER > 0) {
     float v[PER > 0 ? PER : 1];
 #pragma unroll
-    for (int j = 0; j < PER; j++) v[j] = lane + 32 * j < a.cols ? as_float(x[lane + 32 * j]) * scale : -INFINITY;
+    for (int j = 0; j < PER; j++) v[j] = lane + 32 * j < a.cols ? scaled(lane + 32 * j) : -INFINITY;
 #pragma unroll
     for (int j = 0; j < PER; j++) m = fmaxf(m, v[j]);
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -300,12 +301,12 @@ __global__ void __launch_bounds__(128) softmax_kernel(SoftmaxArgs a) {
       if (lane + 32 * j < a.cols) softmax_out<TIn>(out + lane + 32 * j, v[j] * inv);
     return;
   }
-  for (int c = lane; c < a.cols; c += 32) m = fmaxf(m, as_float(x[c]) * scale);
+  for (int c = lane; c < a.cols; c += 32) m = fmaxf(m, scaled(c));
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  for (int c = lane; c < a.cols; c += 32) sum += expf(as_float(x[c]) * scale - m);
+  for (int c = lane; c < a.cols; c += 32) sum += expf(scaled(c) - m);
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = 1.0f / sum;
-  for (int c = lane; c < a.cols; c += 32) softmax_out<TIn>(out + c, expf(as_float(x[c]) * scale - m) * inv);
+  for (int c = lane; c < a.cols; c += 32) softmax_out<TIn>(out + c, expf(scaled(c) - m) * inv);
 }
 
 unsigned grid_for(long long n) {
