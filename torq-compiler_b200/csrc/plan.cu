@@ -82,6 +82,13 @@ struct Builder {
     return reinterpret_cast<const T*>(constants.data() + t.const_offset);
   }
 
+  bool same_shape(int a, int b) const {
+    if (tensors[a].rank != tensors[b].rank) return false;
+    for (uint32_t d = 0; d < tensors[a].rank; d++)
+      if (tensors[a].shape[d] != tensors[b].shape[d]) return false;
+    return true;
+  }
+
   size_t numel(int id) const {
     const auto& t = tensors[id];
     size_t n = 1;
@@ -626,6 +633,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
     }
     // The last concatenation of a chain copies all operands of the chain at once (concat_kernel) when they are intermediates in
     // 16-byte units; operands that are the caller's own buffers keep their copies.
+    auto adds_up = [&](const tb200_op_t& op) {  // the op's own check of its shapes, which a fused op would not get
+      const auto& x0 = tensors[op.in0]; const auto& x1 = tensors[op.in1]; const auto& o = tensors[op.out0];
+      if (x0.rank < 1 || x1.rank < 1 || o.rank < 1 || x0.dtype != TB200_I8 || x1.dtype != TB200_I8 || o.dtype != TB200_I8) return false;
+      const size_t c0 = x0.shape[x0.rank - 1], c1 = x1.shape[x1.rank - 1], co = o.shape[o.rank - 1], rows = b.numel(op.out0) / co;
+      return c0 + c1 == co && b.numel(op.in0) == rows * c0 && b.numel(op.in1) == rows * c1;
+    };
     for (int i = 0; i < (int)ops.size(); i++) {
       const auto& last = ops[i];
       if (last.kind != TB200_OP_CONCAT || last.out0 < 0 || last.out0 >= nt || concat_into[last.out0] >= 0) continue;
@@ -634,7 +647,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       bool fits = true;
       for (int at = i;;) {
         const auto& op = ops[at];
-        fits = fits && op.in0 >= 0 && op.in0 < nt && op.in1 >= 0 && op.in1 < nt;
+        fits = fits && op.in0 >= 0 && op.in0 < nt && op.in1 >= 0 && op.in1 < nt && adds_up(op);
         if (!fits) break;
         leaves.push_back({op.in1, op.in1_mult, op.in1_shift, op.in1_zp, op.out_zp, op.double_round != 0});
         if (concat_into[op.in0] == op.out0) {
@@ -760,7 +773,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
               const int x = side ? mu.in1 : mu.in0, s = side ? mu.in0 : mu.in1;
               // bf16 operands keep their own op: the scalar would be bf16 too
               if (tensors[s].kind != TB200_TENSOR_CONSTANT || b.numel(s) != 1 || tensors[s].dtype != TB200_F32 ||
-                  b.numel(x) != b.numel(op.in0) || b.numel(x) == 1 || tensors[x].dtype != TB200_F32 || tensors[op.in0].dtype != TB200_F32)
+                  tensors[s].rank != tensors[x].rank || !b.same_shape(x, op.in0) || b.numel(x) == 1 || tensors[x].dtype != TB200_F32 || tensors[op.in0].dtype != TB200_F32)
                 continue;
               softmax_scale[i] = t;
               extra_in[i] = x;
@@ -774,7 +787,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             const auto& ca = ops[j];
             if (ca.in0 != op.out0) continue;
             if (ca.kind == TB200_OP_EW && ca.i0 == TB200_EW_CAST && ca.in1 < 0 && !(ca.flags & TB200_FLAG_BOOL_RESULT) && ca.out0 >= 0 && ca.out0 < nt &&
-                (tensors[ca.out0].dtype == TB200_BF16 || tensors[ca.out0].dtype == TB200_F32) && b.numel(ca.out0) == b.numel(op.out0)) {
+                (tensors[ca.out0].dtype == TB200_BF16 || tensors[ca.out0].dtype == TB200_F32) && b.same_shape(ca.out0, op.out0)) {
               softmax_cast[i] = j;
               extra_out[i] = ca.out0;
               fused_away[j] = 1;
