@@ -89,6 +89,10 @@ struct Builder {
     return true;
   }
 
+  // A result that an op fused in front of it may write early: one that only ops behind its own can read. (A state tensor holds
+  // the value of the step before until its op runs.)
+  bool may_write_early(int id) const { return valid_id(id) && (tensors[id].kind == TB200_TENSOR_ACTIVATION || tensors[id].kind == TB200_TENSOR_OUTPUT); }
+
   size_t numel(int id) const {
     const auto& t = tensors[id];
     size_t n = 1;
@@ -690,7 +694,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       const auto& op = ops[i];
       if (op.kind != TB200_OP_TABLE || op.in0 < 0 || op.in0 >= nt || op.out0 < 0 || op.out0 >= nt) continue;
       const int src = op.in0, pc = producer[src];
-      if (pc < 0 || pc >= i || !takes_table(ops[pc]) || uses[src] != 1 || table_after[pc] >= 0 ||
+      if (pc < 0 || pc >= i || !takes_table(ops[pc]) || uses[src] != 1 || table_after[pc] >= 0 || !b.may_write_early(op.out0) ||
           tensors[src].kind != TB200_TENSOR_ACTIVATION || tensors[src].dtype != TB200_I8 || tensors[op.out0].dtype != TB200_I8)
         continue;
       table_after[pc] = i;
@@ -716,7 +720,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       for (int side = 0; side < 2; side++) {
         const int src = side == 0 ? op.in0 : op.in1, other = side == 0 ? op.in1 : op.in0;
         const int pc = producer[src];
-        if (pc < 0 || pc >= i || ops[pc].kind != TB200_OP_CONV2D || uses[src] != 1 || table_after[pc] >= 0 || add_after[pc] >= 0 ||
+        if (pc < 0 || pc >= i || ops[pc].kind != TB200_OP_CONV2D || uses[src] != 1 || table_after[pc] >= 0 || add_after[pc] >= 0 || !b.may_write_early(op.out0) ||
             tensors[src].kind != TB200_TENSOR_ACTIVATION || tensors[src].dtype != TB200_I8 || tensors[op.out0].dtype != TB200_I8 ||
             tensors[other].dtype != TB200_I8 || tensors[other].kind == TB200_TENSOR_CONSTANT)
           continue;
@@ -786,7 +790,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           for (int j = i + 1; j < (int)ops.size(); j++) {
             const auto& ca = ops[j];
             if (ca.in0 != op.out0) continue;
-            if (ca.kind == TB200_OP_EW && ca.i0 == TB200_EW_CAST && ca.in1 < 0 && !(ca.flags & TB200_FLAG_BOOL_RESULT) && ca.out0 >= 0 && ca.out0 < nt &&
+            if (ca.kind == TB200_OP_EW && ca.i0 == TB200_EW_CAST && ca.in1 < 0 && !(ca.flags & TB200_FLAG_BOOL_RESULT) && b.may_write_early(ca.out0) &&
                 (tensors[ca.out0].dtype == TB200_BF16 || tensors[ca.out0].dtype == TB200_F32) && b.same_shape(ca.out0, op.out0)) {
               softmax_cast[i] = j;
               extra_out[i] = ca.out0;
