@@ -251,12 +251,14 @@ static void binary_linear_form(const tb200_op_t& op, BinaryArgs& a) {
   for (double extra : {std::ldexp(1.0, -26), std::ldexp(1.0, -24), 0.0, std::ldexp(1.0, -22), std::ldexp(1.0, -20)}) {
     const long long ma = std::llround(std::ldexp(sa * (1.0 + extra), 24 + f)), mb = std::llround(std::ldexp(sb * (1.0 + extra), 24 + f));
     long long lo = INT64_MIN, hi = INT64_MAX;
-    for (int x = 0; x < 256; x++)
+    for (int x = 0; x < 256 && lo <= hi; x++) {
+      const long long qx = (long long)(x - 128) * 256 * ma;
       for (int y = 0; y < 256; y++) {
-        const long long r = want[x * 256 + y], q = (long long)(x - 128) * 256 * ma + (long long)(y - 128) * 256 * mb;
+        const long long r = want[x * 256 + y], q = qx + (long long)(y - 128) * 256 * mb;
         if (r > a.clamp_min) lo = std::max(lo, r * (1ll << (32 + f)) - q);
         if (r < a.clamp_max) hi = std::min(hi, (r + 1) * (1ll << (32 + f)) - q - 1);
       }
+    }
     if (lo > hi || lo == INT64_MIN || hi == INT64_MAX || std::max(std::llabs(ma), std::llabs(mb)) >= (1ll << 31)) continue;
     a.lin = 1;
     a.lin_f = f;
@@ -605,6 +607,18 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   std::vector<int> add_after(ops.size(), -1);      // conv op -> index of the add fused into its epilogue
   std::vector<char> add_self_is_a(ops.size(), 0);  // the convolution's result is the add's first operand
   std::vector<char> add_fits_small(ops.size(), 0); // the fused add runs in the small-problem kernel
+  // Parameters of an add / sub / mul, null when the op has none. Kept: the linear form looks at 65536 operand pairs several times
+  // over, and an add is asked for two or three times.
+  std::map<int, std::unique_ptr<BinaryArgs>> binary_known;
+  auto binary_args = [&](int i) -> const BinaryArgs* {
+    auto it = binary_known.find(i);
+    if (it == binary_known.end()) {
+      auto a = std::make_unique<BinaryArgs>();
+      if (!binary_args_of(ops[i], *a)) a.reset();
+      it = binary_known.emplace(i, std::move(a)).first;
+    }
+    return it->second.get();
+  };
   // Decoder graphs run op by op: (1) geglu, rope_kv and argmax run in the epilogue of the gemv_w8 right in front of them when they
   // are its only reader (decode_linear.cu) - the reader's step launches both; (2) an rmsnorm directly followed by an rmsnorm of
   // its result runs as one launch. Same arithmetic in the same order, fewer launches.
@@ -741,9 +755,9 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         for (int d = 0; d < 4 && same; d++) same = tensors[other].shape[d] == o.shape[d] && tensors[op.out0].shape[d] == o.shape[d];
         if (!same) continue;
         // the fused form exists for the 32-bit output rescale only
-        BinaryArgs probe{};
-        if (!binary_args_of(op, probe) || probe.epi == 0) continue;
-        add_fits_small[pc] = probe.lin && pointwise_takes_small(M, x.shape[3], OC);
+        const BinaryArgs* probe = binary_args(i);
+        if (!probe || probe->epi == 0) continue;
+        add_fits_small[pc] = probe->lin && pointwise_takes_small(M, x.shape[3], OC);
         if (!all_adds && !(add_fits_small[pc] && tensors[other].kind == TB200_TENSOR_ACTIVATION)) continue;
         add_after[pc] = i;
         add_self_is_a[pc] = side == 0;
@@ -1126,8 +1140,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           const int fused_add = add_after[i];
           Loc lx = x_at, lo = loc(fused_add >= 0 ? ops[fused_add].out0 : result_id), lres{};
           if (fused_add >= 0) {
-            BinaryArgs add{};
-            binary_args_of(ops[fused_add], add);
+            const BinaryArgs& add = *binary_args(fused_add);
             const bool self_a = add_self_is_a[i] != 0;
             sa.add_m_self = self_a ? add.lin_ma : add.lin_mb;
             sa.add_m_other = self_a ? add.lin_mb : add.lin_ma;
@@ -1266,8 +1279,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           Loc lout = y_loc;
           Loc lres{};
           if (fused_add >= 0) {
-            if (!binary_args_of(ops[fused_add], ga.add) || ga.add.epi == 0)
-              return b.fail(TB200_INTERNAL, "op %d: fused add lost its 32-bit rescale", fused_add);
+            ga.add = *binary_args(fused_add);
             ga.add_self_is_a = add_self_is_a[i];
             lout = loc(ops[fused_add].out0);
             lres = loc(add_self_is_a[i] ? ops[fused_add].in1 : ops[fused_add].in0);
@@ -1667,8 +1679,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           return b.fail(TB200_INVALID_ARGUMENT, "op %d: elementwise operands differ in size (no broadcast)", i);
         for (int s : {op.in0_shift, op.in1_shift, op.out_shift})
           if (s < 2 || s > 62) return b.fail(TB200_INVALID_ARGUMENT, "op %d: rescale shift %d outside [2,62]", i, s);
-        BinaryArgs a{};
-        if (!binary_args_of(op, a)) return b.fail(TB200_INVALID_ARGUMENT, "op %d: input left shift outside [0,22]", i);
+        if (!binary_args(i)) return b.fail(TB200_INVALID_ARGUMENT, "op %d: input left shift outside [0,22]", i);
+        BinaryArgs a = *binary_args(i);
         a.n = (long long)n;
         Loc la = loc(op.in0), lb = loc(op.in1), lo = loc(op.out0);
         step.kernel_name = "binary_rescale";
