@@ -821,10 +821,10 @@ cudaError_t launch_linear_mode(const LinearArgs& args, const LinearShape& s, cud
 
 }  // namespace
 
-bool linear_w8_applies(int B, int N, int K) { return linear_shape(B, N, K, kStore, 148).ok; }
-bool linear_geglu_applies(int B, int N, int K) { return N % 2 == 0 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kGeglu, 148).ok; }
+bool linear_w8_applies(int B, int N, int K) { return linear_shape(B, N, K, kStore, current_sm_count()).ok; }
+bool linear_geglu_applies(int B, int N, int K) { return N % 2 == 0 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kGeglu, current_sm_count()).ok; }
 bool linear_rope_applies(int B, int N, int K, int n_q, int n_kv, int D) {
-  return n_kv == 1 && D == 256 && N == (n_q + 2) * 256 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kRope, 148).ok;
+  return n_kv == 1 && D == 256 && N == (n_q + 2) * 256 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kRope, current_sm_count()).ok;
 }
 // whether the arg max over the results can ride along, and the candidates' bytes
 size_t linear_argmax_scratch(int B, int N, int K) {
