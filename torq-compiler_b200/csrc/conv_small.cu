@@ -21,8 +21,9 @@
 #include <atomic>
 
 #include "chunk_divide.h"
-#include "kernels.h"
 #include "dependent_launch.cuh"
+#include "device_memory.cuh"
+#include "kernels.h"
 
 namespace tb200 {
 namespace {
@@ -77,24 +78,6 @@ __device__ __forceinline__ uint32_t load_bytes(const int8_t* p, int n) {
   for (int j = 0; j < 4; j++)
     if (j < n) w |= (uint32_t)(uint8_t)p[j] << (8 * j);
   return w;
-}
-
-// 16 bytes from byte offset off of x (4-byte aligned, total bytes); bytes past the end are undefined
-__device__ __forceinline__ uint4 load16_any(const int8_t* x, int off, int total) {
-  const int w0 = off & ~3;
-  const uint32_t sh = (uint32_t)(off & 3) * 8;
-  uint32_t w[5];
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-    w[i] = 0;
-    const int at = w0 + 4 * i;
-    if (at + 4 <= total) {
-      w[i] = *reinterpret_cast<const uint32_t*>(x + at);
-    } else {
-      for (int j = 0; at + j < total; j++) w[i] |= (uint32_t)(uint8_t)x[at + j] << (8 * j);
-    }
-  }
-  return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
 }
 
 // MODE: what a row of the product is - kRows: lda bytes of memory; kConv: the taps of an output pixel, IC a multiple of 16;
@@ -314,16 +297,6 @@ constexpr int kMidSumPitch = kMidN + 4;  // words
 constexpr int kMidRecv = kMidM * kMidN * 4, kMidSmem = kMidStages * kMidStage + kMidRecv;
 constexpr int kMidGroups = kMidThreads / 128;  // warps that share a chunk's steps
 static_assert(kMidGroups * kMidM * kMidSumPitch * 4 <= kMidStages * kMidStage, "the sums take the stages' place");
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {  // zeros when not valid
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 
 __global__ void __launch_bounds__(kMidThreads, 1) rows_mid_kernel(const ConvSmallArgs a) {
   extern __shared__ __align__(128) unsigned char mid_s[];
@@ -550,7 +523,7 @@ cudaError_t launch_conv_small(const ConvSmallArgs& args, cudaStream_t stream) {
        {{conv_small_kernel<kConv, 1, false, true>, conv_small_kernel<kConv, 2, false, true>, conv_small_kernel<kConv, 3, false, true>}, {conv_small_kernel<kConv, 1, true, true>, conv_small_kernel<kConv, 2, true, true>, conv_small_kernel<kConv, 3, true, true>}}}};
   const bool ragged = a.IC % 16 != 0;
   const Kernel kernel = a.mode == kStem ? conv_small_kernel<kStem, 1, false, false> : kernels[ragged][a.mode == kConv][ks_n > 1][u - 1];
-  return launch_dependent_if(true, kernel, grid, block, smem, stream, a);
+  return launch_dependent(kernel, grid, block, smem, stream, a);
 }
 
 namespace {

@@ -495,7 +495,7 @@ void launch_depthwise(const DwArgs& a, cudaStream_t stream) {
   if (a.wq && depthwise3x3_supported(a) && a.OH <= 65535 && a.N <= 65535 && !small_kernels_off() &&
       (long long)few_strips * (a.C >> 2) * a.OH * a.N <= kFewThreads) {
     const dim3 grid((unsigned)((few_strips * (a.C >> 2) + 127) / 128), (unsigned)a.OH, (unsigned)a.N);
-    auto go = [&](auto kern) { launch_dependent_if(true, kern, grid, dim3(128), 0, stream, a); };
+    auto go = [&](auto kern) { launch_dependent(kern, grid, dim3(128), 0, stream, a); };
     if (a.stride_h == 1) {
       if (a.epi == 1) go(dw3x3_few_kernel<1, 1>);
       else if (a.epi == 2) go(dw3x3_few_kernel<1, 2>);

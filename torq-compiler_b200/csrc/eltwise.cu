@@ -2,8 +2,9 @@
 // standalone rescale (also the building block of a rescaled concat), 2x nearest
 // resize. 128-bit accesses wherever the channel count allows; grids sized in
 // whole multiples of the SM count with grid-stride loops.
-#include "kernels.h"
 #include "dependent_launch.cuh"
+#include "device_memory.cuh"
+#include "kernels.h"
 
 namespace tb200 {
 
@@ -20,12 +21,6 @@ inline unsigned grid_for(long long work_items, int per_block = kThreads) {
 }
 
 // ---- add / sub / mul in TOSA form (ElementWiseBinaryPattern.cpp:385-570, MulPattern.cpp:229-238) ----
-// Four raw table bytes -> one word; lut is indexed by the raw byte.
-__device__ __forceinline__ uint32_t lut_word(const uint8_t* lut, uint32_t w) {
-  const uint32_t b0 = lut[w & 0xff], b1 = lut[(w >> 8) & 0xff], b2 = lut[(w >> 16) & 0xff], b3 = lut[w >> 24];
-  return __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
-}
-
 // add / sub as one linear function of the two bytes: out = clamp((xa * 2^8 * ma + xb * 2^8 * mb + K) >> (32 + F)), the
 // three roundings of the op absorbed in K. The planner takes this form only after it has compared it with the exact op on
 // all 65536 operand pairs (binary_linear_form). Per output: two byte extracts, two multiply-adds and a quarter of the

@@ -18,8 +18,9 @@
 #include <cstdint>
 #include <vector>
 
-#include "kernels.h"
 #include "dependent_launch.cuh"
+#include "device_memory.cuh"
+#include "kernels.h"
 
 namespace tb200 {
 
@@ -33,12 +34,6 @@ inline unsigned grid_for(long long work_items, int per_block = kThreads) {
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   return (unsigned)blocks;
-}
-
-// A fused 256-entry table applied to four packed results; lut is indexed by the raw byte.
-__device__ __forceinline__ uint32_t lut_word(const uint8_t* lut, uint32_t w) {
-  const uint32_t b0 = lut[w & 0xff], b1 = lut[(w >> 8) & 0xff], b2 = lut[(w >> 16) & 0xff], b3 = lut[w >> 24];
-  return __byte_perm(__byte_perm(b0, b1, 0x0040), __byte_perm(b2, b3, 0x0040), 0x5410);
 }
 
 constexpr int kStripThreads = 128;

@@ -6,29 +6,11 @@
 // Bound by memory: a thread makes 16 bytes from five aligned words (neighbours share them in L1). Only words that hold bytes
 // of the tensor are touched.
 #include "dependent_launch.cuh"
+#include "device_memory.cuh"
 #include "kernels.h"
 
 namespace tb200 {
 namespace {
-
-// 16 bytes from byte offset `off` of x (x 4-byte aligned, `total` bytes); bytes past the end are undefined
-__device__ __forceinline__ uint4 load16_any(const int8_t* x, long long off, long long total) {
-  const long long w0 = off & ~3ll;
-  const uint32_t sh = (uint32_t)(off & 3) * 8;
-  const uint32_t* p = reinterpret_cast<const uint32_t*>(x + w0);
-  uint32_t w[5];
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-    w[i] = 0;
-    const long long at = w0 + 4 * i;
-    if (at + 4 <= total) {
-      w[i] = __ldg(p + i);
-    } else if (at < total) {
-      for (int j = 0; at + j < total; j++) w[i] |= (uint32_t)(uint8_t)x[at + j] << (8 * j);
-    }
-  }
-  return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
-}
 
 // out[r][0 .. pitch) <- x[r][0 .. K) followed by unspecified bytes (they meet zero weights); pitch a multiple of 16
 __global__ void __launch_bounds__(256) pad_rows_kernel(const int8_t* x, int8_t* out, long long rows, int K, int pieces) {
