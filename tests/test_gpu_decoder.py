@@ -72,7 +72,13 @@ def _run(device, cfg, batch, prompt_len, gen_len, seed=1234, embed_gain=0.02):
 
 
 @pytest.mark.parametrize("batch", [1, 3])
-def test_small_decoder_matches_reference(device, batch):
+@pytest.mark.parametrize("persistent", [False, True])
+def test_small_decoder_matches_reference(device, batch, persistent, monkeypatch):
+    """Op by op, as one GPU runs it, and as the one kernel that tensor-parallel shards take."""
+    monkeypatch.setenv("TB200_DECODE_FUSED_MAX_B", "8" if persistent else "0")
+    ex = Executable(device, gemma3.build_decode_step(gemma3.SMALL, batch, gemma3.random_weights(gemma3.SMALL, 1, 0.3)).serialize())
+    assert ("decode_step_persistent" in ex.op_kernels()) == persistent
+    ex.destroy()
     # window 24 < sequence: local layers slide; layer 3 of 3 is global
     worst, exact, near_tie, wrong, got = _run(device, gemma3.SMALL, batch, prompt_len=40, gen_len=24)
     assert worst <= FLAT_LOGIT_REL_TOL, worst
@@ -119,8 +125,8 @@ MID = gemma3.GemmaConfig(layers=2, hidden=1024, intermediate=2048, vocab=4096, w
 
 @pytest.mark.parametrize("cfg,batch", [(gemma3.SMALL, 8), (gemma3.SMALL, 32), (MID, 3), (MID, 16)])
 def test_op_by_op_launch_fusions_change_no_bit(device, cfg, batch):
-    """Run op by op, the planner lets the reader of a split-K product finalize the partial sums and runs
-    two norms in a row as one launch. The arithmetic and its order are the same: logits and ids must be
+    """Run op by op, the planner launches a product together with the op that reads it (RoPE and the cache append, GeGLU, the
+    arg max) and runs two norms in a row as one launch. The arithmetic and its order are the same: logits and ids must be
     bit-identical with the fusions switched off (TB200_NO_DECODER_FUSION=1 when the plan is built)."""
     params = gemma3.random_weights(cfg, 77, 0.3)
     blob = gemma3.build_decode_step(cfg, batch, params, with_logits=True).serialize()
@@ -133,9 +139,9 @@ def test_op_by_op_launch_fusions_change_no_bit(device, cfg, batch):
         os.environ.pop("TB200_NO_DECODER_FUSION", None)
         os.environ.pop("TB200_DECODE_PER_OP", None)
     names_f, names_p = fused.op_kernels(), plain.op_kernels()
-    assert any(n.startswith("rmsnorm_pair") for n in names_f) and "rope_kv_from_partials" in names_f
-    assert "geglu_from_partials" in names_f and fused.launch_count < plain.launch_count
-    assert not any("partials" in n or "pair" in n for n in names_p)
+    together = {"rmsnorm_pair", "linear_w8_rope_kv", "linear_w8_geglu"}
+    assert together <= set(names_f) and fused.launch_count < plain.launch_count
+    assert not together & set(names_p) and {"rmsnorm", "linear_w8", "rope_kv", "geglu", "attn_decode"} <= set(names_p)
     rng = np.random.default_rng(5)
     d_tok, d_pos = device.alloc(batch * 4), device.alloc(4)
     outs = [(device.alloc(batch * 4), device.alloc(batch * cfg.vocab * 4)) for _ in range(2)]

@@ -148,6 +148,7 @@ def test_profile_csv_uses_the_reference_event_names(device, tmp_path):
         ex = Executable(device, g.serialize())
         out = np.empty(ex.outputs_info[0].shape, np.int8)
         ex.invoke_host([x], [out])
+        kernel = ex.op_kernels()[0]
         d_in = device.alloc(x.nbytes)
         d_in.upload(x)
         device.wait()
@@ -179,7 +180,7 @@ def test_profile_csv_uses_the_reference_event_names(device, tmp_path):
                  "DISPATCH_SYNC_BINDINGS_OUT_END", "DISPATCH_END", "HOST_COPY_BEGIN"):
         assert want in names, want
     ops = [r for r in rows if r["event"] == "NSS_START_BEGIN"]
-    assert ops and ops[0]["dispatch_name"] == "gemm_i8_tcgen05" and int(ops[0]["action_id"]) == 0
+    assert ops and ops[0]["dispatch_name"] == kernel == "gemm_small_i8_mma" and int(ops[0]["action_id"]) == 0
 
 
 def test_two_devices_in_one_process(device):

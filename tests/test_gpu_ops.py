@@ -91,7 +91,8 @@ IGEMM_CASES = [
 
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("case", IGEMM_CASES)
-def test_conv2d_implicit_gemm(device, case, mode):
+def test_conv2d_implicit_gemm(device, case, mode, monkeypatch):
+    """On the tensor-core kernel of the large sizes (small problems kept off theirs), and as the planner decides."""
     from torq_b200.runtime import Executable
     shape, OC, k, stride, pad, izp = case
     rng = np.random.default_rng(1234)
@@ -104,11 +105,14 @@ def test_conv2d_implicit_gemm(device, case, mode):
     y = g.conv2d(g.input(shape), w, bias, m, s, stride=(stride, stride), pad=pad, input_zp=izp, out_zp=-7, clamp=(-128, 127),
                  requant_mode=mode)
     g.output(y)
-    ex = Executable(device, g.serialize())
     # 16 input channels make 16-byte operand rows: where neither halo patches nor pixel pairs apply, the dp4a kernel takes those
-    assert ex.op_kernels() == ["conv2d_c16_dp4a" if shape[3] == 16 and stride == 2 and shape[2] % 2 else "conv_igemm_i8_tcgen05"]
-    ex.destroy()
-    _check(device, g, [x])
+    large = "conv2d_c16_dp4a" if shape[3] == 16 and stride == 2 and shape[2] % 2 else "conv_igemm_i8_tcgen05"
+    for no_small in ("1", "0"):
+        monkeypatch.setenv("TB200_NO_SMALL", no_small)
+        ex = Executable(device, g.serialize())
+        assert ex.op_kernels()[0] in ([large] if no_small == "1" else [large, "conv_small_i8_mma"])
+        ex.destroy()
+        _check(device, g, [x])
 
 
 def test_conv2d_per_tensor_scale_and_relu6_clamp(device):
@@ -365,12 +369,14 @@ def test_chain_with_intermediates_and_host_call(device):
     ((3, 14, 14, 64), 64, True, False),     # single rounding: the record without the sign term
     ((1, 9, 7, 160), 80, False, True),      # ragged last tile
 ])
-def test_pointwise_conv_with_fused_residual_add(device, shape, OC, conv_first, double_round):
+@pytest.mark.parametrize("no_small,kernel", [("1", "gemm_i8_tcgen05"), ("0", "gemm_small_i8_mma")])
+def test_pointwise_conv_with_fused_residual_add(device, shape, OC, conv_first, double_round, no_small, kernel, monkeypatch):
     """With TB200_ADD_FUSION=1 a rescaled add whose one operand is the only use of a 1x1 convolution's result runs in
     that convolution's epilogue (one launch, the product never stored): bit-exact against the oracle, which runs the
     two ops apart, and against the default plan (two launches); a product with a second reader keeps its own launch."""
     import os
     from torq_b200.runtime import Executable
+    monkeypatch.setenv("TB200_NO_SMALL", no_small)
     rng = np.random.default_rng(shape[1] * 31 + OC)
     x = rng.integers(-128, 128, shape, dtype=np.int8)
     r = rng.integers(-128, 128, shape[:3] + (OC,), dtype=np.int8)
@@ -392,12 +398,12 @@ def test_pointwise_conv_with_fused_residual_add(device, shape, OC, conv_first, d
     g = build(False)
     apart = _check(device, g, [x, r])[0]
     ex = Executable(device, g.serialize())
-    assert ex.op_kernels() == ["gemm_i8_tcgen05", "binary_rescale"]
+    assert ex.op_kernels() == [kernel, "binary_rescale"]
     ex.destroy()
     os.environ["TB200_ADD_FUSION"] = "1"
     try:
         ex = Executable(device, g.serialize())
-        assert ex.op_kernels() == ["gemm_i8_tcgen05", "(add in the convolution's epilogue)"] and ex.launch_count == 1, ex.op_kernels()
+        assert ex.op_kernels() == [kernel, "(add in the convolution's epilogue)"] and ex.launch_count == 1, ex.op_kernels()
         ex.destroy()
         got = _check(device, g, [x, r])[0]
         assert (apart == got).all()
@@ -420,9 +426,9 @@ GEMM_CASES = [
 
 
 @pytest.mark.parametrize("M,K,N", GEMM_CASES)
-def test_pointwise_conv_tensor_core_sweep(device, M, K, N):
-    """1x1 convolution = row-major GEMM; checked against the oracle and, for the same blob,
-    against the CUDA-core kernel (TB200_FORCE_SIMT=1)."""
+def test_pointwise_conv_tensor_core_sweep(device, M, K, N, monkeypatch):
+    """1x1 convolution = row-major GEMM on the tensor-core kernel of the large sizes (small problems kept off theirs) and as
+    the planner decides; checked against the oracle and, for the same blob, against the CUDA-core kernel (TB200_FORCE_SIMT=1)."""
     import os
     rng = np.random.default_rng(1234 + M + K + N)
     a = rng.integers(-128, 128, (1, 1, M, K), dtype=np.int8)
@@ -432,11 +438,14 @@ def test_pointwise_conv_tensor_core_sweep(device, M, K, N):
     g = Graph()
     y = g.conv2d(g.input(a.shape), w, bias, m, s, input_zp=-6, out_zp=4, clamp=(-120, 115))
     g.output(y)
-    got = _check(device, g, [a])[0]
     from torq_b200.runtime import Executable
-    ex = Executable(device, g.serialize())
-    assert ex.op_kernels() == ["gemm_i8_tcgen05" if M > 4 or K % 16 else "fc_rows_dp4a"]
-    ex.destroy()
+    large = "gemm_i8_tcgen05" if M > 4 or K % 16 else "fc_rows_dp4a"
+    for no_small in ("1", "0"):
+        monkeypatch.setenv("TB200_NO_SMALL", no_small)
+        ex = Executable(device, g.serialize())
+        assert ex.op_kernels()[0] in ([large] if no_small == "1" else [large, "gemm_small_i8_mma", "gemm_mid_i8_mma"])
+        ex.destroy()
+        got = _check(device, g, [a])[0]
     os.environ["TB200_FORCE_SIMT"] = "1"
     try:
         ex = Executable(device, g.serialize())
@@ -493,14 +502,17 @@ def test_chained_concats_are_written_in_place(device):
 
 @pytest.mark.parametrize("shape,OC,k,dil", [((1, 12, 12, 64), 32, 1, 1),    # 1x1: tensor-core GEMM
                                             ((2, 14, 14, 32), 48, 3, 1),    # 3x3: tensor-core implicit GEMM
-                                            ((1, 18, 18, 16), 20, 3, 1),    # 16 channels: direct dp4a kernel
+                                            ((1, 18, 18, 16), 20, 3, 1),    # 20 filters: tensor-core implicit GEMM, padded result trimmed
                                             ((1, 20, 20, 3), 16, 3, 1),     # stem kernel
                                             ((1, 11, 11, 24), 10, 3, 2)])   # dilation: generic CUDA-core kernel
-def test_table_fused_into_conv_epilogue(device, shape, OC, k, dil):
+@pytest.mark.parametrize("no_small", ["1", "0"])
+def test_table_fused_into_conv_epilogue(device, shape, OC, k, dil, no_small, monkeypatch):
     """conv -> table (SiLU as a 256-entry table follows every convolution of the detector): when the table is
-    the convolution's only reader it runs in the convolution's epilogue; same bytes as the two-kernel form."""
+    the convolution's only reader it runs in the convolution's epilogue; same bytes as the two-kernel form. On the kernels
+    named above (small problems kept off theirs), and as the planner decides."""
     import os
     from torq_b200.runtime import Executable
+    monkeypatch.setenv("TB200_NO_SMALL", no_small)
     rng = np.random.default_rng(1234)
     x = rng.integers(-128, 128, shape, dtype=np.int8)
     w = rng.integers(-127, 128, (OC, k, k, shape[3]), dtype=np.int8)
@@ -511,14 +523,15 @@ def test_table_fused_into_conv_epilogue(device, shape, OC, k, dil):
     y = g.conv2d(g.input(shape), w, np.round(rng.normal(0, 2000, OC)).astype(np.int32), m, s, dilation=(dil, dil),
                  pad=(p, p, p, p), input_zp=-4, out_zp=3)
     g.output(g.table(y, table))
+    trim = int(no_small == "1" and OC == 20)
     ex = Executable(device, g.serialize())
-    assert ex.launch_count == 1, ex.op_kernels()
+    assert ex.launch_count == 1 + trim, ex.op_kernels()
     ex.destroy()
     fused = _check(device, g, [x])[0]
     os.environ["TB200_NO_TABLE_FUSION"] = "1"
     try:
         ex = Executable(device, g.serialize())
-        assert ex.launch_count == 2
+        assert ex.launch_count == 2 + trim
         ex.destroy()
         assert (run_graph_gpu(device, g, [x])[0] == fused).all()
     finally:

@@ -1100,8 +1100,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
                                       op.pad_b == 0 && op.pad_l == 0 && op.pad_r == 0);
         const long long M = (long long)N * OH * OW;
         // Small problems (conv_small.cu): the same two families of products, on kernels that are latency-bound differently.
-        // The step keeps the name of the family, whichever kernel the size picks.
-        auto plan_small = [&](const char* family, int rows_per_group, Loc x_at, cudaError_t (*launcher)(const ConvSmallArgs&, cudaStream_t)) {
+        auto plan_small = [&](const char* name, int rows_per_group, Loc x_at, cudaError_t (*launcher)(const ConvSmallArgs&, cudaStream_t)) {
           const int G = rows_per_group;  // rows read as one (block-diagonal weights) to make a row a multiple of 16 bytes
           ConvSmallArgs sa{};
           const bool stem = !pointwise && IC == 3;
@@ -1148,7 +1147,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             sa.add_clamp_min = add.clamp_min; sa.add_clamp_max = add.clamp_max;
             lres = loc(self_a ? ops[fused_add].in1 : ops[fused_add].in0);
           }
-          step.kernel_name = family;
+          step.kernel_name = name;
           step.launch = [=](const ExecContext& c) {
             ConvSmallArgs k = sa;
             k.x = (const int8_t*)lx.resolve(c);
@@ -1165,7 +1164,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         const bool few_rows = M <= 4 && K % 16 == 0 && K <= 12288;  // fc_rows below
         if (add_after[i] >= 0 ? add_fits_small[i] != 0
                               : pointwise && op.weight_zp == 0 && !force_simt() && !few_rows && pointwise_takes_small(M, K, OC)) {
-          plan_small("gemm_i8_tcgen05", pointwise_small_group(M, K), loc(op.in0), launch_conv_small);
+          plan_small("gemm_small_i8_mma", pointwise_small_group(M, K), loc(op.in0), launch_conv_small);
           break;
         }
         const int IC16 = (IC + 15) / 16 * 16, OC16 = (OC + 15) / 16 * 16;
@@ -1175,7 +1174,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             (IC != 16 || OC != OC16 || conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).halo ||
              conv_tc_geometry_padded(N, OH, OW, W, IC, OC, KH, KW, op.stride_h, op.pad_l).s2) &&
             conv_small_applies(M, OC, KH * KW, IC)) {
-          plan_small("conv_igemm_i8_tcgen05", 1, loc(op.in0), launch_conv_small);
+          plan_small("conv_small_i8_mma", 1, loc(op.in0), launch_conv_small);
           break;
         }
         // Rows that are no multiple of 16 bytes (ragged_rows.cu): the layer runs on padded copies in scratch. A product whose rows
@@ -1217,7 +1216,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           }
         }
         if (mid) {
-          plan_small("gemm_i8_tcgen05", 1, x_loc, launch_rows_mid);
+          plan_small("gemm_mid_i8_mma", 1, x_loc, launch_rows_mid);
           break;
         }
         // At most four rows: a weight-streaming dp4a kernel instead of 128-row tensor-core tiles (the weights are the
@@ -1472,7 +1471,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         // leave few pixels of a frame beyond that)
         if (!fc && IC == 3 && KH == 3 && KW == 3 && op.stride_h == op.stride_w && op.dil_h == 1 && op.dil_w == 1 && op.weight_zp == 0 &&
             !force_simt() && conv_small_applies(M, OC, 1, 16) && b.numel(op.in0) < (size_t)INT32_MAX) {
-          plan_small("conv2d_stem333_dp4a", 1, loc(op.in0), launch_conv_small);
+          plan_small("conv2d_stem333_i8_mma", 1, loc(op.in0), launch_conv_small);
           break;
         }
         const int Kpad = (int)((K + 31) / 32 * 32);
@@ -1936,13 +1935,13 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           const LinearStep l{loc(op.in0), w_off, s_off, B, N, K};
           if (gemv_deferred[i]) {
             linear[i] = l;
-            step.kernel_name = "gemv_w8_splitk_partials";
+            step.kernel_name = "(product in the launch of the op behind it)";
             step.launches = 0;
             step.launch = [](const ExecContext&) {};
             break;
           }
           const Loc ly = loc(op.out0);
-          step.kernel_name = "gemv_w8";
+          step.kernel_name = "linear_w8";
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
             k.y = ly.resolve(c);
@@ -1984,7 +1983,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         const float theta = op.f0, eps = op.f1;
         if (gemv_before[i] >= 0) {
           const LinearStep l = linear[gemv_before[i]];
-          step.kernel_name = "rope_kv_from_partials";
+          step.kernel_name = "linear_w8_rope_kv";
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
             k.pos = (const int32_t*)lp.resolve(c);
@@ -2023,7 +2022,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         // the append right in front of it, to the same caches at the same position: a launch of its own at head size 256
         const bool early = i > 0 && ops[i - 1].kind == TB200_OP_ROPE_KV && ops[i - 1].out1 == op.in2 && ops[i - 1].in2 == op.weights &&
                            ops[i - 1].in1 == op.in1;
-        step.kernel_name = "attn_decode_splitT";
+        step.kernel_name = "attn_decode";
         step.launch = [=](const ExecContext& c) {
           launch_attn_decode((const uint16_t*)lq.resolve(c), (const int32_t*)lp.resolve(c), (const uint16_t*)lk.resolve(c),
                              (const uint16_t*)lv.resolve(c), (uint16_t*)lo.resolve(c), B, n_q, T, window, scale, early, c.stream);
@@ -2038,7 +2037,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         Loc lx = loc(op.in0), lo = loc(op.out0);
         if (gemv_before[i] >= 0) {
           const LinearStep l = linear[gemv_before[i]];
-          step.kernel_name = "geglu_from_partials";
+          step.kernel_name = "linear_w8_geglu";
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
             k.y = lo.resolve(c);
@@ -2065,6 +2064,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         step.launches = 2;
         if (gemv_before[i] >= 0) {  // the product leaves candidates of every block behind its logits
           const LinearStep l = linear[gemv_before[i]];
+          step.kernel_name = "linear_w8_argmax";
           scratch_need = std::max(scratch_need, linear_argmax_scratch(l.B, l.N, l.K));
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
