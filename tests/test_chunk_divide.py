@@ -10,13 +10,19 @@ PROGRAM = r'''
 #include "chunk_divide.h"
 int main() {
   for (int d = 1; d <= tb200::kMaxChunks; d++) {
-    const uint32_t inv = tb200::divide_constant(d);
+    const tb200::ChunkDivisor by = tb200::chunk_divisor(d);
     for (int c = 0; c < tb200::kMaxChunks + 4; c++)
-      if (tb200::divide_by(c, inv) != c / d) {
-        printf("%d / %d gives %d\n", c, d, tb200::divide_by(c, inv));
+      if (tb200::divide_chunk(c, by) != c / d) {
+        printf("%d / %d gives %d\n", c, d, tb200::divide_chunk(c, by));
         return 1;
       }
   }
+  for (int kw = 1; kw <= tb200::kMaxTaps; kw++)
+    for (int tap = 0; tap < tb200::kMaxTaps + 4; tap++)
+      if (tb200::divide_tap(tap, tb200::tap_divisor(kw)) != tap / kw) {
+        printf("tap %d / %d\n", tap, kw);
+        return 1;
+      }
   return 0;
 }
 '''

@@ -20,7 +20,6 @@
 
 #include <atomic>
 
-#include "chunk_divide.h"
 #include "dependent_launch.cuh"
 #include "device_memory.cuh"
 #include "kernels.h"
@@ -158,8 +157,8 @@ __global__ void __launch_bounds__(SPLIT ? 256 : 128, SPLIT ? 2 : 4) conv_small_k
         }
       }
     } else if (MODE == kConv) {
-      const int tap = divide_by(c, a.inv_icb), icb = c - tap * a.icb;
-      const int kh = divide_by(tap, a.inv_kw), kw = tap - kh * a.KW;
+      const int tap = divide_chunk(c, a.by_icb), icb = c - tap * a.icb;
+      const int kh = divide_tap(tap, a.inv_kw), kw = tap - kh * a.KW;
       const int off = (kh * a.W + kw) * a.IC + icb * 16;
 #pragma unroll
       for (int r = 0; r < 2; r++) {
@@ -455,7 +454,7 @@ int conv_small_columns(int OC) { return ceil_div(OC, kTileN) * kTileN; }
 constexpr long long kSmallCost = 29000;
 
 bool conv_small_applies(long long M, int OC, int taps, int IC) {
-  if (small_kernels_off() || IC < 1 || taps < 1 || taps > 64 || (long long)taps * ceil_div(IC, 16) > kMaxChunks) return false;
+  if (small_kernels_off() || IC < 1 || taps < 1 || taps > kMaxTaps || (long long)taps * ceil_div(IC, 16) > kMaxChunks) return false;
   const long long tiles = (long long)ceil_div(M, kTileM) * ceil_div(OC, kTileN);
   // unaligned rows take five loads for one: worth it up to half of that (3x3 28x28 x 100 -> 77, cost 12 k, 8.8 us against 12.9
   // padded; FullyConnected 500 x 1001 -> 1003, 21 k, 19.4 us against about 11)
@@ -499,8 +498,8 @@ cudaError_t launch_conv_small(const ConvSmallArgs& args, cudaStream_t stream) {
   a.steps = a.mode == kStem ? 1 : conv_small_steps(taps, a.IC);
   a.icb = a.mode == kStem ? 1 : ceil_div(a.IC, 16);
   a.chunks = taps * a.icb;
-  a.inv_icb = divide_constant(a.icb);
-  a.inv_kw = divide_constant(a.KW);
+  a.by_icb = chunk_divisor(a.icb);
+  a.inv_kw = tap_divisor(a.KW);
   a.vec = a.ldc % 8 == 0 && ((uintptr_t)a.out & 7) == 0 && ((uintptr_t)a.res & 7) == 0;
   // K is split over 2 or 4 warps while the grid stays within about twelve warps per SM, over 8 (whose sums take longer to
   // meet) only up to six. One layer, us with 1 / 2 / 4 / 8 warps per tile: 98 tiles, 3 steps 3.0 / 2.3 / 2.0 / 2.1;

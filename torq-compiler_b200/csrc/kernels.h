@@ -7,6 +7,7 @@
 #include <atomic>
 #include <vector>
 
+#include "chunk_divide.h"
 #include "common.cuh"
 
 namespace tb200 {
@@ -248,7 +249,8 @@ struct ConvSmallArgs {
   long long add_k;
   // filled by the launcher
   int m_tiles, n_tiles, steps, chunks, icb, ks_log2, vec;
-  uint32_t inv_icb, inv_kw;  // divide_constant
+  ChunkDivisor by_icb;
+  uint32_t inv_kw;  // tap_divisor
 };
 bool conv_small_applies(long long M, int OC, int taps, int IC);  // is this the faster kernel for the size
 int conv_small_steps(int taps, int IC);
