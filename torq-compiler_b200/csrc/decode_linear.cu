@@ -9,7 +9,10 @@
 //   * the op behind a product runs in its epilogue where a block holds what it needs: GeGLU (a warp's tile is 16 gate rows
 //     and the 16 matching up rows), head norm + RoPE + cache append (a cluster of eight blocks holds a head), the arg max
 //     over the logits.
-// Measured at the Gemma-3-1B shape, 32 sequences at position 1024, us per launch before -> after: see each kernel.
+// Measured at the Gemma-3-1B shape at position 1024, launches serialised, us per launch (split-K kernels of decoder.cu, 32 sequences)
+// -> here with 32 / one sequence: attention 10.6 + 3.4 -> 9.2 / 6.2, gate/up + GeGLU 10.5 + 4.4 -> 11.7 / 7.5, norms 8.6 -> 2.4, LM head
+// 125 -> 96 / 62, arg max 24 -> 2.3; q/k/v + head norm + RoPE 8.2 / 5.5, o and down 7.9 / 5.7 on average. A whole step, launches
+// overlapping: 1.20 / 0.81 ms.
 #include <cuda_bf16.h>
 
 #include <algorithm>

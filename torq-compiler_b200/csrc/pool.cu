@@ -10,7 +10,9 @@
 //  * Average: the rescale depends only on the number of taps inside the image. The planner gives per count a record
 //    {M', K} for which (sum * 2^16 * M' + K) >> 40 is TOSA's result for every sum that can occur (checked there); one
 //    multiply-add, the result's byte is bits 8..15 of the high word, and the 16-bit saturating pack is the int8 clamp.
-// What bounds it: HBM at large sizes. 64x112x112x64, 3x3 stride 2 (64 MB): max 21.3 -> 13 us, average 27.8 -> 14 us.
+// 64x112x112x64, 3x3 stride 2 (64 MB; kernel alone): max with a table behind it 21 + a table pass -> 13.3 us, average 28 -> 15.8 us. What
+// bounds it: the latency of its loads. A third of the warps fit (52 .. 64 registers), they wait for memory three quarters of
+// the time, issue slots are 42 .. 50 % used and DRAM 28 .. 35 %.
 //
 // The kernels below it take every other window: one thread per output pixel and 16, 4 or 1 channels; avgpool_warp_kernel
 // spreads the taps of a large window over a warp (the global pool at the end of a classifier).
