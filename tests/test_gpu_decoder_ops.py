@@ -51,7 +51,8 @@ def test_embed_and_rmsnorm(device):
 
 @pytest.mark.parametrize("B,K,N,splits", [(1, 1152, 1536, 0), (1, 6912, 1152, 0), (3, 512, 200, 1), (3, 1024, 77, 2),
                                           (8, 2048, 64, 4), (32, 1152, 256, 0), (1, 1152, 4096, 1),
-                                          # batches above 8: the tensor-core kernel (K % 64 == 0), ragged N, K splits
+                                          # slices left to the planner (0) take the decode step's product where K % 64 == 0, given
+                                          # ones the split-K kernels: CUDA cores up to two tokens, tensor cores above; ragged N
                                           (9, 1152, 1536, 0), (32, 6912, 1152, 0), (17, 256, 200, 0), (32, 1152, 4100, 1),
                                           (12, 1024, 77, 2), (24, 2048, 130, 5),
                                           (16, 1040, 64, 0),   # K % 64 != 0: stays on the CUDA-core kernel
@@ -73,6 +74,44 @@ def test_gemv_w8(device, B, K, N, splits, f32):
         assert err <= 1e-5, err
         return
     _close(got, _bf(want), floor=0.05)
+
+
+@pytest.mark.parametrize("H", [1, 30, 2052, 4096, 4099, 5000])
+def test_rmsnorm_widths(device, H):
+    """Rows in registers (a multiple of four up to 4096) and rows read twice (every other width)."""
+    rng = np.random.default_rng(H)
+    x, r = (to_bf16(rng.normal(0, 1, (3, H)).astype(np.float32)) for _ in range(2))
+    w = to_bf16(rng.normal(0, 0.1, H).astype(np.float32))
+    g = Graph()
+    g.output(g.rmsnorm(g.input((3, H), "bf16"), w, 1e-6, residual=g.input((3, H), "bf16")))
+    t, rt, wt = (torch.from_numpy(from_bf16(v)) for v in (x, r, w))
+    want = _bf(rt + _bf(t * torch.rsqrt((t * t).mean(-1, keepdim=True) + 1e-6) * (1 + wt)))
+    # two ulp of the norm and of the sum, also where the two cancel
+    got = from_bf16(run_graph_gpu(device, g, [x, r])[0])
+    assert (np.abs(got - want.numpy()) <= ULP2 * (np.abs(want.numpy()) + np.abs((want - rt).numpy()))).all()
+
+
+@pytest.mark.parametrize("D,n_q,n_kv", [(64, 3, 1), (128, 2, 2), (256, 3, 2), (10, 1, 1)])
+def test_rope_of_other_heads(device, D, n_q, n_kv):
+    """Head sizes and numbers of KV heads that no attention op here takes: the rotated queries."""
+    rng = np.random.default_rng(D)
+    B, T, theta = 3, 20, 10000.0
+    qw, kw = (to_bf16(rng.normal(0, 0.1, D).astype(np.float32)) for _ in range(2))
+    g = Graph()
+    kc, vc = g.state((B, T, n_kv * D), "bf16"), g.state((B, T, n_kv * D), "bf16")
+    qkv = to_bf16(rng.normal(0, 1, (B, (n_q + 2 * n_kv) * D)).astype(np.float32))
+    g.output(g.rope_kv(g.input(qkv.shape, "bf16"), g.input((1,), "i32"), qw, kw, kc, vc, n_q=n_q, n_kv=n_kv, head_dim=D, theta=theta, eps=1e-6))
+    pos, half = 7, D // 2
+    got = run_graph_gpu(device, g, [qkv, np.array([pos], np.int32)])[0]
+    q = torch.from_numpy(from_bf16(qkv))[:, :n_q * D].reshape(B, n_q, D)
+    q = _bf(q * torch.rsqrt((q * q).mean(-1, keepdim=True) + 1e-6) * (1 + torch.from_numpy(from_bf16(qw))))
+    inv = torch.pow(torch.tensor(theta), -torch.arange(half, dtype=torch.float32) / half)
+    cs, sn = torch.cos(pos * inv), torch.sin(pos * inv)
+    a, b = q[..., :half], q[..., half:]
+    want = torch.cat([a * cs - b * sn, b * cs + a * sn], -1).reshape(B, -1).numpy()
+    # a rotated pair may cancel: two ulp of its terms
+    bound = torch.cat([a.abs() * cs.abs() + b.abs() * sn.abs(), b.abs() * cs.abs() + a.abs() * sn.abs()], -1).reshape(B, -1).numpy()
+    assert (np.abs(from_bf16(got) - want) <= ULP2 * bound + 1e-6).all()
 
 
 def test_rope_kv_and_attention(device):
