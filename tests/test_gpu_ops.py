@@ -44,7 +44,9 @@ CONV_CASES = [
 
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("case", CONV_CASES)
-def test_conv2d(device, case, mode):
+@pytest.mark.parametrize("no_small", ["0", "1"])  # as the planner decides, and on the kernels of the large sizes
+def test_conv2d(device, case, mode, no_small, monkeypatch):
+    monkeypatch.setenv("TB200_NO_SMALL", no_small)
     shape, OC, k, stride, dil, pad, izp, wzp = case
     rng = np.random.default_rng(1234)
     x = rng.integers(-128, 128, shape, dtype=np.int8)
@@ -153,7 +155,9 @@ DW_CASES = [
 
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("case", DW_CASES)
-def test_depthwise(device, case, mode):
+@pytest.mark.parametrize("no_small", ["0", "1"])  # few outputs take a kernel of their own
+def test_depthwise(device, case, mode, no_small, monkeypatch):
+    monkeypatch.setenv("TB200_NO_SMALL", no_small)
     shape, k, M, stride, pad, izp = case
     rng = np.random.default_rng(1234)
     x = rng.integers(-128, 128, shape, dtype=np.int8)
@@ -172,7 +176,11 @@ def test_depthwise(device, case, mode):
                                        (33, 100, 130, 3), (256, 1280, 1000, -2),
                                        # the large corners of the FC sweep (M up to 4096, K = N up to 8192)
                                        (64, 4096, 4096, -7), (1, 8192, 8192, 0), (512, 8192, 8192, -7), (4096, 4096, 4096, 0)])
-def test_fully_connected(device, M, K, N, azp):
+@pytest.mark.parametrize("no_small", ["0", "1"])
+def test_fully_connected(device, M, K, N, azp, no_small, monkeypatch):
+    if no_small == "1" and M > 256:
+        pytest.skip("the same kernel either way")
+    monkeypatch.setenv("TB200_NO_SMALL", no_small)
     rng = np.random.default_rng(1234)
     a = rng.integers(-128, 128, (M, K), dtype=np.int8)
     w = rng.integers(-127, 128, (N, K), dtype=np.int8)
@@ -272,6 +280,8 @@ def test_matmul_int32(device):
     ((1, 20, 20, 48), (5, 5), (1, 1), (2, 2, 2, 2)),     # SPPF window
     ((2, 11, 12, 6), (2, 2), (2, 2), (0, 0, 0, 0)),
     ((1, 7, 7, 128), (7, 7), (1, 1), (0, 0, 0, 0)),      # avgpool2d.mlir (global)
+    # windows without a strip kernel: 16, 4 and 1 channels per thread
+    ((2, 13, 12, 32), (3, 3), (3, 3), (1, 1, 1, 1)), ((1, 10, 9, 20), (2, 3), (1, 2), (0, 1, 1, 1)), ((1, 9, 8, 5), (4, 4), (2, 2), (1, 2, 2, 1)),
 ])
 def test_pools(device, shape, kernel, stride, pad):
     rng = np.random.default_rng(1234)

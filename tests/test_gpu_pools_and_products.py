@@ -55,7 +55,7 @@ def test_table_behind_a_pool_at_the_strips_grid_limits(device, kind, shape):
 
 
 @pytest.mark.parametrize("n", [1, 15, 16, 4099])
-@pytest.mark.parametrize("scales", [(0.02, 0.1, 0.05), (0.07, 0.03, 0.09), (0.05, 0.05, 0.02)])
+@pytest.mark.parametrize("scales", [(0.02, 0.1, 0.05), (0.07, 0.03, 0.09), (0.05, 0.05, 0.02), (0.05, 0.05, 0.0008)])  # the last too steep for the linear form
 def test_rescaled_add_covers_every_operand_pair(device, n, scales):
     rng = np.random.default_rng(n)
     m0, m1, mo = add_rescale_params(*scales)
