@@ -136,3 +136,49 @@ def test_folded_scalar_rounds_as_the_multiplication_does(device, cols):
         ex.destroy()
         got.append(run_graph_gpu(device, g, [x])[0])
     assert (got[0].view(np.uint32) == got[1].view(np.uint32)).all(), int((got[0] != got[1]).sum())
+
+
+def _pools_and_add(shape, k, s, table, max_first, fn="add", pad_value=-128):
+    """fn of the max pool (a table behind it) and the average pool of one tensor."""
+    rng = np.random.default_rng(shape[1])
+    m0, m1, mo = add_rescale_params(0.02, 0.03, 0.04)
+    pad = ((k - 1) // 2, k // 2) * 2
+    g = Graph()
+    x = g.input(shape)
+    mx = g.maxpool2d(x, (k, k), (s, s), pad, pad_value=pad_value)
+    if table:
+        mx = g.table(mx, rng.integers(-128, 128, 256).astype(np.int8))
+    av = g.avg_pool2d(x, (k, k), (s, s), pad, input_zp=-9, output_zp=100)  # saturates
+    a, b = (mx, av) if max_first else (av, mx)
+    g.output(getattr(g, fn)(a, b, a_zp=-7, a_ms=m0, b_zp=10, b_ms=m1, out_ms=mo, out_zp=2, clamp=(-120, 127) if table else (-128, 127)))
+    return g
+
+
+@pytest.mark.parametrize("k,s", [(2, 2), (3, 1), (3, 2), (5, 1)])
+@pytest.mark.parametrize("shape", [(1, 5, 7, 3), (2, 9, 6, 20), (1, 13, 11, 32), (3, 40, 33, 64), (9, 112, 107, 32), (20, 61, 64, 64), (5, 90, 91, 100)])
+@pytest.mark.parametrize("table,max_first,fn", [(True, True, "add"), (False, False, "add"), (True, False, "sub")])
+def test_two_pools_and_their_sum_in_one_launch(device, k, s, shape, table, max_first, fn):
+    g = _pools_and_add(shape, k, s, table, max_first, fn)
+    ex = Executable(device, g.serialize())
+    assert ex.launch_count == 1 and ex.op_kernels()[-1] == "pool_add", ex.op_kernels()
+    ex.destroy()
+    _check(device, g, [np.random.default_rng(k).integers(-128, 128, shape, dtype=np.int8)])
+
+
+def test_two_pools_and_their_sum_one_by_one(device):
+    """Another pad value, or a result that lies over the pooled tensor: the three ops as they are."""
+    shape = (2, 24, 24, 16)
+    x = np.random.default_rng(0).integers(-128, 128, shape, dtype=np.int8)
+    g = _pools_and_add(shape, 3, 2, True, True, pad_value=-77)
+    ex = Executable(device, g.serialize())
+    assert ex.launch_count == 3, ex.op_kernels()
+    ex.destroy()
+    _check(device, g, [x])
+    g = _pools_and_add(shape, 3, 1, True, True)
+    ex = Executable(device, g.serialize())
+    buf = device.alloc(x.nbytes)
+    buf.upload(x)
+    ex.dispatch([buf], [buf])
+    got = buf.download(shape, np.int8)
+    buf.free(), ex.destroy()
+    assert (got == run_graph(g, [x])[0]).all()

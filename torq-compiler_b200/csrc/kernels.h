@@ -107,6 +107,15 @@ struct PoolArgs {
 bool pool_strip_applies(const PoolArgs& a);  // by window and strides, element type, N and OH (grid limits); the rest is not looked at
 // Records {M', -, K} by tap count (index 0 unused) of pool_strip_kernel's average; false when a count has no exact one.
 bool pool_avg_records(int taps, int input_zp, int output_zp, std::vector<int4>& out);
+// add / sub of the max pool and the average pool of one tensor over the same windows (pool_add_kernel): the two pools never reach memory.
+// pool.lut: a table behind the max pool, or null. The add's linear form with its factors sorted by pool.
+struct PoolAddArgs {
+  PoolArgs pool;
+  int m_max, m_avg, f, clamp_min, clamp_max;
+  long long k;
+};
+bool pool_add_applies(const PoolArgs& a);  // by window, strides, sizes and pad value
+cudaError_t launch_pool_add(const PoolAddArgs& a, cudaStream_t stream);
 void launch_maxpool(const PoolArgs& a, cudaStream_t stream);
 void launch_avgpool(const PoolArgs& a, cudaStream_t stream);
 

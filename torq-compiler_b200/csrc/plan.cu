@@ -631,6 +631,11 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   // untransposed tensor), the multiplication of softmax's operand by a scalar, and the cast of its result.
   std::vector<int> folded_transpose(ops.size(), -1);  // matmul op -> the tensor its transposed operand is read from
   std::vector<int> softmax_scale(ops.size(), -1), softmax_cast(ops.size(), -1);  // softmax op -> the ew op fused into it
+  // An add / sub of the max pool (with or without a table behind it) and the average pool of one tensor over the same windows
+  // runs as one kernel in the add's place. The pools are planned as by themselves and their launches kept: a caller whose
+  // result buffer overlaps the pooled tensor gets the ops one by one.
+  std::vector<int> max_of_add(ops.size(), -1), avg_of_add(ops.size(), -1);  // add / sub op -> its two pools
+  std::vector<char> held(ops.size(), 0);                                    // pool op whose launch the add behind it makes or replaces
   {
     std::vector<int> uses(nt, 0), producer(nt, -1);
     for (int i = 0; i < (int)ops.size(); i++) {
@@ -815,6 +820,47 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         }
       }
     }
+    for (int i = 0; i < (int)ops.size(); i++) {
+      const auto& op = ops[i];
+      if ((op.kind != TB200_OP_ADD && op.kind != TB200_OP_SUB) || fused_away[i] || !b.valid_id(op.in0) || !b.valid_id(op.in1) || !b.valid_id(op.out0) ||
+          op.in0 == op.in1 || tensors[op.out0].dtype != TB200_I8)
+        continue;
+      int pool[2] = {-1, -1};  // by kind: max, average
+      for (int src : {op.in0, op.in1}) {
+        if (tensors[src].kind != TB200_TENSOR_ACTIVATION || tensors[src].dtype != TB200_I8 || uses[src] != 1) break;
+        int p = producer[src];
+        if (p >= 0 && p < i && ops[p].kind == TB200_OP_TABLE && fused_away[p]) {
+          const int from = producer[ops[p].in0];
+          p = from >= 0 && ops[from].kind == TB200_OP_MAXPOOL && table_after[from] == p ? from : -1;
+        }
+        if (p < 0 || p >= i || (ops[p].kind != TB200_OP_MAXPOOL && ops[p].kind != TB200_OP_AVGPOOL)) break;
+        pool[ops[p].kind == TB200_OP_AVGPOOL] = p;
+      }
+      if (pool[0] < 0 || pool[1] < 0) continue;
+      const auto& mx = ops[pool[0]]; const auto& av = ops[pool[1]];
+      const int x = mx.in0;
+      if (x != av.in0 || !b.act_i8(x, 4) || !b.act_i8(mx.out0, 4) || !b.act_i8(av.out0, 4) || !b.same_shape(mx.out0, av.out0) ||
+          (tensors[x].kind != TB200_TENSOR_INPUT && tensors[x].kind != TB200_TENSOR_ACTIVATION) || mx.kh != av.kh || mx.kw != av.kw ||
+          mx.stride_h != av.stride_h || mx.stride_w != av.stride_w || mx.pad_t != av.pad_t || mx.pad_l != av.pad_l || table_after[pool[1]] >= 0 ||
+          b.numel(op.in0) != b.numel(mx.out0) || b.numel(op.in1) != b.numel(mx.out0) || b.numel(op.out0) != b.numel(mx.out0))
+        continue;
+      // the pools move to the add's place: nothing in between may write where the caller's input could lie
+      bool clear = true;
+      for (int j = std::min(pool[0], pool[1]); j < i; j++)
+        for (int id : {ops[j].out0, ops[j].out1, extra_out[j]})
+          clear = clear && (id < 0 || (id < nt && id != x && tensors[id].kind == TB200_TENSOR_ACTIVATION));
+      PoolArgs a{};
+      a.KH = mx.kh; a.KW = mx.kw; a.stride_h = mx.stride_h; a.stride_w = mx.stride_w; a.pad_value = mx.pad_value;
+      a.N = tensors[mx.out0].shape[0]; a.OH = tensors[mx.out0].shape[1]; a.OW = tensors[mx.out0].shape[2]; a.C = tensors[mx.out0].shape[3];
+      std::vector<int4> rec;
+      if (!clear || !pool_add_applies(a) || !pool_avg_records(a.KH * a.KW, av.in0_zp, av.out_zp, rec)) continue;
+      const BinaryArgs* lin = binary_args(i);
+      if (!lin || !lin->lin) continue;
+      max_of_add[i] = pool[0];
+      avg_of_add[i] = pool[1];
+      held[pool[0]] = held[pool[1]] = 1;
+      extra_in[i] = x;
+    }
     const char* no_dec = getenv("TB200_NO_DECODER_FUSION");
     for (int i = 0; i + 1 < (int)ops.size() && !(no_dec && *no_dec && *no_dec != '0'); i++) {
       const auto& op = ops[i];
@@ -949,6 +995,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   auto report = [](cudaError_t e, const ExecContext& c) {
     if (e != cudaSuccess && c.launch_error) *c.launch_error = e;
   };
+  struct PlannedPool { PoolArgs args; Loc x; size_t lut_off, rec_off; bool has_lut; std::function<void(const ExecContext&)> launch; };
+  std::map<int, PlannedPool> pools;  // held pool ops
   bool needs_fusion = false;  // the graph holds ops that exist only inside the fused decode step
   // ---- one step per op ----
   for (int i = 0; i < (int)ops.size(); i++) {
@@ -1665,6 +1713,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           if (is_max) launch_maxpool(k, c.stream);
           else launch_avgpool(k, c.stream);
         };
+        if (held[i]) {
+          pools[i] = PlannedPool{a, lx, lut_off, rec_off, fused_table >= 0, step.launch};
+          step.kernel_name = "(pool in the add behind it)";
+          step.launches = 0;
+          step.launch = [](const ExecContext&) {};
+        }
         break;
       }
       case TB200_OP_ADD:
@@ -1690,6 +1744,31 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           k.out = (int8_t*)lo.resolve(c);
           launch_binary(k, c.stream);
         };
+        if (max_of_add[i] >= 0) {
+          const PlannedPool mx = pools[max_of_add[i]], av = pools[avg_of_add[i]];
+          const bool max_first = op.in0 == (mx.has_lut ? ops[table_after[max_of_add[i]]].out0 : ops[max_of_add[i]].out0);
+          PoolAddArgs pa{};
+          pa.pool = mx.args;
+          pa.m_max = max_first ? a.lin_ma : a.lin_mb;
+          pa.m_avg = max_first ? a.lin_mb : a.lin_ma;
+          pa.f = a.lin_f; pa.k = a.lin_k; pa.clamp_min = a.clamp_min; pa.clamp_max = a.clamp_max;
+          const size_t x_bytes = (size_t)pa.pool.N * pa.pool.H * pa.pool.W * pa.pool.C;
+          step.kernel_name = "pool_add";
+          step.launch = [=, one_by_one = step.launch](const ExecContext& c) {
+            PoolAddArgs k = pa;
+            k.pool.x = (const int8_t*)mx.x.resolve(c);
+            k.pool.out = (int8_t*)lo.resolve(c);
+            if (k.pool.x < k.pool.out + n && k.pool.out < k.pool.x + x_bytes) {  // the result lies over the tensor that is still being read
+              mx.launch(c);
+              av.launch(c);
+              one_by_one(c);
+              return;
+            }
+            k.pool.lut = mx.has_lut ? (const int8_t*)(c.consts + mx.lut_off) : nullptr;
+            k.pool.by_count = (const int4*)(c.consts + av.rec_off);
+            report(launch_pool_add(k, c.stream), c);
+          };
+        }
         break;
       }
       case TB200_OP_TABLE: {

@@ -18,6 +18,7 @@
 // spreads the taps of a large window over a warp (the global pool at the end of a classifier).
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include "dependent_launch.cuh"
@@ -39,6 +40,46 @@ inline unsigned grid_for(long long work_items, int per_block = kThreads) {
 }
 
 constexpr int kStripThreads = 128;
+
+// Sum and packed unsigned maximum of N words of two 16-bit fields (three operands to an instruction).
+template <int N>
+__device__ __forceinline__ uint32_t sum_of(const uint32_t (&v)[N]) {
+  uint32_t s = v[0];
+#pragma unroll
+  for (int i = 1; i < N; i++) s += v[i];
+  return s;
+}
+// The same for sums below 2048 on the other arithmetic pipe: the bit pattern of a 16-bit float below 2^-13 is its value in units of
+// 2^-24, and sums of such floats are exact.
+template <int N>
+__device__ __forceinline__ uint32_t row_sum(const uint32_t (&v)[N]) {
+  static_assert(N * 255 < 2048, "bit patterns count units only below 2048");
+  uint32_t s = v[0];
+#pragma unroll
+  for (int i = 1; i < N; i++) asm("add.rn.f16x2 %0, %0, %1;" : "+r"(s) : "r"(v[i]));
+  return s;
+}
+template <int N>
+__device__ __forceinline__ uint32_t max_u16x2_of(const uint32_t (&v)[N]) {
+  uint32_t m = v[0];
+  int i = 1;
+#pragma unroll
+  for (; i + 1 < N; i += 2) m = __vimax3_u16x2(m, v[i], v[i + 1]);
+  return i < N ? __vmaxu2(m, v[i]) : m;
+}
+template <int N>
+__device__ __forceinline__ uint32_t max_s16x2_of(const uint32_t (&v)[N]) {
+  uint32_t m = v[0];
+  int i = 1;
+#pragma unroll
+  for (; i + 1 < N; i += 2) m = __vimax3_s16x2(m, v[i], v[i + 1]);
+  return i < N ? max_s16x2(m, v[i]) : m;
+}
+__device__ __forceinline__ uint32_t pack_sat_s16x2(int lo, int hi) {
+  uint32_t r;
+  asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(r) : "r"(hi), "r"(lo));
+  return r;
+}
 
 // VW: 32-bit words of channels per thread (4 or 1), or 0 for a single channel.
 template <int VW, int K, int S, int ROWS, bool AVG, bool LUT>
@@ -168,6 +209,167 @@ __global__ void __launch_bounds__(kStripThreads) pool_strip_kernel(PoolArgs a) {
     out += (size_t)a.OW * a.C;
   }
 }
+
+// add / sub of the max pool (with an optional table behind it) and the average pool of one tensor: one pass over the input where the
+// three ops make three passes and move 2.25 times the bytes. A thread owns one output column of 16, 4 or 1 channels and a strip of
+// rows; the rows the next step needs are loaded before the last ones are reduced. Both reductions work on the same unpacked bytes
+// (biased by 128, two to a word as 16-bit fields: unsigned maxima and sums). What follows the maximum (table, factor and constant of
+// the add's linear form) is one 64-bit entry per byte value, filled by the block before it waits for the launch ahead; the average's
+// byte is multiplied in by one multiply-add.
+// 64x112x112x64, 3x3 stride 2, table behind the maximum (kernel alone, buffers out of L2): three launches 39 us, this one 20.1. What bounds
+// it: integer instructions, about 115 per four outputs and most of them on one pipe (measured: the sums of a row on the float pipe
+// 20.7 -> 20.1; input staged in shared memory, which halves what L2 is asked for, 27; all loads of a strip up front and no loop 22.5).
+// Four rows to a strip: 1, 2, 3, 4, 7, 14 rows take 29, 22.9, 21.0, 20.1, 20.5, 23.6 us (halo rows against waves of blocks).
+template <int VW, int K, int S>
+__global__ void __launch_bounds__(kStripThreads, VW == 4 ? 4 : 7) pool_add_kernel(const PoolAddArgs pa, int cols, int strips, int strip_rows, int threads) {
+  const PoolArgs& a = pa.pool;
+  __shared__ long long from_max[256];
+  for (int v = threadIdx.x; v < 256; v += kStripThreads) {  // v: the byte biased by 128
+    const int q = a.lut ? (int)a.lut[v] : v - 128;
+    from_max[v] = (long long)(q * 256) * (long long)pa.m_max + pa.k;
+  }
+  __syncthreads();
+  grid_dependency_wait();
+  grid_dependency_release();
+  constexpr int VB = VW == 0 ? 1 : 4 * VW;  // channels per thread
+  constexpr int NW = VW == 0 ? 1 : VW;
+  const int idx = blockIdx.x * kStripThreads + threadIdx.x;
+  if (idx >= threads) return;
+  const int strip_of_all = idx / cols, col = idx - strip_of_all * cols;
+  const int n = strip_of_all / strips, oh0 = (strip_of_all - n * strips) * strip_rows;
+  const int nrows = min(strip_rows, a.OH - oh0);
+  const int groups = a.C / VB;
+  const int ow = col / groups, g = col - ow * groups;
+  const int iw0 = ow * S - a.pad_l, ih0 = oh0 * S - a.pad_t;
+  const long long row_bytes = (long long)a.W * a.C;
+  const int8_t* px = a.x + (size_t)n * a.H * row_bytes + (long long)ih0 * row_bytes + (long long)iw0 * a.C + g * VB;
+  int8_t* out = a.out + (((size_t)n * a.OH + oh0) * a.OW + ow) * a.C + g * VB;
+  const bool narrow = pa.clamp_min != -128 || pa.clamp_max != 127;
+  const uint32_t lo2 = (uint32_t)(pa.clamp_min & 0xffff) * 0x10001u, hi2 = (uint32_t)(pa.clamp_max & 0xffff) * 0x10001u;
+  struct Raw {
+    uint32_t w[K][NW];
+  };
+  // horizontal reductions of one input row: bytes 0 and 2 (e), 1 and 3 (o) of every word, sums (s) and maxima (m)
+  struct Row {
+    uint32_t se[NW], so[NW], me[NW], mo[NW];
+  };
+  // EDGE: some window of the warp may hang over the frame
+  auto strip = [&](auto edge) {
+    constexpr bool EDGE = decltype(edge)::value;
+    bool col_ok[K];
+    int ncol = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      col_ok[k] = !EDGE || (iw0 + k >= 0 && iw0 + k < a.W);
+      ncol += col_ok[k];
+    }
+    auto load_row = [&](int ih, Raw& r) {
+      const bool row_ok = !EDGE || (ih >= 0 && ih < a.H);
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        if (EDGE) {
+#pragma unroll
+          for (int j = 0; j < NW; j++) r.w[k][j] = 0x80808080u;  // outside: nothing to the sum, the lowest value to the maximum
+        }
+        if (row_ok && col_ok[k]) {
+          const int8_t* p = px + (size_t)k * a.C;
+          if (VW == 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(p);
+            r.w[k][0] = v.x; r.w[k][NW > 1 ? 1 : 0] = v.y; r.w[k][NW > 2 ? 2 : 0] = v.z; r.w[k][NW > 3 ? 3 : 0] = v.w;
+          } else if (VW == 1) {
+            r.w[k][0] = *reinterpret_cast<const uint32_t*>(p);
+          } else {
+            r.w[k][0] = (uint32_t)(uint8_t)*p;
+          }
+        }
+      }
+      px += row_bytes;
+    };
+    auto reduce = [&](const Raw& raw) {
+      Row r;
+#pragma unroll
+      for (int j = 0; j < NW; j++) {
+        uint32_t e[K], o[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          e[k] = (raw.w[k][j] ^ 0x80808080u) & 0x00ff00ffu;
+          o[k] = VW == 0 ? 0u : __byte_perm(raw.w[k][j], 0, 0x4341) ^ 0x00800080u;
+        }
+        r.se[j] = row_sum<K>(e);
+        r.me[j] = max_u16x2_of<K>(e);
+        r.so[j] = VW == 0 ? 0u : row_sum<K>(o);
+        r.mo[j] = VW == 0 ? 0u : max_u16x2_of<K>(o);
+      }
+      return r;
+    };
+    int ih = ih0;
+    Row rows[K];  // the window's
+    Raw next[S];  // the rows the next step adds, on their way while the last ones are reduced
+#pragma unroll
+    for (int i = 0; i < K - S; i++) {
+      Raw raw;
+      load_row(ih++, raw);
+      rows[S + i] = reduce(raw);
+    }
+#pragma unroll
+    for (int i = 0; i < S; i++) load_row(ih++, next[i]);
+    int4 c = __ldg(a.by_count + K * K);
+#pragma unroll 1
+    for (int r = 0; r < nrows; r++) {
+#pragma unroll
+      for (int i = 0; i < K - S; i++) rows[i] = rows[S + i];
+#pragma unroll
+      for (int i = 0; i < S; i++) rows[K - S + i] = reduce(next[i]);
+      if (r + 1 < nrows) {
+#pragma unroll
+        for (int i = 0; i < S; i++) load_row(ih++, next[i]);
+      }
+      if (EDGE) {
+        const int top = ih0 + r * S;
+        c = __ldg(a.by_count + ncol * (min(top + K, a.H) - max(top, 0)));
+      }
+      const unsigned long long kk = ((unsigned long long)(uint32_t)c.w << 32) | (uint32_t)c.z;
+      auto average = [&](uint32_t sum_high) { return (int)(((unsigned long long)sum_high * (uint32_t)c.x + kk) >> 32); };
+      uint32_t res[NW];
+#pragma unroll
+      for (int j = 0; j < NW; j++) {
+        uint32_t t[K];
+#pragma unroll
+        for (int i = 0; i < K; i++) t[i] = rows[i].se[j];
+        const uint32_t se = sum_of<K>(t);
+#pragma unroll
+        for (int i = 0; i < K; i++) t[i] = rows[i].me[j];
+        const uint32_t me = max_u16x2_of<K>(t);
+#pragma unroll
+        for (int i = 0; i < K; i++) t[i] = rows[i].so[j];
+        const uint32_t so = sum_of<K>(t);
+#pragma unroll
+        for (int i = 0; i < K; i++) t[i] = rows[i].mo[j];
+        const uint32_t mo = max_u16x2_of<K>(t);
+        // the average's bytes in the high byte of 16-bit fields (saturated as the op does), then the linear form
+        const uint32_t qe = pack_sat_s16x2(average(se << 16), average(se & 0xffff0000u));
+        const int h0 = mad_wide_hi(sx8_shl8<1>(qe), pa.m_avg, from_max[me & 0xffffu]) >> pa.f;
+        const int h2 = VW == 0 ? h0 : mad_wide_hi(sx8_shl8<3>(qe), pa.m_avg, from_max[me >> 16]) >> pa.f;
+        int h1 = h0, h3 = h0;
+        if (VW != 0) {
+          const uint32_t qo = pack_sat_s16x2(average(so << 16), average(so & 0xffff0000u));
+          h1 = mad_wide_hi(sx8_shl8<1>(qo), pa.m_avg, from_max[mo & 0xffffu]) >> pa.f;
+          h3 = mad_wide_hi(sx8_shl8<3>(qo), pa.m_avg, from_max[mo >> 16]) >> pa.f;
+        }
+        res[j] = narrow ? clamp_pack4(h0, h1, h2, h3, lo2, hi2) : sat_pack4(h0, h1, h2, h3);
+      }
+      if (VW == 4)
+        *reinterpret_cast<uint4*>(out) = make_uint4(res[0], res[NW > 1 ? 1 : 0], res[NW > 2 ? 2 : 0], res[NW > 3 ? 3 : 0]);
+      else if (VW == 1) *reinterpret_cast<uint32_t*>(out) = res[0];
+      else *out = (int8_t)res[0];
+      out += (size_t)a.OW * a.C;
+    }
+  };
+  const bool inside = iw0 >= 0 && iw0 + K <= a.W && ih0 >= 0 && ih0 + (nrows - 1) * S + K <= a.H;
+  if (__all_sync(__activemask(), inside)) strip(std::false_type{});
+  else strip(std::true_type{});
+}
+
 
 // ---- any other window ----
 // I: index type, 32 bits where the tensor allows (a 64-bit division costs more than a window of loads)
@@ -475,7 +677,36 @@ bool try_strip(const PoolArgs& a, cudaStream_t stream) {
   return true;
 }
 bool fits32(const PoolArgs& a) { return (long long)a.N * a.OH * a.OW * a.C < (1ll << 30); }
+
+template <int VW, int K, int S>
+cudaError_t launch_pool_add_strips(const PoolAddArgs& a, int rows, cudaStream_t stream) {
+  const int vb = VW == 0 ? 1 : 4 * VW, cols = a.pool.OW * (a.pool.C / vb), strips = (a.pool.OH + rows - 1) / rows;
+  const int threads = a.pool.N * strips * cols;  // pool_add_applies: fits
+  return launch_dependent(pool_add_kernel<VW, K, S>, dim3((unsigned)((threads + kStripThreads - 1) / kStripThreads)), dim3(kStripThreads), 0,
+                          stream, a, cols, strips, rows, threads);
+}
+// As in launch_strip_shape, and the strip shortened step by step: two rows halve what a warp has to do in turn at the cost of a quarter
+// more input rows. Words of 4 channels take strips of 8 where there is work for them (27.3 -> 23.8 us at the size above).
+template <int K, int S>
+cudaError_t launch_pool_add_shape(const PoolAddArgs& pa, cudaStream_t stream) {
+  const PoolArgs& a = pa.pool;
+  const uintptr_t at = (uintptr_t)a.x | (uintptr_t)a.out;
+  const long long pixels = (long long)a.N * a.OH * a.OW, want = 148ll * 512, wide = pixels * (a.C / 16) / want, words = pixels * (a.C / 4) / want;
+  if ((at & 15) == 0 && (a.C & 15) == 0 && wide >= 1) return launch_pool_add_strips<4, K, S>(pa, wide >= 4 ? 4 : wide >= 2 ? 2 : 1, stream);
+  if ((at & 3) == 0 && (a.C & 3) == 0) return launch_pool_add_strips<1, K, S>(pa, words >= 8 ? 8 : words >= 4 ? 4 : 1, stream);
+  return launch_pool_add_strips<0, K, S>(pa, 4, stream);
+}
 }  // namespace
+
+bool pool_add_applies(const PoolArgs& a) {
+  return pool_strip_applies(a) && a.pad_value == -128 && (long long)a.N * a.OH * a.OW * a.C < (1ll << 31) - kStripThreads;
+}
+
+cudaError_t launch_pool_add(const PoolAddArgs& a, cudaStream_t stream) {
+  if (a.pool.KH == 2) return launch_pool_add_shape<2, 2>(a, stream);
+  if (a.pool.KH == 5) return launch_pool_add_shape<5, 1>(a, stream);
+  return a.pool.stride_h == 1 ? launch_pool_add_shape<3, 1>(a, stream) : launch_pool_add_shape<3, 2>(a, stream);
+}
 
 void launch_maxpool(const PoolArgs& a, cudaStream_t stream) {
   if (try_strip<false>(a, stream)) return;
