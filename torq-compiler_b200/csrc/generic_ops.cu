@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 
 #include "../../include/torq_b200_ops.h"
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace tb200 {
@@ -275,6 +276,8 @@ template <typename TIn, typename TOut, int PER>
 __global__ void __launch_bounds__(128) softmax_kernel(SoftmaxArgs a) {
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  grid_dependency_release();
   if (row >= a.rows) return;
   const TIn* x = reinterpret_cast<const TIn*>(a.x) + row * a.cols;
   TOut* out = reinterpret_cast<TOut*>(a.out) + row * a.cols;
@@ -424,10 +427,10 @@ void launch_softmax(const SoftmaxArgs& a, cudaStream_t stream) {
   auto sized = [&](auto in, auto out) {
     typedef decltype(in) I;
     typedef decltype(out) O;
-    if (a.cols <= 256) softmax_kernel<I, O, 8><<<blocks, 128, 0, stream>>>(a);
-    else if (a.cols <= 512) softmax_kernel<I, O, 16><<<blocks, 128, 0, stream>>>(a);
-    else if (a.cols <= 1024) softmax_kernel<I, O, 32><<<blocks, 128, 0, stream>>>(a);
-    else softmax_kernel<I, O, 0><<<blocks, 128, 0, stream>>>(a);
+    if (a.cols <= 256) launch_dependent(softmax_kernel<I, O, 8>, dim3(blocks), dim3(128), 0, stream, a);
+    else if (a.cols <= 512) launch_dependent(softmax_kernel<I, O, 16>, dim3(blocks), dim3(128), 0, stream, a);
+    else if (a.cols <= 1024) launch_dependent(softmax_kernel<I, O, 32>, dim3(blocks), dim3(128), 0, stream, a);
+    else launch_dependent(softmax_kernel<I, O, 0>, dim3(blocks), dim3(128), 0, stream, a);
   };
   if (a.dtype == TB200_F32) {
     if (a.out_dtype == TB200_F32) sized(0.f, 0.f);

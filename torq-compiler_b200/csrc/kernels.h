@@ -91,7 +91,7 @@ bool depthwise3x3_supported(const DwArgs& a);
 size_t depthwise3x3_pack(const int8_t* w, int C, int stride, uint32_t* out);
 
 // raw integer matmul (matmul_tile.cu), b is [K][N], or [N][K] when b_transposed
-void launch_matmul_int(const void* a, const void* b, void* out, bool in_i16, bool out_i16, int M, int K, int N, int a_zp,
+cudaError_t launch_matmul_int(const void* a, const void* b, void* out, bool in_i16, bool out_i16, int M, int K, int N, int a_zp,
                        int b_zp, bool b_transposed, cudaStream_t stream);
 
 struct PoolArgs {
@@ -432,7 +432,7 @@ void launch_reduce(const ReduceArgs& a, cudaStream_t stream);
 // (the caller has copied values to out first). Indices outside [0, K) give zero rows / are skipped.
 void launch_gather_rows(const void* values, const int32_t* idx, void* out, int N, int K, int W, int row_bytes, cudaStream_t stream);
 void launch_scatter_rows(const void* updates, const int32_t* idx, void* out, int N, int K, int W, int row_bytes, cudaStream_t stream);
-void launch_matmul_f(const void* a, const void* b, void* out, int M, int K, int N, int in_dtype, int out_dtype, bool b_transposed,
+cudaError_t launch_matmul_f(const void* a, const void* b, void* out, int M, int K, int N, int in_dtype, int out_dtype, bool b_transposed,
                      cudaStream_t stream);
 struct DepthwiseFArgs {
   const void* x;     // [N, H, W, C]

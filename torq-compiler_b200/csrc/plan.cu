@@ -1641,7 +1641,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           const int azp = op.in0_zp, bzp = op.weight_zp;
           step.kernel_name = "matmul_int";
           step.launch = [=](const ExecContext& c) {
-            launch_matmul_int(lx.resolve(c), lw.resolve(c), lo.resolve(c), in16, out16, M, K, N, azp, bzp, tb_fold, c.stream);
+            report(launch_matmul_int(lx.resolve(c), lw.resolve(c), lo.resolve(c), in16, out16, M, K, N, azp, bzp, tb_fold, c.stream), c);
           };
           break;
         }
@@ -1658,7 +1658,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         int azp = op.in0_zp, bzp = op.weight_zp;
         step.kernel_name = "matmul_int";
         step.launch = [=](const ExecContext& c) {
-          launch_matmul_int(lx.resolve(c), c.consts + w_off, lo.resolve(c), false, false, M, K, N, azp, bzp, false, c.stream);
+          report(launch_matmul_int(lx.resolve(c), c.consts + w_off, lo.resolve(c), false, false, M, K, N, azp, bzp, false, c.stream), c);
         };
         break;
       }
@@ -2357,7 +2357,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         Loc la = loc(op.in0), lb = loc(tb_fold ? folded_transpose[i] : op.in1), lo = loc(op.out0);
         step.kernel_name = "matmul_f";
         step.launch = [=](const ExecContext& c) {
-          launch_matmul_f(la.resolve(c), lb.resolve(c), lo.resolve(c), M, K, N, idt, odt, tb_fold, c.stream);
+          report(launch_matmul_f(la.resolve(c), lb.resolve(c), lo.resolve(c), M, K, N, idt, odt, tb_fold, c.stream), c);
         };
         break;
       }
