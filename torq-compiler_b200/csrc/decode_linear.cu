@@ -736,8 +736,12 @@ __global__ void __launch_bounds__(512) rmsnorm_row_kernel(const uint16_t* __rest
       if (w2) wv2[k] = __ldg(reinterpret_cast<const uint2*>(w2 + i));
     }
   }
-  grid_dependency_wait();
+  // Lets the product behind it in before its own wait: a norm runs for a microsecond, and a product that came only then asked for its
+  // weights and scales 2 us after its activations were there. The product reads nothing but constants before its wait, and what
+  // runs before a norm in a chain (the products, the embedding) releases after its wait, so no chain stacks up further.
+  // One step of the 1B shape at position 1024: 808 -> 748 us (one sequence), 1215 -> 1167 us (32); products that release first, too: 747 / 1210.
   grid_dependency_release();
+  grid_dependency_wait();
   const size_t base = (size_t)blockIdx.x * H;
   float v[V][4], r[V][4], ss = 0.f;
 #pragma unroll
