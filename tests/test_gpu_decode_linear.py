@@ -38,6 +38,39 @@ def test_products(device, B, K, N):
     assert (ids == got.argmax(-1)).all()
 
 
+@pytest.mark.parametrize("B,K,N", [(1, 1152, 40), (2, 6912, 33), (7, 64, 32), (8, 1152, 30001)])
+@pytest.mark.parametrize("spread", [0, 8, 40, 120])
+def test_products_of_few_tokens_over_magnitudes(device, B, K, N, spread):
+    """Up to eight tokens the activations enter as fixed-point numbers: magnitudes 2^-spread .. 1 side by side, subnormals at the far end.
+    Against 64 bits; the bound is that of an fp32 sum of K terms: K 2^-24 of the sum of magnitudes."""
+    rng = np.random.default_rng(B + K + spread)
+    x = to_bf16((rng.normal(0, 1, (B, K)) * np.exp2(rng.uniform(-spread, 0, (B, K)) - (100 if spread == 40 else 0))).astype(np.float32))
+    x[0, : K // 2] = 0
+    w = rng.integers(-128, 128, (N, K), dtype=np.int8)
+    s = to_bf16(np.ones(N, np.float32))
+    g = Graph()
+    g.output(g.gemv_w8(g.input((B, K), "bf16"), w, s, out_dtype="f32"))
+    got = run_graph_gpu(device, g, [x])[0].astype(np.float64)
+    xd, wd = from_bf16(x).astype(np.float64), w.astype(np.float64)
+    bound = K * 2.0 ** -24 * (np.abs(xd) @ np.abs(wd).T) + 1e-44
+    assert (np.abs(got - xd @ wd.T) <= bound).all(), np.max(np.abs(got - xd @ wd.T) / bound)
+
+
+@pytest.mark.parametrize("B,K,N", [(1, 64, 40), (3, 1152, 33), (8, 1152, 30001)])
+def test_products_of_few_tokens_with_infinities_and_nans(device, B, K, N):
+    rng = np.random.default_rng(K)
+    x, w, s, _ = _product(rng, B, K, N)
+    x[0, 5], x[B - 1, K - 1] = 0x7f80, (0x7fc0 if B > 1 else 0x7f80)
+    g = Graph()
+    g.output(g.gemv_w8(g.input((B, K), "bf16"), w, s, out_dtype="f32"))
+    got = run_graph_gpu(device, g, [x])[0]
+    with np.errstate(invalid="ignore"):
+        want = (from_bf16(x)[:, None, :] * w.astype(np.float32)[None]).sum(-1) * from_bf16(s)[None]
+    assert (np.isnan(got) == np.isnan(want)).all() and (np.isposinf(got) == np.isposinf(want)).all() and (np.isneginf(got) == np.isneginf(want)).all()
+    ok = np.isfinite(want)
+    assert not ok.any() or np.abs(got[ok] - want[ok]).max() <= 1e-5 * np.abs(want[ok]).max()
+
+
 @pytest.mark.parametrize("B,K,I", [(1, 64, 1), (5, 1152, 17), (32, 1152, 6912), (17, 4096, 100)])
 def test_geglu_behind_the_product(device, B, K, I):
     rng = np.random.default_rng(B + K + I)

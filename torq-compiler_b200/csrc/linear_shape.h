@@ -2,7 +2,7 @@
 // Host code only, so that the layout can be checked without a GPU.
 //
 // Shared memory of a block, in order:
-//   [0, x_bytes)                  staged activations
+//   [0, x_bytes)                  staged activations: rows, behind them room for the sums of a norm in front; or slices, and a shift per token
 //   [x_bytes, + rings)            every warp's weight ring; both are overwritten by the groups' sums once all warps have multiplied
 //   [scale_off, + rt * 32 * 4)    scales of the block's rows
 //   [recv_off, smem)              what other blocks of the cluster store into this one: nothing else uses it, because a peer that
@@ -17,6 +17,12 @@ enum { kStore = 0, kGeglu = 1, kRope = 2, kStream = 3 };
 constexpr int kTileRows = 32, kBlk = 64, kStageBytes = kTileRows * kBlk, kStreamStages = 4;
 constexpr int kRopeTokens = 8;  // most tokens a warp finishes in the RoPE epilogue
 constexpr int kSmemMax = 227 * 1024 - 1024;
+// Up to kSlicedTokens tokens the product over the vocabulary multiplies integers: a bf16 activation is four int8 slices of a 31-bit
+// fixed-point number, a slice a column of the instruction. Its weights then need no conversion. The products of the layers keep bf16: their
+// results are rounded to bf16 and go through every layer behind them, where two sums that differ in the last bit of fp32 end almost a
+// percent apart.
+// Up to kNormTokens the norm in front of a product runs in it.
+constexpr int kSlicedTokens = 8, kSlices = 4, kNormTokens = 2;
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
@@ -30,8 +36,8 @@ inline int linear_groups(int N, int K) {
 }
 
 struct LinearShape {
-  int tk, kg, ck, rt, stages, x_pitch, x_bytes, scale_off, recv_off, smem, tiles, grid;
-  bool ok;
+  int tk, kg, ck, rt, stages, x_pitch, x_bytes, side_off, scale_off, recv_off, smem, tiles, grid;
+  bool ok, sliced;
 };
 
 // bytes other blocks store into one: the RoPE epilogue's sums of squares and partner values, or the sums of a cluster's K slices
@@ -46,13 +52,21 @@ inline LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
   const int tok = ceil_div(B, 8) * 8, blocks = K / kBlk;
   s.tk = linear_groups(N, K);
   if (mode == kStore && s.tk == 1) mode = kStream;
+  s.sliced = mode == kStream && B <= kSlicedTokens;
   s.tiles = mode == kGeglu ? ceil_div(N / 2, 16) : ceil_div(N, kTileRows);
   auto fit = [&](int kg, int ck, int rt, int stages) {
     s.kg = kg; s.ck = ck; s.rt = rt; s.stages = stages;
     int widest = 0;
     for (int r = 0; r < ck; r++) widest = std::max(widest, blocks * (r * kg + kg) / s.tk - blocks * (r * kg) / s.tk);
-    s.x_pitch = (widest * kBlk * 2 + 127) / 128 * 128 + 16;
-    s.x_bytes = (tok * s.x_pitch + 127) / 128 * 128;
+    if (s.sliced) {  // [column][K], two columns to 128 bytes of banks
+      s.x_pitch = (widest * kBlk + 127) / 128 * 128 + 64;
+      s.side_off = ceil_div(B * kSlices, 8) * 8 * s.x_pitch;
+      s.x_bytes = (s.side_off + B * 4 + 127) / 128 * 128;
+    } else {
+      s.x_pitch = (widest * kBlk * 2 + 127) / 128 * 128 + 16;
+      s.side_off = tok * s.x_pitch;
+      s.x_bytes = (s.side_off + (B <= kNormTokens && (mode == kGeglu || mode == kRope) ? kNormTokens * 2 * 16 * 4 : 0) + 127) / 128 * 128;
+    }
     const int warps = kg * rt;
     const int sums = warps * kTileRows * (tok + 1) * 4;
     s.scale_off = std::max(s.x_bytes + warps * stages * kStageBytes, mode == kStream ? 16 * tok * 8 : (sums + 127) / 128 * 128);

@@ -315,6 +315,8 @@ bool force_simt() {
 // Result bytes from which cutting a padded result back beats byte stores from the product: 1000 x 1003 26.2 -> 19.7 us,
 // 4096 x 8190 328 -> 59 us; below, the second launch costs what it saves.
 constexpr long long kTrimBytes = 1 << 18;
+// Most of a later product's weights that an earlier one asks for: a quarter of L2.
+constexpr size_t kPrefetchBytes = 32 << 20;
 static int bytes16_row_group(long long K) {  // rows that together are a multiple of 16 bytes
   int g16 = 16;
   while (K % g16 != 0) g16 >>= 1;  // gcd(K, 16)
@@ -625,6 +627,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   std::vector<int> gemv_before(ops.size(), -1);    // reader op -> the gemv_w8 op that runs in its step
   std::vector<char> gemv_deferred(ops.size(), 0);
   std::vector<int> norm_second(ops.size(), -1);    // rmsnorm op -> the rmsnorm op fused into it
+  std::vector<int> norm_of(ops.size(), -1);        // reader of a deferred product -> the rmsnorm op (pair) that runs in its step, too
+  std::vector<char> norm_deferred(ops.size(), 0);
   std::vector<int> extra_out(ops.size(), -1);      // tensor an op writes on behalf of the op fused into it
   std::vector<int> extra_in(ops.size(), -1);       // tensor an op reads on behalf of the op fused into it
   // Attention written op by op: a rank-2 transpose that only feeds a matmul's second operand (the product reads the
@@ -865,7 +869,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
     for (int i = 0; i + 1 < (int)ops.size() && !(no_dec && *no_dec && *no_dec != '0'); i++) {
       const auto& op = ops[i];
       const auto& nx = ops[i + 1];
-      auto ok2d = [&](int id, int dtype) {
+      auto ok2d = [&](int id, uint32_t dtype) {
         return id >= 0 && id < nt && tensors[id].rank == 2 && tensors[id].dtype == dtype;
       };
       if (op.kind == TB200_OP_GEMV_W8 && ok2d(op.in0, TB200_BF16) && ok2d(op.weights, TB200_I8) && op.i0 <= 0 && op.i1 == 0 && nx.in0 == op.out0) {
@@ -889,6 +893,26 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         fused_away[i + 1] = 1;
         extra_out[i] = nx.out0;
       }
+    }
+    // A norm (or a pair) directly in front of a product that runs in its reader's step (3) runs in that launch too where the product's
+    // kernel can. Only the product reads the normed rows, which then never reach memory.
+    for (int i = 0; i + 2 < (int)ops.size() && !(no_dec && *no_dec && *no_dec != '0'); i++) {
+      const int last = norm_second[i] >= 0 ? norm_second[i] : i, p = last + 1;
+      if (ops[i].kind != TB200_OP_RMSNORM || fused_away[i] || p + 1 >= (int)ops.size() || !gemv_deferred[p] || ops[p].in0 != ops[last].out0) continue;
+      const auto& first = ops[i];
+      const int normed = ops[last].out0;
+      auto rows = [&](int id) { return b.is_t(id, TB200_BF16, 2) && b.same_shape(id, normed); };
+      if (tensors[normed].kind != TB200_TENSOR_ACTIVATION || uses[normed] != 1 || (ops[p + 1].kind != TB200_OP_GEGLU && ops[p + 1].kind != TB200_OP_ROPE_KV) ||
+          !rows(first.in0) || !rows(first.out0) || (first.in1 >= 0 && !rows(first.in1)) ||
+          !linear_norm_applies(tensors[ops[p].in0].shape[0], tensors[ops[p].weights].shape[0], tensors[ops[p].weights].shape[1], ops[p + 1].kind == TB200_OP_GEGLU))
+        continue;
+      // it runs two or three ops behind its place, and the ops in between run in the same launch
+      if (last != i && !b.may_write_early(first.out0)) continue;
+      bool constant = true;
+      for (int id : {first.in0, first.in1}) constant = constant && (id < 0 || tensors[id].kind == TB200_TENSOR_ACTIVATION || tensors[id].kind == TB200_TENSOR_INPUT);
+      if (!constant) continue;
+      norm_of[p + 1] = i;
+      norm_deferred[i] = 1;
     }
   }
   for (int i = 0; i < (int)ops.size(); i++) {
@@ -925,6 +949,10 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       if (tensors[op.out0].kind == TB200_TENSOR_ACTIVATION) root[op.out0] = root[op.in0];
     }
   }
+  for (int i = 0; i < (int)ops.size(); i++)
+    if (norm_of[i] >= 0)
+      for (int id : {ops[norm_of[i]].in0, ops[norm_of[i]].in1, ops[norm_of[i]].out0})
+        if (id >= 0) last_use[root[id]] = std::max(last_use[root[id]], i);
   for (int i = 0; i < (int)ops.size(); i++)
     for (const auto& l : concat_leaves[i]) last_use[root[l.id]] = std::max(last_use[root[l.id]], i);
   auto bytes_of = [&](int id) {
@@ -982,7 +1010,9 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   }
 
   size_t scratch_need = 0;
-  struct LinearStep { Loc x; size_t w_off, s_off; int B, N, K; };
+  struct NormStep { Loc x, res, out; size_t w_off, w2_off; float eps, eps2; bool has_res, pair; };
+  std::map<int, NormStep> norms;  // deferred rmsnorm ops
+  struct LinearStep { Loc x; size_t w_off, s_off; int B, N, K; size_t next_off, next_bytes; };
   std::vector<LinearStep> linear(ops.size(), LinearStep{});  // deferred gemv_w8 ops
   auto linear_args = [](const LinearStep& l, const ExecContext& c) {
     LinearArgs k{};
@@ -990,7 +1020,17 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
     k.W = (const int8_t*)(c.consts + l.w_off);
     k.scale = (const uint16_t*)(c.consts + l.s_off);
     k.B = l.B; k.N = l.N; k.K = l.K;
+    k.next = l.next_bytes ? (const int8_t*)(c.consts + l.next_off) : nullptr;
+    k.next_bytes = (uint32_t)l.next_bytes;
     return k;
+  };
+  auto norm_args = [](LinearArgs& k, const NormStep& n, const ExecContext& c) {
+    k.norm_x = (const uint16_t*)n.x.resolve(c);
+    k.norm_res = n.has_res ? (const uint16_t*)n.res.resolve(c) : nullptr;
+    k.norm_w = (const uint16_t*)(c.consts + n.w_off);
+    k.norm_w2 = n.pair ? (const uint16_t*)(c.consts + n.w2_off) : nullptr;
+    k.norm_out = n.pair ? (uint16_t*)n.out.resolve(c) : nullptr;
+    k.norm_eps = n.eps; k.norm_eps2 = n.eps2;
   };
   auto report = [](cudaError_t e, const ExecContext& c) {
     if (e != cudaSuccess && c.launch_error) *c.launch_error = e;
@@ -1978,6 +2018,13 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             lo2 = loc(ops[second].out0);
             eps2 = ops[second].f0;
           }
+          if (norm_deferred[i]) {
+            norms[i] = NormStep{lx, lr, lo, w_off, w2_off, eps, eps2, has_res, second >= 0};
+            step.kernel_name = "(norm in the launch of the product behind it)";
+            step.launches = 0;
+            step.launch = [](const ExecContext&) {};
+            break;
+          }
           step.kernel_name = second >= 0 ? "rmsnorm_pair" : "rmsnorm";
           step.launch = [=](const ExecContext& c) {
             launch_rmsnorm_row((const uint16_t*)lx.resolve(c), has_res ? (const uint16_t*)lr.resolve(c) : nullptr,
@@ -2011,7 +2058,17 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         if (!b.add_raw_const(op.weights, (size_t)N * K, "weights", i, w_off)) return b.status;
         if (!b.add_raw_const(op.bias, (size_t)N * 2, "scales", i, s_off)) return b.status;
         if (op.i0 <= 0 && op.i1 == 0 && K == tensors[op.in0].shape[1] && linear_w8_applies(B, N, K)) {
-          const LinearStep l{loc(op.in0), w_off, s_off, B, N, K};
+          // the product after the next one: its weights have that long to come from memory
+          size_t next_off = 0, next_bytes = 0;
+          for (int j = i + 1, seen = 0; j < (int)ops.size(); j++) {
+            if (ops[j].kind != TB200_OP_GEMV_W8 || ++seen < 2) continue;
+            if (b.is_t(ops[j].weights, TB200_I8, 2) && tensors[ops[j].weights].kind == TB200_TENSOR_CONSTANT) {
+              next_bytes = std::min<size_t>(tensors[ops[j].weights].const_bytes, kPrefetchBytes);
+              if (!b.add_raw_const(ops[j].weights, next_bytes, "weights", j, next_off)) return b.status;
+            }
+            break;
+          }
+          const LinearStep l{loc(op.in0), w_off, s_off, B, N, K, next_off, next_bytes};
           if (gemv_deferred[i]) {
             linear[i] = l;
             step.kernel_name = "(product in the launch of the op behind it)";
@@ -2062,9 +2119,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         const float theta = op.f0, eps = op.f1;
         if (gemv_before[i] >= 0) {
           const LinearStep l = linear[gemv_before[i]];
-          step.kernel_name = "linear_w8_rope_kv";
+          const bool has_norm = norm_of[i] >= 0;
+          const NormStep norm = has_norm ? norms[norm_of[i]] : NormStep{};
+          step.kernel_name = has_norm ? "norm_linear_w8_rope_kv" : "linear_w8_rope_kv";
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
+            if (has_norm) norm_args(k, norm, c);
             k.pos = (const int32_t*)lp.resolve(c);
             k.qw = (const uint16_t*)(c.consts + qw_off);
             k.kw = (const uint16_t*)(c.consts + kw_off);
@@ -2116,9 +2176,12 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         Loc lx = loc(op.in0), lo = loc(op.out0);
         if (gemv_before[i] >= 0) {
           const LinearStep l = linear[gemv_before[i]];
-          step.kernel_name = "linear_w8_geglu";
+          const bool has_norm = norm_of[i] >= 0;
+          const NormStep norm = has_norm ? norms[norm_of[i]] : NormStep{};
+          step.kernel_name = has_norm ? "norm_linear_w8_geglu" : "linear_w8_geglu";
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
+            if (has_norm) norm_args(k, norm, c);
             k.y = lo.resolve(c);
             report(launch_linear_geglu(k, c.stream), c);
           };
