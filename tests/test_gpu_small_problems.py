@@ -6,6 +6,7 @@ import pytest
 
 from torq_b200.oplist import Graph
 from torq_b200.quant import quantize_multipliers
+from torq_b200.runtime import Executable
 from oracle_exec import run_graph
 from gpu_exec import run_graph_gpu
 
@@ -114,3 +115,26 @@ def test_few_dozen_rows(device, M, K, N, table, monkeypatch):
                           input_zp=-7, out_zp=3)
     g.output(g.table(y, rng.permutation(np.arange(-128, 128)).astype(np.int8)) if table else y)
     _both(device, g, [rng.integers(-128, 128, (M, K), dtype=np.int8)], monkeypatch)
+
+
+@pytest.mark.parametrize("shape,OC,stride,pad", [((1, 211, 90, 3), 16, 2, (0, 1, 0, 1)), ((3, 70, 75, 3), 32, 1, (1, 1, 1, 1)), ((2, 65, 43, 3), 48, 2, (1, 1, 1, 1)),
+                                                 ((37, 5, 7, 3), 64, 1, (2, 0, 2, 0)), ((40, 31, 17, 3), 16, 1, (1, 1, 1, 1)),
+                                                 ((3, 67, 132, 3), 16, 2, (0, 1, 0, 1)), ((2, 30, 140, 3), 32, 2, (1, 1, 1, 1)), ((5, 9, 64, 3), 96, 2, (1, 0, 2, 3)),
+                                                 ((2, 90, 4, 3), 16, 2, (1, 1, 1, 1))])
+@pytest.mark.parametrize("table", [False, True])
+@pytest.mark.parametrize("double_round,clamp", [(True, (-128, 127)), (False, (3, 100))])
+def test_stem_of_large_frames(device, shape, OC, stride, pad, table, double_round, clamp, monkeypatch):
+    """The stem kernel of the frames the small-problem kernels leave: pixel counts that end inside a warp, rows shorter than a warp, windows
+    over every edge, one and several passes over the channels."""
+    monkeypatch.setenv("TB200_NO_SMALL", "1")
+    rng = np.random.default_rng(OC + shape[1])
+    g = Graph()
+    m, s = quantize_multipliers(rng.uniform(0.002, 0.004, OC))
+    y = g.conv2d(g.input(shape), rng.integers(-127, 128, (OC, 3, 3, 3), dtype=np.int8), rng.integers(-3000, 3000, OC).astype(np.int32), m, s,
+                 stride=(stride, stride), pad=pad, input_zp=-7, out_zp=3, double_round=double_round, clamp=clamp)
+    g.output(g.table(y, rng.integers(-128, 128, 256).astype(np.int8)) if table else y)
+    ex = Executable(device, g.serialize())
+    assert ex.op_kernels()[0] == "conv2d_stem333_mma", ex.op_kernels()
+    ex.destroy()
+    x = rng.integers(-128, 128, shape, dtype=np.int8)
+    assert (run_graph_gpu(device, g, [x])[0] == run_graph(g, [x])[0]).all()

@@ -8,8 +8,11 @@
 //   sum (x-izp)(w-wzp) = sum x*w - izp*sum(w) - wzp*sum(x) + K*izp*wzp
 // with sums over ALL K taps; the izp terms are constants per output channel and
 // arrive folded into ChanParams::bias. int32 wrap-around keeps this exact.
+#include <algorithm>
+
 #include "kernels.h"
 #include "dependent_launch.cuh"
+#include "device_memory.cuh"
 
 namespace tb200 {
 
@@ -339,114 +342,285 @@ __global__ void __launch_bounds__(128) conv2d_c16_kernel(ConvArgs a) {
   }
 }
 
-// The 3x3 window over 3 channels (the stem of an image network) with the compact 32-bit epilogue records. A thread
-// owns kStemPix output pixels (adjacent threads adjacent pixels). A kernel row of a pixel is 9 consecutive bytes of
-// the input: three aligned words and two funnel shifts bring them in (pixels whose window leaves the image, or whose
-// words would reach past the tensor, gather byte by byte with the input zero point outside). The 27 bytes are packed
-// into 7 dp4a operands once and run against every output channel's 7 weight words (two 16-byte shared-memory loads
-// per channel, shared by the thread's pixels): 7 dp4a + about 7 instructions of rescale per output.
-constexpr int kStemPix = 4;
-template <int EPI, bool LUT>
-__global__ void __launch_bounds__(128) conv2d_stem333_kernel(ConvArgs a) {
+// The 3x3 window over 3 channels (the stem of an image network) with the compact 32-bit epilogue records, on warp-level matrix
+// instructions. A thread gathers a pixel: a kernel row is 9 consecutive bytes of the input, three aligned words and two funnel shifts
+// (pixels whose window leaves the image, or whose words would reach past the tensor, gather byte by byte with the input zero
+// point outside). The 27 bytes, packed into 8 words, are a row of 32 of the product's left operand: the warp leaves its 32 rows in
+// shared memory and reads them back as fragments (ldmatrix), a k32 instruction then gives 16 pixels x 8 channels. Fragment column f
+// of instruction j is channel (W / 4) (f / 2) + 2 j + f % 2 of a group of W, so that a lane ends with W / 4 consecutive channels of a pixel.
+// What bounds it: integer issue, a third of it the gathering, half the rescale. Before, with 7 dp4a per output and 64-bit divisions per
+// pixel: 25 instructions per output, 256 x 224 x 224 -> 32 channels 133 us, 64 x 640 x 640 -> 16 channels with a table 183 us; here 82 and 134.
+constexpr int kStemPix = 8;  // most pixels a thread gathers, one after the other
+// W: channels per pass over the fragments (16 or 32). I: index type, 32 bits where every offset fits.
+template <int EPI, bool LUT, int W, typename I>
+__global__ void __launch_bounds__(128) conv2d_stem333_kernel(ConvArgs a, int pixels) {
+  constexpr int NJ = W / 8, CH = W / 4;  // instructions per 16 pixels, channels a lane ends with
+  __shared__ __align__(16) uint4 rows_s[4][64];  // [warp][32 pixels x 2 halves]
+  __shared__ uint8_t lut_s[LUT ? 256 : 4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  if (LUT)
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) lut_s[LUT ? i : 0] = (uint8_t)a.lut[(int)(int8_t)i + 128];  // by the raw byte
+  // weights and records of the first W channels (all of them in most stems)
+  uint2 b[NJ];
+  int4 q[CH];
+  auto constants = [&](int oc0) {
+#pragma unroll
+    for (int j = 0; j < NJ; j++) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(a.w + (size_t)(oc0 + CH * (g >> 1) + 2 * j + (g & 1)) * a.Kpad) + t;
+      b[j] = make_uint2(__ldg(w), __ldg(w + 4));
+    }
+#pragma unroll
+    for (int c = 0; c < CH; c++) q[c] = __ldg(a.q4 + oc0 + CH * t + c);
+  };
+  constants(0);
   grid_dependency_wait();
   grid_dependency_release();
-  extern __shared__ __align__(16) uint32_t stem_s[];  // [OC][8] weight words (word 7 zero), [OC] Q4 records, 256-byte table
-  uint4* w_s = reinterpret_cast<uint4*>(stem_s);
-  int4* q_s = reinterpret_cast<int4*>(stem_s + (size_t)a.OC * 8);
-  const int8_t* lut_s = reinterpret_cast<const int8_t*>(stem_s + (size_t)a.OC * 12);
-  if (LUT)
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) reinterpret_cast<int8_t*>(stem_s + (size_t)a.OC * 12)[i] = a.lut[i];
-  for (int i = threadIdx.x; i < a.OC * 8; i += blockDim.x) {
-    const int oc = i >> 3, kw = i & 7;
-    stem_s[i] = kw < 7 ? *reinterpret_cast<const uint32_t*>(a.w + (size_t)oc * a.Kpad + kw * 4) : 0u;
+  if (LUT) __syncthreads();
+  const I P = (I)a.N * a.OH * a.OW;
+  I p0 = ((I)blockIdx.x * 4 + warp) * (32 * pixels);  // the warp's pixels
+  if (p0 >= P) return;
+  // this lane's pixel
+  int ow, oh, n;
+  {
+    const I p = p0 + lane < P ? p0 + lane : 0, r = p / (I)a.OW;
+    ow = (int)(p - r * (I)a.OW);
+    n = (int)(r / (I)a.OH);
+    oh = (int)(r - (I)n * a.OH);
   }
-  for (int i = threadIdx.x; i < a.OC; i += blockDim.x) q_s[i] = a.q4[i];
-  __syncthreads();
-  const long long P = (long long)a.N * a.OH * a.OW;
-  const long long p_base = (long long)blockIdx.x * (128 * kStemPix) + threadIdx.x;
   const uint32_t zp_byte = (uint32_t)(a.input_zp & 0xff);
-  uint32_t patch[kStemPix][7];
+  const uint32_t lo2 = (uint32_t)(a.clamp_min & 0xffff) * 0x10001u, hi2 = (uint32_t)(a.clamp_max & 0xffff) * 0x10001u;
+  const I row_bytes = (I)a.W * 3;
+  uint4* mine = rows_s[warp];
+  const uint32_t base = smem_u32(mine);
+  const int swap = lane >> 2 & 1;  // half h of row r lies at 2 r + (h ^ (r >> 2 & 1)): eight rows' halves in different banks
+  const uint32_t frag = base + (uint32_t)(2 * (lane & 15) + ((lane >> 4) ^ swap)) * 16;
+  // the three words of each kernel row of the lane's pixel, asked for a pixel ahead
+  uint32_t word[3][3], sh[3];
+  bool inside;
+  int ih0, iw0;
+  auto ask = [&]() {
+    ih0 = oh * a.stride_h - a.pad_t;
+    iw0 = ow * a.stride_w - a.pad_l;
+    const I off0 = (((I)n * a.H + ih0) * a.W + iw0) * 3;
+    inside = ih0 >= 0 && ih0 + 2 < a.H && iw0 >= 0 && iw0 + 2 < a.W && ((off0 + 2 * row_bytes) & ~(I)3) + 12 <= (I)a.x_bytes;
+    if (!inside) return;
 #pragma unroll
-  for (int px = 0; px < kStemPix; px++) {
-    const long long p = p_base + px * 128;
-    const long long pp = p < P ? p : 0;
-    const int ow = (int)(pp % a.OW);
-    const long long t = pp / a.OW;
-    const int oh = (int)(t % a.OH);
-    const int n = (int)(t / a.OH);
-    const int ih0 = oh * a.stride_h - a.pad_t, iw0 = ow * a.stride_w - a.pad_l;
+    for (int kh = 0; kh < 3; kh++) {
+      const I off = off0 + kh * row_bytes;
+      const uint32_t* wp = reinterpret_cast<const uint32_t*>(a.x + (off & ~(I)3));
+#pragma unroll
+      for (int k = 0; k < 3; k++) word[kh][k] = __ldg(wp + k);
+      sh[kh] = (uint32_t)(off & 3) * 8;
+    }
+  };
+  ask();
+  for (int px = 0; px < pixels && p0 < P; px++, p0 += 32) {
     uint32_t row[3][3];  // per kernel row: bytes 0-3, 4-7, 8 (upper bytes of the third word are not used)
-    const long long off0 = (((long long)n * a.H + ih0) * a.W + iw0) * 3;
-    const bool inside = ih0 >= 0 && ih0 + 2 < a.H && iw0 >= 0 && iw0 + 2 < a.W &&
-                        ((off0 + 2ll * a.W * 3) & ~3ll) + 12 <= a.x_bytes;
     if (inside) {
 #pragma unroll
       for (int kh = 0; kh < 3; kh++) {
-        const long long off = off0 + (long long)kh * a.W * 3;
-        const uint32_t* wp = reinterpret_cast<const uint32_t*>(a.x + (off & ~3ll));
-        const uint32_t w0 = __ldg(wp), w1 = __ldg(wp + 1), w2 = __ldg(wp + 2);
-        const uint32_t sh = (uint32_t)(off & 3) * 8;
-        row[kh][0] = __funnelshift_r(w0, w1, sh);
-        row[kh][1] = __funnelshift_r(w1, w2, sh);
-        row[kh][2] = w2 >> sh;
+        row[kh][0] = __funnelshift_r(word[kh][0], word[kh][1], sh[kh]);
+        row[kh][1] = __funnelshift_r(word[kh][1], word[kh][2], sh[kh]);
+        row[kh][2] = word[kh][2] >> sh[kh];
       }
     } else {
       const int8_t* xin = a.x + (size_t)n * a.H * a.W * 3;
 #pragma unroll
       for (int kh = 0; kh < 3; kh++) {
         const int ih = ih0 + kh;
-        uint32_t b[12];
+        uint32_t c[9];
 #pragma unroll
         for (int j = 0; j < 9; j++) {
           const int iw = iw0 + j / 3;
-          b[j] = (ih >= 0 && ih < a.H && iw >= 0 && iw < a.W) ? (uint32_t)(uint8_t)xin[((size_t)ih * a.W + iw) * 3 + j % 3] : zp_byte;
+          c[j] = (ih >= 0 && ih < a.H && iw >= 0 && iw < a.W) ? (uint32_t)(uint8_t)xin[((size_t)ih * a.W + iw) * 3 + j % 3] : zp_byte;
         }
-        row[kh][0] = b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24);
-        row[kh][1] = b[4] | (b[5] << 8) | (b[6] << 16) | (b[7] << 24);
-        row[kh][2] = b[8];
+        row[kh][0] = c[0] | (c[1] << 8) | (c[2] << 16) | (c[3] << 24);
+        row[kh][1] = c[4] | (c[5] << 8) | (c[6] << 16) | (c[7] << 24);
+        row[kh][2] = c[8];
       }
     }
-    // K order (kh, kw, ic): bytes 0-8 row 0, 9-17 row 1, 18-26 row 2, byte 27 meets a zero weight
-    patch[px][0] = row[0][0];
-    patch[px][1] = row[0][1];
-    patch[px][2] = (row[0][2] & 0xffu) | (row[1][0] << 8);
-    patch[px][3] = __funnelshift_r(row[1][0], row[1][1], 24);
-    patch[px][4] = (row[1][1] >> 24) | ((row[1][2] & 0xffu) << 8) | (row[2][0] << 16);
-    patch[px][5] = __funnelshift_r(row[2][0], row[2][1], 16);
-    patch[px][6] = (row[2][1] >> 16) | ((row[2][2] & 0xffu) << 16);
+    // K order (kh, kw, ic): bytes 0-8 row 0, 9-17 row 1, 18-26 row 2, bytes 27-31 meet zero weights
+    mine[2 * lane + swap] = make_uint4(row[0][0], row[0][1], __byte_perm(row[0][2], row[1][0], 0x6540), __funnelshift_r(row[1][0], row[1][1], 24));
+    mine[2 * lane + (swap ^ 1)] = make_uint4(__byte_perm(row[1][1], __byte_perm(row[1][2], row[2][0], 0x5400), 0x7653), __funnelshift_r(row[2][0], row[2][1], 16),
+                                             __byte_perm(row[2][1], row[2][2], 0x0432), 0u);
+    // the next pixel of this lane; behind the last one: read, never stored
+    for (ow += 32; ow >= a.OW;) {
+      ow -= a.OW;
+      if (++oh == a.OH) {
+        oh = 0;
+        n++;
+      }
+    }
+    if (p0 + 32 + lane >= P) ow = oh = n = 0;
+    ask();
+    __syncwarp();
+    uint32_t f[2][4];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(f[m][0]), "=r"(f[m][1]), "=r"(f[m][2]), "=r"(f[m][3]) : "r"(frag + m * 512) : "memory");
+    __syncwarp();  // read before the next pixels are written
+    const bool all = p0 + 32 <= P;
+    int8_t* out = a.out + (size_t)(p0 + g) * a.OC + CH * t;
+    for (int oc0 = 0; oc0 < a.OC; oc0 += W, out += W) {
+      if (a.OC > W) constants(oc0);
+      int8_t* o = out;
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        int acc[NJ][4];
+#pragma unroll
+        for (int j = 0; j < NJ; j++)
+          asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                       : "=r"(acc[j][0]), "=r"(acc[j][1]), "=r"(acc[j][2]), "=r"(acc[j][3])
+                       : "r"(f[m][0]), "r"(f[m][1]), "r"(f[m][2]), "r"(f[m][3]), "r"(b[j].x), "r"(b[j].y), "r"(0));
+#pragma unroll
+        for (int h = 0; h < 2; h++, o += 8 * a.OC) {
+          uint32_t res[CH / 4];
+#pragma unroll
+          for (int k = 0; k < CH / 4; k++) {
+            int r[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              const int v = acc[2 * k + (c >> 1)][2 * h + (c & 1)];
+              r[c] = EPI == 1 ? scale_q4_sign(v, q[4 * k + c]) : scale_q4(v, q[4 * k + c]);
+            }
+            res[k] = clamp_pack4(r[0], r[1], r[2], r[3], lo2, hi2);
+            if (LUT) res[k] = lut_word(lut_s, res[k]);
+          }
+          if (all || p0 + 16 * m + 8 * h + g < P) {
+            if (CH == 8) *reinterpret_cast<uint2*>(o) = make_uint2(res[0], res[CH / 4 - 1]);
+            else *reinterpret_cast<uint32_t*>(o) = res[0];
+          }
+        }
+      }
+    }
   }
-  for (int oc0 = 0; oc0 < a.OC; oc0 += 16) {
-    uint32_t packed[kStemPix][4];
+}
+
+// The same at stride 2 on rows of whole words (a width that is a multiple of 4): no pixel is gathered. A warp takes 32 pixels of a result
+// row: three kernel rows of 50 words, loaded as they lie (every word is inside the frame or outside), left in shared memory and read
+// back as fragments. Windows of pixels two apart start 12 bytes apart, so the even pixels are one 16-row operand and the odd ones another, each
+// with the weights at its own byte shift: nine words of K, a k32 and a k16 instruction. The words of the next 32 pixels are on their way
+// while these are multiplied and rescaled. STEM2
+template <int EPI, bool LUT, int W>
+__global__ void __launch_bounds__(128, 4) conv2d_stem333_s2_kernel(ConvArgs a, int tiles, int tiles_x, int per_warp) {
+  constexpr int NJ = W / 8, CH = W / 4;  // as above
+  constexpr int kWords = 50, kPitch = 56;
+  __shared__ uint32_t rows_s[4][3 * kPitch];
+  __shared__ uint32_t w_s[2 * NJ * 3 * 32];  // [even / odd][instruction][word t, word t + 4, word 8][lane]
+  __shared__ uint8_t lut_s[LUT ? 256 : 4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int oc0 = blockIdx.y * W;
+  const int sb = -3 * a.pad_l;  // first byte of the window of pixel 0; 32 pixels on is 192 bytes on
+  if (LUT)
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) lut_s[LUT ? i : 0] = (uint8_t)a.lut[(int)(int8_t)i + 128];
+  for (int i = threadIdx.x; i < 2 * NJ * 3 * 32; i += blockDim.x) {
+    const int l = i & 31, k = (i >> 5) % 3, j = (i >> 5) / 3 % NJ, odd = (i >> 5) / (3 * NJ);
+    const int word = k == 2 ? 8 : (l & 3) + 4 * k, kh = word / 3, first = 4 * (word % 3) - ((sb + 6 * odd) & 3);
+    const int8_t* w = a.w + (size_t)(oc0 + CH * (l >> 3) + 2 * j + (l >> 2 & 1)) * a.Kpad + 9 * kh;
+    uint32_t v = 0;
+    for (int e = 0; e < 4; e++)
+      if (first + e >= 0 && first + e < 9 && (k < 2 || (l & 3) == 0)) v |= (uint32_t)(uint8_t)w[first + e] << (8 * e);
+    w_s[i] = v;
+  }
+  int4 q[CH];
 #pragma unroll
-    for (int g = 0; g < 4; g++) {
-      int q[kStemPix][4];
+  for (int c = 0; c < CH; c++) q[c] = __ldg(a.q4 + oc0 + CH * t + c);
+  __syncthreads();
+  uint32_t b[2][NJ][3];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int oc = min(oc0 + 4 * g + j, a.OC - 1);
-        const uint4 wa = w_s[oc * 2], wb = w_s[oc * 2 + 1];
-        const int4 c = q_s[oc];
+  for (int o = 0; o < 2; o++)
 #pragma unroll
-        for (int px = 0; px < kStemPix; px++) {
-          int acc = __dp4a((int)patch[px][0], (int)wa.x, 0);
-          acc = __dp4a((int)patch[px][1], (int)wa.y, acc);
-          acc = __dp4a((int)patch[px][2], (int)wa.z, acc);
-          acc = __dp4a((int)patch[px][3], (int)wa.w, acc);
-          acc = __dp4a((int)patch[px][4], (int)wb.x, acc);
-          acc = __dp4a((int)patch[px][5], (int)wb.y, acc);
-          acc = __dp4a((int)patch[px][6], (int)wb.z, acc);
-          const int r = EPI == 1 ? scale_q4_sign(acc, c) : scale_q4(acc, c);
-          q[px][j] = max(a.clamp_min, min(a.clamp_max, r));
-          if (LUT) q[px][j] = lut_s[q[px][j] + 128];  // a fused 256-entry table
-        }
+    for (int j = 0; j < NJ; j++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) b[o][j][k] = w_s[((o * NJ + j) * 3 + k) * 32 + lane];
+  grid_dependency_wait();
+  grid_dependency_release();
+  int tile = (blockIdx.x * 4 + warp) * per_warp;
+  const int last = min(tiles, tile + per_warp);
+  if (tile >= last) return;
+  int r = tile / tiles_x, tx = tile - r * tiles_x;  // r: result row over all images
+  int n = r / a.OH, oh = r - n * a.OH;
+  const uint32_t zp_word = (uint32_t)(a.input_zp & 0xff) * 0x01010101u;
+  const uint32_t lo2 = (uint32_t)(a.clamp_min & 0xffff) * 0x10001u, hi2 = (uint32_t)(a.clamp_max & 0xffff) * 0x10001u;
+  const int row_bytes = a.W * 3;
+  uint32_t word[3][2];
+  auto ask = [&]() {
+    const int ih0 = oh * 2 - a.pad_t, col = (sb & ~3) + tx * 192 + 4 * lane;
+#pragma unroll
+    for (int kh = 0; kh < 3; kh++) {
+      const bool row_ok = (unsigned)(ih0 + kh) < (unsigned)a.H;
+      const int8_t* row = a.x + ((n * a.H + ih0 + kh) * row_bytes + col);
+      word[kh][0] = word[kh][1] = zp_word;
+      if (row_ok && (unsigned)col < (unsigned)row_bytes) word[kh][0] = __ldg(reinterpret_cast<const uint32_t*>(row));
+      if (row_ok && lane < kWords - 32 && (unsigned)(col + 128) < (unsigned)row_bytes) word[kh][1] = __ldg(reinterpret_cast<const uint32_t*>(row + 128));
+    }
+  };
+  ask();
+  uint32_t* mine = rows_s[warp];
+  // where this lane's words of the even pixel 2 g lie: word t, word t + 4, word 8 of its window
+  auto at = [&](int w) { return mine + 3 * g + w / 3 * kPitch + w % 3; };
+  const uint32_t* const f0 = at(t);
+  const uint32_t* const f1 = at(t + 4);
+  const uint32_t* const f2 = at(8);
+  const int odd_words = ((sb & 3) + 6) >> 2;
+  for (; tile < last; tile++) {
+#pragma unroll
+    for (int kh = 0; kh < 3; kh++) {
+      mine[kh * kPitch + lane] = word[kh][0];
+      if (lane < kWords - 32) mine[kh * kPitch + 32 + lane] = word[kh][1];
+    }
+    int8_t* out = a.out + ((size_t)(r * a.OW + tx * 32 + 2 * g) * a.OC + oc0 + CH * t);
+    const int left = a.OW - tx * 32 - 2 * g;  // pixels from this lane's first on
+    if (++tx == tiles_x) {
+      tx = 0;
+      r++;
+      if (++oh == a.OH) {
+        oh = 0;
+        n++;
+      }
+    }
+    if (tile + 1 < last) ask();
+    __syncwarp();
+    uint32_t f[2][6];
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+      const int d = o ? odd_words : 0;
+      f[o][0] = f0[d]; f[o][1] = f0[d + 24]; f[o][2] = f1[d]; f[o][3] = f1[d + 24]; f[o][4] = f2[d]; f[o][5] = f2[d + 24];
+    }
+    __syncwarp();  // read before the next rows are written
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+      int acc[NJ][4];
+#pragma unroll
+      for (int j = 0; j < NJ; j++) {
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                     : "=r"(acc[j][0]), "=r"(acc[j][1]), "=r"(acc[j][2]), "=r"(acc[j][3])
+                     : "r"(f[o][0]), "r"(f[o][1]), "r"(f[o][2]), "r"(f[o][3]), "r"(b[o][j][0]), "r"(b[o][j][1]), "r"(0));
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                     : "+r"(acc[j][0]), "+r"(acc[j][1]), "+r"(acc[j][2]), "+r"(acc[j][3])
+                     : "r"(f[o][4]), "r"(f[o][5]), "r"(b[o][j][2]));
       }
 #pragma unroll
-      for (int px = 0; px < kStemPix; px++) packed[px][g] = pack4(q[px][0], q[px][1], q[px][2], q[px][3]);
-    }
+      for (int h = 0; h < 2; h++) {  // pixels 2 (g + 8 h) + o
+        uint32_t res[CH / 4];
 #pragma unroll
-    for (int px = 0; px < kStemPix; px++) {
-      const long long p = p_base + px * 128;
-      if (p >= P) continue;
-      *reinterpret_cast<uint4*>(a.out + (size_t)p * a.OC + oc0) = make_uint4(packed[px][0], packed[px][1], packed[px][2], packed[px][3]);
+        for (int k = 0; k < CH / 4; k++) {
+          int v[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            const int sum = acc[2 * k + (c >> 1)][2 * h + (c & 1)];
+            v[c] = EPI == 1 ? scale_q4_sign(sum, q[4 * k + c]) : scale_q4(sum, q[4 * k + c]);
+          }
+          res[k] = clamp_pack4(v[0], v[1], v[2], v[3], lo2, hi2);
+          if (LUT) res[k] = lut_word(lut_s, res[k]);
+        }
+        if (16 * h + o < left) {
+          int8_t* p = out + (16 * h + o) * a.OC;
+          if (CH == 8) *reinterpret_cast<uint2*>(p) = make_uint2(res[0], res[CH / 4 - 1]);
+          else *reinterpret_cast<uint32_t*>(p) = res[0];
+        }
+      }
     }
   }
 }
@@ -557,7 +731,7 @@ static bool conv_stem333_applies(const ConvArgs& a) {
 
 const char* conv2d_simt_kernel_name(const ConvArgs& a) {
   if (conv_c16_applies(a)) return "conv2d_c16_dp4a";
-  if (conv_stem333_shape(a)) return "conv2d_stem333_dp4a";
+  if (conv_stem333_shape(a)) return "conv2d_stem333_mma";
   return (a.IC <= 4 && a.K <= 64 && a.OC <= 256 && a.weight_zp == 0) ? "conv2d_smallic_dp4a" : "conv2d_simt";
 }
 
@@ -582,15 +756,36 @@ void launch_conv2d_simt(const ConvArgs& a, cudaStream_t stream) {
     return;
   }
   if (conv_stem333_applies(a)) {
-    const unsigned blocks = (unsigned)((P + 128 * kStemPix - 1) / (128 * kStemPix));
-    const size_t smem = (size_t)a.OC * (32 + 16) + 256;
-    if (a.lut) {
-      if (a.epi == 1) launch_dependent(conv2d_stem333_kernel<1, true>, dim3(blocks), dim3(128), smem, stream, a);
-      else launch_dependent(conv2d_stem333_kernel<2, true>, dim3(blocks), dim3(128), smem, stream, a);
+    // a frame or two: as many blocks as there is work for
+    const int pixels = (int)std::max(1ll, std::min((long long)kStemPix, P / (128ll * 148 * 6)));
+    const unsigned blocks = (unsigned)((P + 128 * pixels - 1) / (128 * pixels));
+    // 32-bit offsets where the last pixel of the last block still has one
+    const bool small = P + 128 * kStemPix < (1ll << 31) && a.x_bytes < (1ll << 31) - 64;
+    const bool words = a.stride_h == 2 && a.stride_w == 2 && (a.W & 3) == 0;
+    const int tiles_x = (a.OW + 31) / 32, tiles = small && words ? a.N * a.OH * tiles_x : 0;
+    const int per_warp = std::max(1, (tiles + 148 * 4 * 4 - 1) / (148 * 4 * 4));  // one wave of blocks, their weights laid out once
+    const dim3 tile_grid((unsigned)((tiles + 4 * per_warp - 1) / (4 * per_warp)));
+#define TB200_STEM(EPI, LUT, W)                                                                                                       \
+  do {                                                                                                                                \
+    if (small && words)                                                                                                               \
+      launch_dependent(conv2d_stem333_s2_kernel<EPI, LUT, W>, dim3(tile_grid.x, (unsigned)(a.OC / W)), dim3(128), 0, stream, a, tiles, tiles_x, per_warp); \
+    else if (small) launch_dependent(conv2d_stem333_kernel<EPI, LUT, W, int>, dim3(blocks), dim3(128), 0, stream, a, pixels);         \
+    else launch_dependent(conv2d_stem333_kernel<EPI, LUT, W, long long>, dim3(blocks), dim3(128), 0, stream, a, pixels);              \
+  } while (0)
+#define TB200_STEM_EPI(LUT, W)               \
+  do {                                       \
+    if (a.epi == 1) TB200_STEM(1, LUT, W);   \
+    else TB200_STEM(2, LUT, W);              \
+  } while (0)
+    if (a.OC % 32 == 0) {
+      if (a.lut) TB200_STEM_EPI(true, 32);
+      else TB200_STEM_EPI(false, 32);
     } else {
-      if (a.epi == 1) launch_dependent(conv2d_stem333_kernel<1, false>, dim3(blocks), dim3(128), smem, stream, a);
-      else launch_dependent(conv2d_stem333_kernel<2, false>, dim3(blocks), dim3(128), smem, stream, a);
+      if (a.lut) TB200_STEM_EPI(true, 16);
+      else TB200_STEM_EPI(false, 16);
     }
+#undef TB200_STEM_EPI
+#undef TB200_STEM
     return;
   }
   if (a.IC <= 4 && a.K <= 64 && a.OC <= 256 && a.weight_zp == 0) {
