@@ -14,7 +14,8 @@ IDENT = ((1 << 30), 30)
 
 
 @pytest.mark.parametrize("shape,channels,rescaled", [((1, 1, 1), (16, 16), ()), ((2, 9, 7), (16, 48, 32), (1,)), ((1, 20, 21), (128, 16, 16, 64), (0, 3)),
-                                                     ((3, 64, 64), (32, 32), (0, 1)), ((1, 5, 3), (16,) * 8, (2, 7)), ((1, 6, 5), (16, 24), (1,))])
+                                                     ((3, 64, 64), (32, 32), (0, 1)), ((1, 5, 3), (16,) * 8, (2, 7)), ((1, 6, 5), (16, 24), (1,)),
+                                                     ((40, 64, 64), (16, 48, 16), (1, 2)), ((37, 65, 67), (32, 64), ()), ((41, 64, 64), (96, 32, 32), (0, 2))])
 def test_concat_of_intermediates(device, shape, channels, rescaled):
     rng = np.random.default_rng(sum(channels))
     g = Graph()

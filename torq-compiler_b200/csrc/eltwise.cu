@@ -2,6 +2,8 @@
 // standalone rescale (also the building block of a rescaled concat), 2x nearest
 // resize. 128-bit accesses wherever the channel count allows; grids sized in
 // whole multiples of the SM count with grid-stride loops.
+#include <algorithm>
+
 #include "dependent_launch.cuh"
 #include "device_memory.cuh"
 #include "kernels.h"
@@ -124,12 +126,22 @@ __global__ void __launch_bounds__(kThreads) table_kernel(const int8_t* __restric
 
 // ---- concatenation along the channels (ConcatOpPattern: every operand rescaled to the result's scale) ----
 // All operands of a chain in one launch that writes whole rows. Bound by memory: a copy per operand wrote pieces of 16 .. 256
-// bytes of every row and paid a launch for each - the 38 copies of YOLOv8n took 388 us at 64 frames, 13 launches of this
-// kernel take 257 us (128 us of HBM time). A thread
+// bytes of every row and paid a launch for each - the 38 copies of YOLOv8n took 388 us at 64 frames, 13 launches 221 us of this kernel
+// alone and 135 us with the wide one below (128 us of HBM time). A thread
 // has kConcatFlight units in flight; a unit's row comes from one 32-bit division.
 constexpr int kConcatFlight = 4;
-template <bool LUT>
+enum { kAsIs = 0, kTables = 1, kLinear = 2 };
+// A rescale as one multiply-add with 16 fraction bits per byte, where the planner found one that gives the table exactly.
+__device__ __forceinline__ uint4 rescale_linear(const uint4& v, int m, int k) {
+  auto word = [&](uint32_t w) {
+    const int q0 = (int)(int8_t)w * m + k, q1 = (int)(int8_t)(w >> 8) * m + k, q2 = (int)(int8_t)(w >> 16) * m + k, q3 = ((int)w >> 24) * m + k;
+    return sat_pack4(q0 >> 16, q1 >> 16, q2 >> 16, q3 >> 16);
+  };
+  return make_uint4(word(v.x), word(v.y), word(v.z), word(v.w));
+}
+template <int MODE>
 __global__ void __launch_bounds__(kThreads) concat_kernel(const __grid_constant__ ConcatArgs a) {
+  constexpr bool LUT = MODE == kTables;
   __shared__ uint8_t lut[LUT ? kConcatMax : 1][256];
   if (LUT) {
     for (int o = 0; o < a.n; o++)
@@ -173,8 +185,36 @@ __global__ void __launch_bounds__(kThreads) concat_kernel(const __grid_constant_
         const uint8_t* t = lut[LUT ? op[u] : 0];
         v[u] = make_uint4(lut_word(t, v[u].x), lut_word(t, v[u].y), lut_word(t, v[u].z), lut_word(t, v[u].w));
       }
+      if (MODE == kLinear && a.lin_m[op[u]] != 0) v[u] = rescale_linear(v[u], a.lin_m[op[u]], a.lin_k[op[u]]);
       reinterpret_cast<uint4*>(a.out)[i] = v[u];
     }
+  }
+}
+
+// Large concatenations of operands in whole 32-byte sectors: blockIdx.y is the operand, whose units a block reads as they lie (no choice of
+// the operand per unit); a unit's row comes from one multiplication. Operands of 16 channels stay above: halves of sectors from
+// different blocks cost more than the choice (160 x 160 x three of 16: 55 us here, 43 above). The nine concatenations of the detector at 64 frames
+// that copy 121 -> 67 us, three of those that rescale 56 -> 25 us.
+template <bool LIN>
+__global__ void __launch_bounds__(kThreads) concat_wide_kernel(const __grid_constant__ ConcatArgs a) {
+  grid_dependency_wait();
+  grid_dependency_release();
+  const int o = blockIdx.y, units = a.units[o], m = LIN ? a.lin_m[o] : 0, k = LIN ? a.lin_k[o] : 0;
+  const uint32_t total = (uint32_t)a.rows * (uint32_t)units, per_row = a.per_row[o];
+  const uint4* x = reinterpret_cast<const uint4*>(a.x[o]);
+  uint4* out = reinterpret_cast<uint4*>(a.out) + a.first[o];
+  const uint32_t i0 = blockIdx.x * (kThreads * kConcatFlight) + threadIdx.x;
+  uint4 v[kConcatFlight];
+#pragma unroll
+  for (int u = 0; u < kConcatFlight; u++)
+    if (i0 + u * kThreads < total) v[u] = __ldcs(x + i0 + u * kThreads);
+#pragma unroll
+  for (int u = 0; u < kConcatFlight; u++) {
+    const uint32_t i = i0 + u * kThreads;
+    if (i >= total) break;
+    if (LIN && m != 0) v[u] = rescale_linear(v[u], m, k);
+    const uint32_t r = __umulhi(i, per_row);
+    out[(size_t)r * a.row_units + (i - r * units)] = v[u];
   }
 }
 
@@ -311,10 +351,27 @@ void launch_table(const int8_t* x, const int8_t* table, int8_t* out, long long n
 void launch_concat(const ConcatArgs& a, cudaStream_t stream) {
   bool lut = false;
   for (int o = 0; o < a.n; o++) lut |= a.lut[o] != nullptr;
+  // from about four units a thread of a full chip on; the quotient by multiplication is exact below 2^32 / units
+  ConcatArgs w = a;
+  int widest = 0;
+  bool linear = true, sectors = true;
+  for (int o = 0; o < a.n; o++) {
+    w.per_row[o] = (uint32_t)((0x100000000ull + a.units[o] - 1) / a.units[o]);
+    widest = std::max(widest, a.units[o]);
+    sectors = sectors && a.units[o] % 2 == 0;
+    linear = linear && (!a.lut[o] || a.lin_m[o] != 0);
+  }
+  if (linear && sectors && a.rows * a.row_units >= 4ll * kThreads * 4 * current_sm_count() && a.rows * a.row_units < (1ll << 31) && a.rows * widest < (1ll << 32) / widest) {
+    const dim3 wide((unsigned)((a.rows * widest + kThreads * kConcatFlight - 1) / (kThreads * kConcatFlight)), (unsigned)a.n);
+    if (lut) launch_dependent(concat_wide_kernel<true>, wide, dim3(kThreads), 0, stream, w);
+    else launch_dependent(concat_wide_kernel<false>, wide, dim3(kThreads), 0, stream, w);
+    return;
+  }
   const long long blocks = (a.rows * a.row_units + kThreads - 1) / kThreads, most = 8ll * current_sm_count();
   const dim3 grid((unsigned)(blocks < most ? blocks : most));
-  if (lut) launch_dependent(concat_kernel<true>, grid, dim3(kThreads), 0, stream, a);
-  else launch_dependent(concat_kernel<false>, grid, dim3(kThreads), 0, stream, a);
+  if (lut && linear) launch_dependent(concat_kernel<kLinear>, grid, dim3(kThreads), 0, stream, a);
+  else if (lut) launch_dependent(concat_kernel<kTables>, grid, dim3(kThreads), 0, stream, a);
+  else launch_dependent(concat_kernel<kAsIs>, grid, dim3(kThreads), 0, stream, a);
 }
 
 void launch_rescale(const RescaleArgs& a, cudaStream_t stream) {

@@ -155,6 +155,9 @@ struct ConcatArgs {
   const int8_t* x[kConcatMax];    // [rows, 16 * units]
   const uint8_t* lut[kConcatMax]; // indexed by the raw byte, or null = as they are
   int units[kConcatMax], first[kConcatMax];  // 16-byte units per row of the operand, and of the result in front of it
+  // the table as one multiply-add with 16 fraction bits, clamp((x * lin_m + lin_k) >> 16), where that is exact for every byte (lin_m != 0)
+  int lin_m[kConcatMax], lin_k[kConcatMax];
+  uint32_t per_row[kConcatMax];  // filled by the launcher: 2^32 / units, rounded up
   int n, row_units;
   long long rows;
   int8_t* out;

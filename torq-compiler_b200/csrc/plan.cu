@@ -269,6 +269,25 @@ static void binary_linear_form(const tb200_op_t& op, BinaryArgs& a) {
   }
 }
 
+// A table over the raw byte that rescales by a factor: m, k with clamp((x * m + k) >> 16) == table[x] for every byte x, or m = 0.
+static void table_linear_form(const int8_t* table, double factor, int& m, int& k) {
+  m = k = 0;
+  if (std::fabs(factor) >= 100.0) return;
+  for (int nudge : {0, 1, -1, 2, -2}) {
+    const long long mm = std::llround(std::ldexp(factor, 16)) + nudge;
+    long long lo = INT32_MIN / 2, hi = INT32_MAX / 2;
+    for (int x = -128; x < 128; x++) {
+      const long long r = table[(uint8_t)x];
+      if (r > -128) lo = std::max(lo, r * 65536 - x * mm);
+      if (r < 127) hi = std::min(hi, (r + 1) * 65536 - 1 - x * mm);
+    }
+    if (mm == 0 || lo > hi) continue;
+    m = (int)mm;
+    k = (int)(lo + (hi - lo) / 2);
+    return;
+  }
+}
+
 // The parameters of a rescaled add / sub / mul without its pointers and size. The operand-side rescales are functions
 // of one byte: both tables are evaluated here as the kernel does, the value that reaches the output rescale is
 // bounded, and the 32-bit form of that rescale is taken when it is exact. False: a left shift outside [0, 22].
@@ -1913,6 +1932,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
               table[v] = (uint8_t)(int8_t)std::max(-128ll, std::min(127ll, r));
             }
             lut_off.back() = b.add_const(table, 256);
+            table_linear_form((const int8_t*)table, std::ldexp((double)l.mult, -l.shift), ca.lin_m[k], ca.lin_k[k]);
           }
           const Loc to = loc(op.out0);
           step.kernel_name = "concat_rescale";
