@@ -357,8 +357,12 @@ __global__ void __launch_bounds__(kMidThreads, 1) rows_mid_kernel(const ConvSmal
   for (int c = 0; c < chunks; c++) {
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();  // chunk c has arrived for everyone, and chunk c - 1 has been read by everyone
-    load_w();
-    load_x();
+    if (c + 2 < chunks) {
+      load_w();
+      load_x();
+    } else {
+      asm volatile("cp.async.commit_group;" ::: "memory");  // the wait above counts groups
+    }
     const uint32_t xs = stage + g * kMidPitch + t * 16, ws = stage + kMidX + nt * 8192 + lane * 16;
     stage = stage == base + (kMidStages - 1) * kMidStage ? base : stage + kMidStage;
 #pragma unroll
@@ -378,6 +382,12 @@ __global__ void __launch_bounds__(kMidThreads, 1) rows_mid_kernel(const ConvSmal
       }
     }
   }
+  // the records of the channels this lane finishes: on their way while the sums meet
+  const int chan = nb * kMidN + 4 * lane, left = a.N - chan;
+  int4 q[4];
+  if (a.epi && left > 0)
+#pragma unroll
+    for (int j = 0; j < 4; j++) q[j] = __ldg(a.q4 + chan + j);
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   int* sums = reinterpret_cast<int*>(mid_s);
@@ -413,12 +423,7 @@ __global__ void __launch_bounds__(kMidThreads, 1) rows_mid_kernel(const ConvSmal
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
-  const int chan = nb * kMidN + 4 * lane, left = a.N - chan;
   if (left <= 0) return;
-  int4 q[4];
-  if (a.epi)
-#pragma unroll
-    for (int j = 0; j < 4; j++) q[j] = __ldg(a.q4 + chan + j);
   for (int r = warp; r < 1 << share_log2; r += kMidThreads / 32) {
     const int row = (rank << share_log2) + r;
     if (row0 + row >= a.M) break;
