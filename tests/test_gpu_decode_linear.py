@@ -122,3 +122,43 @@ def test_attention_over_short_and_long_caches(device, n_q, B, window):
     for b in [d_in, d_pos] + outs:
         b.free()
     ex.destroy()
+
+
+@pytest.mark.parametrize("behind", ["geglu", "rope_kv"])
+@pytest.mark.parametrize("B", [1, 2])
+def test_norms_in_front_of_a_product_over_the_callers_own_rows(device, B, behind):
+    """A residual updated in place, and a result bound over rows that the norm reads: the product's blocks read these rows while others
+    store, so the norm has to run before it. The same bits as with buffers of their own, which the norm in the product's launch takes."""
+    H, I, n_q, D, T = 1152, 6912, 4, 256, 8
+    rng = np.random.default_rng(B)
+    x, r = (to_bf16(rng.normal(0, 1, (B, H)).astype(np.float32)) for _ in range(2))
+    w1, w2, wd = (to_bf16(rng.normal(0, 0.1, n).astype(np.float32)) for n in (H, H, D))
+    N = 2 * I if behind == "geglu" else (n_q + 2) * D
+    _, w, s, _ = _product(rng, B, H, N)
+    g = Graph()
+    xi, ri = g.input((B, H), "bf16"), g.input((B, H), "bf16")
+    y1 = g.rmsnorm(xi, w1, 1e-6, residual=ri)
+    y = g.gemv_w8(g.rmsnorm(y1, w2, 1e-6), w, s)
+    if behind == "geglu":
+        y, width = g.geglu(y), I
+    else:
+        pos = g.input((1,), "i32")
+        kc, vc = g.state((B, T, D), "bf16"), g.state((B, T, D), "bf16")
+        y, width = g.rope_kv(y, pos, wd, wd, kc, vc, n_q=n_q, n_kv=1, head_dim=D, theta=10000.0, eps=1e-6), n_q * D
+    g.output(y1), g.output(y)
+    ex = Executable(device, g.serialize())
+    assert any(k.startswith("norm_linear_w8") for k in ex.op_kernels()), ex.op_kernels()
+    bx, br, b1, by = (device.alloc(2 * B * max(H, width)) for _ in range(4))
+    bp = device.alloc(4)
+    bp.upload(np.array([3], np.int32))
+    want = None
+    for o1, oy in ((b1, by), (br, by), (bx, by), (b1, bx), (b1, br), (br, bx)):
+        for _ in range(1 if want is None else 20):
+            bx.upload(x), br.upload(r)
+            ex.dispatch([bx, br] + ([bp] if behind == "rope_kv" else []), [o1, oy])
+            got = [o1.download((B, H), np.uint16), oy.download((B, width), np.uint16)]
+            want = want or got
+            assert all((a == b).all() for a, b in zip(got, want)), (o1 is b1, oy is by)
+    for b in (bx, br, b1, by, bp):
+        b.free()
+    ex.destroy()

@@ -914,7 +914,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
       }
     }
     // A norm (or a pair) directly in front of a product that runs in its reader's step (3) runs in that launch too where the product's
-    // kernel can. Only the product reads the normed rows, which then never reach memory.
+    // kernel can. Only the product reads the normed rows, which then never reach memory. They keep their place in the arena: a caller whose
+    // buffers lie over one another gets the norm as a launch of its own (run_norm).
     for (int i = 0; i + 2 < (int)ops.size() && !(no_dec && *no_dec && *no_dec != '0'); i++) {
       const int last = norm_second[i] >= 0 ? norm_second[i] : i, p = last + 1;
       if (ops[i].kind != TB200_OP_RMSNORM || fused_away[i] || p + 1 >= (int)ops.size() || !gemv_deferred[p] || ops[p].in0 != ops[last].out0) continue;
@@ -1029,7 +1030,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
   }
 
   size_t scratch_need = 0;
-  struct NormStep { Loc x, res, out; size_t w_off, w2_off; float eps, eps2; bool has_res, pair; };
+  struct NormStep { Loc x, res, out, out2; size_t w_off, w2_off; float eps, eps2; bool has_res, pair; int rows, H; };
   std::map<int, NormStep> norms;  // deferred rmsnorm ops
   struct LinearStep { Loc x; size_t w_off, s_off; int B, N, K; size_t next_off, next_bytes; };
   std::vector<LinearStep> linear(ops.size(), LinearStep{});  // deferred gemv_w8 ops
@@ -1043,12 +1044,29 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
     k.next_bytes = (uint32_t)l.next_bytes;
     return k;
   };
-  auto norm_args = [](LinearArgs& k, const NormStep& n, const ExecContext& c) {
-    k.norm_x = (const uint16_t*)n.x.resolve(c);
-    k.norm_res = n.has_res ? (const uint16_t*)n.res.resolve(c) : nullptr;
-    k.norm_w = (const uint16_t*)(c.consts + n.w_off);
-    k.norm_w2 = n.pair ? (const uint16_t*)(c.consts + n.w2_off) : nullptr;
-    k.norm_out = n.pair ? (uint16_t*)n.out.resolve(c) : nullptr;
+  // Every block of the product reads the norm's rows, no block waits for another, and the first that are done store: into rows that lie over
+  // those (a residual updated in place) the norm has to be through before the product starts, and keeps its own launch.
+  auto run_norm = [](LinearArgs& k, const NormStep& n, const void* result, size_t result_bytes, const ExecContext& c) {
+    struct Range { const void* at; size_t bytes; };
+    const size_t rows_bytes = (size_t)n.rows * n.H * 2;
+    const uint16_t *x = (const uint16_t*)n.x.resolve(c), *res = n.has_res ? (const uint16_t*)n.res.resolve(c) : nullptr;
+    uint16_t* const out = (uint16_t*)n.out.resolve(c);
+    const uint16_t *w = (const uint16_t*)(c.consts + n.w_off), *w2 = n.pair ? (const uint16_t*)(c.consts + n.w2_off) : nullptr;
+    const Range reads[] = {{x, rows_bytes}, {res, res ? rows_bytes : 0}, {k.pos, k.pos ? sizeof(int32_t) : 0}};
+    const Range writes[] = {{result, result_bytes}, {out, n.pair ? rows_bytes : 0}};
+    bool apart = true;
+    for (const Range& r : reads)
+      for (const Range& o : writes)
+        apart = apart && (!r.bytes || !o.bytes || (const char*)r.at + r.bytes <= (const char*)o.at || (const char*)o.at + o.bytes <= (const char*)r.at);
+    if (!apart) {
+      launch_rmsnorm_row(x, res, w, out, w2, n.pair ? (uint16_t*)n.out2.resolve(c) : nullptr, n.rows, n.H, n.eps, n.eps2, c.stream);
+      return;
+    }
+    k.norm_x = x;
+    k.norm_res = res;
+    k.norm_w = w;
+    k.norm_w2 = w2;
+    k.norm_out = n.pair ? out : nullptr;
     k.norm_eps = n.eps; k.norm_eps2 = n.eps2;
   };
   auto report = [](cudaError_t e, const ExecContext& c) {
@@ -2039,7 +2057,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             eps2 = ops[second].f0;
           }
           if (norm_deferred[i]) {
-            norms[i] = NormStep{lx, lr, lo, w_off, w2_off, eps, eps2, has_res, second >= 0};
+            norms[i] = NormStep{lx, lr, lo, lo2, w_off, w2_off, eps, eps2, has_res, second >= 0, rows, H};
             step.kernel_name = "(norm in the launch of the product behind it)";
             step.launches = 0;
             step.launch = [](const ExecContext&) {};
@@ -2144,7 +2162,6 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           step.kernel_name = has_norm ? "norm_linear_w8_rope_kv" : "linear_w8_rope_kv";
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
-            if (has_norm) norm_args(k, norm, c);
             k.pos = (const int32_t*)lp.resolve(c);
             k.qw = (const uint16_t*)(c.consts + qw_off);
             k.kw = (const uint16_t*)(c.consts + kw_off);
@@ -2152,6 +2169,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
             k.kcache = (uint16_t*)lk.resolve(c);
             k.vcache = (uint16_t*)lv.resolve(c);
             k.n_q = n_q; k.T = T; k.theta = theta; k.eps = eps;
+            if (has_norm) run_norm(k, norm, k.q_out, (size_t)B * n_q * D * 2, c);
             report(launch_linear_rope(k, c.stream), c);
           };
           break;
@@ -2201,8 +2219,8 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
           step.kernel_name = has_norm ? "norm_linear_w8_geglu" : "linear_w8_geglu";
           step.launch = [=](const ExecContext& c) {
             LinearArgs k = linear_args(l, c);
-            if (has_norm) norm_args(k, norm, c);
             k.y = lo.resolve(c);
+            if (has_norm) run_norm(k, norm, k.y, (size_t)B * I * 2, c);
             report(launch_linear_geglu(k, c.stream), c);
           };
           break;
