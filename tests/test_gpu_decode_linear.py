@@ -56,6 +56,37 @@ def test_products_of_few_tokens_over_magnitudes(device, B, K, N, spread):
     assert (np.abs(got - xd @ wd.T) <= bound).all(), np.max(np.abs(got - xd @ wd.T) / bound)
 
 
+@pytest.mark.parametrize("B,K,N", [(1, 1152, 30001), (2, 4096, 28500), (5, 1152, 28500), (8, 1600, 30001)])
+@pytest.mark.parametrize("gap", [16, 22, 30])
+def test_rows_with_an_outlier_keep_what_lies_below_it(device, B, K, N, gap):
+    """One activation of a row 2^gap above the rest, meeting weights of zero: what is left is the sum of the others, to the bound of an fp32
+    sum of K terms. Rows without an outlier beside it give the same bits as without such neighbours, and the arg max ranges over both."""
+    rng = np.random.default_rng(B + K + gap)
+    x = rng.normal(0, 1, (B, K)).astype(np.float32)
+    x = np.where(np.abs(x) < 2.0 ** -9, 2.0 ** -9, x)
+    plain = to_bf16(x)
+    at = [b * K // B for b in range(B)]
+    outliers = [b for b in range(B) if b % 2 == 0]
+    for b in outliers:
+        x[b, at[b]] = 2.0 ** gap
+    w = rng.integers(-128, 128, (N, K), dtype=np.int8)
+    w[:, at] = 0
+    g = Graph()
+    y = g.gemv_w8(g.input((B, K), "bf16"), w, to_bf16(np.ones(N, np.float32)), out_dtype="f32")
+    g.output(y), g.output(g.argmax(y))
+    bits = to_bf16(x)
+    got, ids = run_graph_gpu(device, g, [bits])
+    xd = torch.from_numpy(from_bf16(bits)).double()
+    wd = torch.from_numpy(w).double()
+    xd[outliers, [at[b] for b in outliers]] = 0.0  # meets zeros only
+    want, bound = (xd @ wd.T).numpy(), K * 2.0 ** -24 * (xd.abs() @ wd.abs().T).numpy()
+    assert (np.abs(got - want) <= bound).all(), np.max(np.abs(got - want) / bound)
+    assert (ids == got.argmax(-1)).all()
+    rest = [b for b in range(B) if b not in outliers]
+    beside = run_graph_gpu(device, g, [plain])[0]
+    assert (got[rest].view(np.uint32) == beside[rest].view(np.uint32)).all()
+
+
 @pytest.mark.parametrize("B,K,N", [(1, 64, 40), (3, 1152, 33), (8, 1152, 30001)])
 def test_products_of_few_tokens_with_infinities_and_nans(device, B, K, N):
     rng = np.random.default_rng(K)

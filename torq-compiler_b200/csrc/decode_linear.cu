@@ -101,9 +101,10 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 //            cand_v, the block's arg-max candidates per token. SLICED (up to eight tokens): int8 instructions on the weights as they are and
 //            on four int8 slices of every activation, exact integer sums joined in fp32. The conversion of weights to bf16 was what bounded it:
 //            302 MB of weights for one token 62.2 -> 49.1 us (46 us of HBM time), against 64 bits the error falls from 1.2e-7 to 0.3e-7.
+//            Tokens whose row four slices do not hold exactly go through the weights once more in bf16.
 // ---------------------------------------------------------------------------------------------------------------
 
-constexpr int kNonFinite = 0x7fffffff;  // in place of a shift: the group's activations of a token hold an infinity or a NaN
+constexpr int kNoSlices = 0x7fffffff;  // in place of a shift: four slices do not hold the token's activations exactly
 
 template <int NT, int MODE, bool SLICED>
 __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
@@ -211,16 +212,20 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
   const int warps = blockDim.x >> 5;
   if constexpr (SLICED) {
     // A warp slices a token: x = d0 + 2^8 d1 + 2^16 d2 + 2^24 d3 in units of 2^-shift, the largest of the row just below 2^30, digits in
-    // [-128, 127]. A value down to 2^-22 of the largest is exact, below that it is off by at most 2^-31 of the largest.
+    // [-128, 127]. Exact where no value's exponent but a zero's is more than 22 below the largest one's. A smaller value would lose bits that
+    // an fp32 sum keeps (all that is left of the sum where the large ones meet zero weights), so such a row is left to the bf16 form, as one
+    // with an infinity or a NaN is. Of rows of 1152 normal values one in 2300 goes there.
     constexpr int kHold = 10;  // 128 values each, kept between the two passes over them
     for (int b = warp; b < a.B; b += warps) {
       const uint16_t* src = a.x + (size_t)b * a.K + 4 * lane;
       auto load = [&](int i) { return 128 * i + 4 * lane < a.K ? __ldcg(reinterpret_cast<const uint2*>(src + 128 * i)) : make_uint2(0, 0); };
       uint2 hold[kHold];
-      uint32_t top = 0;  // largest magnitude, as bits
+      uint32_t top = 0, low = 0xffffffffu;  // largest magnitude, as bits, and the smallest that is not zero, less one
       auto widen = [&](const uint2& u) {
         top = __vmaxu2(top, u.x & 0x7fff7fffu);
         top = __vmaxu2(top, u.y & 0x7fff7fffu);
+        low = __vminu2(low, __vsub2(u.x & 0x7fff7fffu, 0x00010001u));  // (a zero becomes the largest)
+        low = __vminu2(low, __vsub2(u.y & 0x7fff7fffu, 0x00010001u));
       };
 #pragma unroll
       for (int i = 0; i < kHold; i++) hold[i] = load(i);
@@ -228,8 +233,11 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
       for (int i = 0; i < kHold; i++) widen(hold[i]);
       for (int i = kHold; 128 * i < a.K; i++) widen(load(i));
       const uint32_t e = __reduce_max_sync(0xffffffffu, max(top >> 16, top & 0xffffu)) >> 7;  // its exponent, biased
+      const uint32_t least = __reduce_min_sync(0xffffffffu, min(low >> 16, low & 0xffffu));
       const int shift = 29 + 127 - max((int)e, 1), first = min(shift, 126);
-      if (lane == 0) shifts[b] = e == 255 ? kNonFinite : shift;
+      // the seven bits behind the smallest one's exponent end at or above a unit (a row of zeros has no smallest one)
+      const bool exact = e != 255 && (least == 0xffffu || max((int)e, 1) - max((int)((least + 1) >> 7), 1) <= 22);
+      if (lane == 0) shifts[b] = exact ? shift : kNoSlices;
       const float s0 = pow2(first), s1 = pow2(shift - first);
       const uint32_t dst = x_addr + (uint32_t)(b * kSlices * a.x_pitch + 4 * lane);
       auto slice = [&](const uint2& u, int i) {
@@ -327,52 +335,53 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
   if (MODE != kStream && (int)threadIdx.x < a.rt * kTileRows) scale_s[threadIdx.x] = bf2f(scale_r);
   __syncthreads();
 
-  // the product of one weight row and one token, element by element: for activations that hold infinities or NaNs
-  auto plain_dot = [&](int n, int b) {
-    float v = 0.f;
-    for (int k = 0; k < a.K; k++) v += (float)a.W[(size_t)n * a.K + k] * bf2f(a.x[(size_t)b * a.K + k]);
-    return v;
-  };
-  int stage = 0, kb = 0, tile = tile0;
-  // Sums of this warp: [16-row half][tile of eight columns][...]. Sliced: columns are the slices of two tokens, 2 t + tig / 2 for this lane;
-  // else eight tokens.
+  // Sums of this warp: [16-row half][tile of eight columns][...]. Of slices (ci): columns are the slices of two tokens, 2 t + tig / 2 for this
+  // lane; else (cs) eight tokens.
   // Independent chains of accumulation where the tokens leave room: a dependent matrix instruction waits 28 cycles.
-  constexpr int kSets = SLICED || NT > 2 ? 1 : NT == 2 ? 2 : 4;
-  float cs[kSets][2][NT][4];
+  constexpr int kTiles = kTok / 8, kSets = kTiles > 2 ? 1 : kTiles == 2 ? 2 : 4;
+  float cs[kSets][2][kTiles][4];
   int ci[2][NT][4];
   auto& c = cs[0];
-  float best_v[NT][2];
-  int best_i[NT][2];
+  float best_v[kTiles][2], best_sliced_v[NT];
+  int best_i[kTiles][2], best_sliced_i[NT];
 #pragma unroll
-  for (int t = 0; t < NT; t++) {
+  for (int t = 0; t < kTiles; t++) {
     best_v[t][0] = best_v[t][1] = -INFINITY;
     best_i[t][0] = best_i[t][1] = 0x7fffffff;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      ci[0][t][j] = ci[1][t][j] = 0;
+    for (int j = 0; j < 4; j++)
 #pragma unroll
       for (int q = 0; q < kSets; q++) cs[q][0][t][j] = cs[q][1][t][j] = 0.f;
-    }
   }
-  int shift[NT];  // of this lane's token in each tile
-  if (SLICED)
 #pragma unroll
-    for (int t = 0; t < NT; t++) shift[t] = 2 * t + (tig >> 1) < a.B ? shifts[2 * t + (tig >> 1)] : 0;
+  for (int t = 0; t < NT; t++) {
+    best_sliced_v[t] = -INFINITY;
+    best_sliced_i[t] = 0x7fffffff;
+#pragma unroll
+    for (int j = 0; j < 4; j++) ci[0][t][j] = ci[1][t][j] = 0;
+  }
+  // Every token takes one of the two forms by what is in its own row, so its result does not depend on the tokens beside it.
+  uint32_t sliced_tokens = 0;  // a bit each
+  int shift[NT] = {};          // of this lane's token in each tile
+  if constexpr (SLICED) {
+    for (int b = 0; b < a.B; b++) sliced_tokens |= (uint32_t)(shifts[b] != kNoSlices) << b;
+#pragma unroll
+    for (int t = 0; t < NT; t++) shift[t] = sliced_tokens >> (2 * t + (tig >> 1)) & 1 ? shifts[2 * t + (tig >> 1)] : 0;
+  }
   // a lane's finished sum of row 16 mt + 8 (tig % 2) + g for its token of tile t (two lanes hold two slices each and finish a row each)
-  auto finished = [&](int mt, int t, int n) {
+  auto finished = [&](int mt, int t) {
     const float lo = (float)ci[mt][t][0] + 256.f * (float)ci[mt][t][1], hi = (float)ci[mt][t][2] + 256.f * (float)ci[mt][t][3];  // rows g, g + 8
     const float other = __shfl_xor_sync(0xffffffffu, tig & 1 ? lo : hi, 1);
     const float v = tig & 1 ? 65536.f * hi + other : 65536.f * other + lo;
     const int first = min(shift[t], 126);
-    if (shift[t] == kNonFinite) return plain_dot(n, 2 * t + (tig >> 1));
     return v * pow2(-first) * pow2(first - shift[t]);
   };
   auto fold = [&]() {  // the chains into the first, which the others start from zero after
-    if (SLICED || kSets == 1) return;
+    if (kSets == 1) return;
 #pragma unroll
     for (int mt = 0; mt < 2; mt++)
 #pragma unroll
-      for (int t = 0; t < NT; t++)
+      for (int t = 0; t < kTiles; t++)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           if (kSets == 4) c[mt][t][j] = (c[mt][t][j] + cs[1 % kSets][mt][t][j]) + (cs[2 % kSets][mt][t][j] + cs[3 % kSets][mt][t][j]);
@@ -381,100 +390,127 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
           for (int q = 1; q < kSets; q++) cs[q][mt][t][j] = 0.f;
         }
   };
-  const uint32_t xrow = x_addr + (uint32_t)(g * a.x_pitch + (wb0 - kb0) * kBlk * (SLICED ? 1 : 2) + tig * (SLICED ? 16 : 32));
-  for (int i = 0; i < total; i++) {
-    if (MODE == kStream) {  // the ring is a.stages deep and one group is committed per block from here on
-      if (SLICED || i >= a.stages) cp_wait<kStreamStages - 1>();
-      __syncwarp();
-    }
-    const uint32_t src = ring + stage * kStageBytes + g * kBlk + tig * 16;
-    const uint4 w0 = lds128(src), w1 = lds128(src + 8 * kBlk), w2 = lds128(src + 16 * kBlk), w3 = lds128(src + 24 * kBlk);
-    if (MODE == kStream) {
-      __syncwarp();  // read by every lane before any of them refills the stage
-      if (issued < total) {
-        issue();
-        issued++;
+  auto multiply = [&](auto of_slices, uint32_t x_row, int x_pitch) {
+    constexpr bool kInts = decltype(of_slices)::value;
+    int stage = 0, kb = 0, tile = tile0;
+    const uint32_t xrow = x_row + (uint32_t)((wb0 - kb0) * kBlk * (kInts ? 1 : 2) + tig * (kInts ? 16 : 32));
+    for (int i = 0; i < total; i++) {
+      if (MODE == kStream) {  // the ring is a.stages deep and one group is committed per block from here on
+        if (kInts || i >= a.stages) cp_wait<kStreamStages - 1>();
+        __syncwarp();
       }
-      cp_commit();
-    }
-    if constexpr (SLICED) {
-#pragma unroll
-      for (int t = 0; t < NT; t++) {
-        const uint4 x = lds128(xrow + (uint32_t)(t * 8 * a.x_pitch + kb * kBlk));
-        mma_s8(ci[0][t], w0.x, w1.x, w0.y, w1.y, x.x, x.y);
-        mma_s8(ci[1][t], w2.x, w3.x, w2.y, w3.y, x.x, x.y);
-        mma_s8(ci[0][t], w0.z, w1.z, w0.w, w1.w, x.z, x.w);
-        mma_s8(ci[1][t], w2.z, w3.z, w2.w, w3.w, x.z, x.w);
+      const uint32_t src = ring + stage * kStageBytes + g * kBlk + tig * 16;
+      const uint4 w0 = lds128(src), w1 = lds128(src + 8 * kBlk), w2 = lds128(src + 16 * kBlk), w3 = lds128(src + 24 * kBlk);
+      if (MODE == kStream) {
+        __syncwarp();  // read by every lane before any of them refills the stage
+        if (issued < total) {
+          issue();
+          issued++;
+        }
+        cp_commit();
       }
-    } else {
-      const uint32_t ww[4][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}, {w2.x, w2.y, w2.z, w2.w}, {w3.x, w3.y, w3.z, w3.w}};
-      uint4 x0[NT], x1[NT];
-#pragma unroll
-      for (int t = 0; t < NT; t++) {
-        const uint32_t xa = xrow + (uint32_t)(t * 8 * a.x_pitch + kb * kBlk * 2);
-        x0[t] = lds128(xa);
-        x1[t] = lds128(xa + 16);
-      }
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        uint32_t f[4][2];
-#pragma unroll
-        for (int r = 0; r < 4; r++) s8x4_to_bf16x4(ww[r][m], f[r][0], f[r][1]);
+      if constexpr (kInts) {
 #pragma unroll
         for (int t = 0; t < NT; t++) {
-          const uint32_t b0 = m == 0 ? x0[t].x : m == 1 ? x0[t].z : m == 2 ? x1[t].x : x1[t].z;
-          const uint32_t b1 = m == 0 ? x0[t].y : m == 1 ? x0[t].w : m == 2 ? x1[t].y : x1[t].w;
-          mma_bf16(cs[m % kSets][0][t], f[0][0], f[1][0], f[0][1], f[1][1], b0, b1);
-          mma_bf16(cs[m % kSets][1][t], f[2][0], f[3][0], f[2][1], f[3][1], b0, b1);
+          const uint4 x = lds128(xrow + (uint32_t)(t * 8 * x_pitch + kb * kBlk));
+          mma_s8(ci[0][t], w0.x, w1.x, w0.y, w1.y, x.x, x.y);
+          mma_s8(ci[1][t], w2.x, w3.x, w2.y, w3.y, x.x, x.y);
+          mma_s8(ci[0][t], w0.z, w1.z, w0.w, w1.w, x.z, x.w);
+          mma_s8(ci[1][t], w2.z, w3.z, w2.w, w3.w, x.z, x.w);
+        }
+      } else {
+        const uint32_t ww[4][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}, {w2.x, w2.y, w2.z, w2.w}, {w3.x, w3.y, w3.z, w3.w}};
+        uint4 x0[kTiles], x1[kTiles];
+#pragma unroll
+        for (int t = 0; t < kTiles; t++) {
+          const uint32_t xa = xrow + (uint32_t)(t * 8 * x_pitch + kb * kBlk * 2);
+          x0[t] = lds128(xa);
+          x1[t] = lds128(xa + 16);
+        }
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          uint32_t f[4][2];
+#pragma unroll
+          for (int r = 0; r < 4; r++) s8x4_to_bf16x4(ww[r][m], f[r][0], f[r][1]);
+#pragma unroll
+          for (int t = 0; t < kTiles; t++) {
+            const uint32_t b0 = m == 0 ? x0[t].x : m == 1 ? x0[t].z : m == 2 ? x1[t].x : x1[t].z;
+            const uint32_t b1 = m == 0 ? x0[t].y : m == 1 ? x0[t].w : m == 2 ? x1[t].y : x1[t].w;
+            mma_bf16(cs[m % kSets][0][t], f[0][0], f[1][0], f[0][1], f[1][1], b0, b1);
+            mma_bf16(cs[m % kSets][1][t], f[2][0], f[3][0], f[2][1], f[3][1], b0, b1);
+          }
         }
       }
-    }
-    if (++stage == a.stages) stage = 0;
-    if (++kb == nb) {
-      kb = 0;
-      fold();
-      if (MODE == kStream) {
-        auto take = [&](int n, float s, float sum, int b, float& best, int& at) {
-          const float v = sum * s;
-          if (n >= a.N || b >= a.B) return;
-          if (a.y_f32) ((float*)a.y)[(size_t)b * a.N + n] = v;
-          else ((uint16_t*)a.y)[(size_t)b * a.N + n] = f2bf(v);
-          if (v > best) {  // a warp's rows come in rising order: ties keep the lower index
-            best = v;
-            at = n;
-          }
-        };
-        if constexpr (SLICED) {
-#pragma unroll
-          for (int mt = 0; mt < 2; mt++) {
-            const int n = tile * kTileRows + 16 * mt + 8 * (tig & 1) + g;
-            const float s = n < a.N ? bf2f(__ldg(a.scale + n)) : 0.f;
-#pragma unroll
-            for (int t = 0; t < NT; t++) {
-              take(n, s, finished(mt, t, min(n, a.N - 1)), 2 * t + (tig >> 1), best_v[t][0], best_i[t][0]);
-#pragma unroll
-              for (int j = 0; j < 4; j++) ci[mt][t][j] = 0;
+      if (++stage == a.stages) stage = 0;
+      if (++kb == nb) {
+        kb = 0;
+        if (!kInts) fold();
+        if (MODE == kStream) {
+          auto take = [&](int n, float s, float sum, int b, float& best, int& at) {
+            const float v = sum * s;
+            if (n >= a.N || b >= a.B || (SLICED && (sliced_tokens >> b & 1) != kInts)) return;
+            if (a.y_f32) ((float*)a.y)[(size_t)b * a.N + n] = v;
+            else ((uint16_t*)a.y)[(size_t)b * a.N + n] = f2bf(v);
+            if (v > best) {  // a warp's rows come in rising order: ties keep the lower index
+              best = v;
+              at = n;
             }
-          }
-        } else {
+          };
+          if constexpr (kInts) {
 #pragma unroll
-          for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              const int n = tile * kTileRows + 16 * mt + 8 * h + g;
+            for (int mt = 0; mt < 2; mt++) {
+              const int n = tile * kTileRows + 16 * mt + 8 * (tig & 1) + g;
               const float s = n < a.N ? bf2f(__ldg(a.scale + n)) : 0.f;
 #pragma unroll
-              for (int t = 0; t < NT; t++)
+              for (int t = 0; t < NT; t++) {
+                take(n, s, finished(mt, t), 2 * t + (tig >> 1), best_sliced_v[t], best_sliced_i[t]);
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                  take(n, s, c[mt][t][2 * h + e], 8 * t + 2 * tig + e, best_v[t][e], best_i[t][e]);
-                  c[mt][t][2 * h + e] = 0.f;
-                }
+                for (int j = 0; j < 4; j++) ci[mt][t][j] = 0;
+              }
             }
+          } else {
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                const int n = tile * kTileRows + 16 * mt + 8 * h + g;
+                const float s = n < a.N ? bf2f(__ldg(a.scale + n)) : 0.f;
+#pragma unroll
+                for (int t = 0; t < kTiles; t++)
+#pragma unroll
+                  for (int e = 0; e < 2; e++) {
+                    take(n, s, c[mt][t][2 * h + e], 8 * t + 2 * tig + e, best_v[t][e], best_i[t][e]);
+                    c[mt][t][2 * h + e] = 0.f;
+                  }
+              }
+          }
+          tile += tile_step;
         }
-        tile += tile_step;
       }
     }
+  };
+  if constexpr (SLICED) {
+    if (sliced_tokens) multiply(std::true_type(), x_addr + (uint32_t)(g * a.x_pitch), a.x_pitch);
+    if (sliced_tokens != (1u << a.B) - 1) {  // once more for the rows left to bf16, staged where the slices were (they take half of that)
+      __syncthreads();
+      const int pitch = (a.K * 2 + 127) / 128 * 128 + 16;
+      for (int b = warp; b < a.B; b += warps)
+        for (int v = lane; v < a.K / 8; v += 32) cp_async16(x_addr + (uint32_t)(b * pitch + 16 * v), a.x + (size_t)b * a.K + 8 * v, true);
+      cp_commit();
+      if (sliced_tokens) {
+        is_tile = tile0;
+        is_kb = is_stage = 0;
+        for (issued = 0; issued < a.stages && issued < total; issued++) {
+          issue();
+          cp_commit();
+        }
+      }
+      cp_wait<0>();
+      __syncthreads();
+      multiply(std::false_type(), x_addr + (uint32_t)(min(g, a.B - 1) * pitch), pitch);
+    }
+  } else {
+    multiply(std::false_type(), x_addr + (uint32_t)(g * a.x_pitch), a.x_pitch);
   }
 
   if constexpr (MODE == kStream) {
@@ -483,27 +519,29 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     __syncthreads();
     float* sv = reinterpret_cast<float*>(sm);
     int* si = reinterpret_cast<int*>(sm) + 16 * kTok;
+    // a lane's best of a token, against those of the other lanes that hold the token
+    auto leave = [&](float v, int n, int b, bool sliced) {
 #pragma unroll
-    for (int t = 0; t < NT; t++)
-#pragma unroll
-      for (int e = 0; e < (SLICED ? 1 : 2); e++) {
-        float v = best_v[t][e];
-        int n = best_i[t][e];
-#pragma unroll
-        for (int o = SLICED ? 1 : 4; o < 32; o = SLICED && o == 1 ? 4 : o << 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-          const int on = __shfl_xor_sync(0xffffffffu, n, o);
-          if (ov > v || (ov == v && on < n)) {
-            v = ov;
-            n = on;
-          }
-        }
-        const int b = SLICED ? 2 * t + (tig >> 1) : 8 * t + 2 * tig + e;
-        if (g == 0) {
-          sv[warp * kTok + b] = v;
-          si[warp * kTok + b] = n;
+      for (int o = sliced ? 1 : 4; o < 32; o = o == 1 ? 4 : o << 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+        const int on = __shfl_xor_sync(0xffffffffu, n, o);
+        if (ov > v || (ov == v && on < n)) {
+          v = ov;
+          n = on;
         }
       }
+      if (g == 0 && (!SLICED || (b < a.B && (sliced_tokens >> b & 1) == sliced))) {
+        sv[warp * kTok + b] = v;
+        si[warp * kTok + b] = n;
+      }
+    };
+    if constexpr (SLICED)
+#pragma unroll
+      for (int t = 0; t < NT; t++) leave(best_sliced_v[t], best_sliced_i[t], 2 * t + (tig >> 1), true);
+#pragma unroll
+    for (int t = 0; t < kTiles; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) leave(best_v[t][e], best_i[t][e], 8 * t + 2 * tig + e, false);
     __syncthreads();
     if ((int)threadIdx.x < a.B) {
       float v = sv[threadIdx.x];
