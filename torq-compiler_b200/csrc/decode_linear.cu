@@ -1065,8 +1065,7 @@ cudaError_t launch_linear_mode(const LinearArgs& args, const LinearShape& s, cud
       default: return launch_linear_as<1, MODE, true>(a, s, cluster, stream);
     }
   switch (ceil_div(a.B, 8)) {
-    case 1:
-      if constexpr (MODE != kStream) return launch_linear_as<1, MODE, false>(a, s, cluster, stream);
+    case 1: return launch_linear_as<1, MODE, false>(a, s, cluster, stream);
     case 2: return launch_linear_as<2, MODE, false>(a, s, cluster, stream);
     case 3: return launch_linear_as<3, MODE, false>(a, s, cluster, stream);
     default: return launch_linear_as<4, MODE, false>(a, s, cluster, stream);

@@ -18,7 +18,8 @@ constexpr int kTileRows = 32, kBlk = 64, kStageBytes = kTileRows * kBlk, kStream
 constexpr int kRopeTokens = 8;  // most tokens a warp finishes in the RoPE epilogue
 constexpr int kSmemMax = 227 * 1024 - 1024;
 // Up to kSlicedTokens tokens the product over the vocabulary multiplies integers: a bf16 activation is four int8 slices of a 31-bit
-// fixed-point number, a slice a column of the instruction. Its weights then need no conversion. The products of the layers keep bf16: their
+// fixed-point number, a slice a column of the instruction. Its weights then need no conversion (where the slices leave room for the warps:
+// linear_shape). The products of the layers keep bf16: their
 // results are rounded to bf16 and go through every layer behind them, where two sums that differ in the last bit of fp32 end almost a
 // percent apart.
 // Up to kNormTokens the norm in front of a product runs in it.
@@ -52,7 +53,6 @@ inline LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
   const int tok = ceil_div(B, 8) * 8, blocks = K / kBlk;
   s.tk = linear_groups(N, K);
   if (mode == kStore && s.tk == 1) mode = kStream;
-  s.sliced = mode == kStream && B <= kSlicedTokens;
   s.tiles = mode == kGeglu ? ceil_div(N / 2, 16) : ceil_div(N, kTileRows);
   auto fit = [&](int kg, int ck, int rt, int stages) {
     s.kg = kg; s.ck = ck; s.rt = rt; s.stages = stages;
@@ -75,12 +75,22 @@ inline LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
     return s.smem <= kSmemMax;
   };
   if (mode == kStream) {
-    for (int rt = 16; rt >= 1; rt /= 2)
-      if (fit(1, 1, rt, kStreamStages)) {
-        s.grid = std::min(sms, ceil_div(s.tiles, rt));
-        s.ok = true;
-        return s;
-      }
+    auto warps_that_fit = [&](bool sliced) {
+      s.sliced = sliced;
+      int rt = 16;
+      while (rt >= 1 && !fit(1, 1, rt, kStreamStages)) rt /= 2;
+      return rt;
+    };
+    auto rounds = [&](int rt) { return ceil_div(s.tiles, (long long)sms * rt); };
+    const int rt = warps_that_fit(false), sliced_rt = B <= kSlicedTokens ? warps_that_fit(true) : 0;
+    // Eight tokens' slices leave room for 8 warps from K = 3008 on, 4 from 5056, 2 from 6080 and none from 6848; bf16 rows for 16 below 6144. A
+    // round (a tile for every warp) takes 8.5 us per 1024 of K with 8 warps on slices and 14.3 with 16 on bf16, but still 7.0 and 6.6 with 4
+    // and 2 on slices: so 8 warps for 16 where the rounds say so, and no others. Eight tokens, slices against bf16: K = 3072, N = 100000 (3 rounds and 2) 76.4 / 86.0 us,
+    // 4096 x 60000 (2 and 1) 72.9 / 57.7, 5120 x 50000 (4 warps) 104.9 / 67.9, 6144 x 50000 (2 warps) 239 / 91.
+    if (sliced_rt < 1 || !(sliced_rt >= rt || (sliced_rt == 8 && 5 * rounds(sliced_rt) < 8 * rounds(rt)))) warps_that_fit(false);
+    if ((s.sliced ? sliced_rt : rt) < 1) return LinearShape{};
+    s.grid = std::min(sms, ceil_div(s.tiles, s.rt));
+    s.ok = true;
     return s;
   }
   const int stages = ceil_div(blocks, s.tk);  // every block of a warp has its own place
