@@ -15,10 +15,11 @@ int main() {
   const int ns[] = {1, 31, 32, 100, 768, 1024, 1152, 1536, 6912, 13824, 30001, 262144};
   for (int sms : {108, 132, 148, 160})
     for (int mode : {kStore, kGeglu, kRope})
+     for (bool logits : {false, true})
       for (int n : ns)
         for (int k = 64; k <= 8192; k += 64)
           for (int b = 1; b <= 32; b++) {
-            const LinearShape s = linear_shape(b, n, k, mode, sms);
+            const LinearShape s = linear_shape(b, n, k, mode, sms, logits);
             if (!s.ok) continue;
             const int tok = ceil_div(b, 8) * 8, warps = s.kg * s.rt;
             const int staged = s.x_bytes + warps * s.stages * kStageBytes;  // activations and rings
@@ -52,7 +53,9 @@ int main() {
         const int rows = ((b + 7) / 8 * 8 * ((k * 2 + 127) / 128 * 128 + 16) + 127) / 128 * 128;
         int warps = 16;
         while (warps >= 1 && rows + warps * (4 * 2048 + 128) > kSmemMax) warps /= 2;
-        const LinearShape s = linear_shape(b, n, k, kStore, 148);
+        const LinearShape s = linear_shape(b, n, k, kStore, 148, true);
+        const LinearShape layer = linear_shape(b, n, k, kStore, 148, false);
+        if (layer.sliced || layer.ok != (warps > 0)) bad++, printf("B %d N %d K %d: bf16 result, ok %d, sliced %d\n", b, n, k, layer.ok, layer.sliced);
         if (!warps) {
           if (s.ok && !s.sliced) bad++, printf("B %d N %d K %d: rows do not fit\n", b, n, k);
           continue;
@@ -71,7 +74,7 @@ int main() {
     for (int n : {1536, 13824})
       for (int k = 64; k <= 2048; k += 64)
         for (int b = 1; b <= kNormTokens; b++) {
-          const LinearShape s = linear_shape(b, n, k, mode, 148);
+          const LinearShape s = linear_shape(b, n, k, mode, 148, false);
           if (!s.ok || s.ck != 1) continue;
           norms++;
           if (s.side_off < 8 * 2 * k || s.side_off + 2 * 2 * 16 * 4 > s.x_bytes) bad++, printf("norm: mode %d B %d N %d K %d\n", mode, b, n, k);

@@ -117,6 +117,22 @@ def test_geglu_behind_the_product(device, B, K, I):
     assert (np.abs(got - want) <= 2.0 ** -6 * np.maximum(np.abs(want), 0.05)).all()
 
 
+@pytest.mark.parametrize("B,K,I", [(1, 64, 20), (8, 1152, 14400), (3, 1536, 15000)])
+def test_geglu_behind_a_product_of_one_group_changes_no_bit(device, B, K, I, monkeypatch):
+    """Products whose K no warps share, as wide gate / up ones: the same bits with GeGLU in the launch and behind it."""
+    rng = np.random.default_rng(B + K)
+    x, w, s, _ = _product(rng, B, K, 2 * I)
+    g = Graph()
+    g.output(g.geglu(g.gemv_w8(g.input((B, K), "bf16"), w, s)))
+    got = run_graph_gpu(device, g, [x])[0]
+    monkeypatch.setenv("TB200_NO_DECODER_FUSION", "1")
+    ex = Executable(device, g.serialize())
+    assert ex.op_kernels() == ["linear_w8", "geglu"], ex.op_kernels()
+    ex.destroy()
+    alone = run_graph_gpu(device, g, [x])[0]
+    assert (got == alone).all(), int((got != alone).sum())
+
+
 @pytest.mark.parametrize("n_q,B,window", [(1, 1, 0), (2, 3, 20), (4, 9, 130)])
 def test_attention_over_short_and_long_caches(device, n_q, B, window):
     rng = np.random.default_rng(n_q)

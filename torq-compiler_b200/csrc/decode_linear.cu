@@ -94,11 +94,12 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 // memory then serves two instructions: at 32 tokens these reads bounded a 16-row tile) and one of TK groups of 64-byte
 // blocks of K, whose weights it copies into a ring of its own (cp.async; nothing but the warp itself waits for them). The
 // activations of the block's K range are staged once per block. TK depends on N and K alone, and a result is the sum of its
-// TK groups in order, so it does not depend on the mode or on how groups are spread over warps and blocks.
+// TK groups in order, so it does not depend on the mode or on how groups are spread over warps and blocks (fp32 results that SLICED
+// takes are the exception, whatever stands behind them).
 //   kStore: bf16 or fp32 results.                      kGeglu: bf16(bf16(gelu(gate)) * up), tiles of 16 gate and 16 up rows.
 //   kRope:  a cluster of eight blocks is one head of 256: head norm, RoPE, q out / cache append (arithmetic of rope_kv_kernel).
 //   kStream: one group and a warp per tile, blocks stay and walk the tiles (the LM head); fp32 or bf16 results and, with
-//            cand_v, the block's arg-max candidates per token. SLICED (up to eight tokens): int8 instructions on the weights as they are and
+//            cand_v, the block's arg-max candidates per token. SLICED (fp32 results of up to eight tokens): int8 instructions on the weights as they are and
 //            on four int8 slices of every activation, exact integer sums joined in fp32. The conversion of weights to bf16 was what bounded it:
 //            302 MB of weights for one token 62.2 -> 49.1 us (46 us of HBM time), against 64 bits the error falls from 1.2e-7 to 0.3e-7.
 //            Tokens whose row four slices do not hold exactly go through the weights once more in bf16.
@@ -1074,36 +1075,36 @@ cudaError_t launch_linear_mode(const LinearArgs& args, const LinearShape& s, cud
 
 }  // namespace
 
-bool linear_w8_applies(int B, int N, int K) { return linear_shape(B, N, K, kStore, current_sm_count()).ok; }
-bool linear_geglu_applies(int B, int N, int K) { return N % 2 == 0 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kGeglu, current_sm_count()).ok; }
+bool linear_w8_applies(int B, int N, int K, bool f32) { return linear_shape(B, N, K, kStore, current_sm_count(), f32).ok; }
+bool linear_geglu_applies(int B, int N, int K) { return N % 2 == 0 && linear_w8_applies(B, N, K, false) && linear_shape(B, N, K, kGeglu, current_sm_count(), false).ok; }
 bool linear_rope_applies(int B, int N, int K, int n_q, int n_kv, int D) {
-  return n_kv == 1 && D == 256 && N == (n_q + 2) * 256 && linear_w8_applies(B, N, K) && linear_shape(B, N, K, kRope, current_sm_count()).ok;
+  return n_kv == 1 && D == 256 && N == (n_q + 2) * 256 && linear_w8_applies(B, N, K, false) && linear_shape(B, N, K, kRope, current_sm_count(), false).ok;
 }
 bool linear_norm_applies(int B, int N, int K, bool geglu) {
-  const LinearShape s = linear_shape(B, N, K, geglu ? kGeglu : kRope, current_sm_count());
+  const LinearShape s = linear_shape(B, N, K, geglu ? kGeglu : kRope, current_sm_count(), false);
   return B <= kNormTokens && s.ok && s.ck == 1 && rmsnorm_row_applies(K) && K <= 4 * 512 && s.kg * s.rt >= ceil_div(K / 4, 32);
 }
-// whether the arg max over the results can ride along, and the candidates' bytes
+// whether the arg max over fp32 results can ride along, and the candidates' bytes
 size_t linear_argmax_scratch(int B, int N, int K) {
-  const LinearShape s = linear_shape(B, N, K, kStore, current_sm_count());
+  const LinearShape s = linear_shape(B, N, K, kStore, current_sm_count(), true);
   return s.ok && s.tk == 1 ? (size_t)B * s.grid * 8 : 0;
 }
 
 cudaError_t launch_linear(const LinearArgs& a, cudaStream_t stream) {
-  const LinearShape s = linear_shape(a.B, a.N, a.K, kStore, current_sm_count());
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kStore, current_sm_count(), a.y_f32 != 0);
   if (!s.ok) return cudaErrorInvalidConfiguration;
   return s.tk == 1 ? launch_linear_mode<kStream>(a, s, stream) : launch_linear_mode<kStore>(a, s, stream);
 }
 cudaError_t launch_linear_geglu(const LinearArgs& a, cudaStream_t stream) {
-  const LinearShape s = linear_shape(a.B, a.N, a.K, kGeglu, current_sm_count());
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kGeglu, current_sm_count(), false);
   return s.ok ? launch_linear_mode<kGeglu>(a, s, stream) : cudaErrorInvalidConfiguration;
 }
 cudaError_t launch_linear_rope(const LinearArgs& a, cudaStream_t stream) {
-  const LinearShape s = linear_shape(a.B, a.N, a.K, kRope, current_sm_count());
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kRope, current_sm_count(), false);
   return s.ok ? launch_linear_mode<kRope>(a, s, stream) : cudaErrorInvalidConfiguration;
 }
 cudaError_t launch_linear_argmax(LinearArgs a, void* scratch, int32_t* out, cudaStream_t stream) {
-  const LinearShape s = linear_shape(a.B, a.N, a.K, kStore, current_sm_count());
+  const LinearShape s = linear_shape(a.B, a.N, a.K, kStore, current_sm_count(), a.y_f32 != 0);
   if (!s.ok || s.tk != 1) return cudaErrorInvalidConfiguration;
   a.cand_v = (float*)scratch;
   a.cand_i = (int32_t*)scratch + (size_t)a.B * s.grid;

@@ -779,7 +779,7 @@ extern "C" int tb200_gemv_w8_noalloc(int cuda_ordinal, void* stream, const void*
     scratch = g_noalloc_scratch_ptr[cuda_ordinal];
   }
   (void)cudaGetLastError();  // an earlier, unrelated error of the host must not be reported as this call's
-  if (own_choice && linear_w8_applies(B, N, K)) {  // as an executable's gemv_w8: no partial sums in memory at all
+  if (own_choice && linear_w8_applies(B, N, K, y_is_f32 != 0)) {  // as an executable's gemv_w8: no partial sums in memory at all
     LinearArgs a{};
     a.x = (const uint16_t*)x_bf16; a.W = (const int8_t*)w_i8; a.scale = (const uint16_t*)scale_bf16;
     a.y = y; a.y_f32 = y_is_f32 ? 1 : 0; a.B = B; a.N = N; a.K = K; a.serial = 1;

@@ -330,7 +330,7 @@ struct LinearArgs {
   int32_t* cand_i;
   int kg, ck, rt, stages, x_pitch, x_bytes, side_off, scale_off, recv_off, inv_b, tiles, work_blocks;
 };
-bool linear_w8_applies(int B, int N, int K);
+bool linear_w8_applies(int B, int N, int K, bool f32);  // f32: of the results
 bool linear_geglu_applies(int B, int N, int K);
 bool linear_norm_applies(int B, int N, int K, bool geglu);  // in front of the product with GeGLU or with RoPE behind it
 bool linear_rope_applies(int B, int N, int K, int n_q, int n_kv, int D);

@@ -17,7 +17,7 @@ enum { kStore = 0, kGeglu = 1, kRope = 2, kStream = 3 };
 constexpr int kTileRows = 32, kBlk = 64, kStageBytes = kTileRows * kBlk, kStreamStages = 4;
 constexpr int kRopeTokens = 8;  // most tokens a warp finishes in the RoPE epilogue
 constexpr int kSmemMax = 227 * 1024 - 1024;
-// Up to kSlicedTokens tokens the product over the vocabulary multiplies integers: a bf16 activation is four int8 slices of a 31-bit
+// Up to kSlicedTokens tokens the product over the vocabulary (a stream with fp32 results) multiplies integers: a bf16 activation is four int8 slices of a 31-bit
 // fixed-point number, a slice a column of the instruction. Its weights then need no conversion (where the slices leave room for the warps:
 // linear_shape). The products of the layers keep bf16: their
 // results are rounded to bf16 and go through every layer behind them, where two sums that differ in the last bit of fp32 end almost a
@@ -47,7 +47,8 @@ inline int linear_recv_bytes(int B, int mode, int ck, int rt) {
   return ck > 1 ? (rt * B + ck - 1) / ck * ck * 128 : 0;
 }
 
-inline LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
+// logits: an fp32 result, as the product over the vocabulary has it
+inline LinearShape linear_shape(int B, int N, int K, int mode, int sms, bool logits) {
   LinearShape s{};
   if (K % kBlk != 0 || K < kBlk || B < 1 || B > 32 || N < 1) return s;
   const int tok = ceil_div(B, 8) * 8, blocks = K / kBlk;
@@ -82,7 +83,7 @@ inline LinearShape linear_shape(int B, int N, int K, int mode, int sms) {
       return rt;
     };
     auto rounds = [&](int rt) { return ceil_div(s.tiles, (long long)sms * rt); };
-    const int rt = warps_that_fit(false), sliced_rt = B <= kSlicedTokens ? warps_that_fit(true) : 0;
+    const int rt = warps_that_fit(false), sliced_rt = logits && B <= kSlicedTokens ? warps_that_fit(true) : 0;
     // Eight tokens' slices leave room for 8 warps from K = 3008 on, 4 from 5056, 2 from 6080 and none from 6848; bf16 rows for 16 below 6144. A
     // round (a tile for every warp) takes 8.5 us per 1024 of K with 8 warps on slices and 14.3 with 16 on bf16, but still 7.0 and 6.6 with 4
     // and 2 on slices: so 8 warps for 16 where the rounds say so, and no others. Eight tokens, slices against bf16: K = 3072, N = 100000 (3 rounds and 2) 76.4 / 86.0 us,

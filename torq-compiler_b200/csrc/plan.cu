@@ -2095,7 +2095,7 @@ int build_plan(const std::vector<tb200_tensor_t>& tensors, const std::vector<tb2
         size_t w_off, s_off;
         if (!b.add_raw_const(op.weights, (size_t)N * K, "weights", i, w_off)) return b.status;
         if (!b.add_raw_const(op.bias, (size_t)N * 2, "scales", i, s_off)) return b.status;
-        if (op.i0 <= 0 && op.i1 == 0 && K == tensors[op.in0].shape[1] && linear_w8_applies(B, N, K)) {
+        if (op.i0 <= 0 && op.i1 == 0 && K == tensors[op.in0].shape[1] && linear_w8_applies(B, N, K, y_f32 != 0)) {
           // the product after the next one: its weights have that long to come from memory
           size_t next_off = 0, next_bytes = 0;
           for (int j = i + 1, seen = 0; j < (int)ops.size(); j++) {
