@@ -16,12 +16,14 @@ IDENT = ((1 << 30), 30)
 @pytest.mark.parametrize("shape,channels,rescaled", [((1, 1, 1), (16, 16), ()), ((2, 9, 7), (16, 48, 32), (1,)), ((1, 20, 21), (128, 16, 16, 64), (0, 3)),
                                                      ((3, 64, 64), (32, 32), (0, 1)), ((1, 5, 3), (16,) * 8, (2, 7)), ((1, 6, 5), (16, 24), (1,)),
                                                      ((40, 64, 64), (16, 48, 16), (1, 2)), ((37, 65, 67), (32, 64), ()), ((41, 64, 64), (96, 32, 32), (0, 2))])
-def test_concat_of_intermediates(device, shape, channels, rescaled):
+@pytest.mark.parametrize("factor", [lambda k: 0.6 + 0.2 * k, lambda k: 0.31 + 0.02 * k], ids=["one multiply-add", "tables"])
+def test_concat_of_intermediates(device, shape, channels, rescaled, factor):
+    """Rescales that one multiply-add gives for every byte, and ones below a half, whose double rounding none does."""
     rng = np.random.default_rng(sum(channels))
     g = Graph()
     xs = [rng.integers(-128, 128, shape + (c,), dtype=np.int8) for c in channels]
     parts = [g.table(g.input(x.shape), rng.permutation(np.arange(-128, 128)).astype(np.int8)) for x in xs]
-    ms = [quantize_multiplier(0.6 + 0.2 * k) if k in rescaled else IDENT for k in range(len(parts))]
+    ms = [quantize_multiplier(factor(k)) if k in rescaled else IDENT for k in range(len(parts))]
     zp = [4 if k not in rescaled else k - 3 for k in range(len(parts))]
     acc = g.concat(parts[0], parts[1], a_zp=zp[0], a_ms=ms[0], b_zp=zp[1], b_ms=ms[1], out_zp=4)
     for k in range(2, len(parts)):

@@ -41,7 +41,8 @@ def test_products(device, B, K, N):
 @pytest.mark.parametrize("B,K,N", [(1, 1152, 40), (2, 6912, 33), (7, 64, 32), (8, 1152, 30001)])
 @pytest.mark.parametrize("spread", [0, 8, 40, 120])
 def test_products_of_few_tokens_over_magnitudes(device, B, K, N, spread):
-    """Up to eight tokens the activations enter as fixed-point numbers: magnitudes 2^-spread .. 1 side by side, subnormals at the far end.
+    """The two sizes whose K no warps share take the activations as fixed-point numbers, the others as they are: magnitudes 2^-spread .. 1
+    side by side, subnormals at the far end.
     Against 64 bits; the bound is that of an fp32 sum of K terms: K 2^-24 of the sum of magnitudes."""
     rng = np.random.default_rng(B + K + spread)
     x = to_bf16((rng.normal(0, 1, (B, K)) * np.exp2(rng.uniform(-spread, 0, (B, K)) - (100 if spread == 40 else 0))).astype(np.float32))

@@ -120,12 +120,12 @@ def test_few_dozen_rows(device, M, K, N, table, monkeypatch):
 @pytest.mark.parametrize("shape,OC,stride,pad", [((1, 211, 90, 3), 16, 2, (0, 1, 0, 1)), ((3, 70, 75, 3), 32, 1, (1, 1, 1, 1)), ((2, 65, 43, 3), 48, 2, (1, 1, 1, 1)),
                                                  ((37, 5, 7, 3), 64, 1, (2, 0, 2, 0)), ((40, 31, 17, 3), 16, 1, (1, 1, 1, 1)),
                                                  ((3, 67, 132, 3), 16, 2, (0, 1, 0, 1)), ((2, 30, 140, 3), 32, 2, (1, 1, 1, 1)), ((5, 9, 64, 3), 96, 2, (1, 0, 2, 3)),
-                                                 ((2, 90, 4, 3), 16, 2, (1, 1, 1, 1))])
+                                                 ((2, 90, 4, 3), 16, 2, (1, 1, 1, 1)), ((37, 101, 77, 3), 16, 1, (1, 1, 1, 1)), ((5, 230, 299, 3), 48, 1, (0, 1, 1, 0))])
 @pytest.mark.parametrize("table", [False, True])
 @pytest.mark.parametrize("double_round,clamp", [(True, (-128, 127)), (False, (3, 100))])
 def test_stem_of_large_frames(device, shape, OC, stride, pad, table, double_round, clamp, monkeypatch):
     """The stem kernel of the frames the small-problem kernels leave: pixel counts that end inside a warp, rows shorter than a warp, windows
-    over every edge, one and several passes over the channels."""
+    over every edge, one and several passes over the channels, one pixel a thread and (from 1536 an SM on) several."""
     monkeypatch.setenv("TB200_NO_SMALL", "1")
     rng = np.random.default_rng(OC + shape[1])
     g = Graph()
