@@ -39,7 +39,7 @@ int main() {
 '''
 
 # A product over the vocabulary (one group of K): [bf16 rows][warps' rings][scales], as many warps of 16, 8, 4, 2, 1 as fit. Slices may not
-# take it away, nor leave it fewer warps (8 for 16 where that is less than 1.6 times as many rounds); and what stands at side_off (a shift
+# take it away, nor leave it fewer warps (8 for 16 where that is less than 1.8 times as many rounds); and what stands at side_off (a shift
 # per token; the sums of a norm in front: two tokens, two norms, 16 warps) lies behind the activations and inside their bytes.
 VOCABULARY = r'''
 #include <cstdio>
@@ -64,7 +64,7 @@ int main() {
         sliced += s.ok && s.sliced;
         const int held = s.sliced ? (b * kSlices + 7) / 8 * 8 * k : b * 2 * k;
         const int tiles = (n + 31) / 32, r8 = (tiles + 8 * 148 - 1) / (8 * 148), r16 = (tiles + 16 * 148 - 1) / (16 * 148);
-        const bool enough = s.kg * s.rt >= warps || (warps == 16 && s.kg * s.rt == 8 && s.sliced && r8 < 1.6 * r16);
+        const bool enough = s.kg * s.rt >= warps || (warps == 16 && s.kg * s.rt == 8 && s.sliced && r8 < 1.8 * r16);
         if (!s.ok || s.tk != 1 || !enough || s.side_off < held || (s.sliced && s.side_off + 4 * b > s.x_bytes)) {
           if (!bad++) printf("B %d N %d K %d: ok %d, %d warps (%d), side_off %d, x_bytes %d\n", b, n, k, s.ok, s.rt, warps, s.side_off, s.x_bytes);
         }

@@ -85,10 +85,11 @@ inline LinearShape linear_shape(int B, int N, int K, int mode, int sms, bool log
     auto rounds = [&](int rt) { return ceil_div(s.tiles, (long long)sms * rt); };
     const int rt = warps_that_fit(false), sliced_rt = logits && B <= kSlicedTokens ? warps_that_fit(true) : 0;
     // Eight tokens' slices leave room for 8 warps from K = 3008 on, 4 from 5056, 2 from 6080 and none from 6848; bf16 rows for 16 below 6144. A
-    // round (a tile for every warp) takes 8.5 us per 1024 of K with 8 warps on slices and 14.3 with 16 on bf16, but still 7.0 and 6.6 with 4
-    // and 2 on slices: so 8 warps for 16 where the rounds say so, and no others. Eight tokens, slices against bf16: K = 3072, N = 100000 (3 rounds and 2) 76.4 / 86.0 us,
-    // 4096 x 60000 (2 and 1) 72.9 / 57.7, 5120 x 50000 (4 warps) 104.9 / 67.9, 6144 x 50000 (2 warps) 239 / 91.
-    if (sliced_rt < 1 || !(sliced_rt >= rt || (sliced_rt == 8 && 5 * rounds(sliced_rt) < 8 * rounds(rt)))) warps_that_fit(false);
+    // round (a tile for every warp) takes 7.6 to 8.5 us per 1024 of K with 8 warps on slices and 13.9 to 14.3 with 16 on bf16, but still 7.0
+    // and 6.6 with 4 and 2 on slices: so 8 warps for 16 up to 1.8 times the rounds, and no others. Eight tokens, slices against bf16: K = 3072,
+    // N = 100000 (3 rounds and 2) 76.4 / 86.0 us, 262144 (7 and 4) 159.6 / 166.2, 75000 (2 and 1) 57.1 / 51.5, 4096 x 60000 (2 and 1) 72.9 / 57.7,
+    // 5120 x 50000 (4 warps) 104.9 / 67.9, 6144 x 50000 (2 warps) 239 / 91.
+    if (sliced_rt < 1 || !(sliced_rt >= rt || (sliced_rt == 8 && 5 * rounds(sliced_rt) < 9 * rounds(rt)))) warps_that_fit(false);
     if ((s.sliced ? sliced_rt : rt) < 1) return LinearShape{};
     s.grid = std::min(sms, ceil_div(s.tiles, s.rt));
     s.ok = true;
