@@ -69,9 +69,11 @@ def test_rescaled_add_covers_every_operand_pair(device, n, scales):
         _check(device, g, [a, b])
 
 
-# the last row: stages' edges of the 16 x 16, 32 x 32 and 64 x 32 tiles, aligned rows and odd ones
+# the second row: stages' edges of the 16 x 16, 32 x 32 and 64 x 32 tiles, aligned rows and odd ones (which take 64 x 64 where there are
+# enough); the third: 64 x 64 tiles of aligned rows, over the edges of tiles and stages
 @pytest.mark.parametrize("M,K,N", [(1, 1, 1), (16, 128, 17), (33, 130, 31), (160, 65, 190), (300, 36, 900), (520, 129, 512),
-                                   (40, 256, 16), (17, 515, 24), (31, 769, 33), (300, 64, 304), (310, 191, 297), (1300, 63, 520), (1291, 128, 512)])
+                                   (40, 256, 16), (17, 515, 24), (31, 769, 33), (300, 64, 304), (310, 191, 297), (1300, 63, 520), (1291, 128, 512),
+                                   (2500, 64, 1008), (2441, 80, 1008)])
 @pytest.mark.parametrize("dtype", ["bf16", "f32", "i16", "i8"])
 @pytest.mark.parametrize("transposed", [False, True])
 def test_tiled_products(device, M, K, N, dtype, transposed):
