@@ -757,14 +757,15 @@ void launch_conv2d_simt(const ConvArgs& a, cudaStream_t stream) {
     return;
   }
   if (conv_stem333_applies(a)) {
+    const int sms = current_sm_count();
     // a frame or two: as many blocks as there is work for
-    const int pixels = (int)std::max(1ll, std::min((long long)kStemPix, P / (128ll * 148 * 6)));
+    const int pixels = (int)std::max(1ll, std::min((long long)kStemPix, P / (128ll * sms * 6)));
     const unsigned blocks = (unsigned)((P + 128 * pixels - 1) / (128 * pixels));
     // 32-bit offsets where the last pixel of the last block still has one
     const bool small = P + 128 * kStemPix < (1ll << 31) && a.x_bytes < (1ll << 31) - 64;
     const bool words = a.stride_h == 2 && a.stride_w == 2 && (a.W & 3) == 0;
     const int tiles_x = (a.OW + 31) / 32, tiles = small && words ? a.N * a.OH * tiles_x : 0;
-    const int per_warp = std::max(1, (tiles + 148 * 4 * 4 - 1) / (148 * 4 * 4));  // one wave of blocks, their weights laid out once
+    const int per_warp = std::max(1, (tiles + sms * 4 * 4 - 1) / (sms * 4 * 4));  // one wave of blocks, their weights laid out once
     const dim3 tile_grid((unsigned)((tiles + 4 * per_warp - 1) / (4 * per_warp)));
 #define TB200_STEM(EPI, LUT, W)                                                                                                       \
   do {                                                                                                                                \

@@ -691,7 +691,7 @@ template <int K, int S>
 cudaError_t launch_pool_add_shape(const PoolAddArgs& pa, cudaStream_t stream) {
   const PoolArgs& a = pa.pool;
   const uintptr_t at = (uintptr_t)a.x | (uintptr_t)a.out;
-  const long long pixels = (long long)a.N * a.OH * a.OW, want = 148ll * 512, wide = pixels * (a.C / 16) / want, words = pixels * (a.C / 4) / want;
+  const long long pixels = (long long)a.N * a.OH * a.OW, want = 512ll * current_sm_count(), wide = pixels * (a.C / 16) / want, words = pixels * (a.C / 4) / want;
   if ((at & 15) == 0 && (a.C & 15) == 0 && wide >= 1) return launch_pool_add_strips<4, K, S>(pa, wide >= 4 ? 4 : wide >= 2 ? 2 : 1, stream);
   if ((at & 3) == 0 && (a.C & 3) == 0) return launch_pool_add_strips<1, K, S>(pa, words >= 8 ? 8 : words >= 4 ? 4 : 1, stream);
   return launch_pool_add_strips<0, K, S>(pa, 4, stream);
