@@ -14,9 +14,10 @@
 //   * up to two sequences the norms in front of the q/k/v and the gate/up product run in it: every block norms the rows for itself, which costs
 //     less than a launch whose result it would have to wait for.
 // Measured at the Gemma-3-1B shape at position 1024, launches serialised, us per launch (split-K kernels of decoder.cu, 32 sequences)
-// -> here with 32 / one sequence: attention 10.6 + 3.4 -> 9.2 / 6.2, gate/up + GeGLU 10.5 + 4.4 -> 11.7 / 7.5, norms 8.6 -> 2.4, LM head
-// 125 -> 96 / 49, arg max 24 -> 2.3; q/k/v + head norm + RoPE 8.2 / 5.5, o and down 7.9 / 5.7 on average. A whole step, launches
-// overlapping: 1.13 / 0.69 ms (0.70 without the later product's weights asked for, 0.75 with the norms as launches of their own).
+// -> here with 32 / one sequence (one sequence: with their norms): attention 10.6 + 3.4 -> 9.2 / 6.3, gate/up + GeGLU 10.5 + 4.4 -> 11.1 /
+// 7.9, norms 8.6 -> 2.4, LM head 125 -> 94.5 / 50.3, arg max 24 -> 2.3; q/k/v + head norm + RoPE 8.8 / 7.5, o and down 7.5 / 5.2 on average. A
+// whole step, launches overlapping: 1.13 / 0.67 ms. What the last steps gave when they were made, one sequence: 0.81 -> 0.75 ms by norms that
+// release before their wait, 0.75 -> 0.70 by norms inside products, 0.01 by the later product's weights.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -49,14 +50,7 @@ __device__ __forceinline__ int cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return (int)r;
 }
-// a float of another block of the cluster, at the address the same float has in this block
-__device__ __forceinline__ float ld_peer(uint32_t addr, int rank) {
-  uint32_t a;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
+// into a float of another block of the cluster, at the address the same float has in this block
 __device__ __forceinline__ void st_peer(uint32_t addr, int rank, float v) {
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
@@ -981,8 +975,8 @@ __global__ void __launch_bounds__(512) rmsnorm_row_kernel(const uint16_t* __rest
     }
   }
   // Lets the product behind it in before its own wait: a norm runs for a microsecond, and a product that came only then asked for its
-  // weights and scales 2 us after its activations were there. The product reads nothing but constants before its wait, and what
-  // runs before a norm in a chain (the products, the embedding) releases after its wait, so no chain stacks up further.
+  // weights and scales 2 us after its activations were there. Before its wait the product reads constants, and the position, which it reads
+  // again behind it; and what runs before a norm in a chain (the products, the embedding) releases after its wait, so no chain stacks up.
   // One step of the 1B shape at position 1024: 808 -> 748 us (one sequence), 1215 -> 1167 us (32); products that release first, too: 747 / 1210.
   grid_dependency_release();
   grid_dependency_wait();

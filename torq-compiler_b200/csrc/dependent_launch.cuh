@@ -27,10 +27,11 @@ inline bool dependent_launch_enabled() {
 // A kernel lets the next one in only after its own wait has returned (grid_dependency_wait before grid_dependency_release):
 // releasing first let chains of short kernels stack up a dozen deep, holding the registers and block slots of the one that
 // had work. Measured on one-image inferences (56 and 120 launches of a few microseconds): released first 269 and 313 us,
-// released after the wait 256 and 287 us, fully serialised 274 and 393 us. One kernel releases first: the decoder's norm
-// (rmsnorm_row), whose few blocks hold next to nothing while the product behind it is made resident (8 steps of one sequence
-// 6467 -> 5987 us). In a decoder two never follow each other, so nothing stacks up; with the products releasing first as well,
-// 32 sequences took 9677 us instead of 9333.
+// released after the wait 256 and 287 us, fully serialised 274 and 393 us. Two kernels release first. The tcgen05 products
+// (gemm_tcgen05): persistent blocks that hold an SM's shared memory until they end. And the decoder's norm (rmsnorm_row), whose few
+// blocks hold next to nothing while the product behind it is made resident (8 steps of one sequence 6467 -> 5987 us); with the
+// decoder's products releasing first as well, 32 sequences took 9677 us instead of 9333. Where the planner fuses norms, two of them
+// never follow each other, so nothing stacks up; with TB200_NO_DECODER_FUSION=1 pairs do, which costs time and nothing else.
 constexpr long long kDependentMinBlocks = 4 * 148;  // persistent kernels: tiles x 2 from which their tail is worth overlapping
 
 template <typename... KArgs, typename... Args>
