@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
   if (MODE != kStream && (int)threadIdx.x < a.rt * kTileRows) scale_s[threadIdx.x] = bf2f(scale_r);
   __syncthreads();
 
+  int stage = 0, kb = 0, tile = tile0;
   // Sums of this warp: [16-row half][tile of eight columns][...]. Of slices (ci): columns are the slices of two tokens, 2 t + tig / 2 for this
   // lane; else (cs) eight tokens.
   // Independent chains of accumulation where the tokens leave room: a dependent matrix instruction waits 28 cycles.
@@ -385,10 +386,10 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
           for (int q = 1; q < kSets; q++) cs[q][mt][t][j] = 0.f;
         }
   };
-  auto multiply = [&](auto of_slices, uint32_t x_row, int x_pitch) {
+  // xrow: this lane's first staged activations. (Positions and addresses outside: with them in here the compiler made the forms of 25 to 32
+  // tokens 2 % slower.)
+  auto multiply = [&](auto of_slices, uint32_t xrow, int x_pitch) {
     constexpr bool kInts = decltype(of_slices)::value;
-    int stage = 0, kb = 0, tile = tile0;
-    const uint32_t xrow = x_row + (uint32_t)((wb0 - kb0) * kBlk * (kInts ? 1 : 2) + tig * (kInts ? 16 : 32));
     for (int i = 0; i < total; i++) {
       if (MODE == kStream) {  // the ring is a.stages deep and one group is committed per block from here on
         if (kInts || i >= a.stages) cp_wait<kStreamStages - 1>();
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
     }
   };
   if constexpr (SLICED) {
-    if (sliced_tokens) multiply(std::true_type(), x_addr + (uint32_t)(g * a.x_pitch), a.x_pitch);
+    if (sliced_tokens) multiply(std::true_type(), x_addr + (uint32_t)(g * a.x_pitch + tig * 16), a.x_pitch);
     if (sliced_tokens != (1u << a.B) - 1) {  // once more for the rows left to bf16, staged where the slices were (they take half of that)
       __syncthreads();
       const int pitch = (a.K * 2 + 127) / 128 * 128 + 16;
@@ -502,10 +503,12 @@ __global__ void __launch_bounds__(512, 1) linear_w8_kernel(const LinearArgs a) {
       }
       cp_wait<0>();
       __syncthreads();
-      multiply(std::false_type(), x_addr + (uint32_t)(min(g, a.B - 1) * pitch), pitch);
+      stage = kb = 0;
+      tile = tile0;
+      multiply(std::false_type(), x_addr + (uint32_t)(min(g, a.B - 1) * pitch + tig * 32), pitch);
     }
   } else {
-    multiply(std::false_type(), x_addr + (uint32_t)(g * a.x_pitch), a.x_pitch);
+    multiply(std::false_type(), x_addr + (uint32_t)(g * a.x_pitch + (wb0 - kb0) * kBlk * 2 + tig * 32), a.x_pitch);
   }
 
   if constexpr (MODE == kStream) {
